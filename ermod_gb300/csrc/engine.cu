@@ -5,7 +5,8 @@
 // Per batch of B placements:
 //   [mixed] place_prep (prep stream) -> pme_a -> pme_b -> gather -> finish (one of two
 //           batch streams) -> reduce + accumulate (aux stream)
-//   [fp64]  place_prep -> spread64 -> D2Z -> influence64 -> Z2D -> mol_energy -> accumulate
+//   [fp64]  place_prep (prep stream) -> spectrum64 -> Z2D -> mol_energy (caller's stream) ->
+//           reduce + accumulate (aux stream)
 // and, when ecorr is on, a flush of the histogram ring every `ring_half` placements on
 // the flush stream while the next batches fill the ring's other half.
 // Status is reported once per call (host API) or per ermod_sync (device API).
@@ -131,6 +132,7 @@ static int free_batch(Engine& e) {
   dfree(b.u_grid);
   dfree(b.u_w);
   dfree(b.u_bvec);
+  dfree(b.u_bvec64);
   dfree(b.u_qmol);
   dfree(b.u_usreal);
   dfree(b.u_radius);
@@ -252,6 +254,7 @@ static int ensure_batch(Engine& e) {
   const int B = e.Bmax;
   BatchArgs& b = e.buf;
   const size_t nr = e.grid_real(), nc = e.grid_cplx();
+  e.tile = e.mixed ? 256 : mol64_tile(e);
   e.ntile = (e.slvmax + e.tile - 1) / e.tile;
   // solute data: kBatchSlots batch slots (the preparation of batch i+1 runs during batch i)
   const size_t NS = kBatchSlots;
@@ -291,9 +294,10 @@ static int ensure_batch(Engine& e) {
     }
     ERMOD_CUDA(dalloc(&b.self_part, NS * B * spectrum_partials(e)));
   } else {
+    ERMOD_CUDA(dalloc(&b.u_bvec64, NS * B * S * 3 * e.Kmax()));
     ERMOD_CUDA(dalloc(&b.spec64, nc * B));
     ERMOD_CUDA(dalloc(&b.phi64, nr * B));
-    ERMOD_CUDA(dalloc(&b.self_part, NS * B * influence64_blocks()));
+    ERMOD_CUDA(dalloc(&b.self_part, NS * B * spectrum64_partials(e)));
   }
   ERMOD_CUDA(dalloc(&b.part, NS * B * e.ntile * e.numslv * 3));
   e.ring_half = e.P.corrcal ? std::max(2 * B, (512 / B) * B) : B;
@@ -306,19 +310,27 @@ static int ensure_batch(Engine& e) {
   ERMOD_CUDA(dalloc(&e.d_ring_nnz, e.ring_cap));
   ERMOD_CUDA(dalloc(&e.d_ring_valid, e.ring_cap));
   if (e.P.corrcal) ERMOD_CUDA(dalloc(&e.d_ring_nz, (size_t)2 * e.ring_cap * e.ermax));
-  // FFT plans
-  if (!e.plans_ready) {
-    int n[3] = {e.geom.K[2], e.geom.K[1], e.geom.K[0]};
-    cufftResult r;
-    if (!e.mixed) {
-      r = cufftPlanMany(&e.plan_d2z, 3, n, nullptr, 1, (int)nr, nullptr, 1, (int)nc, CUFFT_D2Z, B);
-      if (r != CUFFT_SUCCESS) return fail_fft(r, "cufftPlanMany(D2Z)");
-      r = cufftPlanMany(&e.plan_z2d, 3, n, nullptr, 1, (int)nc, nullptr, 1, (int)nr, CUFFT_Z2D, B);
-      if (r != CUFFT_SUCCESS) return fail_fft(r, "cufftPlanMany(Z2D)");
-      cufftSetStream(e.plan_d2z, e.stream);
-      cufftSetStream(e.plan_z2d, e.stream);
+  return ERMOD_OK;
+}
+
+// FP64 path: the batch's inverse transforms, as cuFFT plans of powers of two (a call's last
+// batch may hold any number of placements; each size is planned once, when first needed)
+static int inverse_fft64(Engine& e, const BatchArgs& a) {
+  const size_t nr = e.grid_real(), nc = e.grid_cplx();
+  int done = 0;
+  for (int lg = kFp64MaxLog2; lg >= 0; --lg) {
+    for (; a.nb - done >= (1 << lg); done += 1 << lg) {
+      if (!e.plan_z2d[lg]) {
+        int n[3] = {e.geom.K[2], e.geom.K[1], e.geom.K[0]};
+        cufftHandle plan = 0;
+        cufftResult r = cufftPlanMany(&plan, 3, n, nullptr, 1, (int)nc, nullptr, 1, (int)nr, CUFFT_Z2D, 1 << lg);
+        if (r != CUFFT_SUCCESS) return fail_fft(r, "cufftPlanMany(Z2D)");
+        e.plan_z2d[lg] = plan;
+        if ((r = cufftSetStream(plan, e.stream)) != CUFFT_SUCCESS) return fail_fft(r, "cufftSetStream");
+      }
+      const cufftResult r = cufftExecZ2D(e.plan_z2d[lg], (cufftDoubleComplex*)(a.spec64 + nc * done), a.phi64 + nr * done);
+      if (r != CUFFT_SUCCESS) return fail_fft(r, "cufftExecZ2D");
     }
-    e.plans_ready = true;
   }
   return ERMOD_OK;
 }
@@ -443,7 +455,13 @@ int ermod_create(const ermod_params* p_in, int device, ermod_ctx** out) {
   e.geom.K[0] = K[0];
   e.geom.K[1] = K[1];
   e.geom.K[2] = K[2];
-  e.Bmax = e.mixed ? (p->batch > 0 ? p->batch : 64) : 1;
+  if (e.mixed) {
+    e.Bmax = p->batch > 0 ? p->batch : 64;
+  } else {
+    const size_t one = sizeof(double) * e.grid_real() + sizeof(double2) * e.grid_cplx();
+    e.Bmax = 1;
+    while (2 * e.Bmax <= (1 << kFp64MaxLog2) && 2 * e.Bmax * one <= kFp64GridBytes) e.Bmax *= 2;
+  }
   // four placements per molecule-energy block unless asked otherwise: measured 4% faster
   // than eight on the 33,000-water workload (fewer registers, more blocks in flight)
   e.G = e.mixed ? 4 : 1;
@@ -548,8 +566,8 @@ int ermod_destroy(ermod_ctx* c) {
   dfree(e.d_twiddle64);
   dfree(e.d_status);
   if (e.h_status) cudaFreeHost(e.h_status);
-  if (e.plan_d2z) cufftDestroy(e.plan_d2z);
-  if (e.plan_z2d) cufftDestroy(e.plan_z2d);
+  for (cufftHandle p : e.plan_z2d)
+    if (p) cufftDestroy(p);
   harvest(e);
   for (auto ev : e.ev_pool) cudaEventDestroy(ev);
   if (e.own_stream && e.stream) cudaStreamDestroy(e.stream);
@@ -584,8 +602,8 @@ int ermod_set_stream(ermod_ctx* c, void* stream) {
   if (e.own_stream && e.stream) cudaStreamDestroy(e.stream);
   e.stream = (cudaStream_t)stream;
   e.own_stream = false;
-  if (e.plan_d2z) cufftSetStream(e.plan_d2z, e.stream);
-  if (e.plan_z2d) cufftSetStream(e.plan_z2d, e.stream);
+  for (cufftHandle p : e.plan_z2d)
+    if (p) cufftSetStream(p, e.stream);
   return ERMOD_OK;
 }
 
@@ -953,7 +971,7 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
   const int B = e.Bmax;
   const int S = kMaxSoluteSites;
   const int nbatch = (nplace + B - 1) / B;
-  const size_t parts = e.mixed ? (size_t)spectrum_partials(e) : (size_t)influence64_blocks();
+  const size_t parts = e.mixed ? (size_t)spectrum_partials(e) : (size_t)spectrum64_partials(e);
   // batches run on two alternating streams (mixed path) or on the caller's stream (FP64
   // path, whose cuFFT plans are bound to it); every stream starts after what is
   // already queued on the caller's stream
@@ -991,6 +1009,7 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
     a.u_qf = e.buf.u_qf + (size_t)slot * B * S;
     a.u_grid = e.buf.u_grid + (size_t)slot * B * S;
     a.u_w = e.buf.u_w + (size_t)slot * B * S * 3 * kMaxSplineOrder;
+    if (e.buf.u_bvec64) a.u_bvec64 = e.buf.u_bvec64 + (size_t)slot * B * S * 3 * e.Kmax();
     if (e.buf.u_bvec) a.u_bvec = e.buf.u_bvec + (size_t)slot * B * S * 3 * e.Kmax();
     a.u_radius = e.buf.u_radius + (size_t)slot * B;
     a.u_qmol = e.buf.u_qmol + (size_t)slot * B;
@@ -1048,14 +1067,10 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
       e.phase_end_on(bst);
     } else {
       e.phase_begin_on(PH_SPECTRUM, bst);
-      ERMOD_CUDA(launch_spread64(e, a));
-      cufftResult r = cufftExecD2Z(e.plan_d2z, a.phi64, (cufftDoubleComplex*)a.spec64);
-      if (r != CUFFT_SUCCESS) return fail_fft(r, "cufftExecD2Z");
-      ERMOD_CUDA(launch_influence64(e, a));
+      ERMOD_CUDA(launch_spectrum64(e, a));
       e.phase_end_on(bst);
       e.phase_begin_on(PH_FFT, bst);
-      r = cufftExecZ2D(e.plan_z2d, (cufftDoubleComplex*)a.spec64, a.phi64);
-      if (r != CUFFT_SUCCESS) return fail_fft(r, "cufftExecZ2D");
+      if ((st = inverse_fft64(e, a)) != ERMOD_OK) return st;
       e.phase_end_on(bst);
     }
     e.phase_begin_on(e.mixed ? PH_GATHER : PH_MOL, bst);

@@ -201,8 +201,7 @@ struct Engine {
   bool tmap_ready = false;
 
   // ---- cuFFT -------------------------------------------------------------------------
-  cufftHandle plan_d2z = 0, plan_z2d = 0;
-  bool plans_ready = false;
+  cufftHandle plan_z2d[kFp64MaxLog2 + 1] = {};  // FP64 path: Z2D of 2^i placements, made at first use
 
   // helpers
   int H() const { return geom.K[0] / 2 + 1; }
@@ -247,7 +246,8 @@ struct Engine {
 
 // sizes shared between the launchers and the host code
 int spectrum_partials(const Engine& e);
-int influence64_blocks();
+int spectrum64_partials(const Engine& e);
+int mol64_tile(const Engine& e);  // molecules per block of the FP64 path's molecule kernel
 int accumulate_max_batch();
 size_t frame_cub_bytes(int n);
 size_t brick_cub_bytes(int nsite, int nbricks);

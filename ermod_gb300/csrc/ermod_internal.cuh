@@ -35,25 +35,31 @@ constexpr int kBatchSlots = 3;
 // measured: +0.5% on the 96^3 workload and -2.4% at 48^3, with each kernel's in-pipeline
 // launch time half as long again (it shares the SMs with two other batches)
 constexpr int kBatchStreams = 2;
+// FP64 path: placements per batch, at most 2^kFp64MaxLog2 and as many as keep the batch's
+// grids within kFp64GridBytes (two L2 sizes: 64 placements at 48^3, 16 at 96^3, one from
+// 256^3 on, as before batching)
+constexpr int kFp64MaxLog2 = 6;
+constexpr size_t kFp64GridBytes = (size_t)256 << 20;
 constexpr int kMaxSpecies = 16;
 constexpr int kGridBits = 10;         // packed grid coordinates: K <= 1024 per axis
 constexpr double kPi = 3.1415926535897932;
 
-// B-spline weights M_P(t + j), j = 0..P-1, by the stable Cox-de Boor recursion (FP32)
-template <int P>
-__host__ __device__ __forceinline__ void bspline_w(float t, float w[P]) {
+// B-spline weights M_P(t + j), j = 0..P-1, by the stable Cox-de Boor recursion (FP32: the
+// mixed path's gather; FP64: the FP64 path's solvent sites)
+template <int P, typename T>
+__host__ __device__ __forceinline__ void bspline_w(T t, T (&w)[P]) {
   w[0] = t;
-  w[1] = 1.f - t;
+  w[1] = T(1) - t;
 #pragma unroll
-  for (int j = 2; j < P; ++j) w[j] = 0.f;
+  for (int j = 2; j < P; ++j) w[j] = T(0);
 #pragma unroll
   for (int n = 3; n <= P; ++n) {
-    const float inv = 1.f / (float)(n - 1);
+    const T inv = T(1) / (T)(n - 1);
 #pragma unroll
     for (int j = n - 1; j >= 0; --j) {
-      const float a = (j <= n - 2) ? w[j] : 0.f;
-      const float b = (j >= 1) ? w[j - 1] : 0.f;
-      w[j] = ((t + (float)j) * a + ((float)n - t - (float)j) * b) * inv;
+      const T a = (j <= n - 2) ? w[j] : T(0);
+      const T b = (j >= 1) ? w[j - 1] : T(0);
+      w[j] = ((t + (T)j) * a + ((T)n - t - (T)j) * b) * inv;
     }
   }
 }
@@ -212,15 +218,16 @@ struct BatchArgs {
   int* u_grid;         // [nb][S] packed base grid
   double* u_w;         // [nb][S][3][P] FP64 spline weights
   float2* u_bvec;      // [nb][S][3][Kmax] 1-D structure factors (mixed)
+  double2* u_bvec64;   // the same in FP64 (FP64 path)
   double* u_qmol;      // [nb] molecular charge of the solute
   double* u_usreal;    // [nb] realcal_self value
   float* u_radius;     // [nb] solute bounding radius about site 1 (A)
   // PME
   float2* spec;        // [nb][K3][K2][H] mixed spectrum (engfac * S)
   float* phi;          // [nb][K3][K2][K1] mixed potential
-  double2* spec64;     // FP64 path
-  double* phi64;       // FP64 path
-  double* self_part;   // [nb][K2] (mixed) or [nb][influence64_blocks] (FP64) partial self energies
+  double2* spec64;     // FP64 path: [nb][K3][K2][H] spectrum (engfac * S)
+  double* phi64;       // FP64 path: [nb][K3][K2][K1] potential
+  double* self_part;   // [nb][K2] (mixed) or [nb][spectrum64_partials] (FP64) partial self energies
   // outputs
   int* hist;           // [nb][ermax] instantaneous histogram (insdst)
   double* part;        // [nb][ntile][numslv][3] {sum, min, max}
@@ -249,8 +256,7 @@ cudaError_t launch_place_prep(Engine& e, const BatchArgs& a, const double* sol_x
                               cudaStream_t s);
 cudaError_t launch_pme_mixed(Engine& e, const BatchArgs& a);
 bool pme_fits(int K1, int K2, int K3);
-cudaError_t launch_spread64(Engine& e, const BatchArgs& a);
-cudaError_t launch_influence64(Engine& e, const BatchArgs& a);
+cudaError_t launch_spectrum64(Engine& e, const BatchArgs& a);
 // per-molecule energies and histograms
 cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a);
 cudaError_t launch_gather(Engine& e, const BatchArgs& a);

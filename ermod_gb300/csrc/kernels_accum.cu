@@ -52,14 +52,19 @@ struct AccArgs {
 constexpr int kAccThreads = 256;
 constexpr int kMaxBatch = 512;
 
-// an error in this batch or an earlier one of the call; errors of later batches (already
-// running on the other stream) do not stop this batch's accumulation.  The answer cannot
-// change between the accumulation kernels of a batch: the earlier batches' kernels are
-// complete by then and the error key only decreases.
-__device__ __forceinline__ bool batch_failed(const AccArgs& A) {
+// How many of the batch's placements are accumulated, given the call's first error.  Mixed
+// path: none when the error lies in this batch or an earlier one.  FP64 path: those before
+// the failing placement, as the reference's loop accumulates them.  Errors of later batches
+// (already running on the other stream) do not count.  The answer cannot change between the
+// accumulation kernels of a batch: the earlier batches' kernels are complete by then and the
+// error key only decreases.
+__device__ __forceinline__ int batch_accepted(const AccArgs& A) {
   const volatile unsigned long long* ek = &A.status->err_key;
   const unsigned long long k = *ek;
-  return k != kNoError && (long long)(k >> 36) < (long long)A.a.b0 + A.a.nb;
+  if (k == kNoError) return A.a.nb;
+  const long long before = (long long)(k >> 36) - A.a.b0;
+  if (before >= A.a.nb) return A.a.nb;
+  return (A.ff_keys || before <= 0) ? 0 : (int)before;
 }
 
 // fixed-order block sum: thread t adds elements t, t+256, ... in order, then a fixed tree
@@ -176,7 +181,6 @@ __global__ void __launch_bounds__(kAccThreads) reduce_kernel(AccArgs A) {
 
 __global__ void __launch_bounds__(kAccThreads) accumulate_kernel(AccArgs A) {
   const BatchArgs& a = A.a;
-  const int nb = a.nb;
   __shared__ double sw[kMaxBatch];
   __shared__ double stw[kMaxBatch];
   __shared__ double su0[kMaxBatch];
@@ -184,13 +188,13 @@ __global__ void __launch_bounds__(kAccThreads) accumulate_kernel(AccArgs A) {
   __shared__ double sterm[kMaxBatch];
   __shared__ double sred[2][kAccThreads];
   __shared__ unsigned char srej[kMaxBatch];  // rejected by the configuration check
-  __shared__ int skip;
+  __shared__ int accepted;
   __shared__ double s_voffset;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) srej[b] = (a.skip && a.skip[b]) ? 1 : 0;
+  for (int b = threadIdx.x; b < a.nb; b += blockDim.x) srej[b] = (a.skip && a.skip[b]) ? 1 : 0;
   __syncthreads();
   if (threadIdx.x == 0) {
-    skip = batch_failed(A) ? 1 : 0;
-    if (!skip && A.wgtslf && A.scal[4] == 0.0) {
+    const int nb = accepted = batch_accepted(A);
+    if (nb > 0 && A.wgtslf && A.scal[4] == 0.0) {
       // voffset from the first placement ever accumulated (update_histogram,
       // engproc.F90:779-783); rejected placements never reach it
       int first = 0;
@@ -200,20 +204,19 @@ __global__ void __launch_bounds__(kAccThreads) accumulate_kernel(AccArgs A) {
         A.scal[4] = 1.0;
       }
     }
-    if (!skip && A.rigid && A.scal[6] == 0.0) {
+    if (nb > 0 && A.rigid && A.scal[6] == 0.0) {
       A.scal[5] = a.u_usreal[0];
       A.scal[6] = 1.0;
     }
     s_voffset = A.scal[3];
   }
   __syncthreads();
-  if (skip) {
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-      a.engnmfc[b] = 0.0;
-      A.ring_valid[b] = 0;
-    }
-    return;
+  const int nb = accepted;
+  for (int b = nb + threadIdx.x; b < a.nb; b += blockDim.x) {
+    a.engnmfc[b] = 0.0;
+    A.ring_valid[b] = 0;
   }
+  if (nb == 0) return;
   // weights (parallel); u0 and the eself bins staged for the ordered sums
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     su0[b] = A.u0[b];
@@ -359,8 +362,8 @@ __global__ void __launch_bounds__(kAccThreads) accumulate_kernel(AccArgs A) {
 // intermediate-state mode does this inside accumulate_kernel instead
 __global__ void __launch_bounds__(128) accumulate_bins_kernel(AccArgs A) {
   const BatchArgs& a = A.a;
-  const int nb = a.nb;
-  if (nb <= 0 || batch_failed(A)) return;  // the batch was not accumulated (an error)
+  const int nb = batch_accepted(A);
+  if (nb <= 0) return;  // the batch was not accumulated (an error)
   __shared__ double sw[kMaxBatch];
   for (int b = threadIdx.x; b < nb; b += blockDim.x) sw[b] = a.engnmfc[b];
   __syncthreads();
@@ -663,7 +666,7 @@ cudaError_t launch_accumulate(Engine& e, const BatchArgs& a, cudaStream_t s) {
   A.numslv = e.numslv;
   A.ermax = e.ermax;
   A.esmax = e.esmax;
-  A.nself = e.mixed ? spectrum_partials(e) : influence64_blocks();
+  A.nself = e.mixed ? spectrum_partials(e) : spectrum64_partials(e);
   A.selfcal = e.P.selfcal;
   A.wgtslf = e.P.wgtslf;
   A.soln = e.P.slttype == 1;

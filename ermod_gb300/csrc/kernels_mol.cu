@@ -209,41 +209,6 @@ __device__ __forceinline__ int wrapi(int x, int K) {
   return x;
 }
 
-// fixed-tree block reductions over blockDim.x (power of two) entries
-__device__ __forceinline__ double block_sum(double* sm, double v) {
-  sm[threadIdx.x] = v;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sm[threadIdx.x] += sm[threadIdx.x + st];
-    __syncthreads();
-  }
-  const double r = sm[0];
-  __syncthreads();
-  return r;
-}
-__device__ __forceinline__ long long block_min(long long* sm, long long v) {
-  sm[threadIdx.x] = v;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sm[threadIdx.x] = min(sm[threadIdx.x], sm[threadIdx.x + st]);
-    __syncthreads();
-  }
-  const long long r = sm[0];
-  __syncthreads();
-  return r;
-}
-__device__ __forceinline__ long long block_max(long long* sm, long long v) {
-  sm[threadIdx.x] = v;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sm[threadIdx.x] = max(sm[threadIdx.x], sm[threadIdx.x + st]);
-    __syncthreads();
-  }
-  const long long r = sm[0];
-  __syncthreads();
-  return r;
-}
-
 __device__ __forceinline__ double key_to_double(long long k) {
   k = k ^ ((k >> 63) & 0x7fffffffffffffffll);
   return __longlong_as_double(k);
@@ -431,166 +396,164 @@ __device__ __forceinline__ ff real_mixed(const MolArgs& A, const BatchArgs& a, i
 constexpr long long kKeyPosInf = 0x7ff0000000000000ll;
 constexpr long long kKeyNegInf = (long long)0x800fffffffffffffull;  // ordered key of -inf
 
-// the plain FP64 path: one placement group per block row, one solvent molecule per thread
-template <int P>
-__global__ void __launch_bounds__(256) mol_energy_kernel(MolArgs A) {
-  extern __shared__ int smem_hist[];  // [G][ermax]
-  __shared__ double sred[256];
-  __shared__ long long skey[256];
-  const int tile = blockIdx.x;
-  const int bgrp = blockIdx.y;
+// The plain FP64 path: T = 4 TY threads per (solvent molecule, placement).  FP64 runs at 2
+// FMA per clock and SM on GB300, a warp instruction taking as long with one active lane as
+// with 32, so the work is laid out for full lanes: thread t of a molecule takes the stencil
+// columns c1 = t mod 4, + 4, .. (four consecutive doubles of a grid row side by side in a
+// warp's load, and 21 FP64 instructions per site instead of 148 for the plain triple loop)
+// and the stencil rows c2 = t / 4, + TY, ..; of the real-space pairs it takes every T-th,
+// ordered with the solute site fastest so that neighbouring threads evaluate the same solvent
+// site (the LJ branch is then uniform).  TY = 1 in reference mode, where the batch fills the
+// GPU; TY = 4 for a solution-mode frame of few molecules, whose latency is one molecule's
+// serial chain (mol64_ty).  Per placement, against one thread per molecule and one placement
+// per launch: 148 -> 8.3 us (4,000 waters, 6 sites, 48^3), 260 -> 49 us (33,000 waters, 12
+// sites, 96^3); one frame of 1,000 waters at 32^3 167 -> 33 us.
+constexpr int kMol64Threads = 256;
+template <int P, int TY>
+__global__ void __launch_bounds__(kMol64Threads) mol_energy_kernel(MolArgs A) {
+  constexpr int T = 4 * TY, kMols = kMol64Threads / T;
+  const int tile = blockIdx.x, b = blockIdx.y;
   const BatchArgs& a = A.a;
-  const int G = a.G;
-  const int m = tile * blockDim.x + threadIdx.x;
+  const int sub = threadIdx.x % T;
+  const int m = tile * kMols + threadIdx.x / T;
   const bool valid = m < A.slvmax;
-  for (int i = threadIdx.x; i < G * A.ermax; i += blockDim.x) smem_hist[i] = 0;
-  __syncthreads();
-
   int k = -1, s0 = 0, ns = 0, species = 0;
-  double qmol = 0.0;
   if (valid) {
     k = A.slot_mol[m];
     s0 = A.slot_site[m];
     ns = A.slot_site[m + 1] - s0;
     species = A.slot_species[m];
-    qmol = A.slot_qmol[m];
   }
   const FrameGeom& g = A.g;
   const int K1 = g.K[0], K2 = g.K[1], K3 = g.K[2];
-  const size_t gridn = (size_t)K1 * K2 * K3;
-  const LjK64 k64 = make_k64(A);
-  const double rc = fmax(A.elecut, A.upljcut);
-  const float mol_r = A.frame_scal[0];
-  int sp_off = 0, sp_n = 1, sp_soft = 1;
-  if (valid && species >= 1 && species <= A.numslv) {
-    sp_off = A.spec[3 * (species - 1)];
-    sp_n = A.spec[3 * (species - 1) + 1];
-    sp_soft = A.spec[3 * (species - 1) + 2];
+  const int tg = a.tagslt[b] - 1;
+  const int kskip = (tg >= 0 && tg < A.nummol) ? A.mol_to_k[tg] : -2;
+  // a placement rejected by check_mol_configuration has no molecule (engproc.F90:690-691)
+  const bool active = valid && (k != kskip) && !(a.skip && a.skip[b]);
+  double recip = 0.0, real = 0.0;
+  if (active) {
+    // ---- reciprocal part ----
+    if (!A.bare) {  // bare Coulomb: no reciprocal part
+      const double* phi = a.phi64 + (size_t)b * K1 * K2 * K3;
+      for (int s = 0; s < ns; ++s) {
+        const int idx = s0 + s;
+        const double* w = A.site_w + (size_t)idx * 3 * P;
+        const int gp = A.site_grid[idx];
+        const int g1 = gp & 1023, g2 = (gp >> 10) & 1023, g3 = (gp >> 20) & 1023;
+        double w3[P];
+        int z[P];
+#pragma unroll
+        for (int c3 = 0; c3 < P; ++c3) {
+          w3[c3] = w[2 * P + c3];
+          z[c3] = wrapi(g3 - c3, K3);
+        }
+        double site = 0.0;
+#pragma unroll
+        for (int c1 = sub & 3; c1 < P; c1 += 4) {
+          const double* col = phi + wrapi(g1 - c1, K1);
+          double line = 0.0;
+#pragma unroll
+          for (int c2 = sub >> 2; c2 < P; c2 += TY) {
+            const double* row = col + (size_t)wrapi(g2 - c2, K2) * K1;
+            double t = 0.0;
+#pragma unroll
+            for (int c3 = 0; c3 < P; ++c3) t = fma(w3[c3], row[(size_t)z[c3] * K1 * K2], t);
+            line = fma(w[P + c2], t, line);
+          }
+          site = fma(w[c1], line, site);
+        }
+        recip = fma(A.site_q[idx], site, recip);
+      }
+    }
+    // ---- real space ----
+    const int nu = a.u_nsite[b];
+    const size_t ub = (size_t)b * kMaxSoluteSites;
+    const float rcut = (float)fmax(A.elecut, A.upljcut) + a.u_radius[b] + A.frame_scal[0];
+    double d0 = 0.0;
+    for (int i = 0; i < 3; ++i) {
+      const double h = 0.5 * g.L[i];
+      const double x = fabs(A.site_x[3 * (size_t)s0 + i] - a.u_x[ub * 3 + i]);
+      const double d = g.periodic ? h - fabs(h - x) : x;
+      d0 += d * d;
+    }
+    if (nu > 0 && d0 <= (double)rcut * (double)rcut) {
+      const int npair = nu * ns;
+      int s = sub / nu, su = sub - s * nu;  // pair s nu + su, advanced by T
+      const int ds = T / nu, du = T - ds * nu;
+      for (int p = sub; p < npair; p += T) {
+        real += pair_fp64(A, s0 + s, a.u_x + (ub + su) * 3, a.u_q[ub + su], a.u_pos[ub + su].w,
+                          kPairLj | kPairCoulomb);
+        s += ds;
+        su += du;
+        if (su >= nu) {
+          su -= nu;
+          ++s;
+        }
+      }
+    }
   }
-
-  for (int gi = 0; gi < G; ++gi) {
-    const int b = bgrp * G + gi;
-    if (b >= a.nb) break;  // uniform across the block
-    const int tg = a.tagslt[b] - 1;
-    const int kskip = (tg >= 0 && tg < A.nummol) ? A.mol_to_k[tg] : -2;
-    // a placement rejected by check_mol_configuration has no molecule (engproc.F90:690-691)
-    const bool active = valid && (k != kskip) && !(a.skip && a.skip[b]);
-    double u = 0.0;
+  // the T threads' parts, in a fixed tree (every thread of the warp takes part)
+#pragma unroll
+  for (int o = 1; o < T; o <<= 1) {
+    recip += __shfl_xor_sync(0xffffffffu, recip, o);
+    real += __shfl_xor_sync(0xffffffffu, real, o);
+  }
+  const bool owner = active && sub == 0;
+  double u = 0.0;
+  if (valid && sub == 0) {
     if (active) {
-      // ---- reciprocal part ----
-      double recip = 0.0;
-      if (!A.bare) {  // bare Coulomb: no reciprocal part
-        const double* phi = a.phi64 + (size_t)b * gridn;
-        for (int s = 0; s < ns; ++s) {
-          const int idx = s0 + s;
-          const double chr = A.site_q[idx];
-          const double* w = A.site_w + (size_t)idx * 3 * P;
-          const int gp = A.site_grid[idx];
-          const int g1 = gp & 1023, g2 = (gp >> 10) & 1023, g3 = (gp >> 20) & 1023;
-          for (int c3 = 0; c3 < P; ++c3) {
-            const double fac1 = chr * w[2 * P + c3];
-            const int z = wrapi(g3 - c3, K3);
-            for (int c2 = 0; c2 < P; ++c2) {
-              const double fac2 = fac1 * w[P + c2];
-              const int y = wrapi(g2 - c2, K2);
-              const double* row = phi + ((size_t)z * K2 + y) * K1;
-              for (int c1 = 0; c1 < P; ++c1) {
-                const double fac3 = fac2 * w[c1];
-                recip = recip + fac3 * row[wrapi(g1 - c1, K1)];
-              }
-            }
-          }
-        }
-      }
-      // ---- real space ----
-      double real = 0.0;
-      const int nu = a.u_nsite[b];
-      const size_t ub = (size_t)b * kMaxSoluteSites;
-      const float rcut = (float)rc + a.u_radius[b] + mol_r;
-      double d0 = 0.0;
-      for (int i = 0; i < 3; ++i) {
-        const double h = 0.5 * g.L[i];
-        const double x = fabs(A.site_x[3 * (size_t)s0 + i] - a.u_x[ub * 3 + i]);
-        const double d = g.periodic ? h - fabs(h - x) : x;
-        d0 += d * d;
-      }
-      if (d0 <= (double)rcut * (double)rcut) {
-        for (int su = 0; su < nu; ++su) {
-          const double* ux = a.u_x + (ub + su) * 3;
-          const double qu = a.u_q[ub + su];
-          const int tu = a.u_pos[ub + su].w;
-          for (int s = 0; s < ns; ++s) {
-            const int idx = s0 + s;
-            double dist = 0.0;
-            for (int i = 0; i < 3; ++i) {  // minimum image only when periodic (realcal.F90:202-209)
-              const double h = 0.5 * g.L[i];
-              const double x = fabs(A.site_x[3 * (size_t)idx + i] - ux[i]);
-              const double d = g.periodic ? h - fabs(h - x) : x;
-              dist += d * d;
-            }
-            const int tv = A.site_pos[idx].w;
-            const double ljeps = A.ljene[tv + A.T * tu];
-            if (ljeps > 0) {
-              const double sg2 = A.ljlensq[tv + A.T * tu];
-              if (dist <= k64.lw2)
-                real += lj_low64(A.ljswitch, k64, ljeps, sg2, dist);
-              else if (dist <= k64.up2)
-                real += lj_switch64(A.ljswitch, k64, ljeps, sg2, dist);
-            }
-            if (A.bare) {
-              if (dist < k64.ele2) real += qu * A.site_q[idx] / sqrt(dist);  // realcal_bare
-            } else if (dist <= k64.ele2) {
-              const double r = sqrt(dist);
-              real += qu * A.site_q[idx] * (1.0 - erf(A.screen * r)) / r;
-            }
-          }
-        }
-      }
-      // residual_ene + assembly (engproc.F90:741-752)
-      double epcl;
-      if (A.bare)
-        epcl = 0.0;  // residual_ene returns without a term for bare Coulomb
-      else
-        epcl = kPi * a.u_qmol[b] * qmol / A.screen / A.screen / g.volume;
-      double pairep = -epcl;
-      pairep = pairep + recip;
-      u = real + pairep;
+      // residual_ene + assembly (engproc.F90:741-752); bare Coulomb has no such term
+      const double epcl =
+          A.bare ? 0.0 : kPi * a.u_qmol[b] * A.slot_qmol[m] / A.screen / A.screen / g.volume;
+      u = real + (recip - epcl);
       // ---- getiduv / binsearch ----
-      int ret = 0;
+      int sp_off = 0, sp_n = 1, sp_soft = 1, ret = 0;
+      if (species >= 1 && species <= A.numslv) {
+        sp_off = A.spec[3 * (species - 1)];
+        sp_n = A.spec[3 * (species - 1) + 1];
+        sp_soft = A.spec[3 * (species - 1) + 2];
+      }
       const int code = bin_molecule(A, u, species, sp_off, sp_n, sp_soft, ret);
       if (code)
         atomicMin(&A.status->err_key, make_err_key(a.b0 + b, k + 1, code));
       else
-        hist_add(smem_hist + gi * A.ermax, sp_off + ret - 1);
-      if (a.uvengy_out) a.uvengy_out[(size_t)(a.b0 + b) * (A.slvmax + 1) + k + 1] = u;
-    } else if (valid && a.uvengy_out) {
-      a.uvengy_out[(size_t)(a.b0 + b) * (A.slvmax + 1) + k + 1] = 0.0;
+        hist_add(a.hist + (size_t)b * A.ermax, sp_off + ret - 1);
     }
-    // per-species partials {sum, min, max} of this block (fixed-tree reductions)
-    for (int sp = 1; sp <= A.numslv; ++sp) {
-      const bool mine = active && species == sp;
-      const double s = block_sum(sred, mine ? u : 0.0);
-      const long long mn = block_min(skey, mine ? ordered_key(u) : kKeyPosInf);
-      const long long mx = block_max(skey, mine ? ordered_key(u) : kKeyNegInf);
-      if (threadIdx.x == 0) {
-        double* pt = a.part + (((size_t)b * A.ntile + tile) * A.numslv + (sp - 1)) * 3;
-        pt[0] = s;
-        pt[1] = key_to_double(mn);
-        pt[2] = key_to_double(mx);
-      }
-    }
+    if (a.uvengy_out) a.uvengy_out[(size_t)(a.b0 + b) * (A.slvmax + 1) + k + 1] = u;
   }
-  __syncthreads();
-  // flush the block's histograms
-  for (int gi = 0; gi < G; ++gi) {
-    const int b = bgrp * G + gi;
-    if (b >= a.nb) break;
-    const int* h = smem_hist + gi * A.ermax;
-    int* out = a.hist + (size_t)b * A.ermax;
-    for (int i = threadIdx.x; i < A.ermax; i += blockDim.x) {
-      const int c = h[i];
-      if (c) atomicAdd(out + i, c);
+  // per-species partials {sum, min, max} of this block: fixed trees over the warps, then the
+  // warps in order
+  constexpr int kWarps = kMol64Threads / 32;
+  __shared__ double wsum[kWarps];
+  __shared__ long long wmin[kWarps], wmax[kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int sp = 1; sp <= A.numslv; ++sp) {
+    const bool mine = owner && species == sp;
+    double s = mine ? u : 0.0;
+    long long mn = mine ? ordered_key(u) : kKeyPosInf, mx = mine ? ordered_key(u) : kKeyNegInf;
+    for (int o = 16; o > 0; o >>= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+      mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
+    if (lane == 0) {
+      wsum[warp] = s;
+      wmin[warp] = mn;
+      wmax[warp] = mx;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < kWarps; ++w) {
+        s += wsum[w];
+        mn = min(mn, wmin[w]);
+        mx = max(mx, wmax[w]);
+      }
+      double* pt = a.part + (((size_t)b * A.ntile + tile) * A.numslv + (sp - 1)) * 3;
+      pt[0] = s;
+      pt[1] = key_to_double(mn);
+      pt[2] = key_to_double(mx);
+    }
+    __syncthreads();
   }
 }
 
@@ -1108,16 +1071,18 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
   }
 }
 
-cudaError_t launch_p(Engine& e, const MolArgs& A, dim3 grid, size_t smem) {
+template <int TY>
+cudaError_t launch_mol64(Engine& e, const MolArgs& A) {
+  const dim3 grid(A.ntile, A.a.nb);
   switch (e.P_order) {
     case 4:
-      mol_energy_kernel<4><<<grid, 256, smem, A.a.stream>>>(A);
+      mol_energy_kernel<4, TY><<<grid, kMol64Threads, 0, A.a.stream>>>(A);
       break;
     case 6:
-      mol_energy_kernel<6><<<grid, 256, smem, A.a.stream>>>(A);
+      mol_energy_kernel<6, TY><<<grid, kMol64Threads, 0, A.a.stream>>>(A);
       break;
     case 8:
-      mol_energy_kernel<8><<<grid, 256, smem, A.a.stream>>>(A);
+      mol_energy_kernel<8, TY><<<grid, kMol64Threads, 0, A.a.stream>>>(A);
       break;
     default:
       return cudaErrorInvalidValue;
@@ -1206,20 +1171,17 @@ cudaError_t launch_gather(Engine& e, const BatchArgs& a) {
   return cudaGetLastError();
 }
 
+// the FP64 path's threads per molecule, 4 TY: a solution-mode call holds one placement (or
+// one per solute molecule), so its molecules are split further while that still leaves the
+// GPU room; fixed for a context, so that a placement's sums do not depend on its batch
+static int mol64_ty(const Engine& e) { return e.P.slttype == 1 && e.slvmax < 512 * e.num_sm ? 4 : 1; }
+int mol64_tile(const Engine& e) { return kMol64Threads / (4 * mol64_ty(e)); }
+
 cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a) {
   const MolArgs A = make_mol_args(e, a);
-  const size_t smem = sizeof(int) * (size_t)a.G * e.ermax;
-  dim3 grid(e.ntile, (a.nb + a.G - 1) / a.G);
   e.count_launch();
   cudaError_t err = cudaSuccess;
-  if (!e.mixed) {
-    static SmemAttr attr4, attr6, attr8;
-    if ((err = attr4.ensure(mol_energy_kernel<4>, smem)) != cudaSuccess ||
-        (err = attr6.ensure(mol_energy_kernel<6>, smem)) != cudaSuccess ||
-        (err = attr8.ensure(mol_energy_kernel<8>, smem)) != cudaSuccess)
-      return err;
-    return launch_p(e, A, grid, smem);
-  }
+  if (!e.mixed) return mol64_ty(e) == 4 ? launch_mol64<4>(e, A) : launch_mol64<1>(e, A);
   if (a.G != 8 && a.G != 4) return cudaErrorInvalidValue;
   if (e.P.cltype != 0 && (err = launch_gather(e, a)) != cudaSuccess) return err;
   if (a.phases) {

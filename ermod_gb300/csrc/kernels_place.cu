@@ -3,12 +3,12 @@
 //   place_prep    solute sites of every placement in a batch: wrapped FP64 and
 //                 fixed-point coordinates, calc_spline_molecule (recpcal.F90:408-442,
 //                 FP64 weights on both paths),
-//                 realcal_self (realcal.F90:284-328, FP64) and, for the mixed path,
-//                 the 1-D structure-factor vectors
+//                 realcal_self (realcal.F90:284-328, FP64) and the 1-D structure-factor
+//                 vectors
 //                     b_{s,a}(k) = sum_c theta_{s,a,c} exp(-2 pi i k (g_{s,a} - c) / K_a);
 //                 (the mixed path's spectrum and transforms are in kernels_fft.cu);
-//   spread64 / influence64   the plain FP64 path, literally the reference's order:
-//                 spread, D2Z (cuFFT), self energy + engfac multiply, Z2D (cuFFT).
+//   spectrum64    the plain FP64 path's spectrum engfac S(k) from those vectors, with the
+//                 self energy; its inverse transform is a batched cuFFT Z2D.
 #include "engine.cuh"
 
 namespace ermod {
@@ -142,9 +142,9 @@ __global__ void __launch_bounds__(256) place_prep_kernel(PrepArgs A) {
     a.u_qmol[b] = A.mol_qmol_all[mol];
   }
   __syncthreads();
-  // 1-D structure-factor vectors (mixed path): FP64 weights and twiddles, rounded to FP32
-  // once at the end, so that their errors are independent roundings
-  if (A.mixed) {
+  // 1-D structure-factor vectors: FP64 weights and twiddles; the mixed path rounds them to
+  // FP32 once at the end, so that their errors are independent roundings
+  if (!A.bare) {
     const int Kx = g.K[0], Ky = g.K[1], Kz = g.K[2];
     const int Kmax = max(Kx, max(Ky, Kz));
     const int total = ns * 3 * Kmax;
@@ -170,7 +170,10 @@ __global__ void __launch_bounds__(256) place_prep_kernel(PrepArgs A) {
         re = fma(th[c], w.x, re);
         im = fma(th[c], w.y, im);
       }
-      a.u_bvec[(us * 3 + ax) * Kmax + k] = make_float2((float)re, (float)im);
+      if (A.mixed)
+        a.u_bvec[(us * 3 + ax) * Kmax + k] = make_float2((float)re, (float)im);
+      else
+        a.u_bvec64[(us * 3 + ax) * Kmax + k] = make_double2(re, im);
     }
   }
   // bounding radius about site 1 (minimum image; FP32, padded to stay conservative)
@@ -225,69 +228,80 @@ __global__ void __launch_bounds__(256) place_prep_kernel(PrepArgs A) {
 }
 
 // ---- FP64 path ----------------------------------------------------------------------
-struct Spread64Args {
-  const double* u_q;
-  const double* u_w;
-  const int* u_grid;
+struct Spec64Args {
+  const double2* bvec;  // [nb][S][3][Kmax]
+  const double* u_q;    // [nb][S]
   const int* u_nsite;
-  double* grid;  // [nb][K3][K2][K1]
-  int K1, K2, K3, P;
+  const double* engfac;  // [K3][K2][H]
+  double2* spec;         // [nb][K3][K2][H]
+  double* self_part;     // [nb][spectrum64_partials]
+  int K1, K2, K3, H, Kmax, R;
 };
 
-// one block per placement; sites in order, the P^3 stencil points of a site in parallel
-__global__ void spread64_kernel(Spread64Args A) {
-  const int b = blockIdx.x;
+// The FP64 spectrum engfac(k) S(k), S = sum_s q_s b1_s(k1) b2_s(k2) b3_s(k3): exactly the R2C
+// transform of the spread charges (recpcal.F90:357-384) without the K^3 grid, the spread and
+// the forward transform, and with the self energy 0.5 sum_k engfac |S|^2 (recpcal.F90:385-394)
+// in the same pass.  CTA per (k2, R values of k3, placement): the R x ns row factors
+// q b2 b3 in shared memory, a thread per point of R rows of H.  Bound by the FP64 pipe: 4 FMA
+// per point and site, which at 2 per clock and SM is 35 us for 12 sites at 96^3; measured 50 us a
+// placement there (4.1 us for 6 sites at 48^3), against 149 us (45 us) for the spread, cuFFT's
+// D2Z and the influence pass in its place, one placement at a time.
+constexpr int kSpec64Threads = 256;
+__global__ void __launch_bounds__(kSpec64Threads) spectrum64_kernel(Spec64Args A) {
+  extern __shared__ double2 sc[];  // [ns][R]: q_s b2_s(k2) b3_s(k3)
+  const int k2 = blockIdx.x, k3a = blockIdx.y * A.R, b = blockIdx.z;
+  const int nr = min(A.R, A.K3 - k3a);
   const int ns = A.u_nsite[b];
-  const int P = A.P, P3 = P * P * P;
-  double* grid = A.grid + (size_t)b * A.K1 * A.K2 * A.K3;
-  for (int s = 0; s < ns; ++s) {
-    const size_t us = (size_t)b * kMaxSoluteSites + s;
-    const int gp = A.u_grid[us];
-    const int g1 = gp & 1023, g2 = (gp >> 10) & 1023, g3 = (gp >> 20) & 1023;
-    const double chr = A.u_q[us];
-    const double* w = A.u_w + us * 3 * kMaxSplineOrder;
-    for (int t = threadIdx.x; t < P3; t += blockDim.x) {
-      const int cg1 = t % P, cg2 = (t / P) % P, cg3 = t / (P * P);
-      int r1 = (g1 - cg1) % A.K1, r2 = (g2 - cg2) % A.K2, r3 = (g3 - cg3) % A.K3;
-      if (r1 < 0) r1 += A.K1;
-      if (r2 < 0) r2 += A.K2;
-      if (r3 < 0) r3 += A.K3;
-      const double factor = chr * w[cg1] * w[kMaxSplineOrder + cg2] * w[2 * kMaxSplineOrder + cg3];
-      grid[((size_t)r3 * A.K2 + r2) * A.K1 + r1] += factor;
+  const double2* bv = A.bvec + (size_t)b * kMaxSoluteSites * 3 * A.Kmax;
+  for (int t = threadIdx.x; t < ns * nr; t += blockDim.x) {
+    const int s = t / nr, r = t - s * nr;
+    const double q = A.u_q[(size_t)b * kMaxSoluteSites + s];
+    const double2 b2 = bv[(size_t)(s * 3 + 1) * A.Kmax + k2], b3 = bv[(size_t)(s * 3 + 2) * A.Kmax + k3a + r];
+    const double x = q * b2.x, y = q * b2.y;
+    sc[s * A.R + r] = make_double2(x * b3.x - y * b3.y, x * b3.y + y * b3.x);
+  }
+  __syncthreads();
+  const bool even = (A.K1 % 2) == 0;
+  double self = 0.0;
+  for (int t = threadIdx.x; t < nr * A.H; t += blockDim.x) {
+    const int r = t / A.H, k1 = t - r * A.H;
+    double re = 0.0, im = 0.0;
+    for (int s = 0; s < ns; ++s) {
+      const double2 c = sc[s * A.R + r];
+      const double2 e = __ldg(bv + (size_t)s * 3 * A.Kmax + k1);
+      re = fma(c.x, e.x, fma(-c.y, e.y, re));
+      im = fma(c.x, e.y, fma(c.y, e.x, im));
     }
-    __syncthreads();
+    const size_t at = ((size_t)(k3a + r) * A.K2 + k2) * A.H + k1;
+    const double ef = A.engfac[at];
+    const double en = ef * (re * re + im * im);
+    self += (k1 == 0 || (even && k1 == A.H - 1)) ? 0.5 * en : en;
+    A.spec[(size_t)b * A.K3 * A.K2 * A.H + at] = make_double2(ef * re, ef * im);
+  }
+  __shared__ double red[kSpec64Threads / 32];
+  for (int o = 16; o > 0; o >>= 1) self += __shfl_xor_sync(0xffffffffu, self, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = self;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kSpec64Threads / 32; ++w) self += red[w];
+    A.self_part[((size_t)b * gridDim.y + blockIdx.y) * A.K2 + k2] = self;
   }
 }
 
-struct Infl64Args {
-  double2* spec;          // [nb][K3][K2][H]
-  const double* engfac;
-  double* self_part;      // [nb][nblk]
-  int K1, K2, K3, H;
-  size_t n;
-  int nblk;
-};
-
-__global__ void __launch_bounds__(256) influence64_kernel(Infl64Args A) {
-  const int b = blockIdx.y;
-  double s = 0.0;
-  const bool even = (A.K1 % 2) == 0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += (size_t)gridDim.x * blockDim.x) {
-    const int k1 = (int)(i % A.H);
-    double2 z = A.spec[(size_t)b * A.n + i];
-    const double ef = A.engfac[i];
-    const double e = ef * (z.x * z.x + z.y * z.y);
-    s += (k1 == 0 || (even && k1 == A.H - 1)) ? 0.5 * e : e;
-    A.spec[(size_t)b * A.n + i] = make_double2(ef * z.x, ef * z.y);
+// k3 rows per CTA: the count up to 16 whose R H points leave the fewest of the CTA's thread
+// rounds idle
+int spec64_rows(int H) {
+  int best = 1;
+  double use = 0.0;
+  for (int R = 1; R <= 16; ++R) {
+    const int n = R * H, rounds = (n + kSpec64Threads - 1) / kSpec64Threads;
+    const double u = (double)n / (rounds * kSpec64Threads);
+    if (u > use + 1e-9) {
+      use = u;
+      best = R;
+    }
   }
-  __shared__ double red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int st = 128; st > 0; st >>= 1) {
-    if (threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) A.self_part[(size_t)b * A.nblk + blockIdx.x] = red[0];
+  return best;
 }
 
 Coef make_coef(int order, double screen) {
@@ -337,39 +351,31 @@ cudaError_t launch_place_prep(Engine& e, const BatchArgs& a, const double* sol_x
   return cudaGetLastError();
 }
 
-cudaError_t launch_spread64(Engine& e, const BatchArgs& a) {
-  Spread64Args A{};
-  A.u_q = a.u_q;
-  A.u_w = a.u_w;
-  A.u_grid = a.u_grid;
-  A.u_nsite = a.u_nsite;
-  A.grid = a.phi64;
-  A.K1 = e.geom.K[0];
-  A.K2 = e.geom.K[1];
-  A.K3 = e.geom.K[2];
-  A.P = e.P_order;
-  cudaError_t err = cudaMemsetAsync(a.phi64, 0, sizeof(double) * e.grid_real() * a.nb, a.stream);
-  if (err != cudaSuccess) return err;
-  spread64_kernel<<<a.nb, 128, 0, a.stream>>>(A);
-  e.count_launch();
-  return cudaGetLastError();
+int spectrum64_partials(const Engine& e) {
+  const int R = spec64_rows(e.H());
+  return e.geom.K[1] * ((e.geom.K[2] + R - 1) / R);
 }
 
-int influence64_blocks() { return 152 * 2; }
-
-cudaError_t launch_influence64(Engine& e, const BatchArgs& a) {
-  Infl64Args A{};
-  A.spec = a.spec64;
+cudaError_t launch_spectrum64(Engine& e, const BatchArgs& a) {
+  Spec64Args A{};
+  A.bvec = a.u_bvec64;
+  A.u_q = a.u_q;
+  A.u_nsite = a.u_nsite;
   A.engfac = e.d_engfac;
+  A.spec = a.spec64;
   A.self_part = a.self_part;
   A.K1 = e.geom.K[0];
   A.K2 = e.geom.K[1];
   A.K3 = e.geom.K[2];
   A.H = e.H();
-  A.n = e.grid_cplx();
-  A.nblk = influence64_blocks();
-  dim3 grid(A.nblk, a.nb);
-  influence64_kernel<<<grid, 256, 0, a.stream>>>(A);
+  A.Kmax = e.Kmax();
+  A.R = spec64_rows(A.H);
+  const size_t smem = sizeof(double2) * kMaxSoluteSites * A.R;
+  static SmemAttr attr;
+  cudaError_t err = attr.ensure(spectrum64_kernel, smem);
+  if (err != cudaSuccess) return err;
+  const dim3 grid(A.K2, (A.K3 + A.R - 1) / A.R, a.nb);
+  spectrum64_kernel<<<grid, kSpec64Threads, smem, a.stream>>>(A);
   e.count_launch();
   return cudaGetLastError();
 }
