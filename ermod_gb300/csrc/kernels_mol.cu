@@ -68,6 +68,7 @@ struct MolArgs {
   float fxf[3];    // fixed-point unit per axis (box length / 2^32)
   float screen_f;  // Ewald beta
   float rc_f;      // max(elecut, upljcut)
+  int real_lanes;  // finish kernel: threads sharing a near molecule's solute sites
   int bare;        // cltype 0: bare Coulomb within elecut (no cutoff when non-periodic), no reciprocal space
                    // or residual
   LjK k32;         // LJ switching constants
@@ -292,43 +293,40 @@ __device__ __forceinline__ double pair_fp64(const MolArgs& A, int idx, const dou
   return e;
 }
 
-// FP64 pairs recorded per thread by the finish kernel's first pass (see mol_finish_kernel)
+// The finish kernel's FP64 pairs (see mol_finish_kernel): recorded per thread and window of its
+// real-space pass, and gathered in the block's list until it is full or the pass ends
 constexpr int kBigPerThread = 8;
-// that pass's scratch (ints): the recorded pairs, their compacted list (16-bit), the
-// threads' first sites and one double per thread
-constexpr int kFinishScratchInts = 256 * kBigPerThread + 256 * kBigPerThread / 2 + 256 + 2 * 256;
+constexpr int kBigList = 1024;
+// that pass's scratch (ints): the list (pairs, their near items as 16 bits, their values), the
+// threads' recorded pairs, the molecules' first sites, and the list of near (molecule,
+// placement) items (16 bits)
+__host__ __device__ constexpr int finish_scratch_ints(int G) {
+  return kBigList + kBigList / 2 + 2 * kBigList + 256 * kBigPerThread + 256 + G * 256 / 2;
+}
 // the dynamic shared memory of the finish kernel before its edge keys: the block
-// histograms (when in shared memory) or the FP64 pass's scratch, whichever is larger
+// histograms (when in shared memory) or the real-space pass's scratch, whichever is larger
 __host__ __device__ __forceinline__ int finish_region_ints(int G, int ermax, int hist_global) {
   const int h = hist_global ? 0 : G * ermax;
-  return h > kFinishScratchInts ? h : kFinishScratchInts;
+  return h > finish_scratch_ints(G) ? h : finish_scratch_ints(G);
 }
-// a recorded pair: its FP64 parts (2 bits), placement j of the block (3 bits), solute site
-// (8 bits), site of the solvent molecule (13 bits)
-__device__ __forceinline__ int big_item(int parts, int j, int su, int s) {
-  return (parts << 24) | (j << 21) | (su << 13) | s;
-}
+// a recorded pair: its FP64 parts (2 bits), solute site (8 bits), site of the solvent
+// molecule (13 bits)
+__device__ __forceinline__ int big_item(int parts, int su, int s) { return (parts << 21) | (su << 13) | s; }
 
-// real-space LJ + screened Coulomb of one molecule against solute b (mixed path):
-// fixed-point displacements and FP32 pair terms, summed as a float-float number.  An FP32
-// LJ or Coulomb term above kFp64Lj / kFp64Coulomb in magnitude (or not finite) is left out
-// of the sum and counted in nbig (in the thread's scan order); the count's values in
-// [win, win + kBigPerThread) are recorded with their parts in items[count - win], and bit j
-// of fix is set.  kSum: sum the FP32 terms (the first pass); else only record (the later
-// rounds of a thread with more pairs than one round takes).
 constexpr int kMolSiteCache = 3;  // molecule sites held in registers by the real-space pass
 
-template <bool kSum>
-__device__ __forceinline__ ff real_mixed(const MolArgs& A, const BatchArgs& a, int b, int s0, int ns,
-                                         const LjK& k32, float rcut, int4 p0, int4 u0, int j, int* items,
-                                         int win, int& nbig, unsigned& fix) {
+// real-space LJ + screened Coulomb of one molecule against solute b's sites su0, su0 + L, ..
+// (mixed path): fixed-point displacements and FP32 pair terms, summed as a float-float
+// number.  An FP32 LJ or Coulomb term above kFp64Lj / kFp64Coulomb in magnitude (or not
+// finite) is left out of the sum and counted in nbig (in the thread's scan order); the count's
+// values in [win, win + kBigPerThread) are recorded with their parts in items[count - win].
+// (A thread with more pairs than one window takes calls again for the next ones.)
+__device__ __forceinline__ ff real_mixed(const MolArgs& A, const BatchArgs& a, int b, int s0, int ns, int su0, int L,
+                                         int* items, int win, int& nbig) {
+  const LjK& k32 = A.k32;
   const size_t ub = (size_t)b * kMaxSoluteSites;
   const float fx = A.fxf[0], fy = A.fxf[1], fz = A.fxf[2];
-  const float dx = (float)(int)((unsigned)p0.x - (unsigned)u0.x) * fx;
-  const float dy = (float)(int)((unsigned)p0.y - (unsigned)u0.y) * fy;
-  const float dz = (float)(int)((unsigned)p0.z - (unsigned)u0.z) * fz;
   ff real{0.f, 0.f};
-  if (dx * dx + dy * dy + dz * dz > rcut * rcut) return real;
   const int nu = a.u_nsite[b];
   const float beta = A.screen_f;
   // one pair (solute site su at up with charge qu, molecule site s at vp with charge qv)
@@ -354,15 +352,12 @@ __device__ __forceinline__ ff real_mixed(const MolArgs& A, const BatchArgs& a, i
     }
     // parts too large for FP32 (the comparisons are false for NaN and inf)
     const int parts = (fabsf(elj) <= kFp64Lj ? 0 : kPairLj) | (fabsf(eco) <= kFp64Coulomb ? 0 : kPairCoulomb);
-    if (kSum) {
-      if (!(parts & kPairLj)) real = ff_add(real, elj);
-      if (!(parts & kPairCoulomb)) real = ff_add(real, eco);
-    }
+    if (!(parts & kPairLj)) real = ff_add(real, elj);
+    if (!(parts & kPairCoulomb)) real = ff_add(real, eco);
     if (parts) {
       const int r = nbig - win;
-      if (r >= 0 && r < kBigPerThread) items[r] = big_item(parts, j, su, s);
+      if (r >= 0 && r < kBigPerThread) items[r] = big_item(parts, su, s);
       ++nbig;
-      fix |= 1u << j;
     }
   };
   if (ns <= kMolSiteCache) {
@@ -376,7 +371,7 @@ __device__ __forceinline__ ff real_mixed(const MolArgs& A, const BatchArgs& a, i
         vpc[s] = A.site_pos[s0 + s];
         qvc[s] = A.site_rec[s0 + s].w;
       }
-    for (int su = 0; su < nu; ++su) {
+    for (int su = su0; su < nu; su += L) {
       const int4 up = a.u_pos[ub + su];
       const float qu = a.u_qf[ub + su];
 #pragma unroll
@@ -384,7 +379,7 @@ __device__ __forceinline__ ff real_mixed(const MolArgs& A, const BatchArgs& a, i
         if (s < ns) pair(su, up, qu, s, vpc[s], qvc[s]);
     }
   } else {
-    for (int su = 0; su < nu; ++su) {
+    for (int su = su0; su < nu; su += L) {
       const int4 up = a.u_pos[ub + su];
       const float qu = a.u_qf[ub + su];
       for (int s = 0; s < ns; ++s) pair(su, up, qu, s, A.site_pos[s0 + s], A.site_rec[s0 + s].w);
@@ -807,19 +802,28 @@ __device__ __forceinline__ void species_partials(const MolArgs& A, const BatchAr
 // and of the real-space pair terms, the residual, then the G bin searches in lockstep
 // (binary lifting over the float keys of the edges staged in shared memory, finished
 // exactly against the FP64 edges), histograms and per-species partials.
+//
+// The real-space pass: the block's (molecule, placement) items within the solute's bounding
+// sphere + cutoff are compacted into a list, and A.real_lanes threads (a power of two, set by
+// the solutes' sizes alone) share an item's solute sites, their float-float sums joined in a
+// fixed tree.  So a warp's lanes all have pairs to evaluate (2% of the 33,000-water box's
+// molecules lie in reach), a large solute's pairs are not one thread's serial chain, and an
+// item's sum does not depend on the block it falls in.
 template <int G>
 __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const float* __restrict__ site_e) {
-  extern __shared__ int smem_dyn[];
+  extern __shared__ __align__(16) int smem_dyn[];
   // [G][ermax] block histograms, or none when they would not fit beside other blocks: the
   // molecules' counts then go to the batch histograms in global memory (warp-aggregated).
-  // Before the histograms are zeroed, the same region holds the FP64 pass's scratch
+  // Before the histograms are zeroed, the same region holds the real-space pass's scratch
   // (finish_scratch_ints ints).
   int* smem_hist = A.hist_global ? nullptr : smem_dyn;
   int* skeys = smem_dyn + finish_region_ints(G, A.ermax, A.hist_global);  // [ermax] 32-bit edge keys
-  int* sitem = smem_dyn;                                                     // [256][kBigPerThread]
-  unsigned short* slist = reinterpret_cast<unsigned short*>(sitem + 256 * kBigPerThread);
-  int* ss0 = reinterpret_cast<int*>(slist + 256 * kBigPerThread);           // [256]
-  double* sbuf = reinterpret_cast<double*>(ss0 + 256);                      // [256]
+  double* sval = reinterpret_cast<double*>(smem_dyn);                        // [kBigList] FP64 values of the list
+  int* sbig = reinterpret_cast<int*>(sval + kBigList);                       // [kBigList] the list's pairs
+  unsigned short* sbnear = reinterpret_cast<unsigned short*>(sbig + kBigList);  // [kBigList] their near items
+  int* sitem = reinterpret_cast<int*>(sbnear + kBigList);                   // [256][kBigPerThread]
+  int* ss0 = sitem + 256 * kBigPerThread;                                   // [256] first sites
+  unsigned short* snear = reinterpret_cast<unsigned short*>(ss0 + 256);     // [G * 256] molecule | placement << 8
   __shared__ int swarp[8];
   __shared__ float su[G][256];   // totals, hi part (NaN: no molecule)
   __shared__ float sul[G][256];  // totals, lo part
@@ -859,7 +863,6 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
   const bool spec_ok = valid && species >= 1 && species <= A.numslv;
   sspec[threadIdx.x] = (unsigned char)(spec_ok ? species : 0);
   const int ldb = A.ldb;
-  const LjK& k32 = A.k32;
   int sp_off = 0, sp_n = 1, sp_soft = 1;
   if (spec_ok) {
     sp_off = A.spec[3 * (species - 1)];
@@ -869,13 +872,10 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
   __syncthreads();  // sres staged
   // ---- totals of the G placements, as float-float numbers.  First the site terms: the G
   // placements' terms of a site are G consecutive floats (16-byte loads when G, g0 and ldb
-  // are multiples of 4).  The totals then wait in this thread's entries of su (hi) and sul
-  // (lo) until the bin search; the real-space pass adds to them placement by placement in a
-  // rolled loop (one copy of its code) ----
-  unsigned actm = 0u;  // placements whose total is a solvent molecule's energy
-  unsigned fix = 0u;   // placements with pairs left for the FP64 pass
-  int nbig = 0;        // such pairs of this thread (the first kBigPerThread recorded in sitem)
-  int* items = sitem + threadIdx.x * kBigPerThread;
+  // are multiples of 4).  The totals then wait in su (hi) and sul (lo) until the bin search;
+  // the real-space pass adds to them ----
+  unsigned actm = 0u;   // placements whose total is a solvent molecule's energy
+  unsigned nearm = 0u;  // of those, the ones within reach of the solute
   {
     ff rs[G];
 #pragma unroll
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
         const float* row = site_e + (size_t)(s0 + s) * ldb + g0;
         if (G % 4 == 0 && ng == G) {
 #pragma unroll
-          for (int j4 = 0; j4 < G; j4 += 4) {
+          for (int j4 = 0; j4 + 4 <= G; j4 += 4) {
             const float4 v = __ldg(reinterpret_cast<const float4*>(row + j4));
             rs[j4] = ff_add(rs[j4], v.x);
             rs[j4 + 1] = ff_add(rs[j4 + 1], v.y);
@@ -899,46 +899,105 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
         }
       }
     }
+    const int4 p0 = valid ? A.site_pos[s0] : make_int4(0, 0, 0, 0);
 #pragma unroll
     for (int j = 0; j < G; ++j) {
       const bool on = j < ng && valid && k != skskip[j] && !srej[j];
-      if (on) actm |= 1u << j;
+      if (on) {
+        actm |= 1u << j;
+        const int4 u0 = supos[j];
+        const float dx = (float)(int)((unsigned)p0.x - (unsigned)u0.x) * A.fxf[0];
+        const float dy = (float)(int)((unsigned)p0.y - (unsigned)u0.y) * A.fxf[1];
+        const float dz = (float)(int)((unsigned)p0.z - (unsigned)u0.z) * A.fxf[2];
+        if (!(dx * dx + dy * dy + dz * dz > srcut[j] * srcut[j])) nearm |= 1u << j;
+      }
       // residual_ene (engproc.F90:859-869)
       const ff t = on ? ff_add(rs[j], -sres[j] * qmol) : ff{0.f, 0.f};
       su[j][threadIdx.x] = t.hi;
       sul[j][threadIdx.x] = t.lo;
     }
   }
-  const int4 p0 = valid ? A.site_pos[s0] : make_int4(0, 0, 0, 0);
-#pragma unroll 1
-  for (int j = 0; j < G; ++j) {
-    if (!(actm & (1u << j))) continue;
-    // get_uv_energy (engproc.F90:736-753): real + residual + recip
-    const ff r = real_mixed<true>(A, a, g0 + j, s0, ns, k32, srcut[j], p0, supos[j], j, items, 0, nbig, fix);
-    if (r.hi != 0.f || r.lo != 0.f) {
-      const ff t = ff_add2(ff{su[j][threadIdx.x], sul[j][threadIdx.x]}, r);
-      su[j][threadIdx.x] = t.hi;
-      sul[j][threadIdx.x] = t.lo;
+  // ---- real space: get_uv_energy (engproc.F90:736-753) adds it to residual + recip ----
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int near0, nnear;  // this thread's first entry of the block's near list; its length
+  {
+    const int cnt = __popc(nearm);
+    int incl = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
     }
-  }
-  // ---- FP64 pass over the pair parts left out above (overlapping pairs).  The block's
-  // recorded pairs are compacted (an exclusive scan over the threads) and evaluated one
-  // per thread, so that every FP64 instruction of the pass runs on full warps; each owner
-  // then adds its pairs' values in the order it found them.  A thread with more than
-  // kBigPerThread pairs takes further rounds, recording the next ones by a fresh scan. ----
-  if (__syncthreads_or(fix != 0u)) {
+    if (lane == 31) swarp[wid] = incl;
     ss0[threadIdx.x] = s0;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    __syncthreads();
+    near0 = incl - cnt;
+    nnear = 0;
+    for (int w2 = 0; w2 < 8; ++w2) {
+      if (w2 < wid) near0 += swarp[w2];
+      nnear += swarp[w2];
+    }
+    for (unsigned q = nearm; q; q &= q - 1) snear[near0++] = (unsigned short)(threadIdx.x | ((__ffs(q) - 1) << 8));
+    __syncthreads();
+  }
+  // FP64 pass over the listed pair parts (overlapping pairs, left out of the FP32 sums): one
+  // per thread, so that every FP64 instruction runs on full warps; the first pair of each item
+  // then adds the item's values, which lie side by side, in their order
+  int nlist = 0;  // block-uniform
+  auto add_listed = [&] {
+    __syncthreads();
+    for (int q = threadIdx.x; q < nlist; q += 256) {
+      const int it = sbig[q], nr = snear[sbnear[q]];
+      const size_t us = (size_t)(g0 + (nr >> 8)) * kMaxSoluteSites + ((it >> 13) & 0xff);
+      sval[q] = pair_fp64(A, ss0[nr & 0xff] + (it & 0x1fff), a.u_x + us * 3, a.u_q[us], a.u_pos[us].w, it >> 21);
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < nlist; q += 256) {
+      const int near = sbnear[q];
+      if (q > 0 && sbnear[q - 1] == near) continue;
+      const int t = snear[near] & 0xff, j = snear[near] >> 8;
+      ff x{su[j][t], sul[j][t]};
+      for (int i = q; i < nlist && sbnear[i] == near; ++i) x = ff_add2(x, ff_from_double(sval[i]));
+      su[j][t] = x.hi;
+      sul[j][t] = x.lo;
+    }
+    __syncthreads();
+    nlist = 0;
+  };
+  const int L = A.real_lanes, lg = __ffs(L) - 1;
+  int* items = sitem + threadIdx.x * kBigPerThread;
+  for (int base = 0; base < nnear << lg; base += 256) {  // block-uniform
+    const int task = base + threadIdx.x;
+    const int near = task >> lg, su0 = task & (L - 1);
+    const bool on = near < nnear;
+    int t = 0, j = 0, is0 = 0, ins = 0, nbig = 0;
+    if (on) {
+      t = snear[near] & 0xff;
+      j = snear[near] >> 8;
+      is0 = ss0[t];
+      ins = A.slot_site[tile * 256 + t + 1] - is0;
+    }
+    // a thread with more than kBigPerThread FP64 pairs takes further windows
     for (int win = 0;; win += kBigPerThread) {
-      if (win > 0) {  // later round: record pairs win .. win + kBigPerThread - 1 afresh
-        int n2 = 0;
-        unsigned f2 = 0u;
-        if (nbig > win)
-          for (int j = 0; j < G; ++j)
-            if (fix & (1u << j)) real_mixed<false>(A, a, g0 + j, s0, ns, k32, srcut[j], p0, supos[j], j, items, win, n2, f2);
+      if (win == 0 || nbig > win) {
+        ff r{0.f, 0.f};
+        nbig = 0;
+        if (on) r = real_mixed(A, a, g0 + j, is0, ins, su0, L, items, win, nbig);
+        if (win == 0) {
+          for (int o = 1; o < L; o <<= 1) {  // the lower thread's sum plus the upper one's
+            const ff w{__shfl_down_sync(0xffffffffu, r.hi, o), __shfl_down_sync(0xffffffffu, r.lo, o)};
+            if ((su0 & (2 * o - 1)) == 0) r = ff_add2(r, w);
+          }
+          if (on && su0 == 0 && (r.hi != 0.f || r.lo != 0.f)) {
+            const ff v = ff_add2(ff{su[j][t], sul[j][t]}, r);
+            su[j][t] = v.hi;
+            sul[j][t] = v.lo;
+          }
+        }
       }
+      if (!__syncthreads_or(nbig > win)) break;
+      // the window's pairs to the end of the list (an exclusive scan over the threads, so in the
+      // items' order; a window of kBigList entries or more is passed on in parts)
       const int cnt = min(max(nbig - win, 0), kBigPerThread);
-      // exclusive scan of cnt over the block
       int incl = cnt;
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, incl, o);
@@ -947,38 +1006,26 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
       if (lane == 31) swarp[wid] = incl;
       __syncthreads();
       int off = incl - cnt, total = 0;
-      for (int w2 = 0; w2 < (int)(blockDim.x >> 5); ++w2) {
+      for (int w2 = 0; w2 < 8; ++w2) {
         if (w2 < wid) off += swarp[w2];
         total += swarp[w2];
       }
-      if (total == 0) break;  // block-uniform
-      for (int i = 0; i < cnt; ++i) slist[off + i] = (unsigned short)(threadIdx.x * kBigPerThread + i);
-      __syncthreads();
-      for (int base = 0; base < total; base += blockDim.x) {
-        const int q = base + threadIdx.x;
-        double v = 0.0;
-        if (q < total) {
-          const int slot = slist[q];
-          const int t = slot / kBigPerThread, it = sitem[slot];
-          const int j = (it >> 21) & 7, su_ = (it >> 13) & 0xff, sv = it & 0x1fff;
-          const size_t us = (size_t)(g0 + j) * kMaxSoluteSites + su_;
-          v = pair_fp64(A, ss0[t] + sv, a.u_x + us * 3, a.u_q[us], a.u_pos[us].w, it >> 24);
-        }
-        sbuf[threadIdx.x] = v;
-        __syncthreads();
+      // (an item's later windows would not lie beside its first one)
+      if (win > 0 || nlist + total > kBigList) add_listed();
+      for (int p0 = 0; p0 < total; p0 += kBigList) {
+        if (p0 > 0) add_listed();
         for (int i = 0; i < cnt; ++i) {
-          const int qq = off + i - base;
-          if (qq < 0 || qq >= (int)blockDim.x) continue;
-          const int j = (items[i] >> 21) & 7;
-          const ff t = ff_add2(ff{su[j][threadIdx.x], sul[j][threadIdx.x]}, ff_from_double(sbuf[qq]));
-          su[j][threadIdx.x] = t.hi;
-          sul[j][threadIdx.x] = t.lo;
+          const int q = off + i - p0;
+          if (q < 0 || q >= kBigList) continue;
+          sbig[nlist + q] = items[i];
+          sbnear[nlist + q] = (unsigned short)near;
         }
-        __syncthreads();
+        nlist += min(total - p0, kBigList);
       }
     }
-    __syncthreads();  // the scratch is free: the histograms may take the region
   }
+  if (nlist > 0) add_listed();
+  __syncthreads();  // the totals are complete and the scratch is free: the histograms may take the region
   if (!A.hist_global)
     for (int i = threadIdx.x; i < G * A.ermax; i += blockDim.x) smem_hist[i] = 0;
   int ku[G];     // ordered key of the total's hi part
@@ -1116,9 +1163,6 @@ static MolArgs make_mol_args(Engine& e, const BatchArgs& a) {
   A.ldb = e.Bmax;
   A.uvkey = e.d_uvkey;
   A.uvkey_f = e.d_uvkey_f;
-  // finish kernel: block histograms in shared memory up to 64 KB (three blocks per SM
-  // fit); beyond that the counts go straight to global memory
-  A.hist_global = (size_t)a.G * e.ermax * sizeof(int) > 64 * 1024 ? 1 : 0;
   A.spec = e.d_spec;
   A.numslv = e.numslv;
   A.ermax = e.ermax;
@@ -1132,6 +1176,7 @@ static MolArgs make_mol_args(Engine& e, const BatchArgs& a) {
   A.upljcut = e.P.upljcut;
   A.screen = e.P.screen;
   A.bare = (e.P.cltype == 0) ? 1 : 0;
+  A.real_lanes = e.max_solute_sites <= 2 ? 1 : e.max_solute_sites <= 6 ? 2 : e.max_solute_sites <= 16 ? 4 : 8;
   A.resid_fac = A.bare ? 0.0 : kPi / e.P.screen / e.P.screen / e.geom.volume;
   for (int i = 0; i < 3; ++i) A.fxf[i] = (float)e.geom.fx_scale[i];
   A.screen_f = (float)e.P.screen;
@@ -1177,26 +1222,43 @@ cudaError_t launch_gather(Engine& e, const BatchArgs& a) {
 static int mol64_ty(const Engine& e) { return e.P.slttype == 1 && e.slvmax < 512 * e.num_sm ? 4 : 1; }
 int mol64_tile(const Engine& e) { return kMol64Threads / (4 * mol64_ty(e)); }
 
+// placements per molecule-energy block: the caller's choice (4 or 8), else 4, halved while the
+// launch has fewer than 1.5 blocks per SM (2,000 waters, 36 sites, batches of 64: 26.6 ms of
+// 4,000 insertions with 128 blocks of 4, 22.2 with 256 of 2, 22.1 with 512 of 1; with 256 or
+// more blocks of 4 -- 4,000 waters -- fewer placements per block are no faster, and at 33,000
+// waters 2 cost 5%).  A molecule's energy does not depend on the split.
+static int finish_group(const Engine& e, int nb) {
+  int G = e.G;
+  if (e.P.finish_group != 0) return G;
+  while (G > 1 && 2LL * e.ntile * ((nb + G - 1) / G) < 3LL * e.num_sm) G /= 2;
+  return G;
+}
+
 cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a) {
-  const MolArgs A = make_mol_args(e, a);
+  MolArgs A = make_mol_args(e, a);
   e.count_launch();
   cudaError_t err = cudaSuccess;
   if (!e.mixed) return mol64_ty(e) == 4 ? launch_mol64<4>(e, A) : launch_mol64<1>(e, A);
-  if (a.G != 8 && a.G != 4) return cudaErrorInvalidValue;
+  const int G = finish_group(e, a.nb);
+  // block histograms in shared memory up to 64 KB (three blocks per SM fit); beyond that the
+  // counts go straight to global memory
+  A.hist_global = (size_t)G * e.ermax * sizeof(int) > 64 * 1024 ? 1 : 0;
   if (e.P.cltype != 0 && (err = launch_gather(e, a)) != cudaSuccess) return err;
   if (a.phases) {
     e.phase_end_on(a.stream);
     e.phase_begin_on(PH_MOL, a.stream);
   }
   // step 2: per-molecule totals and binning (histograms + edge keys in shared memory)
-  const size_t smem_f = sizeof(int) * ((size_t)finish_region_ints(a.G, e.ermax, A.hist_global) + e.ermax);
-  dim3 g2((a.nb + a.G - 1) / a.G, e.ntile);
+  const size_t smem_f = sizeof(int) * ((size_t)finish_region_ints(G, e.ermax, A.hist_global) + e.ermax);
+  dim3 g2((a.nb + G - 1) / G, e.ntile);
 #define ERMOD_FINISH(GG)                                                                                   \
-  if (a.G == GG) {                                                                                         \
+  if (G == GG) {                                                                                           \
     static SmemAttr attr;                                                                                  \
     if ((err = attr.ensure(mol_finish_kernel<GG>, smem_f)) != cudaSuccess) return err;                     \
-    mol_finish_kernel<GG><<<g2, 256, smem_f, a.stream>>>(A, a.site_e);                                   \
+    mol_finish_kernel<GG><<<g2, 256, smem_f, a.stream>>>(A, a.site_e);                                     \
   }
+  ERMOD_FINISH(1)
+  ERMOD_FINISH(2)
   ERMOD_FINISH(4)
   ERMOD_FINISH(8)
 #undef ERMOD_FINISH
