@@ -129,8 +129,6 @@ static int free_batch(Engine& e) {
   dfree(b.u_pos);
   dfree(b.u_q);
   dfree(b.u_qf);
-  dfree(b.u_grid);
-  dfree(b.u_w);
   dfree(b.u_bvec);
   dfree(b.u_bvec64);
   dfree(b.u_qmol);
@@ -157,11 +155,11 @@ static int free_batch(Engine& e) {
 
 static int free_frame(Engine& e) {
   dfree(e.d_sitepos);
-  dfree(e.d_wrapped);
   dfree(e.d_sort_key);
   dfree(e.d_sort_key_alt);
   dfree(e.d_sort_val);
   dfree(e.d_sort_val_alt);
+  dfree(e.d_sort_count);
   dfree(e.d_cub_tmp);
   dfree(e.d_slot_mol);
   dfree(e.d_slot_site);
@@ -174,9 +172,7 @@ static int free_frame(Engine& e) {
   dfree(e.d_site_w);
   dfree(e.d_site_q);
   dfree(e.d_frame_scal);
-  dfree(e.d_brick_key);
-  dfree(e.d_brick_key_alt);
-  dfree(e.d_brick_val);
+  dfree(e.d_brick_cursor);
   dfree(e.d_brick_site);
   dfree(e.d_brick_count);
   dfree(e.d_brick_start);
@@ -254,7 +250,7 @@ static int ensure_batch(Engine& e) {
   const int B = e.Bmax;
   BatchArgs& b = e.buf;
   const size_t nr = e.grid_real(), nc = e.grid_cplx();
-  e.tile = e.mixed ? 256 : mol64_tile(e);
+  e.tile = mol_tile(e);
   e.ntile = (e.slvmax + e.tile - 1) / e.tile;
   // solute data: kBatchSlots batch slots (the preparation of batch i+1 runs during batch i)
   const size_t NS = kBatchSlots;
@@ -263,8 +259,6 @@ static int ensure_batch(Engine& e) {
   ERMOD_CUDA(dalloc(&b.u_pos, NS * B * S));
   ERMOD_CUDA(dalloc(&b.u_q, NS * B * S));
   ERMOD_CUDA(dalloc(&b.u_qf, NS * B * S));
-  ERMOD_CUDA(dalloc(&b.u_grid, NS * B * S));
-  ERMOD_CUDA(dalloc(&b.u_w, NS * B * S * 3 * kMaxSplineOrder));
   ERMOD_CUDA(dalloc(&b.u_qmol, NS * B));
   ERMOD_CUDA(dalloc(&b.u_usreal, NS * B));
   ERMOD_CUDA(dalloc(&b.u_radius, NS * B));
@@ -731,17 +725,19 @@ int ermod_set_topology(ermod_ctx* c, int nummol, int numatm, const int* mbi, con
   ERMOD_CUDA(cudaMemcpy(e.d_mol_to_k, mol_to_k.data(), sizeof(int) * nummol, cudaMemcpyHostToDevice));
   // frame buffers
   ERMOD_CUDA(dalloc(&e.d_sitepos, 3 * (size_t)numatm));
-  ERMOD_CUDA(dalloc(&e.d_wrapped, 3 * (size_t)numatm));
   ERMOD_CUDA(dalloc(&e.d_sort_key, e.slvmax));
   ERMOD_CUDA(dalloc(&e.d_sort_key_alt, e.slvmax));
   ERMOD_CUDA(dalloc(&e.d_sort_val, e.slvmax));
   ERMOD_CUDA(dalloc(&e.d_sort_val_alt, e.slvmax + 1));
   ERMOD_CUDA(cudaMemset(e.d_sort_val_alt, 0, sizeof(int) * (e.slvmax + 1)));
+  const size_t ncode = (size_t)1 << (3 * kSortMaxBits);
+  ERMOD_CUDA(dalloc(&e.d_sort_count, 2 * ncode));
+  ERMOD_CUDA(cudaMemset(e.d_sort_count, 0, sizeof(int) * ncode));
   e.nbrick[0] = (e.geom.K[0] + kBrickX - 1) / kBrickX;
   e.nbrick[1] = (e.geom.K[1] + kBrickY - 1) / kBrickY;
   e.nbrick[2] = (e.geom.K[2] + kBrickZ - 1) / kBrickZ;
   e.nbricks = e.nbrick[0] * e.nbrick[1] * e.nbrick[2];
-  e.cub_tmp_bytes = std::max(frame_cub_bytes(e.slvmax), brick_cub_bytes(e.nsite_phys, e.nbricks));
+  e.cub_tmp_bytes = frame_cub_bytes(e.slvmax);
   ERMOD_CUDA(dalloc((char**)&e.d_cub_tmp, e.cub_tmp_bytes));
   ERMOD_CUDA(dalloc(&e.d_slot_mol, e.slvmax));
   ERMOD_CUDA(dalloc(&e.d_slot_site, e.slvmax + 1));
@@ -751,9 +747,7 @@ int ermod_set_topology(ermod_ctx* c, int nummol, int numatm, const int* mbi, con
   ERMOD_CUDA(dalloc(&e.d_site_grid, e.nsite_phys));
   if (e.mixed) {
     ERMOD_CUDA(dalloc(&e.d_site_rec, e.nsite_phys));
-    ERMOD_CUDA(dalloc(&e.d_brick_key, e.nsite_phys));
-    ERMOD_CUDA(dalloc(&e.d_brick_key_alt, e.nsite_phys));
-    ERMOD_CUDA(dalloc(&e.d_brick_val, e.nsite_phys));
+    ERMOD_CUDA(dalloc(&e.d_brick_cursor, e.nbricks));
     ERMOD_CUDA(dalloc(&e.d_brick_site, e.nsite_phys));
     ERMOD_CUDA(dalloc(&e.d_brick_count, e.nbricks + 1));
     ERMOD_CUDA(dalloc(&e.d_brick_start, e.nbricks + 1));
@@ -922,7 +916,6 @@ static int frame_launch(Engine& e) {
   if (changed && e.P.cltype != 0) ERMOD_CUDA(launch_greenfunc(e));
   std::memcpy(e.prevcl, e.cell, sizeof(e.cell));
   e.green_valid = true;
-  ERMOD_CUDA(launch_frame_wrap(e));
   ERMOD_CUDA(launch_frame_sort(e));
   ERMOD_CUDA(launch_frame_sites(e));
   if (e.mixed) ERMOD_CUDA(launch_frame_bricks(e));
@@ -994,11 +987,19 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
     }
     ERMOD_CUDA(launch_config_check(e, nplace, d_tag));
   }
-  ERMOD_CUDA(cudaEventRecord(e.ev_done[0], e.stream));
-  ERMOD_CUDA(cudaStreamWaitEvent(e.aux, e.ev_done[0], 0));
-  ERMOD_CUDA(cudaStreamWaitEvent(e.prep, e.ev_done[0], 0));
-  if (dual) {
-    for (int k = 0; k < kBatchStreams; ++k) ERMOD_CUDA(cudaStreamWaitEvent(e.bs[k], e.ev_done[0], 0));
+  // a call of one batch has nothing to overlap: all of it runs on the caller's stream, without
+  // the events between the streams (a solution-mode frame saves some 15 of them)
+  const bool single = nbatch <= 1;
+  const cudaStream_t prep = single ? e.stream : e.prep, aux = single ? e.stream : e.aux,
+                     flush = single ? e.stream : e.flush;
+  e.status_clean = false;
+  if (!single) {
+    ERMOD_CUDA(cudaEventRecord(e.ev_done[0], e.stream));
+    ERMOD_CUDA(cudaStreamWaitEvent(aux, e.ev_done[0], 0));
+    ERMOD_CUDA(cudaStreamWaitEvent(prep, e.ev_done[0], 0));
+    if (dual) {
+      for (int k = 0; k < kBatchStreams; ++k) ERMOD_CUDA(cudaStreamWaitEvent(e.bs[k], e.ev_done[0], 0));
+    }
   }
   auto batch_args = [&](int ib) {
     const int b0 = ib * B, slot = ib % kBatchSlots;
@@ -1015,8 +1016,6 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
     a.u_pos = e.buf.u_pos + (size_t)slot * B * S;
     a.u_q = e.buf.u_q + (size_t)slot * B * S;
     a.u_qf = e.buf.u_qf + (size_t)slot * B * S;
-    a.u_grid = e.buf.u_grid + (size_t)slot * B * S;
-    a.u_w = e.buf.u_w + (size_t)slot * B * S * 3 * kMaxSplineOrder;
     if (e.buf.u_bvec64) a.u_bvec64 = e.buf.u_bvec64 + (size_t)slot * B * S * 3 * e.Kmax();
     if (e.buf.u_bvec) a.u_bvec = e.buf.u_bvec + (size_t)slot * B * S * 3 * e.Kmax();
     a.u_radius = e.buf.u_radius + (size_t)slot * B;
@@ -1028,7 +1027,7 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
     a.u0 = e.d_u0 + (size_t)slot * B;
     a.self_bin = e.d_self_bin + (size_t)slot * B;
     a.slot = slot;
-    a.stream = dual ? e.bs[ib % kBatchStreams] : e.stream;  // streams and slots taken in turn
+    a.stream = (dual && !single) ? e.bs[ib % kBatchStreams] : e.stream;  // streams and slots taken in turn
     a.phases = 1;
     a.mol_bin = e.adj_on ? e.d_mol_bin + (size_t)slot * B * e.slvmax : nullptr;
     a.skip = check ? e.d_skip + b0 : nullptr;
@@ -1043,12 +1042,12 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
   auto issue_prep = [&](int ib) -> int {
     const int slot = ib % kBatchSlots;
     const BatchArgs a = batch_args(ib);
-    if (ib >= kBatchSlots) ERMOD_CUDA(cudaStreamWaitEvent(e.prep, e.ev_acc[slot], 0));  // slot free again
+    if (ib >= kBatchSlots) ERMOD_CUDA(cudaStreamWaitEvent(prep, e.ev_acc[slot], 0));  // slot free again
     const double* sol = d_sol ? d_sol + (size_t)a.b0 * ns_solute * 3 : nullptr;
-    e.phase_begin_on(PH_PREP, e.prep);
-    ERMOD_CUDA(launch_place_prep(e, a, sol, e.P.slttype == 2 ? 2 : 1, e.prep));
-    e.phase_end_on(e.prep);
-    ERMOD_CUDA(cudaEventRecord(e.ev_prep[slot], e.prep));
+    e.phase_begin_on(PH_PREP, prep);
+    ERMOD_CUDA(launch_place_prep(e, a, sol, e.P.slttype == 2 ? 2 : 1, prep));
+    e.phase_end_on(prep);
+    if (!single) ERMOD_CUDA(cudaEventRecord(e.ev_prep[slot], prep));
     return ERMOD_OK;
   };
   if (nbatch > 0 && (st = issue_prep(0)) != ERMOD_OK) return st;
@@ -1060,7 +1059,7 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
     a.hist = e.d_ring_hist + (size_t)(e.ring_off + e.ring_fill) * e.ermax;
     cudaStream_t bst = a.stream;
     if (ibatch >= kBatchSlots) ERMOD_CUDA(cudaStreamWaitEvent(bst, e.ev_acc[slot], 0));  // slot free again
-    ERMOD_CUDA(cudaStreamWaitEvent(bst, e.ev_prep[slot], 0));
+    if (!single) ERMOD_CUDA(cudaStreamWaitEvent(bst, e.ev_prep[slot], 0));
     const int half = e.ring_off ? 1 : 0;
     if (e.flush_pend[half]) {  // the first batch in this half waits for its previous flush
       ERMOD_CUDA(cudaStreamWaitEvent(bst, e.ev_flush[half], 0));
@@ -1084,28 +1083,30 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
     e.phase_begin_on(e.mixed ? PH_GATHER : PH_MOL, bst);
     ERMOD_CUDA(launch_mol_energy(e, a));  // mixed: gather, then (mol_energy phase) finish
     e.phase_end_on(bst);
-    ERMOD_CUDA(cudaEventRecord(e.ev_done[slot], bst));
     // ---- ordered accumulation on the aux stream ----
-    ERMOD_CUDA(cudaStreamWaitEvent(e.aux, e.ev_done[slot], 0));
-    e.phase_begin_on(PH_ACCUM, e.aux);
-    ERMOD_CUDA(launch_accumulate(e, a, e.aux));
-    e.phase_end_on(e.aux);
-    if (e.adj_on) {  // after the weights engnmfc of the batch exist
-      e.phase_begin_on(PH_ADJOINT, e.aux);
-      ERMOD_CUDA(launch_adjoint(e, a, e.aux));
-      e.phase_end_on(e.aux);
+    if (!single) {
+      ERMOD_CUDA(cudaEventRecord(e.ev_done[slot], bst));
+      ERMOD_CUDA(cudaStreamWaitEvent(aux, e.ev_done[slot], 0));
     }
-    ERMOD_CUDA(cudaEventRecord(e.ev_acc[slot], e.aux));
+    e.phase_begin_on(PH_ACCUM, aux);
+    ERMOD_CUDA(launch_accumulate(e, a, aux));
+    e.phase_end_on(aux);
+    if (e.adj_on) {  // after the weights engnmfc of the batch exist
+      e.phase_begin_on(PH_ADJOINT, aux);
+      ERMOD_CUDA(launch_adjoint(e, a, aux));
+      e.phase_end_on(aux);
+    }
+    if (!single) ERMOD_CUDA(cudaEventRecord(e.ev_acc[slot], aux));
     if (e.P.corrcal) {
       e.ring_fill += nb;
       if (e.ring_fill + B > e.ring_half) {  // flush this half; the next batches fill the other
         // after the half's accumulations (the aux stream runs them in order)
-        ERMOD_CUDA(cudaStreamWaitEvent(e.flush, e.ev_acc[slot], 0));
-        e.phase_begin_on(PH_ECORR, e.flush);
-        ERMOD_CUDA(launch_ecorr_flush(e, e.flush));
-        e.phase_end_on(e.flush);
-        ERMOD_CUDA(cudaEventRecord(e.ev_flush[half], e.flush));
-        e.flush_pend[half] = true;
+        if (!single) ERMOD_CUDA(cudaStreamWaitEvent(flush, e.ev_acc[slot], 0));
+        e.phase_begin_on(PH_ECORR, flush);
+        ERMOD_CUDA(launch_ecorr_flush(e, flush));
+        e.phase_end_on(flush);
+        if (!single) ERMOD_CUDA(cudaEventRecord(e.ev_flush[half], flush));
+        e.flush_pend[half] = !single;
         e.ring_off = e.ring_half - e.ring_off;
         e.ring_fill = 0;
       }
@@ -1114,10 +1115,10 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
     }
   }
   if (e.P.corrcal && e.ring_fill > 0) {
-    ERMOD_CUDA(cudaStreamWaitEvent(e.flush, e.ev_acc[(nbatch - 1) % kBatchSlots], 0));
-    e.phase_begin_on(PH_ECORR, e.flush);
-    ERMOD_CUDA(launch_ecorr_flush(e, e.flush));
-    e.phase_end_on(e.flush);
+    if (!single) ERMOD_CUDA(cudaStreamWaitEvent(flush, e.ev_acc[(nbatch - 1) % kBatchSlots], 0));
+    e.phase_begin_on(PH_ECORR, flush);
+    ERMOD_CUDA(launch_ecorr_flush(e, flush));
+    e.phase_end_on(flush);
   }
   // the join below orders every flush before the next call's work
   e.ring_fill = 0;
@@ -1129,7 +1130,7 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
   cudaStream_t others[2 + kBatchStreams] = {e.aux, e.prep};
   for (int k = 0; k < kBatchStreams; ++k) others[2 + k] = e.bs[k];
   const int nj = (dual ? 2 + kBatchStreams : 2);
-  for (int k = 0; k < nj + (e.P.corrcal ? 1 : 0); ++k) {
+  for (int k = 0; !single && k < nj + (e.P.corrcal ? 1 : 0); ++k) {
     const cudaStream_t sk = (k < nj) ? others[k] : e.flush;
     ERMOD_CUDA(cudaEventRecord(e.ev_join[k], sk));
     ERMOD_CUDA(cudaStreamWaitEvent(e.stream, e.ev_join[k], 0));
@@ -1146,10 +1147,11 @@ static int check_ready(Engine& e, int nplace) {
   return ERMOD_OK;
 }
 
-static int reset_status(Engine& e) {  // memsets only, so that a graph capture can hold it
-  static_assert(sizeof(DevStatus) == 24, "DevStatus layout: err_key, first_key, mbin_hit, range_fault");
-  ERMOD_CUDA(cudaMemsetAsync(&e.d_status->err_key, 0xff, 2 * sizeof(unsigned long long), e.stream));  // kNoError
-  ERMOD_CUDA(cudaMemsetAsync(&e.d_status->mbin_hit, 0, 2 * sizeof(int), e.stream));
+// a kernel, so that a graph capture can hold it; skipped while nothing has touched the status
+// since the last reset (the end of every host call resets it)
+static int reset_status(Engine& e, bool force = false) {
+  if (force || !e.status_clean) ERMOD_CUDA(launch_reset_status(e));
+  e.status_clean = true;
   *e.h_status = DevStatus{kNoError, kNoError, 0, 0};
   return ERMOD_OK;
 }
@@ -1720,6 +1722,7 @@ int ermod_generate_placements(ermod_ctx* c, int nplace, int nsite, const double*
     ERMOD_CUDA(cudaMemcpyAsync(e.d_ins, bfcoord, sizeof(double) * 3 * nsite, cudaMemcpyHostToDevice, e.stream));
   ERMOD_CUDA(cudaMemcpyAsync(e.d_ins + 3 * kMaxSoluteSites, mass, sizeof(double) * nsite, cudaMemcpyHostToDevice,
                              e.stream));
+  e.status_clean = false;  // a placement that cannot be made reports it
   ERMOD_CUDA(launch_insert(e, nplace, nsite, *ip, e.d_ins, e.d_ins + 3 * kMaxSoluteSites, sol_d, sws_d));
   return ERMOD_OK;
 }
@@ -1823,7 +1826,7 @@ int ermod_graph_create(int nctx, ermod_ctx* const* ctx, const double* const* sit
                                e.stream)) != cudaSuccess)
       st = fail_cuda(err, "frame copy");
     if (st == ERMOD_OK) st = frame_launch(e);
-    if (st == ERMOD_OK && nplace[i] > 0) st = reset_status(e);
+    if (st == ERMOD_OK && nplace[i] > 0) st = reset_status(e, true);
     if (st == ERMOD_OK && nplace[i] > 0)
       st = run_placements(e, nplace[i], tag_d[i], sol_d ? sol_d[i] : nullptr, sws_d ? sws_d[i] : nullptr, nullptr,
                           nullptr, e.numsite[solute_mol[i] - 1]);
@@ -1851,6 +1854,7 @@ int ermod_graph_launch(ermod_graph* g, void* stream) {
   if (!g || !g->exec) return fail_param("null graph");
   cudaSetDevice(g->device);
   g->launched = (cudaStream_t)stream;
+  for (ermod_ctx* c : g->ctx) c->e.status_clean = false;
   ERMOD_CUDA(cudaGraphLaunch(g->exec, g->launched));
   return ERMOD_OK;
 }

@@ -91,12 +91,12 @@ struct Engine {
   double* d_splfc = nullptr;     // [K1 + K2 + K3]
   float2* d_twiddle = nullptr;   // [K1 + K2 + K3] exp(-2 pi i m / K)
   double2* d_twiddle64 = nullptr;  // the same in FP64 (solute structure factors)
-  double* d_wrapped = nullptr;   // (3, numatm) normalised coordinates
   // spatial sort of physical molecules
   unsigned int* d_sort_key = nullptr;
   unsigned int* d_sort_key_alt = nullptr;
   int* d_sort_val = nullptr;
   int* d_sort_val_alt = nullptr;
+  int* d_sort_count = nullptr;    // [2][2^(3 kSortMaxBits)] counts per code (zero between frames), cursors
   void* d_cub_tmp = nullptr;
   size_t cub_tmp_bytes = 0;
   // slot-ordered solvent layout
@@ -113,10 +113,8 @@ struct Engine {
   float* d_frame_scal = nullptr;  // [0] max molecule radius about its first site (A)
   // sites grouped by 8^3 bricks of the PME grid (the mixed gather's unit of work)
   int nbrick[3] = {1, 1, 1}, nbricks = 1;
-  unsigned int* d_brick_key = nullptr;
-  unsigned int* d_brick_key_alt = nullptr;
-  int* d_brick_val = nullptr;
-  int* d_brick_site = nullptr;   // [nsite_phys] site indices (slot order) sorted by brick
+  int* d_brick_cursor = nullptr;  // [nbricks] scratch
+  int* d_brick_site = nullptr;   // [nsite_phys] site indices (slot order) by brick
   int* d_brick_count = nullptr;  // [nbricks+1]
   int* d_brick_start = nullptr;  // [nbricks+1]
 
@@ -145,6 +143,7 @@ struct Engine {
   // ---- status ----------------------------------------------------------------------
   DevStatus* d_status = nullptr;
   DevStatus* h_status = nullptr;  // pinned
+  bool status_clean = true;  // d_status holds no result of queued work
   int err_placement = -1, err_molecule = -1;
   double err_energy = 0.0;
   int call_b0 = 0;
@@ -248,10 +247,9 @@ struct Engine {
 // sizes shared between the launchers and the host code
 int spectrum_partials(const Engine& e);
 int spectrum64_partials(const Engine& e);
-int mol64_tile(const Engine& e);  // molecules per block of the FP64 path's molecule kernel
+int mol_tile(const Engine& e);  // molecules per block of the molecule kernels
 int accumulate_max_batch();
 size_t frame_cub_bytes(int n);
-size_t brick_cub_bytes(int nsite, int nbricks);
 cudaError_t launch_frame_bricks(Engine& e);
 double host_spline_value(int order, double x);
 

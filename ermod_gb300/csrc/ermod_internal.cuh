@@ -130,6 +130,12 @@ struct SmemAttr {
   }
 };
 
+// the molecules sorted by counting their spatial codes: at most this many, whose codes (at most
+// 4 per molecule) have at most this many bits per axis
+constexpr int kSortMaxMol = 98304;
+constexpr int kSortMaxBits = 6;
+static_assert(4LL * kSortMaxMol < 1LL << (3 * (kSortMaxBits + 1)), "the codes' counts");
+
 // bricks of the mixed path's gather: kBrickX x kBrickY x kBrickZ PME grid points
 constexpr int kBrickX = 16, kBrickY = 8, kBrickZ = 8;
 
@@ -215,8 +221,6 @@ struct BatchArgs {
   int4* u_pos;         // [nb][S] fixed point + ljtype
   double* u_q;         // [nb][S]
   float* u_qf;         // [nb][S] FP32 copy for the mixed kernels
-  int* u_grid;         // [nb][S] packed base grid
-  double* u_w;         // [nb][S][3][P] FP64 spline weights
   float2* u_bvec;      // [nb][S][3][Kmax] 1-D structure factors (mixed)
   double2* u_bvec64;   // the same in FP64 (FP64 path)
   double* u_qmol;      // [nb] molecular charge of the solute
@@ -243,7 +247,7 @@ struct Engine;
 
 // ---- launchers (defined in the .cu files) ---------------------------------------
 // frame preparation
-cudaError_t launch_frame_wrap(Engine& e);
+cudaError_t launch_reset_status(Engine& e);
 cudaError_t launch_carry_status(Engine& e);  // device API: an earlier call's error stops this call
 cudaError_t launch_max_abs(Engine& e, const double* x_d, size_t n, double* host_out);  // syncs e.stream
 cudaError_t launch_frame_sort(Engine& e);

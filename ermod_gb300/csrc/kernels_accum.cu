@@ -67,34 +67,39 @@ __device__ __forceinline__ int batch_accepted(const AccArgs& A) {
   return (A.ff_keys || before <= 0) ? 0 : (int)before;
 }
 
-// fixed-order block sum: thread t adds elements t, t+256, ... in order, then a fixed tree
-__device__ __forceinline__ double block_sum_fixed(double* red, const double* x, int n, int stride) {
+// fixed-order warp sum: lane t adds elements t, t + 32, ... in order, then a fixed tree
+__device__ __forceinline__ double warp_sum_fixed(const double* x, int n, int stride) {
   double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += x[(size_t)i * stride];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
-    __syncthreads();
+  for (int i = threadIdx.x & 31; i < n; i += 32) s += x[(size_t)i * stride];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+__device__ __forceinline__ void warp_min_max(double& mn, double& mx) {
+  for (int o = 16; o > 0; o >>= 1) {
+    mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   }
-  const double r = red[0];
-  __syncthreads();
-  return r;
 }
 
-// one CTA per placement: self energy u0, the self-energy bin check, and the per-species
-// tile partials reduced to flceng / min / max (written to tile slot 0)
-__global__ void __launch_bounds__(kAccThreads) reduce_kernel(AccArgs A) {
+// one placement, by one CTA: self energy u0, the self-energy bin check, and the per-species
+// tile partials reduced to flceng / min / max (written to tile slot 0).  A warp per sum (the
+// self energy's partials, then each species): their block-wide trees took 9 us a launch
+__device__ void reduce_placement(const AccArgs& A, int b) {
   const BatchArgs& a = A.a;
-  const int b = blockIdx.x;
-  __shared__ double red[kAccThreads];
-  const double self = A.bare ? 0.0 : block_sum_fixed(red, a.self_part + (size_t)b * A.nself, A.nself, 1);
-  for (int sp = 0; sp < A.numslv; ++sp) {
-    const double* base = a.part + ((size_t)b * A.ntile * A.numslv + sp) * 3;
+  __shared__ double self_sum;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+  for (int item = warp; item <= A.numslv; item += nwarp) {
+    if (item == 0) {
+      const double s = A.bare ? 0.0 : warp_sum_fixed(a.self_part + (size_t)b * A.nself, A.nself, 1);
+      if (lane == 0) self_sum = s;
+      continue;
+    }
+    const int sp = item - 1;
+    double* base = a.part + ((size_t)b * A.ntile * A.numslv + sp) * 3;
     const int stride = A.numslv * 3;
-    const double s = block_sum_fixed(red, base, A.ntile, stride);
+    const double s = warp_sum_fixed(base, A.ntile, stride);
     double mn = INFINITY, mx = -INFINITY;
-    for (int t = threadIdx.x; t < A.ntile; t += blockDim.x) {
+    for (int t = lane; t < A.ntile; t += 32) {
       const double* pt = base + (size_t)t * stride;
       if (A.ff_keys) {
         mn = fmin(mn, ff_key_to_double(reinterpret_cast<const long long*>(pt)[1]));
@@ -104,30 +109,16 @@ __global__ void __launch_bounds__(kAccThreads) reduce_kernel(AccArgs A) {
         mx = fmax(mx, pt[2]);
       }
     }
-    red[threadIdx.x] = mn;
-    __syncthreads();
-    for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-      if (threadIdx.x < st) red[threadIdx.x] = fmin(red[threadIdx.x], red[threadIdx.x + st]);
-      __syncthreads();
-    }
-    mn = red[0];
-    __syncthreads();
-    red[threadIdx.x] = mx;
-    __syncthreads();
-    for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-      if (threadIdx.x < st) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + st]);
-      __syncthreads();
-    }
-    mx = red[0];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double* out = a.part + ((size_t)b * A.ntile * A.numslv + sp) * 3;  // tile slot 0
-      out[0] = s;
-      out[1] = mn;
-      out[2] = mx;
+    warp_min_max(mn, mx);  // (every lane has read tile slot 0 before lane 0 overwrites it)
+    if (lane == 0) {
+      base[0] = s;
+      base[1] = mn;
+      base[2] = mx;
       if (a.flceng_out) a.flceng_out[(size_t)(a.b0 + b) * A.numslv + sp] = s;
     }
   }
+  __syncthreads();
+  const double self = self_sum;
   if (threadIdx.x == 0 && a.skip && a.skip[b]) {  // rejected by check_mol_configuration
     A.u0[b] = 0.0;
     A.self_bin[b] = -1;
@@ -179,14 +170,16 @@ __global__ void __launch_bounds__(kAccThreads) reduce_kernel(AccArgs A) {
   }
 }
 
-__global__ void __launch_bounds__(kAccThreads) accumulate_kernel(AccArgs A) {
+__global__ void __launch_bounds__(kAccThreads) reduce_kernel(AccArgs A) { reduce_placement(A, blockIdx.x); }
+
+// the batch's weights and scalar sums, by one CTA; every thread returns the number of
+// placements accumulated
+__device__ int accumulate_scalars(const AccArgs& A) {
   const BatchArgs& a = A.a;
   __shared__ double sw[kMaxBatch];
   __shared__ double stw[kMaxBatch];
   __shared__ double su0[kMaxBatch];
   __shared__ int sbin[kMaxBatch];
-  __shared__ double sterm[kMaxBatch];
-  __shared__ double sred[2][kAccThreads];
   __shared__ unsigned char srej[kMaxBatch];  // rejected by the configuration check
   __shared__ int accepted;
   __shared__ double s_voffset;
@@ -216,7 +209,7 @@ __global__ void __launch_bounds__(kAccThreads) accumulate_kernel(AccArgs A) {
     a.engnmfc[b] = 0.0;
     A.ring_valid[b] = 0;
   }
-  if (nb == 0) return;
+  if (nb == 0) return 0;
   // weights (parallel); u0 and the eself bins staged for the ordered sums
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     su0[b] = A.u0[b];
@@ -249,57 +242,49 @@ __global__ void __launch_bounds__(kAccThreads) accumulate_kernel(AccArgs A) {
     A.ring_valid[b] = 1;
   }
   __syncthreads();
-  // ordered scalar sums (placement order, as the reference's loop)
-  if (threadIdx.x == 0) {
-    double engnorm = A.scal[0], engsmpl = A.scal[1], avslf = A.scal[2];
-    double mn = A.minuv[0], mx = A.maxuv[0];
-    for (int b = 0; b < nb; ++b) {
-      if (srej[b]) continue;
-      engnorm = engnorm + sw[b];
-      engsmpl = engsmpl + 1.0;
-      avslf = avslf + stw[b];
-      if (A.selfcal) A.eself[sbin[b]] += sw[b];
-      mn = fmin(mn, su0[b]);
-      mx = fmax(mx, su0[b]);
-    }
-    A.scal[0] = engnorm;
-    A.scal[1] = engsmpl;
-    A.scal[2] = avslf;
-    A.minuv[0] = mn;
-    A.maxuv[0] = mx;
+  // ordered scalar sums (placement order, as the reference's loop), a warp's first thread each:
+  // serial chains of FP64 adds, whose inputs are the shared weights (0 for a rejected
+  // placement, which leaves a sum as it is).  256 placements, one thread for everything: 69 us
+  if (threadIdx.x == 0 || threadIdx.x == 32) {
+    const double* x = threadIdx.x == 0 ? sw : stw;
+    double* to = A.scal + (threadIdx.x == 0 ? 0 : 2);  // engnorm, avslf
+    double v = *to;
+#pragma unroll 8
+    for (int b = 0; b < nb; ++b) v = v + x[b];
+    *to = v;
+  } else if (threadIdx.x == 64 && A.selfcal) {
+    for (int b = 0; b < nb; ++b)
+      if (!srej[b]) A.eself[sbin[b]] += sw[b];
+  } else if (threadIdx.x == 96) {
+    int kept = 0;
+    for (int b = 0; b < nb; ++b) kept += srej[b] ? 0 : 1;
+    A.scal[1] += (double)kept;  // engsmpl: ones, exact in any order
   }
-  // per species: min/max over the batch (order-free tree), slnuv in placement order
-  for (int sp = 0; sp < A.numslv; ++sp) {
+  // per species a warp: min/max over the batch, slnuv in placement order (species -1: the
+  // solute self energies)
+  for (int sp = (int)(threadIdx.x >> 5) - 1; sp < A.numslv; sp += blockDim.x >> 5) {
+    const int lane = threadIdx.x & 31;
     double mn = INFINITY, mx = -INFINITY;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-      const double* pt = a.part + ((size_t)b * A.ntile * A.numslv + sp) * 3;
-      mn = fmin(mn, pt[1]);
-      mx = fmax(mx, pt[2]);
-      if (A.soln) sterm[b] = pt[0] * sw[b];
+    for (int b = lane; b < nb; b += 32) {
+      const double* pt = a.part + ((size_t)b * A.ntile * A.numslv + max(sp, 0)) * 3;
+      if (sp < 0 && srej[b]) continue;
+      mn = fmin(mn, sp < 0 ? su0[b] : pt[1]);
+      mx = fmax(mx, sp < 0 ? su0[b] : pt[2]);
     }
-    sred[0][threadIdx.x] = mn;
-    sred[1][threadIdx.x] = mx;
-    __syncthreads();
-    for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-      if (threadIdx.x < st) {
-        sred[0][threadIdx.x] = fmin(sred[0][threadIdx.x], sred[0][threadIdx.x + st]);
-        sred[1][threadIdx.x] = fmax(sred[1][threadIdx.x], sred[1][threadIdx.x + st]);
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      A.minuv[sp + 1] = fmin(A.minuv[sp + 1], sred[0][0]);
-      A.maxuv[sp + 1] = fmax(A.maxuv[sp + 1], sred[1][0]);
-      if (A.soln) {
+    warp_min_max(mn, mx);
+    if (lane == 0) {
+      A.minuv[sp + 1] = fmin(A.minuv[sp + 1], mn);
+      A.maxuv[sp + 1] = fmax(A.maxuv[sp + 1], mx);
+      if (A.soln && sp >= 0) {
         double sl = A.slnuv[sp];
         for (int b = 0; b < nb; ++b)
-          if (!srej[b]) sl = sl + sterm[b];
+          if (!srej[b]) sl = sl + a.part[((size_t)b * A.ntile * A.numslv + sp) * 3] * sw[b];
         A.slnuv[sp] = sl;
       }
     }
-    __syncthreads();
   }
-  if (!A.zmask) return;  // edens: accumulate_bins_kernel
+  __syncthreads();
+  if (!A.zmask) return nb;  // edens: accumulate_bins
   // edens += engnmfc * insdst, placements in order
   for (int i = threadIdx.x; i < A.ermax; i += blockDim.x) {
     double e = A.edens[i];
@@ -355,45 +340,80 @@ __global__ void __launch_bounds__(kAccThreads) accumulate_kernel(AccArgs A) {
       A.uvintm[sp] = u;
     }
   }
+  return nb;
 }
 
-// edens += engnmfc * insdst (engproc.F90:836-838), one thread per bin, the batch's
-// placements in order (so the FP64 sums are those of the reference's loop); the
-// intermediate-state mode does this inside accumulate_kernel instead
-__global__ void __launch_bounds__(128) accumulate_bins_kernel(AccArgs A) {
-  const BatchArgs& a = A.a;
-  const int nb = batch_accepted(A);
-  if (nb <= 0) return;  // the batch was not accumulated (an error)
-  __shared__ double sw[kMaxBatch];
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) sw[b] = a.engnmfc[b];
-  __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.ermax) return;
-  const int* h = a.hist + i;
+__global__ void __launch_bounds__(kAccThreads) accumulate_kernel(AccArgs A) { accumulate_scalars(A); }
+
+// edens(i) += engnmfc * insdst(i) (engproc.F90:836-838) by one thread, the batch's placements
+// in order (so the FP64 sums are those of the reference's loop); the intermediate-state mode
+// does this inside accumulate_scalars instead.  A serial chain of FMAs; the counts of the next
+// kBinAhead placements load while it runs, and a warp whose bins are all empty skips theirs.
+constexpr int kBinAhead = 16;
+__device__ __forceinline__ void accumulate_bin(const AccArgs& A, int i, int nb, const double* sw) {
+  const int* h = A.a.hist + i;
   const size_t E = (size_t)A.ermax;
   double e = A.edens[i];
-  bool touched = false;
-  int b = 0;
-  for (; b + 8 <= nb; b += 8) {
-    int c[8];
+  int touched = 0;
+  int next[kBinAhead];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) c[u] = __ldg(h + (size_t)(b + u) * E);
+  for (int u = 0; u < kBinAhead; ++u) next[u] = u < nb ? h[(size_t)u * E] : 0;
+  for (int b = 0; b < nb; b += kBinAhead) {
+    int c[kBinAhead], any = 0;
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (c[u]) {
-        e = e + sw[b + u] * (double)c[u];
-        touched = true;
-      }
-  }
-  for (; b < nb; ++b) {
-    const int c = __ldg(h + (size_t)b * E);
-    if (c) {
-      e = e + sw[b] * (double)c;
-      touched = true;
+    for (int u = 0; u < kBinAhead; ++u) {
+      c[u] = next[u];
+      any |= c[u];
+      next[u] = b + kBinAhead + u < nb ? h[(size_t)(b + kBinAhead + u) * E] : 0;
+    }
+    if (any) {
+      touched = 1;
+#pragma unroll
+      for (int u = 0; u < kBinAhead; ++u)
+        if (c[u]) e = fma(sw[b + u], (double)c[u], e);
     }
   }
   if (touched) A.edens[i] = e;
 }
+
+// one warp per block: the FP64 pipe takes 16 clocks per warp instruction and SM, so the bins
+// are spread over the SMs (256 placements of 1,396 bins: 40 us in blocks of 128)
+constexpr int kBinThreads = 32;
+__global__ void __launch_bounds__(kBinThreads) accumulate_bins_kernel(AccArgs A) {
+  const int nb = batch_accepted(A);
+  if (nb <= 0) return;  // the batch was not accumulated (an error)
+  __shared__ double sw[kMaxBatch];
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) sw[b] = A.a.engnmfc[b];
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < A.ermax) accumulate_bin(A, i, nb, sw);
+}
+
+// A batch of one or two placements (a solution-mode frame): the three steps in one launch
+constexpr int kSmallBatch = 2;
+constexpr int kSmallThreads = 512;
+__global__ void __launch_bounds__(kSmallThreads) accumulate_small_kernel(AccArgs A) {
+  for (int b = 0; b < A.a.nb; ++b) reduce_placement(A, b);
+  __syncthreads();
+  const int nb = accumulate_scalars(A);
+  if (nb == 0 || A.zmask) return;
+  __syncthreads();
+  double w[kSmallBatch];
+#pragma unroll
+  for (int b = 0; b < kSmallBatch; ++b) w[b] = b < nb ? A.a.engnmfc[b] : 0.0;
+  for (int i = threadIdx.x; i < A.ermax; i += blockDim.x) {
+    int c[kSmallBatch];
+#pragma unroll
+    for (int b = 0; b < kSmallBatch; ++b) c[b] = b < nb ? A.a.hist[(size_t)b * A.ermax + i] : 0;
+    if (!(c[0] | c[1])) continue;
+    double e = A.edens[i];
+#pragma unroll
+    for (int b = 0; b < kSmallBatch; ++b)
+      if (c[b]) e = fma(w[b], (double)c[b], e);
+    A.edens[i] = e;
+  }
+}
+static_assert(kSmallBatch == 2, "the counts of two placements tested together");
 
 // occupied-bin list per ring entry: entries (bin << 0) with counts beside them
 __global__ void __launch_bounds__(256) ring_compact_kernel(const int* __restrict__ hist, const int* __restrict__ valid,
@@ -700,11 +720,16 @@ cudaError_t launch_accumulate(Engine& e, const BatchArgs& a, cudaStream_t s) {
     A.uvintm = e.d_edintm + e.ermax;
     A.iscal = e.d_edintm + e.ermax + e.numslv;
   }
+  if (a.nb <= kSmallBatch) {
+    accumulate_small_kernel<<<1, kSmallThreads, 0, s>>>(A);
+    e.count_launch();
+    return cudaGetLastError();
+  }
   reduce_kernel<<<a.nb, kAccThreads, 0, s>>>(A);
   accumulate_kernel<<<1, kAccThreads, 0, s>>>(A);
   e.count_launch(2);
   if (!A.zmask) {
-    accumulate_bins_kernel<<<(e.ermax + 127) / 128, 128, 0, s>>>(A);
+    accumulate_bins_kernel<<<(e.ermax + kBinThreads - 1) / kBinThreads, kBinThreads, 0, s>>>(A);
     e.count_launch();
   }
   return cudaGetLastError();

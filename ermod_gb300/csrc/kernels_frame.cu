@@ -1,18 +1,21 @@
 // kernels_frame.cu -- once-per-frame preparation (the engconst prologue).
 //
-//   frame_wrap      realcal_prepare + normalize_periodic (realcal.F90:137-146, 789-885)
-//                   for every atom, FP64, the reference's two wrap passes;
-//   frame_sort      spatial (Morton) order of the physical molecules by the ~4 A cell of
-//                   their first site, so that a CTA's molecules are compact in space
-//                   (coherent near-field branches, PME-grid reuse in L1);
-//   frame_sites     per physical site in slot order: fixed-point coordinates, LJ type,
-//                   charge and the B-spline data of calc_spline_molecule
-//                   (recpcal.F90:408-442) -- replaces recpcal_prepare_solvent
-//                   (engproc.F90:378-382) and the per-placement blockify/sort_block
-//                   rebuild of the reference (realcal.F90:439-525);
+//   frame_key       spatial (Morton) code of each physical molecule's ~4 A cell, from its
+//                   first site wrapped as normalize_periodic does (realcal.F90:789-885)
+//   frame_sort      the molecules in stable order of their codes ("slots"), so that a CTA's
+//                   molecules are compact in space (coherent near-field branches, PME-grid
+//                   reuse in L1), with the slots' site ranges
+//   frame_sites     per physical site in slot order: realcal_prepare + normalize_periodic
+//                   (realcal.F90:137-146, 789-885; FP64, the reference's two wrap passes),
+//                   fixed-point coordinates, LJ type, charge and the B-spline data of
+//                   calc_spline_molecule (recpcal.F90:408-442) -- replaces
+//                   recpcal_prepare_solvent (engproc.F90:378-382) and the per-placement
+//                   blockify/sort_block rebuild of the reference (realcal.F90:439-525)
+//   frame_bricks    the sites listed by brick of the PME grid (the mixed gather's work unit)
 //   greenfunc       recpcal_spline_greenfunc (recpcal.F90:111-152), FP64; for PPPM
 //                   (cltype 3) recpcal_pppm_greenfunc (recpcal.F90:205-319).
 // All of these are HBM-streaming kernels over O(numatm) or O(K^3) elements.
+#include <cooperative_groups.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cmath>
@@ -80,20 +83,6 @@ __device__ __forceinline__ void wrap_atom(const double* __restrict__ pos, int a,
   out[2] = x[2];
 }
 
-__global__ void frame_wrap_kernel(const double* __restrict__ pos, int numatm, FrameGeom g, double* __restrict__ out) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= numatm) return;
-  double w[3];
-  if (g.periodic) {
-    wrap_atom(pos, a, g, w);
-  } else {  // non-periodic: realcal_prepare copies the coordinates as they are
-    for (int i = 0; i < 3; ++i) w[i] = pos[3 * (size_t)a + i];
-  }
-  out[3 * (size_t)a + 0] = w[0];
-  out[3 * (size_t)a + 1] = w[1];
-  out[3 * (size_t)a + 2] = w[2];
-}
-
 __device__ __forceinline__ unsigned int spread3(unsigned int v) {
   v &= 0x3ff;
   v = (v | (v << 16)) & 0x030000ff;
@@ -103,21 +92,190 @@ __device__ __forceinline__ unsigned int spread3(unsigned int v) {
   return v;
 }
 
-__global__ void frame_key_kernel(const double* __restrict__ wrapped, const int* __restrict__ mol_atom0, int slvmax,
-                                 FrameGeom g, int3 ncell, unsigned int* __restrict__ key, int* __restrict__ val) {
+// the coordinates of atom a as the pair terms take them
+__device__ __forceinline__ void normalised(const double* __restrict__ pos, int a, const FrameGeom& g, double out[3]) {
+  if (g.periodic) {
+    wrap_atom(pos, a, g, out);
+  } else {  // non-periodic: realcal_prepare copies the coordinates as they are
+    for (int i = 0; i < 3; ++i) out[i] = pos[3 * (size_t)a + i];
+  }
+}
+
+// the Morton codes and their counts (count zeroed before); also zeroes what the later kernels
+// of the frame add to (the brick counts and the largest molecule radius)
+__global__ void frame_key_kernel(const double* __restrict__ pos, const int* __restrict__ mol_atom0, int slvmax,
+                                 FrameGeom g, int3 ncell, unsigned int* __restrict__ key, int* __restrict__ val,
+                                 int* __restrict__ count, int* __restrict__ brick_count, int nbricks,
+                                 float* __restrict__ frame_scal) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < 4) frame_scal[k] = 0.f;
+  for (int i = k; brick_count && i <= nbricks; i += gridDim.x * blockDim.x) brick_count[i] = 0;
   if (k >= slvmax) return;
-  const int a = mol_atom0[k];
+  double w[3];
+  normalised(pos, mol_atom0[k], g, w);
   int c[3];
   const int n[3] = {ncell.x, ncell.y, ncell.z};
   for (int i = 0; i < 3; ++i) {
     // non-periodic coordinates lie in (-L/2, L/2) of the virtual cube
-    const double f = wrapped[3 * (size_t)a + i] * g.invL[i] + (g.periodic ? 0.0 : 0.5);
+    const double f = w[i] * g.invL[i] + (g.periodic ? 0.0 : 0.5);
     int ci = (int)(f * (double)n[i]);
     c[i] = min(max(ci, 0), n[i] - 1);
   }
-  key[k] = spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2);
-  val[k] = k;
+  const unsigned code = spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2);
+  key[k] = code;
+  if (count)
+    atomicAdd(&count[code], 1);
+  else
+    val[k] = k;
+}
+
+// ---- sorting by small integer codes in one launch --------------------------------------
+// One CTA, or one cluster of 8, of 1024 threads: exclusive scan of the codes' counts, scatter,
+// and within each code the elements in index order.  Integer work on L2-resident arrays, bound
+// by the latency of a few dependent passes, which a radix sort pays per digit and launch: the
+// frame set-up took 13 launches and 76 us of 157 GPU us per frame at 1,000 waters, 130 us at
+// 33,000 (a 30-bit radix sort's four passes alone 42).
+constexpr int kSortThreads = 1024;
+constexpr int kSortCluster = 8;
+
+template <int C>
+__device__ __forceinline__ void sort_sync() {
+  if constexpr (C == 1)
+    __syncthreads();
+  else
+    cooperative_groups::this_cluster().sync();  // orders the cluster's global accesses too
+}
+
+// exclusive prefix sums of get(i), i < n, over the C CTAs of a cluster: put(i, prefix) for each
+// i; returns the total.  Each CTA takes a contiguous range, each thread a contiguous part of it.
+template <int C, class Get, class Put>
+__device__ __forceinline__ int sort_scan(int n, Get get, Put put) {
+  __shared__ int warp_sum[kSortThreads / 32];
+  __shared__ int cta_sum;
+  const int rank = (C == 1) ? 0 : (int)blockIdx.x;
+  const int seg = (n + C - 1) / C, lo = min(n, rank * seg), hi = min(n, lo + seg);
+  const int per = (seg + kSortThreads - 1) / kSortThreads;
+  const int a = min(hi, lo + (int)threadIdx.x * per), b = min(hi, a + per);
+  int own = 0;
+  for (int i = a; i < b; ++i) own += get(i);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = own;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    int w = warp_sum[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += v;
+    }
+    warp_sum[lane] = w;
+    if (lane == 31) cta_sum = w;
+  }
+  sort_sync<C>();
+  int before = incl - own + (warp ? warp_sum[warp - 1] : 0), total = cta_sum;
+  if constexpr (C > 1) {
+    total = 0;
+    for (int r = 0; r < C; ++r) {
+      const int v = *cooperative_groups::this_cluster().map_shared_rank(&cta_sum, r);
+      if (r < rank) before += v;
+      total += v;
+    }
+  }
+  for (int i = a; i < b; ++i) {
+    const int v = get(i);
+    put(i, before);
+    before += v;
+  }
+  sort_sync<C>();  // the prefixes are written, and warp_sum and cta_sum may be used again
+  return total;
+}
+
+struct SortArgs {
+  const unsigned int* key;  // [n] codes
+  int n, ncode;
+  int* count;   // [ncode] counts of the codes; left zero for the next frame
+  int* cursor;  // [ncode] scratch (C > 1; else shared memory)
+  int* tmp;     // [n] scratch
+  const int* mol_nsite;
+  const int* mol_species;
+  const double* mol_qmol;
+  int* slot_mol;
+  int* slot_nsite;  // [n] scratch
+  int* slot_species;
+  double* slot_qmol;
+  int* slot_site;  // [n + 1]
+};
+
+template <int C>
+__global__ void __launch_bounds__(kSortThreads) frame_sort_kernel(SortArgs A) {
+  extern __shared__ int scursor[];
+  int* cursor = (C == 1) ? scursor : A.cursor;
+  const int t0 = (C == 1 ? 0 : blockIdx.x * kSortThreads) + threadIdx.x;
+  constexpr int step = C * kSortThreads;
+  sort_scan<C>(A.ncode, [&](int i) { return A.count[i]; }, [&](int i, int v) { cursor[i] = v; });
+  for (int i = t0; i < A.ncode; i += step) A.count[i] = 0;
+  for (int k = t0; k < A.n; k += step) A.tmp[atomicAdd(&cursor[A.key[k]], 1)] = k;
+  sort_sync<C>();
+  // cursor[code] is now the end of the code's elements; their order among them is that of the
+  // indices (a 4 A cell holds two waters on average)
+  for (int p = t0; p < A.n; p += step) {
+    const int k = A.tmp[p];
+    const unsigned code = A.key[k];
+    const int s = code ? cursor[code - 1] : 0, e = cursor[code];
+    int slot = s;
+    for (int q = s; q < e; ++q) slot += A.tmp[q] < k ? 1 : 0;
+    A.slot_mol[slot] = k;
+    A.slot_nsite[slot] = A.mol_nsite[k];
+    A.slot_species[slot] = A.mol_species[k];
+    A.slot_qmol[slot] = A.mol_qmol[k];
+  }
+  sort_sync<C>();
+  const int total = sort_scan<C>(A.n, [&](int i) { return A.slot_nsite[i]; }, [&](int i, int v) { A.slot_site[i] = v; });
+  if (t0 == 0) A.slot_site[A.n] = total;
+}
+
+// brick of a site: the kBrickX x kBrickY x kBrickZ block of PME grid points holding its stencil
+// base point
+struct BrickGrid {
+  int K[3], nbx, nby;
+  __device__ __forceinline__ int of(int gp) const {
+    int g1 = gp & 1023, g2 = (gp >> 10) & 1023, g3 = (gp >> 20) & 1023;
+    if (g1 >= K[0]) g1 -= K[0];
+    if (g2 >= K[1]) g2 -= K[1];
+    if (g3 >= K[2]) g3 -= K[2];
+    return ((g3 / kBrickZ) * nby + (g2 / kBrickY)) * nbx + (g1 / kBrickX);
+  }
+};
+
+// the sites listed by brick, from the bricks' counts: brick_start[0 .. nbricks], brick_site in
+// no fixed order within a brick (each site's gather is its own)
+template <int C>
+__global__ void __launch_bounds__(kSortThreads) frame_bricks_kernel(const int* __restrict__ site_grid, int nsite,
+                                                                    BrickGrid G, int nbricks,
+                                                                    const int* __restrict__ count, int* gcursor,
+                                                                    int* __restrict__ brick_start,
+                                                                    int* __restrict__ brick_site) {
+  extern __shared__ int scursor[];
+  int* cursor = (C == 1) ? scursor : gcursor;
+  const int total = sort_scan<C>(nbricks, [&](int i) { return count[i]; },
+                                 [&](int i, int v) {
+                                   cursor[i] = v;
+                                   brick_start[i] = v;
+                                 });
+  const int t0 = (C == 1 ? 0 : blockIdx.x * kSortThreads) + threadIdx.x;
+  if (t0 == 0) brick_start[nbricks] = total;
+  for (int i = t0; i < nsite; i += C * kSortThreads) brick_site[atomicAdd(&cursor[G.of(site_grid[i])], 1)] = i;
+}
+
+// the listing alone, grid-wide, from the cursors the scan left (many sites)
+__global__ void brick_fill_kernel(const int* __restrict__ site_grid, int nsite, BrickGrid G, int* cursor,
+                                  int* __restrict__ brick_site) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nsite) brick_site[atomicAdd(&cursor[G.of(site_grid[i])], 1)] = i;
 }
 
 __global__ void frame_slot_kernel(const int* __restrict__ slot_mol, const int* __restrict__ mol_nsite,
@@ -134,7 +292,6 @@ __global__ void frame_slot_kernel(const int* __restrict__ slot_mol, const int* _
 
 struct SiteArgs {
   const double* pos;      // raw sitepos
-  const double* wrapped;  // normalised sitepos
   const int* slot_mol;
   const int* slot_site;
   const int* mol_atom0;
@@ -150,6 +307,8 @@ struct SiteArgs {
   double* site_w;
   double* site_q;
   float* frame_scal;
+  BrickGrid bricks;
+  int* brick_count;  // mixed path
 };
 
 // Four threads per slot (molecule), thread j its sites j, j + 4, ..: water's three sites side
@@ -161,18 +320,26 @@ constexpr int kSiteLanes = 4;
 template <int P>
 __global__ void frame_sites_kernel(SiteArgs A) {
   const int m = (blockIdx.x * blockDim.x + threadIdx.x) / kSiteLanes;
-  double rmax = 0.0;
-  if (m < A.slvmax) {  // (no early return: the warp's maximum below takes every lane)
+  double r2max = 0.0;
+  const FrameGeom& g = A.g;
+  int a0 = 0, ns = 0, s0 = 0;
+  if (m < A.slvmax) {  // (no early return: the shuffles below take every lane)
     const int k = A.slot_mol[m];
-    const int a0 = A.mol_atom0[k];
-    const int ns = A.mol_nsite[k];
-    const int s0 = A.slot_site[m];
-    const FrameGeom& g = A.g;
-    double w0[3] = {A.wrapped[3 * (size_t)a0], A.wrapped[3 * (size_t)a0 + 1], A.wrapped[3 * (size_t)a0 + 2]};
-    for (int s = threadIdx.x % kSiteLanes; s < ns; s += kSiteLanes) {
+    a0 = A.mol_atom0[k];
+    ns = A.mol_nsite[k];
+    s0 = A.slot_site[m];
+  }
+  const int lane = threadIdx.x % kSiteLanes;
+  double w0[3] = {0.0, 0.0, 0.0};  // the molecule's first site
+  if (lane < ns) normalised(A.pos, a0 + lane, g, w0);
+  double w[3] = {w0[0], w0[1], w0[2]};
+#pragma unroll
+  for (int i = 0; i < 3; ++i) w0[i] = __shfl_sync(0xffffffffu, w0[i], 0, kSiteLanes);
+  {
+    for (int s = lane; s < ns; s += kSiteLanes) {
       const int a = a0 + s;
       const int idx = s0 + s;
-      double w[3] = {A.wrapped[3 * (size_t)a], A.wrapped[3 * (size_t)a + 1], A.wrapped[3 * (size_t)a + 2]};
+      if (s != lane) normalised(A.pos, a, g, w);
       // radius about the first site (minimum image)
       double r2 = 0.0;
       for (int i = 0; i < 3; ++i) {
@@ -180,7 +347,7 @@ __global__ void frame_sites_kernel(SiteArgs A) {
         const double d = h - fabs(h - fabs(w[i] - w0[i]));
         r2 += d * d;
       }
-      rmax = fmax(rmax, sqrt(r2));
+      r2max = fmax(r2max, r2);
       // calc_spline_molecule (recpcal.F90:408-442) on the raw coordinates
       const double xst[3] = {A.pos[3 * (size_t)a], A.pos[3 * (size_t)a + 1], A.pos[3 * (size_t)a + 2]};
       int rci[3];
@@ -199,7 +366,9 @@ __global__ void frame_sites_kernel(SiteArgs A) {
           for (int spi = 0; spi < P; ++spi) A.site_w[((size_t)idx * 3 + kk) * P + spi] = wk[spi];
         }
       }
-      A.site_grid[idx] = rci[0] | (rci[1] << kGridBits) | (rci[2] << (2 * kGridBits));
+      const int gp = rci[0] | (rci[1] << kGridBits) | (rci[2] << (2 * kGridBits));
+      A.site_grid[idx] = gp;
+      if constexpr (P == 0) atomicAdd(&A.brick_count[A.bricks.of(gp)], 1);
       const double q = A.charge[a];
       // FP64 wrapped coordinates and charge: the FP64 path's pair terms, and the mixed
       // path's FP64 terms of close pairs
@@ -222,27 +391,9 @@ __global__ void frame_sites_kernel(SiteArgs A) {
   }
   // the largest molecule radius: a warp maximum first, then one atomic per warp on this
   // one address instead of one per molecule
-  float r = (m < A.slvmax) ? (float)rmax * 1.0001f + 1e-4f : 0.f;
+  float r = (m < A.slvmax) ? (float)sqrt(r2max) * 1.0001f + 1e-4f : 0.f;
   for (int off = 16; off > 0; off >>= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, off));
   if ((threadIdx.x & 31) == 0) atomicMax((int*)&A.frame_scal[0], __float_as_int(r));
-}
-
-// brick of every site: the kBrickX x kBrickY x kBrickZ block of PME grid points holding its
-// stencil base point
-__global__ void brick_key_kernel(const int* __restrict__ site_grid, int nsite, int K1, int K2, int K3, int nbx,
-                                 int nby, unsigned int* __restrict__ key, int* __restrict__ val,
-                                 int* __restrict__ count) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsite) return;
-  const int gp = site_grid[i];
-  int g1 = gp & 1023, g2 = (gp >> 10) & 1023, g3 = (gp >> 20) & 1023;
-  if (g1 >= K1) g1 -= K1;
-  if (g2 >= K2) g2 -= K2;
-  if (g3 >= K3) g3 -= K3;
-  const unsigned int bk = (unsigned int)(((g3 / kBrickZ) * nby + (g2 / kBrickY)) * nbx + (g1 / kBrickX));
-  key[i] = bk;
-  val[i] = i;
-  atomicAdd(&count[bk], 1);
 }
 
 // the FP32 copy of engfac keeps rows of H points padded to a multiple of 4 (zeros)
@@ -382,6 +533,14 @@ __global__ void carry_status_kernel(DevStatus* s) {
 
 }  // namespace
 
+__global__ void reset_status_kernel(DevStatus* s) { *s = DevStatus{kNoError, kNoError, 0, 0}; }
+
+cudaError_t launch_reset_status(Engine& e) {
+  reset_status_kernel<<<1, 1, 0, e.stream>>>(e.d_status);
+  e.count_launch();
+  return cudaGetLastError();
+}
+
 cudaError_t launch_carry_status(Engine& e) {
   carry_status_kernel<<<1, 1, 0, e.stream>>>(e.d_status);
   e.count_launch();
@@ -402,25 +561,80 @@ cudaError_t launch_max_abs(Engine& e, const double* x_d, size_t n, double* host_
   return cudaSuccess;
 }
 
-cudaError_t launch_frame_wrap(Engine& e) {
-  frame_wrap_kernel<<<nblk(e.numatm, 256), 256, 0, e.stream>>>(e.d_sitepos, e.numatm, e.geom, e.d_wrapped);
-  e.count_launch();
-  return cudaGetLastError();
+// One CTA while the codes' cursors fit in its shared memory and its threads have few elements,
+// else a cluster of 8 (4,000 molecules: 16 us against 12; 1,000: 7.5 with one CTA; bricks of
+// 3,000 sites 5.7 us with one CTA, of 12,000 12.5 with the cluster)
+constexpr int kSortSharedCodes = 32768;
+constexpr int kSortOneCta = 3 * kSortThreads;
+
+template <class... Params, class... Args>
+static cudaError_t launch_cluster(void (*kern)(Params...), cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kSortCluster);
+  cfg.blockDim = dim3(kSortThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kSortCluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 cudaError_t launch_frame_sort(Engine& e) {
-  int3 nc;
-  nc.x = std::max(1, std::min(1024, (int)(e.geom.L[0] / 4.0)));
-  nc.y = std::max(1, std::min(1024, (int)(e.geom.L[1] / 4.0)));
-  nc.z = std::max(1, std::min(1024, (int)(e.geom.L[2] / 4.0)));
-  frame_key_kernel<<<nblk(e.slvmax, 256), 256, 0, e.stream>>>(e.d_wrapped, e.d_mol_atom0, e.slvmax, e.geom, nc,
-                                                             e.d_sort_key, e.d_sort_val);
+  int nc[3], bits = 1;
+  for (int i = 0; i < 3; ++i) {
+    nc[i] = std::max(1, std::min(1024, (int)(e.geom.L[i] / 4.0)));
+    while ((1 << bits) < nc[i]) ++bits;
+  }
+  // sparse cells (a droplet in its virtual cube): no more codes than 4 per molecule, by doubling
+  // the cell's edge (300 waters, 32,768 codes: 56 us of scanning)
+  while (bits > 1 && (1ll << (3 * bits)) > std::max(4096ll, 4ll * e.slvmax)) {
+    --bits;
+    for (int& n : nc) n = (n + 1) / 2;
+  }
+  // up to kSortMaxMol molecules are sorted by counting (their codes then have at most
+  // kSortMaxBits bits per axis); beyond, the cluster's threads have too many each, and the
+  // radix sort's grid-wide passes are the faster
+  const bool counted = e.slvmax <= kSortMaxMol;
+  const int ncode = 1 << (3 * std::min(bits, kSortMaxBits));
+  frame_key_kernel<<<nblk(e.slvmax, 256), 256, 0, e.stream>>>(
+      e.d_sitepos, e.d_mol_atom0, e.slvmax, e.geom, make_int3(nc[0], nc[1], nc[2]), e.d_sort_key, e.d_sort_val,
+      counted ? e.d_sort_count : nullptr, e.d_brick_count, e.nbricks, e.d_frame_scal);
   e.count_launch();
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
+  if (counted) {
+    SortArgs A{};
+    A.key = e.d_sort_key;
+    A.n = e.slvmax;
+    A.ncode = ncode;
+    A.count = e.d_sort_count;
+    A.cursor = e.d_sort_count + ((size_t)1 << (3 * kSortMaxBits));
+    A.tmp = e.d_sort_val;
+    A.mol_nsite = e.d_mol_nsite;
+    A.mol_species = e.d_mol_species;
+    A.mol_qmol = e.d_mol_qmol;
+    A.slot_mol = e.d_slot_mol;
+    A.slot_nsite = e.d_sort_val_alt;
+    A.slot_species = e.d_slot_species;
+    A.slot_qmol = e.d_slot_qmol;
+    A.slot_site = e.d_slot_site;
+    e.count_launch();
+    if (e.slvmax <= kSortOneCta && ncode <= kSortSharedCodes) {
+      static SmemAttr attr;
+      const size_t smem = sizeof(int) * ncode;
+      if ((err = attr.ensure(frame_sort_kernel<1>, smem)) != cudaSuccess) return err;
+      frame_sort_kernel<1><<<1, kSortThreads, smem, e.stream>>>(A);
+      return cudaGetLastError();
+    }
+    return launch_cluster(frame_sort_kernel<kSortCluster>, e.stream, A);
+  }
   size_t bytes = e.cub_tmp_bytes;
   err = cub::DeviceRadixSort::SortPairs(e.d_cub_tmp, bytes, e.d_sort_key, e.d_sort_key_alt, e.d_sort_val,
-                                        e.d_slot_mol, e.slvmax, 0, 30, e.stream);
+                                        e.d_slot_mol, e.slvmax, 0, 3 * bits, e.stream);
   if (err != cudaSuccess) return err;
   frame_slot_kernel<<<nblk(e.slvmax, 256), 256, 0, e.stream>>>(e.d_slot_mol, e.d_mol_nsite, e.d_mol_species,
                                                               e.d_mol_qmol, e.slvmax, e.d_sort_val_alt,
@@ -434,24 +648,36 @@ cudaError_t launch_frame_sort(Engine& e) {
   return err;
 }
 
+static BrickGrid brick_grid(const Engine& e) {
+  BrickGrid G;
+  for (int i = 0; i < 3; ++i) G.K[i] = e.geom.K[i];
+  G.nbx = e.nbrick[0];
+  G.nby = e.nbrick[1];
+  return G;
+}
+
 cudaError_t launch_frame_bricks(Engine& e) {
-  cudaError_t err = cudaMemsetAsync(e.d_brick_count, 0, sizeof(int) * (e.nbricks + 1), e.stream);
-  if (err != cudaSuccess) return err;
-  brick_key_kernel<<<nblk(e.nsite_phys, 256), 256, 0, e.stream>>>(e.d_site_grid, e.nsite_phys, e.geom.K[0],
-                                                                   e.geom.K[1], e.geom.K[2], e.nbrick[0],
-                                                                   e.nbrick[1], e.d_brick_key, e.d_brick_val,
-                                                                   e.d_brick_count);
-  e.count_launch();
-  if ((err = cudaGetLastError()) != cudaSuccess) return err;
-  int bits = 1;
-  while ((1 << bits) < e.nbricks + 1) ++bits;
-  size_t bytes = e.cub_tmp_bytes;
-  err = cub::DeviceRadixSort::SortPairs(e.d_cub_tmp, bytes, e.d_brick_key, e.d_brick_key_alt, e.d_brick_val,
-                                        e.d_brick_site, e.nsite_phys, 0, bits, e.stream);
-  if (err != cudaSuccess) return err;
-  bytes = e.cub_tmp_bytes;
-  return cub::DeviceScan::ExclusiveSum(e.d_cub_tmp, bytes, e.d_brick_count, e.d_brick_start, e.nbricks + 1,
-                                       e.stream);
+  const BrickGrid G = brick_grid(e);
+  cudaError_t err;
+  // the scan's CTAs list up to 8 sites per thread of theirs; more are listed by a grid-wide launch
+  const bool fill = e.nsite_phys > 8 * kSortThreads;
+  e.count_launch(fill ? 2 : 1);
+  if (e.nsite_phys <= kSortOneCta && e.nbricks <= kSortSharedCodes) {
+    static SmemAttr attr;
+    const size_t smem = sizeof(int) * e.nbricks;
+    if ((err = attr.ensure(frame_bricks_kernel<1>, smem)) != cudaSuccess) return err;
+    frame_bricks_kernel<1><<<1, kSortThreads, smem, e.stream>>>(e.d_site_grid, e.nsite_phys, G, e.nbricks,
+                                                                e.d_brick_count, nullptr, e.d_brick_start,
+                                                                e.d_brick_site);
+    return cudaGetLastError();
+  }
+  err = launch_cluster(frame_bricks_kernel<kSortCluster>, e.stream, (const int*)e.d_site_grid,
+                       fill ? 0 : e.nsite_phys, G, e.nbricks, (const int*)e.d_brick_count, e.d_brick_cursor,
+                       e.d_brick_start, e.d_brick_site);
+  if (err != cudaSuccess || !fill) return err;
+  brick_fill_kernel<<<nblk(e.nsite_phys, 256), 256, 0, e.stream>>>(e.d_site_grid, e.nsite_phys, G, e.d_brick_cursor,
+                                                                   e.d_brick_site);
+  return cudaGetLastError();
 }
 
 size_t frame_cub_bytes(int n) {
@@ -462,20 +688,11 @@ size_t frame_cub_bytes(int n) {
   return std::max(a, b);
 }
 
-size_t brick_cub_bytes(int nsite, int nbricks) {
-  size_t a = 0, b = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, a, (unsigned int*)nullptr, (unsigned int*)nullptr, (int*)nullptr,
-                                  (int*)nullptr, nsite, 0, 32, (cudaStream_t)0);
-  cub::DeviceScan::ExclusiveSum(nullptr, b, (int*)nullptr, (int*)nullptr, nbricks + 1, (cudaStream_t)0);
-  return std::max(a, b);
-}
-
 cudaError_t launch_frame_sites(Engine& e) {
-  cudaError_t err = cudaMemsetAsync(e.d_frame_scal, 0, sizeof(float) * 4, e.stream);
-  if (err != cudaSuccess) return err;
   SiteArgs A{};
   A.pos = e.d_sitepos;
-  A.wrapped = e.d_wrapped;
+  A.bricks = brick_grid(e);
+  A.brick_count = e.d_brick_count;
   A.slot_mol = e.d_slot_mol;
   A.slot_site = e.d_slot_site;
   A.mol_atom0 = e.d_mol_atom0;

@@ -300,7 +300,7 @@ constexpr int kBigList = 1024;
 // that pass's scratch (ints): the list (pairs, their near items as 16 bits, their values), the
 // threads' recorded pairs, the molecules' first sites, and the list of near (molecule,
 // placement) items (16 bits)
-__host__ __device__ constexpr int finish_scratch_ints(int G) {
+__host__ __device__ constexpr int finish_scratch_ints(int G) {  // for the larger tile, 256
   return kBigList + kBigList / 2 + 2 * kBigList + 256 * kBigPerThread + 256 + G * 256 / 2;
 }
 // the dynamic shared memory of the finish kernel before its edge keys: the block
@@ -765,16 +765,16 @@ __device__ __forceinline__ int exact_count(const long long* __restrict__ uvkey, 
 }
 
 // the finish kernel's per-species partials of its block (see mol_finish_kernel)
-template <int G, bool kSum>
-__device__ __forceinline__ void species_partials(const MolArgs& A, const BatchArgs& a, const float (*su)[256],
-                                                 const float (*sul)[256], const unsigned char* sspec, int g0, int ng,
+template <int G, int TILE, bool kSum>
+__device__ __forceinline__ void species_partials(const MolArgs& A, const BatchArgs& a, const float (*su)[TILE],
+                                                 const float (*sul)[TILE], const unsigned char* sspec, int g0, int ng,
                                                  int tile) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int pr = warp; pr < ng * A.numslv; pr += blockDim.x / 32) {
     const int j = pr / A.numslv, sp = pr % A.numslv + 1;
     long long mn = kFfKeyNone, mx = kFfKeyNoneMax;
     double s = 0.0;
-    for (int t = lane; t < blockDim.x; t += 32) {
+    for (int t = lane; t < TILE; t += 32) {
       const float v = su[j][t];
       if (sspec[t] == sp && v == v) {
         const float lo = sul[j][t];
@@ -809,7 +809,10 @@ __device__ __forceinline__ void species_partials(const MolArgs& A, const BatchAr
 // fixed tree.  So a warp's lanes all have pairs to evaluate (2% of the 33,000-water box's
 // molecules lie in reach), a large solute's pairs are not one thread's serial chain, and an
 // item's sum does not depend on the block it falls in.
-template <int G>
+//
+// TILE: molecules per block of 256 threads.  64 in solution mode, where a frame's one placement
+// makes few blocks and the real-space pass takes all 256 threads.
+template <int G, int TILE>
 __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const float* __restrict__ site_e) {
   extern __shared__ __align__(16) int smem_dyn[];
   // [G][ermax] block histograms, or none when they would not fit beside other blocks: the
@@ -825,20 +828,21 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
   int* ss0 = sitem + 256 * kBigPerThread;                                   // [256] first sites
   unsigned short* snear = reinterpret_cast<unsigned short*>(ss0 + 256);     // [G * 256] molecule | placement << 8
   __shared__ int swarp[8];
-  __shared__ float su[G][256];   // totals, hi part (NaN: no molecule)
-  __shared__ float sul[G][256];  // totals, lo part
+  __shared__ float su[G][TILE];   // totals, hi part (NaN: no molecule)
+  __shared__ float sul[G][TILE];  // totals, lo part
   __shared__ float sres[G];      // residual factor x solute charge of the G placements
   __shared__ float srcut[G];     // bounding-sphere cutoff of the real-space sum
   __shared__ int skskip[G];      // slot of the solute molecule itself (not a solvent)
   __shared__ int srej[G];        // placement rejected by check_mol_configuration
   __shared__ int4 supos[G];      // first solute site (fixed point)
-  __shared__ unsigned char sspec[256];
+  __shared__ unsigned char sspec[TILE];
   const int tile = blockIdx.y;
   const int g0 = blockIdx.x * G;
   const BatchArgs& a = A.a;
   const int ng = min(G, a.nb - g0);
-  const int m = tile * blockDim.x + threadIdx.x;
-  const bool valid = m < A.slvmax;
+  const bool mine = TILE == 256 || threadIdx.x < TILE;
+  const int m = tile * TILE + threadIdx.x;
+  const bool valid = mine && m < A.slvmax;
   for (int i = threadIdx.x; i < A.ermax; i += blockDim.x) skeys[i] = A.uvkey_f[i];
   if (threadIdx.x < ng) {
     const int b = g0 + threadIdx.x;
@@ -861,7 +865,7 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
     qmol = (float)A.slot_qmol[m];
   }
   const bool spec_ok = valid && species >= 1 && species <= A.numslv;
-  sspec[threadIdx.x] = (unsigned char)(spec_ok ? species : 0);
+  if (mine) sspec[threadIdx.x] = (unsigned char)(spec_ok ? species : 0);
   const int ldb = A.ldb;
   int sp_off = 0, sp_n = 1, sp_soft = 1;
   if (spec_ok) {
@@ -913,8 +917,10 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
       }
       // residual_ene (engproc.F90:859-869)
       const ff t = on ? ff_add(rs[j], -sres[j] * qmol) : ff{0.f, 0.f};
-      su[j][threadIdx.x] = t.hi;
-      sul[j][threadIdx.x] = t.lo;
+      if (mine) {
+        su[j][threadIdx.x] = t.hi;
+        sul[j][threadIdx.x] = t.lo;
+      }
     }
   }
   // ---- real space: get_uv_energy (engproc.F90:736-753) adds it to residual + recip ----
@@ -974,7 +980,7 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
       t = snear[near] & 0xff;
       j = snear[near] >> 8;
       is0 = ss0[t];
-      ins = A.slot_site[tile * 256 + t + 1] - is0;
+      ins = A.slot_site[tile * TILE + t + 1] - is0;
     }
     // a thread with more than kBigPerThread FP64 pairs takes further windows
     for (int win = 0;; win += kBigPerThread) {
@@ -1032,8 +1038,8 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
   float ulo[G];  // the total's lo part
 #pragma unroll
   for (int j = 0; j < G; ++j) {
-    ku[j] = ordered_key32(su[j][threadIdx.x]);
-    ulo[j] = sul[j][threadIdx.x];
+    ku[j] = mine ? ordered_key32(su[j][threadIdx.x]) : 0;
+    ulo[j] = mine ? sul[j][threadIdx.x] : 0.f;
   }
   if (valid && a.uvengy_out) {
 #pragma unroll
@@ -1094,8 +1100,10 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
     } else if (a.mol_bin && valid && j < ng) {
       a.mol_bin[(size_t)(g0 + j) * A.slvmax + m] = A.ermax;
     }
-    su[j][threadIdx.x] = hv;
-    sul[j][threadIdx.x] = lv;
+    if (mine) {
+      su[j][threadIdx.x] = hv;
+      sul[j][threadIdx.x] = lv;
+    }
   }
   __syncthreads();
   // per-species {sum, min, max} of the block: one warp per (placement, species),
@@ -1104,9 +1112,9 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
   // here unless the species sums are wanted -- they are flceng (engproc.F90:822-825),
   // needed for slnuv (solution mode) and when the caller asks for flceng
   if (A.soln || a.flceng_out != nullptr)
-    species_partials<G, true>(A, a, su, sul, sspec, g0, ng, tile);
+    species_partials<G, TILE, true>(A, a, su, sul, sspec, g0, ng, tile);
   else
-    species_partials<G, false>(A, a, su, sul, sspec, g0, ng, tile);
+    species_partials<G, TILE, false>(A, a, su, sul, sspec, g0, ng, tile);
   if (A.hist_global) return;
   for (int j = 0; j < ng; ++j) {
     const int* h = smem_hist + j * A.ermax;
@@ -1176,7 +1184,10 @@ static MolArgs make_mol_args(Engine& e, const BatchArgs& a) {
   A.upljcut = e.P.upljcut;
   A.screen = e.P.screen;
   A.bare = (e.P.cltype == 0) ? 1 : 0;
+  // two to five solute sites a thread; one in the small tiles of solution mode
   A.real_lanes = e.max_solute_sites <= 2 ? 1 : e.max_solute_sites <= 6 ? 2 : e.max_solute_sites <= 16 ? 4 : 8;
+  if (e.mixed && e.tile < 256)
+    for (A.real_lanes = 1; A.real_lanes < std::min(32, e.max_solute_sites);) A.real_lanes *= 2;
   A.resid_fac = A.bare ? 0.0 : kPi / e.P.screen / e.P.screen / e.geom.volume;
   for (int i = 0; i < 3; ++i) A.fxf[i] = (float)e.geom.fx_scale[i];
   A.screen_f = (float)e.P.screen;
@@ -1220,7 +1231,12 @@ cudaError_t launch_gather(Engine& e, const BatchArgs& a) {
 // one per solute molecule), so its molecules are split further while that still leaves the
 // GPU room; fixed for a context, so that a placement's sums do not depend on its batch
 static int mol64_ty(const Engine& e) { return e.P.slttype == 1 && e.slvmax < 512 * e.num_sm ? 4 : 1; }
-int mol64_tile(const Engine& e) { return kMol64Threads / (4 * mol64_ty(e)); }
+// molecules per block of the molecule kernels: the FP64 path's as above; the mixed path's 256,
+// or 64 in solution mode while that still leaves blocks to fill the GPU
+int mol_tile(const Engine& e) {
+  if (!e.mixed) return kMol64Threads / (4 * mol64_ty(e));
+  return e.P.slttype == 1 && e.P.finish_group == 0 && e.slvmax < 64 * 3 * e.num_sm ? 64 : 256;
+}
 
 // placements per molecule-energy block: the caller's choice (4 or 8), else 4, halved while the
 // launch has fewer than 1.5 blocks per SM (2,000 waters, 36 sites, batches of 64: 26.6 ms of
@@ -1230,6 +1246,7 @@ int mol64_tile(const Engine& e) { return kMol64Threads / (4 * mol64_ty(e)); }
 static int finish_group(const Engine& e, int nb) {
   int G = e.G;
   if (e.P.finish_group != 0) return G;
+  if (e.tile < 256) return 1;
   while (G > 1 && 2LL * e.ntile * ((nb + G - 1) / G) < 3LL * e.num_sm) G /= 2;
   return G;
 }
@@ -1240,9 +1257,9 @@ cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a) {
   cudaError_t err = cudaSuccess;
   if (!e.mixed) return mol64_ty(e) == 4 ? launch_mol64<4>(e, A) : launch_mol64<1>(e, A);
   const int G = finish_group(e, a.nb);
-  // block histograms in shared memory up to 64 KB (three blocks per SM fit); beyond that the
-  // counts go straight to global memory
-  A.hist_global = (size_t)G * e.ermax * sizeof(int) > 64 * 1024 ? 1 : 0;
+  // block histograms in shared memory up to 64 KB (three blocks per SM fit); beyond that, and
+  // for the few molecules of a small tile, the counts go straight to global memory
+  A.hist_global = (e.tile < 256 || (size_t)G * e.ermax * sizeof(int) > 64 * 1024) ? 1 : 0;
   if (e.P.cltype != 0 && (err = launch_gather(e, a)) != cudaSuccess) return err;
   if (a.phases) {
     e.phase_end_on(a.stream);
@@ -1251,16 +1268,17 @@ cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a) {
   // step 2: per-molecule totals and binning (histograms + edge keys in shared memory)
   const size_t smem_f = sizeof(int) * ((size_t)finish_region_ints(G, e.ermax, A.hist_global) + e.ermax);
   dim3 g2((a.nb + G - 1) / G, e.ntile);
-#define ERMOD_FINISH(GG)                                                                                   \
-  if (G == GG) {                                                                                           \
+#define ERMOD_FINISH(GG, TILE)                                                                             \
+  if (G == GG && e.tile == TILE) {                                                                         \
     static SmemAttr attr;                                                                                  \
-    if ((err = attr.ensure(mol_finish_kernel<GG>, smem_f)) != cudaSuccess) return err;                     \
-    mol_finish_kernel<GG><<<g2, 256, smem_f, a.stream>>>(A, a.site_e);                                     \
+    if ((err = attr.ensure(mol_finish_kernel<GG, TILE>, smem_f)) != cudaSuccess) return err;               \
+    mol_finish_kernel<GG, TILE><<<g2, 256, smem_f, a.stream>>>(A, a.site_e);                               \
   }
-  ERMOD_FINISH(1)
-  ERMOD_FINISH(2)
-  ERMOD_FINISH(4)
-  ERMOD_FINISH(8)
+  ERMOD_FINISH(1, 64)
+  ERMOD_FINISH(1, 256)
+  ERMOD_FINISH(2, 256)
+  ERMOD_FINISH(4, 256)
+  ERMOD_FINISH(8, 256)
 #undef ERMOD_FINISH
   e.count_launch();
   return cudaGetLastError();

@@ -59,7 +59,7 @@ struct PrepArgs {
   int self_mode;  // 0: none, 1: all placements, 2: only placement 0 of the batch
   int nummol;
   int bare;  // cltype 0
-  unsigned mK[3], mKmax, m3Kmax;  // ceil(2^32 / d): n / d = umulhi(n, m) for n d < 2^32
+  unsigned mK[3];  // ceil(2^32 / d): n / d = umulhi(n, m) for n d < 2^32
   DevStatus* status;
 };
 
@@ -71,32 +71,76 @@ __device__ __forceinline__ void wrap_coord(const double* v, double x0raw, const 
   out[0] = out[0] - g.L[0] * floor(g.invL[0] * x0b);
 }
 
-// one block per placement of the batch
+// 1-D structure factors of one axis of one placement's solute: FP64 weights
+// (calc_spline_molecule on the raw coordinates) and twiddles; the mixed path rounds them to
+// FP32 once at the end, so that their errors are independent roundings
+__device__ void structure_factors(const PrepArgs& A, int b, int atom0, int ns, int ax) {
+  __shared__ double th[kMaxSoluteSites * kMaxSplineOrder];
+  __shared__ int sgrd[kMaxSoluteSites];
+  const BatchArgs& a = A.a;
+  const FrameGeom& g = A.g;
+  const int P = A.sc.order, K = g.K[ax];
+  for (int t = threadIdx.x; t < ns * P; t += blockDim.x) {
+    const int s = t / P, spi = t - s * P;
+    const double* raw = A.solxyz ? A.solxyz + ((size_t)b * ns + s) * 3 : A.sitepos + 3 * (size_t)(atom0 + s);
+    double factor = g.invcl[ax + 0] * raw[0] + g.invcl[ax + 3] * raw[1] + g.invcl[ax + 6] * raw[2];
+    factor = factor - floor(factor);
+    const double f2 = factor * (double)K;
+    const int rci = (int)f2;
+    th[t] = spline_value(A.sc, f2 - (double)(rci - spi));
+    if (spi == 0) sgrd[s] = rci;
+  }
+  __syncthreads();
+  const int Kmax = max(g.K[0], max(g.K[1], g.K[2]));
+  const double2* tw = A.twiddle64 + (ax == 0 ? 0 : (ax == 1 ? g.K[0] : g.K[0] + g.K[1]));
+  const unsigned mk = A.mK[ax];
+  for (int t = threadIdx.x; t < ns * K; t += blockDim.x) {
+    const int s = (int)__umulhi((unsigned)t, mk), k = t - s * K;
+    const int grd = sgrd[s];
+    double re = 0.0, im = 0.0;
+    for (int c = 0; c < P; ++c) {
+      int gc = grd - c;  // in (-P, K)
+      if (gc < 0) gc += K;
+      const unsigned x = (unsigned)(k * gc);  // < K^2 <= 10^6
+      const int mm = (int)(x - __umulhi(x, mk) * (unsigned)K);
+      const double2 w = tw[mm];
+      re = fma(th[s * P + c], w.x, re);
+      im = fma(th[s * P + c], w.y, im);
+    }
+    const size_t at = (((size_t)b * kMaxSoluteSites + s) * 3 + ax) * Kmax + k;
+    if (A.mixed)
+      a.u_bvec[at] = make_float2((float)re, (float)im);
+    else
+      a.u_bvec64[at] = make_double2(re, im);
+  }
+}
+
+// Four blocks per placement of the batch: the structure factors of each axis, and the rest
+// (coordinates, charges, bounding radius, realcal_self), so that a single placement's FP64
+// chains run side by side and on four SMs' FP64 pipes (one block, one thread per site for the
+// weights: 24 us for 6 sites at 32^3, on a solution-mode frame's critical path).
 __global__ void __launch_bounds__(256) place_prep_kernel(PrepArgs A) {
   const int b = blockIdx.x;
+  const int part = A.bare ? 3 : (int)blockIdx.y;
   const BatchArgs& a = A.a;
   const FrameGeom& g = A.g;
   const int mol = a.tagslt[b] - 1;
-  if (mol < 0 || mol >= A.nummol) {  // device-side inputs are checked here, not trusted
-    if (threadIdx.x == 0) {
+  // device-side inputs are checked here, not trusted
+  const int atom0 = (mol < 0 || mol >= A.nummol) ? 0 : A.mbi0[mol];
+  const int ns = (mol < 0 || mol >= A.nummol) ? 0 : A.mbi0[mol + 1] - atom0;
+  if (ns < 1 || ns > kMaxSoluteSites) {
+    if (part == 3 && threadIdx.x == 0) {
       atomicOr(&A.status->range_fault, 1);
       a.u_nsite[b] = 0;
     }
     return;
   }
-  const int atom0 = A.mbi0[mol];
-  const int ns = A.mbi0[mol + 1] - atom0;
-  const int P = A.sc.order;
+  if (part < 3) {
+    structure_factors(A, b, atom0, ns, part);
+    return;
+  }
   __shared__ double sx[kMaxSoluteSites][3];
   __shared__ double red[256];
-  __shared__ int sgrd[kMaxSoluteSites][3];
-  if (ns > kMaxSoluteSites) {
-    if (threadIdx.x == 0) {
-      atomicOr(&A.status->range_fault, 1);
-      a.u_nsite[b] = 0;
-    }
-    return;
-  }
   for (int s = threadIdx.x; s < ns; s += blockDim.x) {
     const double* raw = A.solxyz ? A.solxyz + ((size_t)b * ns + s) * 3 : A.sitepos + 3 * (size_t)(atom0 + s);
     double w[3];
@@ -123,58 +167,10 @@ __global__ void __launch_bounds__(256) place_prep_kernel(PrepArgs A) {
     a.u_pos[us] = make_int4((int)X[0], (int)X[1], (int)X[2], A.ljtype[atom0 + s]);
     a.u_q[us] = A.charge[atom0 + s];
     a.u_qf[us] = (float)A.charge[atom0 + s];
-    int rci[3];
-    for (int kk = 0; kk < 3; ++kk) {  // calc_spline_molecule on the raw coordinates
-      double factor = g.invcl[kk + 0] * raw[0] + g.invcl[kk + 3] * raw[1] + g.invcl[kk + 6] * raw[2];
-      factor = factor - floor(factor);
-      const double f2 = factor * (double)g.K[kk];
-      rci[kk] = (int)f2;
-      double* uw = a.u_w + (us * 3 + kk) * kMaxSplineOrder;
-      // FP64 weights on both paths: on the mixed path they set the 1-D structure factors,
-      // whose accuracy bounds that of the solute self energy (the weights of placements)
-      for (int spi = 0; spi < P; ++spi) uw[spi] = spline_value(A.sc, f2 - (double)(rci[kk] - spi));
-      sgrd[s][kk] = rci[kk];
-    }
-    a.u_grid[us] = rci[0] | (rci[1] << kGridBits) | (rci[2] << (2 * kGridBits));
   }
   if (threadIdx.x == 0) {
     a.u_nsite[b] = ns;
     a.u_qmol[b] = A.mol_qmol_all[mol];
-  }
-  __syncthreads();
-  // 1-D structure-factor vectors: FP64 weights and twiddles; the mixed path rounds them to
-  // FP32 once at the end, so that their errors are independent roundings
-  if (!A.bare) {
-    const int Kx = g.K[0], Ky = g.K[1], Kz = g.K[2];
-    const int Kmax = max(Kx, max(Ky, Kz));
-    const int total = ns * 3 * Kmax;
-    for (int t = threadIdx.x; t < total; t += blockDim.x) {
-      const int s = (int)__umulhi((unsigned)t, A.m3Kmax);
-      const int r = t - s * 3 * Kmax;
-      const int ax = (int)__umulhi((unsigned)r, A.mKmax);
-      const int k = r - ax * Kmax;
-      const int K = g.K[ax];
-      if (k >= K) continue;
-      const size_t us = (size_t)b * kMaxSoluteSites + s;
-      const int grd = sgrd[s][ax];
-      const double2* tw = A.twiddle64 + (ax == 0 ? 0 : (ax == 1 ? Kx : Kx + Ky));
-      const double* th = a.u_w + (us * 3 + ax) * kMaxSplineOrder;
-      const unsigned mk = A.mK[ax];
-      double re = 0.0, im = 0.0;
-      for (int c = 0; c < P; ++c) {
-        int gc = grd - c;  // in (-P, K)
-        if (gc < 0) gc += K;
-        const unsigned x = (unsigned)(k * gc);  // < K^2 <= 10^6
-        const int mm = (int)(x - __umulhi(x, mk) * (unsigned)K);
-        const double2 w = tw[mm];
-        re = fma(th[c], w.x, re);
-        im = fma(th[c], w.y, im);
-      }
-      if (A.mixed)
-        a.u_bvec[(us * 3 + ax) * Kmax + k] = make_float2((float)re, (float)im);
-      else
-        a.u_bvec64[(us * 3 + ax) * Kmax + k] = make_double2(re, im);
-    }
   }
   // bounding radius about site 1 (minimum image; FP32, padded to stay conservative)
   __shared__ int rmax_bits;
@@ -344,9 +340,7 @@ cudaError_t launch_place_prep(Engine& e, const BatchArgs& a, const double* sol_x
   A.status = e.d_status;
   auto magic = [](unsigned d) { return (unsigned)((0x100000000ull + d - 1) / d); };
   for (int i = 0; i < 3; ++i) A.mK[i] = magic((unsigned)e.geom.K[i]);
-  A.mKmax = magic((unsigned)e.Kmax());
-  A.m3Kmax = magic(3u * (unsigned)e.Kmax());
-  place_prep_kernel<<<a.nb, 256, 0, s>>>(A);
+  place_prep_kernel<<<dim3(a.nb, A.bare ? 1 : 4), 256, 0, s>>>(A);
   e.count_launch();
   return cudaGetLastError();
 }
