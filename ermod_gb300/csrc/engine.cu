@@ -17,6 +17,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "engine.cuh"
@@ -41,6 +42,30 @@ void dfree(T*& p) {
   p = nullptr;
 }
 }  // namespace
+
+// A large output array is often fresh memory whose pages the kernel has yet to make and zero, one
+// thread at a time inside the copy: a few threads write to each page first (a 4,996-bin ecorr,
+// 200 MB: read back in 8.4 ms, with the threads 4.2).  The array is overwritten whole afterwards.
+static void touch_pages(void* p, size_t bytes) {
+  constexpr size_t kPage = 4096, kPart = (size_t)8 << 20;
+  const int n = (int)std::min<size_t>(8, bytes / kPart);
+  if (n < 2) return;
+  const size_t part = (bytes / n + kPage - 1) / kPage * kPage;
+  auto touch = [&](int i) {
+    volatile char* c = static_cast<char*>(p);
+    for (size_t at = i * part, end = std::min(bytes, at + part); at < end; at += kPage) c[at] = 0;
+  };
+  std::vector<std::thread> th;
+  for (int i = 1; i < n; ++i) {
+    try {
+      th.emplace_back(touch, i);
+    } catch (const std::exception&) {  // no thread: the copy makes the pages
+      break;
+    }
+  }
+  touch(0);
+  for (std::thread& t : th) t.join();
+}
 
 void set_error_string(const std::string& s) { g_err = s; }
 
@@ -201,14 +226,11 @@ static int free_bins(Engine& e) {
   dfree(e.d_uvkey_f);
   dfree(e.d_eskey);
   dfree(e.d_spec);
-  dfree(e.d_edens);
+  dfree(e.d_accum);
+  if (e.h_accum) cudaFreeHost(e.h_accum);
+  e.h_accum = nullptr;
   dfree(e.d_ecorr);
   dfree(e.d_ecorr_n);
-  dfree(e.d_eself);
-  dfree(e.d_slnuv);
-  dfree(e.d_minuv);
-  dfree(e.d_maxuv);
-  dfree(e.d_scal);
   return ERMOD_OK;
 }
 
@@ -503,6 +525,11 @@ int ermod_create(const ermod_params* p_in, int device, ermod_ctx** out) {
     ermod_destroy(c);
     return fail_cuda(err, "status allocation");
   }
+  if ((err = cudaMallocHost(&e.h_stage, 2 * kStageBytes)) != cudaSuccess ||
+      (err = cudaEventCreateWithFlags(&e.ev_stage, cudaEventDisableTiming)) != cudaSuccess) {
+    ermod_destroy(c);
+    return fail_cuda(err, "staging allocation");
+  }
   DevStatus s0{kNoError, kNoError, 0, 0};
   cudaMemcpy(e.d_status, &s0, sizeof(s0), cudaMemcpyHostToDevice);
   *e.h_status = s0;
@@ -566,6 +593,9 @@ int ermod_destroy(ermod_ctx* c) {
   dfree(e.d_twiddle64);
   dfree(e.d_status);
   if (e.h_status) cudaFreeHost(e.h_status);
+  if (e.h_stage) cudaFreeHost(e.h_stage);
+  if (e.ev_stage) cudaEventDestroy(e.ev_stage);
+  dfree(e.d_out);
   for (cufftHandle p : e.plan_z2d)
     if (p) cufftDestroy(p);
   harvest(e);
@@ -819,16 +849,20 @@ int ermod_set_bins(ermod_ctx* c, int numslv, const int* uvmax, const int* uvsoft
   ERMOD_CUDA(cudaMemcpy(e.d_uvkey_f, ukf.data(), sizeof(int) * ermax, cudaMemcpyHostToDevice));
   ERMOD_CUDA(cudaMemcpy(e.d_eskey, ek.data(), sizeof(long long) * ek.size(), cudaMemcpyHostToDevice));
   ERMOD_CUDA(cudaMemcpy(e.d_spec, spec.data(), sizeof(int) * spec.size(), cudaMemcpyHostToDevice));
-  ERMOD_CUDA(dalloc(&e.d_edens, ermax));
+  const size_t nes = (size_t)std::max(esmax, 1);
+  e.n_accum = ermax + nes + numslv + 8 + 2 * ((size_t)numslv + 1);
+  ERMOD_CUDA(dalloc(&e.d_accum, e.n_accum));
+  ERMOD_CUDA(cudaMallocHost(&e.h_accum, sizeof(double) * e.n_accum));
+  e.d_edens = e.d_accum;
+  e.d_eself = e.d_edens + ermax;
+  e.d_slnuv = e.d_eself + nes;
+  e.d_scal = e.d_slnuv + numslv;
+  e.d_minuv = e.d_scal + 8;
+  e.d_maxuv = e.d_minuv + numslv + 1;
   if (e.P.corrcal) {
     ERMOD_CUDA(dalloc(&e.d_ecorr, (size_t)ermax * ermax));
     if (e.P.count_mirror) ERMOD_CUDA(dalloc(&e.d_ecorr_n, (size_t)ermax * ermax));
   }
-  ERMOD_CUDA(dalloc(&e.d_eself, std::max(esmax, 1)));
-  ERMOD_CUDA(dalloc(&e.d_slnuv, numslv));
-  ERMOD_CUDA(dalloc(&e.d_minuv, numslv + 1));
-  ERMOD_CUDA(dalloc(&e.d_maxuv, numslv + 1));
-  ERMOD_CUDA(dalloc(&e.d_scal, 8));
   // enginit's initial values (engproc.F90:255-260): minuv = infty, maxuv = -infty, voffset = -infty
   std::vector<double> mn(numslv + 1, 1.0e50), mx(numslv + 1, -1.0e50);
   ERMOD_CUDA(cudaMemcpy(e.d_minuv, mn.data(), sizeof(double) * (numslv + 1), cudaMemcpyHostToDevice));
@@ -940,10 +974,21 @@ int ermod_frame(ermod_ctx* c, const double* sitepos, const double* cell, double 
   }
   int st = frame_common(e, cell, sws, extent);
   if (st) return st;
-  ERMOD_CUDA(cudaMemcpyAsync(e.d_sitepos, sitepos, sizeof(double) * 3 * e.numatm, cudaMemcpyHostToDevice, e.stream));
+  // a small frame goes through pinned memory, so that the caller's array is free at once and the
+  // placements are queued while the frame is prepared; a large one is copied from the caller's
+  // array and waited for (the second copy on the host would cost more than the overlap gives)
+  const size_t bytes = sizeof(double) * 3 * (size_t)e.numatm;
+  const bool staged = bytes <= kStageBytes;
+  if (staged) {
+    ERMOD_CUDA(cudaEventSynchronize(e.ev_stage));
+    std::memcpy(e.h_stage, sitepos, bytes);
+  }
+  ERMOD_CUDA(cudaMemcpyAsync(e.d_sitepos, staged ? (const void*)e.h_stage : sitepos, bytes, cudaMemcpyHostToDevice,
+                             e.stream));
+  if (staged) ERMOD_CUDA(cudaEventRecord(e.ev_stage, e.stream));
   st = frame_launch(e);
   if (st) return st;
-  ERMOD_CUDA(cudaStreamSynchronize(e.stream));
+  if (!staged) ERMOD_CUDA(cudaStreamSynchronize(e.stream));
   return ERMOD_OK;
 }
 
@@ -1252,23 +1297,44 @@ int ermod_placements(ermod_ctx* c, int nplace, const int* tagslt, const double* 
                                e.stream));
   if (sws) ERMOD_CUDA(cudaMemcpyAsync(e.d_sws, sws, sizeof(double) * nplace, cudaMemcpyHostToDevice, e.stream));
   e.phase_end();
-  double* d_uv = nullptr;
-  double* d_fl = nullptr;
-  if (uv_out) ERMOD_CUDA(dalloc(&d_uv, (size_t)nplace * (e.slvmax + 1)));
-  if (fl_out) ERMOD_CUDA(dalloc(&d_fl, (size_t)nplace * e.numslv));
+  // device outputs: a workspace kept up to kOutKept doubles (an allocation and its release took
+  // 40 us of a small call), larger ones for the call alone
+  const size_t n_uv = uv_out ? (size_t)nplace * (e.slvmax + 1) : 0, n_fl = fl_out ? (size_t)nplace * e.numslv : 0;
+  const size_t n_out = n_uv + n_fl;
+  double* d_tmp = nullptr;
+  if (n_out > kOutKept) {
+    ERMOD_CUDA(dalloc(&d_tmp, n_out));
+  } else if (n_out > e.cap_out) {
+    dfree(e.d_out);
+    e.cap_out = 0;
+    ERMOD_CUDA(dalloc(&e.d_out, n_out));
+    e.cap_out = n_out;
+  }
+  double* d_uv = d_tmp ? d_tmp : e.d_out;
+  double* d_fl = d_uv + n_uv;
   st = reset_status(e);
-  if (!st) st = run_placements(e, nplace, e.d_tagslt, sol ? e.d_solxyz : nullptr, sws ? e.d_sws : nullptr, d_uv, d_fl, ns);
-  if (!st) {
-    if (uv_out)
-      st = cudaMemcpyAsync(uv_out, d_uv, sizeof(double) * (size_t)nplace * (e.slvmax + 1), cudaMemcpyDeviceToHost,
-                           e.stream) == cudaSuccess ? ERMOD_OK : ERMOD_E_CUDA;
-    if (fl_out && !st)
-      st = cudaMemcpyAsync(fl_out, d_fl, sizeof(double) * (size_t)nplace * e.numslv, cudaMemcpyDeviceToHost,
-                           e.stream) == cudaSuccess ? ERMOD_OK : ERMOD_E_CUDA;
+  if (!st)
+    st = run_placements(e, nplace, e.d_tagslt, sol ? e.d_solxyz : nullptr, sws ? e.d_sws : nullptr,
+                        uv_out ? d_uv : nullptr, fl_out ? d_fl : nullptr, ns);
+  const bool staged = sizeof(double) * n_out <= kStageBytes;
+  char* stage = e.h_stage + kStageBytes;
+  if (!st && n_out > 0) {
+    cudaError_t err = cudaSuccess;
+    if (staged) {
+      err = cudaMemcpyAsync(stage, d_uv, sizeof(double) * n_out, cudaMemcpyDeviceToHost, e.stream);
+    } else {
+      if (uv_out) err = cudaMemcpyAsync(uv_out, d_uv, sizeof(double) * n_uv, cudaMemcpyDeviceToHost, e.stream);
+      if (fl_out && err == cudaSuccess)
+        err = cudaMemcpyAsync(fl_out, d_fl, sizeof(double) * n_fl, cudaMemcpyDeviceToHost, e.stream);
+    }
+    if (err != cudaSuccess) st = fail_cuda(err, "outputs");
   }
   const int st2 = ermod_sync(c);
-  if (d_uv) cudaFree(d_uv);
-  if (d_fl) cudaFree(d_fl);
+  if (!st && staged) {
+    if (uv_out) std::memcpy(uv_out, stage, sizeof(double) * n_uv);
+    if (fl_out) std::memcpy(fl_out, stage + sizeof(double) * n_uv, sizeof(double) * n_fl);
+  }
+  dfree(d_tmp);
   return st ? st : st2;
 }
 
@@ -1277,13 +1343,11 @@ int ermod_clear(ermod_ctx* c) {  // engclear (engproc.F90:276-288)
   Engine& e = c->e;
   if (!e.bins_ready) return fail_param("ermod_set_bins must come first");
   cudaSetDevice(e.device);
-  ERMOD_CUDA(cudaMemsetAsync(e.d_edens, 0, sizeof(double) * e.ermax, e.stream));
+  // edens, eself, slnuv and engnorm, engsmpl, avslf
+  ERMOD_CUDA(cudaMemsetAsync(e.d_accum, 0, sizeof(double) * (size_t)(e.d_scal + 3 - e.d_accum), e.stream));
   if (e.d_ecorr) ERMOD_CUDA(cudaMemsetAsync(e.d_ecorr, 0, sizeof(double) * (size_t)e.ermax * e.ermax, e.stream));
   if (e.d_ecorr_n)
     ERMOD_CUDA(cudaMemsetAsync(e.d_ecorr_n, 0, sizeof(long long) * (size_t)e.ermax * e.ermax, e.stream));
-  ERMOD_CUDA(cudaMemsetAsync(e.d_eself, 0, sizeof(double) * std::max(e.esmax, 1), e.stream));
-  ERMOD_CUDA(cudaMemsetAsync(e.d_slnuv, 0, sizeof(double) * e.numslv, e.stream));
-  ERMOD_CUDA(cudaMemsetAsync(e.d_scal, 0, sizeof(double) * 3, e.stream));  // engnorm, engsmpl, avslf
   if (e.d_edintm)  // engclear's hunk of the intermediate-state extension
     ERMOD_CUDA(cudaMemsetAsync(e.d_edintm, 0, sizeof(double) * ((size_t)e.ermax + e.numslv + 3), e.stream));
   if (e.adj_on) {
@@ -1593,27 +1657,31 @@ int ermod_get_accum(ermod_ctx* c, double* edens, double* ecorr, double* eself, d
   if (!c) return fail_param("null context");
   Engine& e = c->e;
   if (!e.bins_ready) return fail_param("ermod_set_bins must come first");
+  if (ecorr && !e.d_ecorr) return fail_param("corrcal is off");
+  if (ecorr_count && !e.d_ecorr_n) return fail_param("count_mirror is off");
   cudaSetDevice(e.device);
+  // the small accumulators by one copy into pinned memory (one copy each, waited for, took 72 us)
+  ERMOD_CUDA(cudaMemcpyAsync(e.h_accum, e.d_accum, sizeof(double) * e.n_accum, cudaMemcpyDeviceToHost, e.stream));
   ERMOD_CUDA(cudaStreamSynchronize(e.stream));
   const size_t E = e.ermax;
-  if (edens) ERMOD_CUDA(cudaMemcpy(edens, e.d_edens, sizeof(double) * E, cudaMemcpyDeviceToHost));
   if (ecorr) {
-    if (!e.d_ecorr) return fail_param("corrcal is off");
+    touch_pages(ecorr, sizeof(double) * E * E);
     ERMOD_CUDA(cudaMemcpy(ecorr, e.d_ecorr, sizeof(double) * E * E, cudaMemcpyDeviceToHost));
   }
   if (ecorr_count) {
-    if (!e.d_ecorr_n) return fail_param("count_mirror is off");
+    touch_pages(ecorr_count, sizeof(long long) * E * E);
     ERMOD_CUDA(cudaMemcpy(ecorr_count, e.d_ecorr_n, sizeof(long long) * E * E, cudaMemcpyDeviceToHost));
   }
-  if (eself && e.esmax > 0) ERMOD_CUDA(cudaMemcpy(eself, e.d_eself, sizeof(double) * e.esmax, cudaMemcpyDeviceToHost));
-  if (slnuv) ERMOD_CUDA(cudaMemcpy(slnuv, e.d_slnuv, sizeof(double) * e.numslv, cudaMemcpyDeviceToHost));
-  if (minuv) ERMOD_CUDA(cudaMemcpy(minuv, e.d_minuv, sizeof(double) * (e.numslv + 1), cudaMemcpyDeviceToHost));
-  if (maxuv) ERMOD_CUDA(cudaMemcpy(maxuv, e.d_maxuv, sizeof(double) * (e.numslv + 1), cudaMemcpyDeviceToHost));
-  if (scalars) {
-    double s[8];
-    ERMOD_CUDA(cudaMemcpy(s, e.d_scal, sizeof(s), cudaMemcpyDeviceToHost));
-    for (int i = 0; i < 5; ++i) scalars[i] = s[i];
-  }
+  const double* h = e.h_accum;
+  auto out = [&](double* to, const double* d, size_t n) {
+    if (to) std::memcpy(to, h + (d - e.d_accum), sizeof(double) * n);
+  };
+  out(edens, e.d_edens, E);
+  out(eself, e.d_eself, e.esmax);
+  out(slnuv, e.d_slnuv, e.numslv);
+  out(minuv, e.d_minuv, e.numslv + 1);
+  out(maxuv, e.d_maxuv, e.numslv + 1);
+  out(scalars, e.d_scal, 5);
   return ERMOD_OK;
 }
 

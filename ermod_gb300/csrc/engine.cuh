@@ -70,6 +70,11 @@ struct Engine {
   int* d_spec = nullptr;         // [numslv][3] {uvoff, uvmax, uvsoft}
 
   // ---- accumulators ----------------------------------------------------------------
+  // d_edens, d_eself, d_slnuv, d_scal, d_minuv, d_maxuv lie in one block in this order, which
+  // is cleared by one memset and read back by one copy into h_accum
+  double* d_accum = nullptr;
+  double* h_accum = nullptr;  // pinned
+  size_t n_accum = 0;
   double* d_edens = nullptr;
   double* d_ecorr = nullptr;
   long long* d_ecorr_n = nullptr;
@@ -124,6 +129,12 @@ struct Engine {
   double* d_solxyz = nullptr;     // [cap_place][S][3]
   double* d_sws = nullptr;        // [cap_place]
   int cap_place = 0;
+  double* d_out = nullptr;        // [cap_out] uvengy and flceng of a host call
+  size_t cap_out = 0;
+  // pinned staging of a host call's small transfers: a frame's coordinates in the first
+  // kStageBytes, results in the second.  ev_stage: the last coordinate copy has left it
+  char* h_stage = nullptr;
+  cudaEvent_t ev_stage = nullptr;
   BatchArgs buf{};                // device buffers sized for Bmax (pointers only)
   // histogram ring for ecorr (corrcal) / per-batch histograms
   // histogram ring of the ecorr flush: two halves of ring_half entries; batches fill the

@@ -40,6 +40,10 @@ constexpr int kBatchStreams = 2;
 // 256^3 on, as before batching)
 constexpr int kFp64MaxLog2 = 6;
 constexpr size_t kFp64GridBytes = (size_t)256 << 20;
+// host API: transfers up to this size go through pinned staging; device outputs kept up to
+// this many doubles (64 MB)
+constexpr size_t kStageBytes = (size_t)256 << 10;
+constexpr size_t kOutKept = (size_t)8 << 20;
 constexpr int kMaxSpecies = 16;
 constexpr int kGridBits = 10;         // packed grid coordinates: K <= 1024 per axis
 constexpr double kPi = 3.1415926535897932;

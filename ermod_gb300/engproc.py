@@ -175,8 +175,8 @@ class EnergyRepresentation:
     def accum(self, with_count: bool = False):
         E, S, N = self.ermax, self.esmax, self.numslv
         edens = np.zeros(E)
-        ecorr = np.zeros(E * E) if self.params.get("corrcal") else None
-        cnt = np.zeros(E * E, np.int64) if with_count else None
+        ecorr = np.empty(E * E) if self.params.get("corrcal") else None  # written whole
+        cnt = np.empty(E * E, np.int64) if with_count else None
         eself = np.zeros(max(S, 1))
         slnuv = np.zeros(N)
         mn, mx = np.zeros(N + 1), np.zeros(N + 1)
