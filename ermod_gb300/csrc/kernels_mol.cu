@@ -556,13 +556,14 @@ __global__ void __launch_bounds__(kMol64Threads) mol_energy_kernel(MolArgs A) {
 // ---- TMA + mbarrier helpers (inline PTX, sm_90+ forms, valid on sm_103a) -------------
 
 // Mixed path, step 1 -- gather by bricks.  CTA per (kBrickX x kBrickY x kBrickZ brick of the
-// PME grid, run of placement groups of 4).  One 5-D TMA box copy per group brings the
+// PME grid, run of placement groups of 4).  One TMA box copy per group brings the
 // brick's stencil halo of the group's interleaved potential grids into shared memory as
 // [z][y][x][4], in kGatherStages buffers so that the next groups' copies are in flight
 // while this one is used; each thread takes a site of the brick (its B-spline weights
 // computed once for all groups, FP32 stable recursion) and accumulates
 // q theta theta theta phi for the four placements with one 16-byte shared load per
-// stencil point.
+// stencil point.  Bound by those loads (66% of the shared-memory wavefronts, a launch of 256
+// placements at 96^3 in 340 us); 160-thread CTAs, three to an SM, measured 2% slower.
 constexpr int kGatherThreads = 256;
 constexpr int kGatherStages = 2;  // halo buffers (TMA copies in flight) per gather CTA
 
@@ -636,13 +637,12 @@ __global__ void __launch_bounds__(kGatherThreads) gather_tma_kernel(
   }
   __syncthreads();
   // padded coordinates: the halo of brick (bx, by, bz) starts at (kBrickX bx,
-  // kBrickY by, kBrickZ bz); the innermost box coordinate (the placement within the
-  // group) is 0
+  // kBrickY by, kBrickZ bz), four floats (the group's placements) per x
   if (threadIdx.x == 0) {
     for (int g = g_begin; g < min(g_end, g_begin + kGatherStages); ++g) {
       const int st = g - g_begin;
       mbar_expect_tx(&bar[st], box_bytes);
-      tma_load_5d(halo_base + (size_t)st * hstride, &tmap, 0, bx * kBrickX, by * kBrickY, bz * kBrickZ, g, &bar[st]);
+      tma_load_4d(halo_base + (size_t)st * hstride, &tmap, 4 * bx * kBrickX, by * kBrickY, bz * kBrickZ, g, &bar[st]);
     }
   }
   const int h = P - 1;
@@ -730,8 +730,8 @@ __global__ void __launch_bounds__(kGatherThreads) gather_tma_kernel(
     if (threadIdx.x == 0 && g + kGatherStages < g_end) {
       fence_proxy_async_smem();
       mbar_expect_tx(&bar[slot], box_bytes);
-      tma_load_5d(halo_base + (size_t)slot * hstride, &tmap, 0, bx * kBrickX, by * kBrickY, bz * kBrickZ, g + kGatherStages,
-                  &bar[slot]);
+      tma_load_4d(halo_base + (size_t)slot * hstride, &tmap, 4 * bx * kBrickX, by * kBrickY, bz * kBrickZ,
+                  g + kGatherStages, &bar[slot]);
     }
   }
 }
@@ -1205,7 +1205,10 @@ static MolArgs make_mol_args(Engine& e, const BatchArgs& a) {
 cudaError_t launch_gather(Engine& e, const BatchArgs& a) {
   cudaError_t err = cudaSuccess;
   const int ngroups = (a.nb + 3) / 4;
-  const int gpc = std::min(ngroups, 8);
+  // groups per CTA: 16 (site set-up and the first copies' latency paid once for them), 8 where 16
+  // would leave fewer than four rounds of the two CTAs an SM holds
+  int gpc = std::min(ngroups, 16);
+  if ((long long)e.nbricks * ((ngroups + gpc - 1) / gpc) < 8LL * e.num_sm) gpc = std::min(ngroups, 8);
   dim3 g1(e.nbricks, (ngroups + gpc - 1) / gpc);
   const int K1 = e.geom.K[0], K2 = e.geom.K[1], K3 = e.geom.K[2];
   const size_t npt = (size_t)e.gbox[0] * e.gbox[1] * e.gbox[2];
