@@ -696,13 +696,11 @@ int ermod_set_topology(ermod_ctx* c, int nummol, int numatm, const int* mbi, con
   std::vector<int> mol_to_k(nummol, -1);
   e.total_charge_phys = 0.0;
   e.max_mol_sites = 0;
-  e.max_solute_sites = 0;
   for (int i = 0; i < nummol; ++i) {
     e.numsite[i] = e.mbi0[i + 1] - e.mbi0[i];
     double s = 0.0;  // mol_charge (setconf.F90:832-834)
     for (int a = e.mbi0[i]; a < e.mbi0[i + 1]; ++a) s += charge[a];
     e.mol_charge[i] = s;
-    if (sluvid[i] != 0) e.max_solute_sites = std::max(e.max_solute_sites, e.numsite[i]);
     if (sluvid[i] == 0 || sluvid[i] == 1) {  // tagpt (engproc.F90:336-348)
       mol_to_k[i] = (int)e.tagpt.size();
       e.tagpt.push_back(i);

@@ -68,7 +68,8 @@ struct MolArgs {
   float fxf[3];    // fixed-point unit per axis (box length / 2^32)
   float screen_f;  // Ewald beta
   float rc_f;      // max(elecut, upljcut)
-  int real_lanes;  // finish kernel: threads sharing a near molecule's solute sites
+  float fx_scale_f;  // finish kernel: 2^bits of the fixed-point sums of FP32 pair terms
+  float reach2_f;    // finish kernel: the larger squared cutoff of LJ and Coulomb
   int bare;        // cltype 0: bare Coulomb within elecut (no cutoff when non-periodic), no reciprocal space
                    // or residual
   LjK k32;         // LJ switching constants
@@ -293,15 +294,21 @@ __device__ __forceinline__ double pair_fp64(const MolArgs& A, int idx, const dou
   return e;
 }
 
-// The finish kernel's FP64 pairs (see mol_finish_kernel): recorded per thread and window of its
-// real-space pass, and gathered in the block's list until it is full or the pass ends
-constexpr int kBigPerThread = 8;
+// ---- the finish kernel's real-space pass -------------------------------------------------
+// Its FP64 pairs are gathered in a list per block; more than that many and each item's thread
+// finds its own again.
 constexpr int kBigList = 1024;
-// that pass's scratch (ints): the list (pairs, their near items as 16 bits, their values), the
-// threads' recorded pairs, the molecules' first sites, and the list of near (molecule,
-// placement) items (16 bits)
+// a pair: near item (11 bits: at most 8 placements of 256 molecules), solute site (8 bits), site
+// of the solvent molecule (13 bits)
+__device__ __forceinline__ unsigned pair_key(int near, int su, int s) {
+  return ((unsigned)near << 21) | ((unsigned)su << 13) | (unsigned)s;
+}
+constexpr int kPairQueue = 64;  // pairs within the cutoffs waiting in a warp's queue: at most 31 + 32
+// the pass's scratch (ints): the list (values, pairs, their order as 16 bits, their FP64 parts as
+// bytes), the warps' queues, the fixed-point sums of the near items, the molecules' first
+// sites, and the list of near (molecule, placement) items (16 bits)
 __host__ __device__ constexpr int finish_scratch_ints(int G) {  // for the larger tile, 256
-  return kBigList + kBigList / 2 + 2 * kBigList + 256 * kBigPerThread + 256 + G * 256 / 2;
+  return 2 * kBigList + kBigList + kBigList / 2 + kBigList / 4 + 8 * kPairQueue + 2 * 256 * G + 256 + G * 256 / 2;
 }
 // the dynamic shared memory of the finish kernel before its edge keys: the block
 // histograms (when in shared memory) or the real-space pass's scratch, whichever is larger
@@ -309,83 +316,50 @@ __host__ __device__ __forceinline__ int finish_region_ints(int G, int ermax, int
   const int h = hist_global ? 0 : G * ermax;
   return h > finish_scratch_ints(G) ? h : finish_scratch_ints(G);
 }
-// a recorded pair: its FP64 parts (2 bits), solute site (8 bits), site of the solvent
-// molecule (13 bits)
-__device__ __forceinline__ int big_item(int parts, int su, int s) { return (parts << 21) | (su << 13) | s; }
 
-constexpr int kMolSiteCache = 3;  // molecule sites held in registers by the real-space pass
+__device__ __forceinline__ float pair_r2(const MolArgs& A, const int4& vp, const int4& up) {
+  const float ex = (float)(int)((unsigned)vp.x - (unsigned)up.x) * A.fxf[0];
+  const float ey = (float)(int)((unsigned)vp.y - (unsigned)up.y) * A.fxf[1];
+  const float ez = (float)(int)((unsigned)vp.z - (unsigned)up.z) * A.fxf[2];
+  return ex * ex + ey * ey + ez * ez;
+}
 
-// real-space LJ + screened Coulomb of one molecule against solute b's sites su0, su0 + L, ..
-// (mixed path): fixed-point displacements and FP32 pair terms, summed as a float-float
-// number.  An FP32 LJ or Coulomb term above kFp64Lj / kFp64Coulomb in magnitude (or not
-// finite) is left out of the sum and counted in nbig (in the thread's scan order); the count's
-// values in [win, win + kBigPerThread) are recorded with their parts in items[count - win].
-// (A thread with more pairs than one window takes calls again for the next ones.)
-__device__ __forceinline__ ff real_mixed(const MolArgs& A, const BatchArgs& a, int b, int s0, int ns, int su0, int L,
-                                         int* items, int win, int& nbig) {
+// the FP32 terms of one pair at squared distance r2: LJ (0 beyond its cutoff) and screened or
+// bare Coulomb; returns the parts too large for FP32 (above kFp64Lj / kFp64Coulomb in
+// magnitude, or not finite: the comparisons are false for NaN and inf)
+__device__ __forceinline__ int pair_fp32(const MolArgs& A, const int4& vp, const int4& up, float qu, float qv, float r2,
+                                         float& elj, float& eco) {
   const LjK& k32 = A.k32;
-  const size_t ub = (size_t)b * kMaxSoluteSites;
-  const float fx = A.fxf[0], fy = A.fxf[1], fz = A.fxf[2];
-  ff real{0.f, 0.f};
-  const int nu = a.u_nsite[b];
-  const float beta = A.screen_f;
-  // one pair (solute site su at up with charge qu, molecule site s at vp with charge qv)
-  auto pair = [&](int su, const int4& up, float qu, int s, const int4& vp, float qv) {
-    const float ex = (float)(int)((unsigned)vp.x - (unsigned)up.x) * fx;
-    const float ey = (float)(int)((unsigned)vp.y - (unsigned)up.y) * fy;
-    const float ez = (float)(int)((unsigned)vp.z - (unsigned)up.z) * fz;
-    const float r2 = ex * ex + ey * ey + ez * ez;
-    float elj = 0.f, eco = 0.f;
-    const float ljeps = A.ljene_f[vp.w + A.T * up.w];
-    if (ljeps > 0.f) {
-      const float sg2 = A.ljlensq_f[vp.w + A.T * up.w];
-      if (r2 <= k32.lw2)
-        elj = lj_low<float>(A.ljswitch, k32, ljeps, sg2, r2);
-      else if (r2 <= k32.up2)
-        elj = lj_switch<float>(A.ljswitch, k32, ljeps, sg2, r2);
-    }
-    if (A.bare) {
-      if (r2 < k32.ele2) eco = qu * qv / sqrtf(r2);  // realcal_bare
-    } else if (r2 <= k32.ele2) {
-      const float r = sqrtf(r2);
-      eco = qu * qv * erfcf(beta * r) / r;
-    }
-    // parts too large for FP32 (the comparisons are false for NaN and inf)
-    const int parts = (fabsf(elj) <= kFp64Lj ? 0 : kPairLj) | (fabsf(eco) <= kFp64Coulomb ? 0 : kPairCoulomb);
-    if (!(parts & kPairLj)) real = ff_add(real, elj);
-    if (!(parts & kPairCoulomb)) real = ff_add(real, eco);
-    if (parts) {
-      const int r = nbig - win;
-      if (r >= 0 && r < kBigPerThread) items[r] = big_item(parts, su, s);
-      ++nbig;
-    }
-  };
-  if (ns <= kMolSiteCache) {
-    // small molecules (water): their sites' positions and charges held in registers for
-    // every solute site
-    int4 vpc[kMolSiteCache];
-    float qvc[kMolSiteCache];
-#pragma unroll
-    for (int s = 0; s < kMolSiteCache; ++s)
-      if (s < ns) {
-        vpc[s] = A.site_pos[s0 + s];
-        qvc[s] = A.site_rec[s0 + s].w;
-      }
-    for (int su = su0; su < nu; su += L) {
-      const int4 up = a.u_pos[ub + su];
-      const float qu = a.u_qf[ub + su];
-#pragma unroll
-      for (int s = 0; s < kMolSiteCache; ++s)
-        if (s < ns) pair(su, up, qu, s, vpc[s], qvc[s]);
-    }
-  } else {
-    for (int su = su0; su < nu; su += L) {
-      const int4 up = a.u_pos[ub + su];
-      const float qu = a.u_qf[ub + su];
-      for (int s = 0; s < ns; ++s) pair(su, up, qu, s, A.site_pos[s0 + s], A.site_rec[s0 + s].w);
-    }
+  elj = 0.f;
+  eco = 0.f;
+  const float ljeps = A.ljene_f[vp.w + A.T * up.w];
+  if (ljeps > 0.f) {
+    const float sg2 = A.ljlensq_f[vp.w + A.T * up.w];
+    if (r2 <= k32.lw2)
+      elj = lj_low<float>(A.ljswitch, k32, ljeps, sg2, r2);
+    else if (r2 <= k32.up2)
+      elj = lj_switch<float>(A.ljswitch, k32, ljeps, sg2, r2);
   }
-  return real;
+  if (A.bare) {
+    if (r2 < k32.ele2) eco = qu * qv / sqrtf(r2);  // realcal_bare
+  } else if (r2 <= k32.ele2) {
+    const float r = sqrtf(r2);
+    eco = qu * qv * erfcf(A.screen_f * r) / r;
+  }
+  return (fabsf(elj) <= kFp64Lj ? 0 : kPairLj) | (fabsf(eco) <= kFp64Coulomb ? 0 : kPairCoulomb);
+}
+
+// Sums of FP32 terms as 64-bit integers of 2^-A.fx_bits kcal/mol (2^-44 unless the molecules'
+// pairs could overflow it: no term is above 16): exact additions, so that the sum does not
+// depend on the order in which a block's threads add.  Two words, the low one's carry passed on.
+__device__ __forceinline__ void fixed_add(unsigned* lo, unsigned* hi, long long v) {
+  const unsigned l = (unsigned)v, old = atomicAdd(lo, l);
+  atomicAdd(hi, (unsigned)((unsigned long long)v >> 32) + (old + l < old ? 1u : 0u));
+}
+__device__ __forceinline__ ff fixed_to_ff(unsigned lo, unsigned hi, float unit) {
+  const long long v = (long long)(((unsigned long long)hi << 32) | lo);
+  const float h = __ll2float_rn(v);
+  return ff{h * unit, __ll2float_rn(v - __float2ll_rn(h)) * unit};
 }
 
 constexpr long long kKeyPosInf = 0x7ff0000000000000ll;
@@ -804,16 +778,19 @@ __device__ __forceinline__ void species_partials(const MolArgs& A, const BatchAr
 // exactly against the FP64 edges), histograms and per-species partials.
 //
 // The real-space pass: the block's (molecule, placement) items within the solute's bounding
-// sphere + cutoff are compacted into a list, and A.real_lanes threads (a power of two, set by
-// the solutes' sizes alone) share an item's solute sites, their float-float sums joined in a
-// fixed tree.  So a warp's lanes all have pairs to evaluate (2% of the 33,000-water box's
-// molecules lie in reach), a large solute's pairs are not one thread's serial chain, and an
-// item's sum does not depend on the block it falls in.
+// sphere + cutoff are compacted into a list (2% of the 33,000-water box's molecules); a thread
+// takes an item and a solute site, and the pairs within the cutoffs -- a fifth of the tested
+// ones for a 36-site solute -- go through a queue per warp, so that the evaluation, ten times
+// as long as the test, runs on full warps.  Its terms are added as fixed-point integers, in
+// any order.  (A few threads per item, each walking its pairs: 19 of 32 lanes active and four
+// times the instructions, 438 us for 256 insertions of a 36-site solute into 2,000 waters,
+// now 280; 12 sites into 33,000 waters 340, now 314.)
 //
+// Four blocks per SM (64 registers): 2-3% faster over a whole run than three of 80.
 // TILE: molecules per block of 256 threads.  64 in solution mode, where a frame's one placement
 // makes few blocks and the real-space pass takes all 256 threads.
 template <int G, int TILE>
-__global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const float* __restrict__ site_e) {
+__global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const float* __restrict__ site_e) {
   extern __shared__ __align__(16) int smem_dyn[];
   // [G][ermax] block histograms, or none when they would not fit beside other blocks: the
   // molecules' counts then go to the batch histograms in global memory (warp-aggregated).
@@ -821,13 +798,16 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
   // (finish_scratch_ints ints).
   int* smem_hist = A.hist_global ? nullptr : smem_dyn;
   int* skeys = smem_dyn + finish_region_ints(G, A.ermax, A.hist_global);  // [ermax] 32-bit edge keys
-  double* sval = reinterpret_cast<double*>(smem_dyn);                        // [kBigList] FP64 values of the list
-  int* sbig = reinterpret_cast<int*>(sval + kBigList);                       // [kBigList] the list's pairs
-  unsigned short* sbnear = reinterpret_cast<unsigned short*>(sbig + kBigList);  // [kBigList] their near items
-  int* sitem = reinterpret_cast<int*>(sbnear + kBigList);                   // [256][kBigPerThread]
-  int* ss0 = sitem + 256 * kBigPerThread;                                   // [256] first sites
-  unsigned short* snear = reinterpret_cast<unsigned short*>(ss0 + 256);     // [G * 256] molecule | placement << 8
+  double* sval = reinterpret_cast<double*>(smem_dyn);                           // [kBigList] FP64 values of the list
+  unsigned* sbig = reinterpret_cast<unsigned*>(sval + kBigList);                // [kBigList] the list's pairs
+  unsigned short* sorder = reinterpret_cast<unsigned short*>(sbig + kBigList);  // [kBigList] in the pairs' order
+  unsigned char* sparts = reinterpret_cast<unsigned char*>(sorder + kBigList);  // [kBigList] the parts left out
+  unsigned* squeue = reinterpret_cast<unsigned*>(sparts + kBigList);            // [8][kPairQueue]
+  unsigned* sfix = squeue + 8 * kPairQueue;                                     // [2][G * 256] sums, low and high words
+  int* ss0 = reinterpret_cast<int*>(sfix + 2 * 256 * G);                        // [256] first sites
+  unsigned short* snear = reinterpret_cast<unsigned short*>(ss0 + 256);         // [G * 256] molecule | placement << 8
   __shared__ int swarp[8];
+  __shared__ int snlist, snu;    // pairs in the FP64 list; the placements' most solute sites
   __shared__ float su[G][TILE];   // totals, hi part (NaN: no molecule)
   __shared__ float sul[G][TILE];  // totals, lo part
   __shared__ float sres[G];      // residual factor x solute charge of the G placements
@@ -943,94 +923,122 @@ __global__ void __launch_bounds__(256, 3) mol_finish_kernel(MolArgs A, const flo
       nnear += swarp[w2];
     }
     for (unsigned q = nearm; q; q &= q - 1) snear[near0++] = (unsigned short)(threadIdx.x | ((__ffs(q) - 1) << 8));
-    __syncthreads();
-  }
-  // FP64 pass over the listed pair parts (overlapping pairs, left out of the FP32 sums): one
-  // per thread, so that every FP64 instruction runs on full warps; the first pair of each item
-  // then adds the item's values, which lie side by side, in their order
-  int nlist = 0;  // block-uniform
-  auto add_listed = [&] {
-    __syncthreads();
-    for (int q = threadIdx.x; q < nlist; q += 256) {
-      const int it = sbig[q], nr = snear[sbnear[q]];
-      const size_t us = (size_t)(g0 + (nr >> 8)) * kMaxSoluteSites + ((it >> 13) & 0xff);
-      sval[q] = pair_fp64(A, ss0[nr & 0xff] + (it & 0x1fff), a.u_x + us * 3, a.u_q[us], a.u_pos[us].w, it >> 21);
+    for (int i = threadIdx.x; i < nnear; i += 256) sfix[i] = sfix[256 * G + i] = 0u;
+    if (threadIdx.x == 0) {
+      snlist = 0;
+      snu = 0;
+      for (int j = 0; j < ng; ++j) snu = max(snu, a.u_nsite[g0 + j]);
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < nlist; q += 256) {
-      const int near = sbnear[q];
-      if (q > 0 && sbnear[q - 1] == near) continue;
+  }
+  if (nnear > 0) {  // block-uniform
+    const int nu_max = snu;
+    const unsigned magic = nu_max > 1 ? (unsigned)((0x100000000ull + nu_max - 1) / nu_max) : 0u;
+    const float scale = A.fx_scale_f, reach2 = A.reach2_f;
+    unsigned* queue = squeue + wid * kPairQueue;
+    int nq = 0;  // warp-uniform
+    // the last n pairs of the warp's queue, one per lane
+    auto evaluate = [&](int n) {
+      __syncwarp();
+      if (lane < n) {
+        const unsigned key = queue[nq - n + lane];
+        const int near = key >> 21, su_ = (key >> 13) & 0xff, s = key & 0x1fff;
+        const int nr = snear[near], site = ss0[nr & 0xff] + s;
+        const size_t us = (size_t)(g0 + (nr >> 8)) * kMaxSoluteSites + su_;
+        const int4 vp = A.site_pos[site], up = a.u_pos[us];
+        float elj, eco;
+        const int parts = pair_fp32(A, vp, up, a.u_qf[us], A.site_rec[site].w, pair_r2(A, vp, up), elj, eco);
+        long long v = 0;
+        if (!(parts & kPairLj)) v = __float2ll_rn(elj * scale);
+        if (!(parts & kPairCoulomb)) v += __float2ll_rn(eco * scale);
+        if (v != 0) fixed_add(sfix + near, sfix + 256 * G + near, v);
+        if (parts) {
+          const int q = atomicAdd(&snlist, 1);
+          if (q < kBigList) {
+            sbig[q] = key;
+            sparts[q] = (unsigned char)parts;
+          }
+        }
+      }
+      __syncwarp();
+      nq -= n;
+    };
+    for (int task0 = wid * 32; task0 < nnear * nu_max; task0 += 256) {  // warp-uniform
+      const int task = task0 + lane;
+      const int near = nu_max > 1 ? (int)__umulhi((unsigned)task, magic) : task, su_ = task - near * nu_max;
+      int is0 = 0, ins = 0, b = 0;
+      if (near < nnear) {
+        const int nr = snear[near];
+        b = g0 + (nr >> 8);
+        is0 = ss0[nr & 0xff];
+        if (su_ < a.u_nsite[b]) ins = A.slot_site[tile * TILE + (nr & 0xff) + 1] - is0;
+      }
+      const int4 up = a.u_pos[(size_t)b * kMaxSoluteSites + su_];
+      for (int s = 0; __any_sync(0xffffffffu, s < ins); ++s) {
+        const bool in = s < ins && pair_r2(A, A.site_pos[is0 + s], up) <= reach2;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) queue[nq + __popc(m & ((1u << lane) - 1u))] = pair_key(near, su_, s);
+        nq += __popc(m);
+        if (nq >= 32) evaluate(32);
+      }
+    }
+    if (nq > 0) evaluate(nq);
+    __syncthreads();
+    // FP64 pass over the listed pair parts (overlapping pairs, left out of the FP32 sums): one
+    // per thread, so that every FP64 instruction runs on full warps; an item's values are added
+    // in the order of its pairs (solute site, molecule site), by the thread of the first
+    const int nlist = snlist;
+    if (nlist <= kBigList) {
+      for (int q = threadIdx.x; q < nlist; q += 256) {
+        const unsigned key = sbig[q];
+        int rank = 0;
+        for (int i = 0; i < nlist; ++i) rank += sbig[i] < key ? 1 : 0;
+        sorder[rank] = (unsigned short)q;
+        const int nr = snear[key >> 21];
+        const size_t us = (size_t)(g0 + (nr >> 8)) * kMaxSoluteSites + ((key >> 13) & 0xff);
+        sval[q] = pair_fp64(A, ss0[nr & 0xff] + (int)(key & 0x1fff), a.u_x + us * 3, a.u_q[us], a.u_pos[us].w, sparts[q]);
+      }
+      __syncthreads();
+    }
+    for (int near = threadIdx.x; near < nnear; near += 256) {
       const int t = snear[near] & 0xff, j = snear[near] >> 8;
-      ff x{su[j][t], sul[j][t]};
-      for (int i = q; i < nlist && sbnear[i] == near; ++i) x = ff_add2(x, ff_from_double(sval[i]));
+      const ff r = fixed_to_ff(sfix[near], sfix[256 * G + near], 1.f / scale);
+      const ff x = ff_add2(ff{su[j][t], sul[j][t]}, r);
       su[j][t] = x.hi;
       sul[j][t] = x.lo;
     }
     __syncthreads();
-    nlist = 0;
-  };
-  const int L = A.real_lanes, lg = __ffs(L) - 1;
-  int* items = sitem + threadIdx.x * kBigPerThread;
-  for (int base = 0; base < nnear << lg; base += 256) {  // block-uniform
-    const int task = base + threadIdx.x;
-    const int near = task >> lg, su0 = task & (L - 1);
-    const bool on = near < nnear;
-    int t = 0, j = 0, is0 = 0, ins = 0, nbig = 0;
-    if (on) {
-      t = snear[near] & 0xff;
-      j = snear[near] >> 8;
-      is0 = ss0[t];
-      ins = A.slot_site[tile * TILE + t + 1] - is0;
-    }
-    // a thread with more than kBigPerThread FP64 pairs takes further windows
-    for (int win = 0;; win += kBigPerThread) {
-      if (win == 0 || nbig > win) {
-        ff r{0.f, 0.f};
-        nbig = 0;
-        if (on) r = real_mixed(A, a, g0 + j, is0, ins, su0, L, items, win, nbig);
-        if (win == 0) {
-          for (int o = 1; o < L; o <<= 1) {  // the lower thread's sum plus the upper one's
-            const ff w{__shfl_down_sync(0xffffffffu, r.hi, o), __shfl_down_sync(0xffffffffu, r.lo, o)};
-            if ((su0 & (2 * o - 1)) == 0) r = ff_add2(r, w);
+    if (nlist <= kBigList) {
+      for (int r = threadIdx.x; r < nlist; r += 256) {
+        const unsigned near = sbig[sorder[r]] >> 21;
+        if (r > 0 && sbig[sorder[r - 1]] >> 21 == near) continue;
+        const int t = snear[near] & 0xff, j = snear[near] >> 8;
+        ff x{su[j][t], sul[j][t]};
+        for (int i = r; i < nlist && sbig[sorder[i]] >> 21 == near; ++i) x = ff_add2(x, ff_from_double(sval[sorder[i]]));
+        su[j][t] = x.hi;
+        sul[j][t] = x.lo;
+      }
+    } else {  // more than the list holds: each item's pairs again, in the same order
+      for (int near = threadIdx.x; near < nnear; near += 256) {
+        const int t = snear[near] & 0xff, j = snear[near] >> 8, b = g0 + j;
+        const int is0 = ss0[t], ins = A.slot_site[tile * TILE + t + 1] - is0, nu = a.u_nsite[b];
+        const size_t ub = (size_t)b * kMaxSoluteSites;
+        ff x{su[j][t], sul[j][t]};
+        for (int u = 0; u < nu; ++u)
+          for (int s = 0; s < ins; ++s) {
+            const int4 vp = A.site_pos[is0 + s], up = a.u_pos[ub + u];
+            const float r2 = pair_r2(A, vp, up);
+            if (!(r2 <= reach2)) continue;
+            float elj, eco;
+            const int parts = pair_fp32(A, vp, up, a.u_qf[ub + u], A.site_rec[is0 + s].w, r2, elj, eco);
+            if (parts)
+              x = ff_add2(x, ff_from_double(pair_fp64(A, is0 + s, a.u_x + (ub + u) * 3, a.u_q[ub + u], up.w, parts)));
           }
-          if (on && su0 == 0 && (r.hi != 0.f || r.lo != 0.f)) {
-            const ff v = ff_add2(ff{su[j][t], sul[j][t]}, r);
-            su[j][t] = v.hi;
-            sul[j][t] = v.lo;
-          }
-        }
-      }
-      if (!__syncthreads_or(nbig > win)) break;
-      // the window's pairs to the end of the list (an exclusive scan over the threads, so in the
-      // items' order; a window of kBigList entries or more is passed on in parts)
-      const int cnt = min(max(nbig - win, 0), kBigPerThread);
-      int incl = cnt;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      if (lane == 31) swarp[wid] = incl;
-      __syncthreads();
-      int off = incl - cnt, total = 0;
-      for (int w2 = 0; w2 < 8; ++w2) {
-        if (w2 < wid) off += swarp[w2];
-        total += swarp[w2];
-      }
-      // (an item's later windows would not lie beside its first one)
-      if (win > 0 || nlist + total > kBigList) add_listed();
-      for (int p0 = 0; p0 < total; p0 += kBigList) {
-        if (p0 > 0) add_listed();
-        for (int i = 0; i < cnt; ++i) {
-          const int q = off + i - p0;
-          if (q < 0 || q >= kBigList) continue;
-          sbig[nlist + q] = items[i];
-          sbnear[nlist + q] = (unsigned short)near;
-        }
-        nlist += min(total - p0, kBigList);
+        su[j][t] = x.hi;
+        sul[j][t] = x.lo;
       }
     }
   }
-  if (nlist > 0) add_listed();
   __syncthreads();  // the totals are complete and the scratch is free: the histograms may take the region
   if (!A.hist_global)
     for (int i = threadIdx.x; i < G * A.ermax; i += blockDim.x) smem_hist[i] = 0;
@@ -1184,16 +1192,17 @@ static MolArgs make_mol_args(Engine& e, const BatchArgs& a) {
   A.upljcut = e.P.upljcut;
   A.screen = e.P.screen;
   A.bare = (e.P.cltype == 0) ? 1 : 0;
-  // two to five solute sites a thread; one in the small tiles of solution mode
-  A.real_lanes = e.max_solute_sites <= 2 ? 1 : e.max_solute_sites <= 6 ? 2 : e.max_solute_sites <= 16 ? 4 : 8;
-  if (e.mixed && e.tile < 256)
-    for (A.real_lanes = 1; A.real_lanes < std::min(32, e.max_solute_sites);) A.real_lanes *= 2;
   A.resid_fac = A.bare ? 0.0 : kPi / e.P.screen / e.P.screen / e.geom.volume;
   for (int i = 0; i < 3; ++i) A.fxf[i] = (float)e.geom.fx_scale[i];
   A.screen_f = (float)e.P.screen;
   A.rc_f = (float)std::max(A.elecut, e.P.upljcut);
   A.k64 = make_k64(A);
   A.k32 = to_f32(A.k64);
+  A.reach2_f = std::max(A.k32.up2, A.k32.ele2);
+  // terms of at most 16 = 2^4: 2^(44 + 4) each, 2^15 pairs of a molecule with a solute in 63 bits
+  int fx_bits = 44;
+  for (long long pairs = (long long)e.max_mol_sites * kMaxSoluteSites; pairs > (1 << 15); pairs /= 2) --fx_bits;
+  A.fx_scale_f = std::ldexp(1.f, fx_bits);
   A.a = a;
   A.ntile = e.ntile;
   A.status = e.d_status;
