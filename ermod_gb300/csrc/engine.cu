@@ -169,6 +169,8 @@ static int free_batch(Engine& e) {
   dfree(e.d_ring_hist);
   dfree(e.d_ring_w);
   dfree(e.d_ring_nz);
+  dfree(e.d_ring_act);
+  dfree(e.d_ring_digits);
   dfree(e.d_ring_nnz);
   dfree(e.d_ring_valid);
   dfree(e.d_u0);
@@ -227,7 +229,7 @@ static int free_bins(Engine& e) {
   dfree(e.d_eskey);
   dfree(e.d_spec);
   dfree(e.d_accum);
-  if (e.h_accum) cudaFreeHost(e.h_accum);
+  if (e.h_accum && e.h_accum != e.stage_out()) cudaFreeHost(e.h_accum);
   e.h_accum = nullptr;
   dfree(e.d_ecorr);
   dfree(e.d_ecorr_n);
@@ -328,7 +330,11 @@ static int ensure_batch(Engine& e) {
   ERMOD_CUDA(dalloc(&e.d_ring_w, e.ring_cap));
   ERMOD_CUDA(dalloc(&e.d_ring_nnz, e.ring_cap));
   ERMOD_CUDA(dalloc(&e.d_ring_valid, e.ring_cap));
-  if (e.P.corrcal) ERMOD_CUDA(dalloc(&e.d_ring_nz, (size_t)2 * e.ring_cap * e.ermax));
+  if (e.P.corrcal) {
+    if (!e.mixed) ERMOD_CUDA(dalloc(&e.d_ring_nz, (size_t)2 * e.ring_cap * e.ermax));
+    ERMOD_CUDA(dalloc(&e.d_ring_act, ecorr_scratch_ints(e.ermax)));
+    if (!e.d_ecorr_n) ERMOD_CUDA(dalloc(&e.d_ring_digits, ecorr_digits_bytes(e.ermax)));
+  }
   return ERMOD_OK;
 }
 
@@ -524,15 +530,12 @@ int ermod_create(const ermod_params* p_in, int device, ermod_ctx** out) {
   cudaEventCreateWithFlags(&e.ev_flush[0], cudaEventDisableTiming);
   cudaEventCreateWithFlags(&e.ev_flush[1], cudaEventDisableTiming);
   for (int s = 0; s < 3 + kBatchStreams; ++s) cudaEventCreateWithFlags(&e.ev_join[s], cudaEventDisableTiming);
-  if ((err = dalloc(&e.d_status, 1)) != cudaSuccess || (err = cudaMallocHost(&e.h_status, sizeof(DevStatus))) != cudaSuccess) {
+  if ((err = dalloc(&e.d_status, 1)) != cudaSuccess || (err = cudaMallocHost(&e.h_stage, 2 * kStageBytes + sizeof(DevStatus))) != cudaSuccess ||
+      (err = cudaEventCreateWithFlags(&e.ev_stage, cudaEventDisableTiming)) != cudaSuccess) {
     ermod_destroy(c);
     return fail_cuda(err, "status allocation");
   }
-  if ((err = cudaMallocHost(&e.h_stage, 2 * kStageBytes)) != cudaSuccess ||
-      (err = cudaEventCreateWithFlags(&e.ev_stage, cudaEventDisableTiming)) != cudaSuccess) {
-    ermod_destroy(c);
-    return fail_cuda(err, "staging allocation");
-  }
+  e.h_status = reinterpret_cast<DevStatus*>(e.h_stage + 2 * kStageBytes);
   DevStatus s0{kNoError, kNoError, 0, 0};
   cudaMemcpy(e.d_status, &s0, sizeof(s0), cudaMemcpyHostToDevice);
   *e.h_status = s0;
@@ -595,7 +598,6 @@ int ermod_destroy(ermod_ctx* c) {
   dfree(e.d_twiddle);
   dfree(e.d_twiddle64);
   dfree(e.d_status);
-  if (e.h_status) cudaFreeHost(e.h_status);
   if (e.h_stage) cudaFreeHost(e.h_stage);
   if (e.ev_stage) cudaEventDestroy(e.ev_stage);
   dfree(e.d_out);
@@ -853,7 +855,10 @@ int ermod_set_bins(ermod_ctx* c, int numslv, const int* uvmax, const int* uvsoft
   const size_t nes = (size_t)std::max(esmax, 1);
   e.n_accum = ermax + nes + numslv + 8 + 2 * ((size_t)numslv + 1);
   ERMOD_CUDA(dalloc(&e.d_accum, e.n_accum));
-  ERMOD_CUDA(cudaMallocHost(&e.h_accum, sizeof(double) * e.n_accum));
+  if (sizeof(double) * e.n_accum <= kStageBytes)
+    e.h_accum = e.stage_out();
+  else
+    ERMOD_CUDA(cudaMallocHost(&e.h_accum, sizeof(double) * e.n_accum));
   e.d_edens = e.d_accum;
   e.d_eself = e.d_edens + ermax;
   e.d_slnuv = e.d_eself + nes;
@@ -1318,7 +1323,7 @@ int ermod_placements(ermod_ctx* c, int nplace, const int* tagslt, const double* 
     st = run_placements(e, nplace, e.d_tagslt, sol ? e.d_solxyz : nullptr, sws ? e.d_sws : nullptr,
                         uv_out ? d_uv : nullptr, fl_out ? d_fl : nullptr, ns);
   const bool staged = sizeof(double) * n_out <= kStageBytes;
-  char* stage = e.h_stage + kStageBytes;
+  double* stage = e.stage_out();
   if (!st && n_out > 0) {
     cudaError_t err = cudaSuccess;
     if (staged) {
@@ -1333,7 +1338,7 @@ int ermod_placements(ermod_ctx* c, int nplace, const int* tagslt, const double* 
   const int st2 = ermod_sync(c);
   if (!st && staged) {
     if (uv_out) std::memcpy(uv_out, stage, sizeof(double) * n_uv);
-    if (fl_out) std::memcpy(fl_out, stage + sizeof(double) * n_uv, sizeof(double) * n_fl);
+    if (fl_out) std::memcpy(fl_out, stage + n_uv, sizeof(double) * n_fl);
   }
   dfree(d_tmp);
   return st ? st : st2;

@@ -72,7 +72,7 @@ struct Engine {
   // d_edens, d_eself, d_slnuv, d_scal, d_minuv, d_maxuv lie in one block in this order, which
   // is cleared by one memset and read back by one copy into h_accum
   double* d_accum = nullptr;
-  double* h_accum = nullptr;  // pinned
+  double* h_accum = nullptr;  // pinned: the staging of results, or its own when larger
   size_t n_accum = 0;
   double* d_edens = nullptr;
   double* d_ecorr = nullptr;
@@ -130,10 +130,11 @@ struct Engine {
   int cap_place = 0;
   double* d_out = nullptr;        // [cap_out] uvengy and flceng of a host call
   size_t cap_out = 0;
-  // pinned staging of a host call's small transfers: a frame's coordinates in the first
-  // kStageBytes, results in the second.  ev_stage: the last coordinate copy has left it
+  // pinned: a frame's coordinates in the first kStageBytes, a call's results in the second (each
+  // call waits for its own), then the status.  ev_stage: the last coordinate copy has left it
   char* h_stage = nullptr;
   cudaEvent_t ev_stage = nullptr;
+  double* stage_out() const { return reinterpret_cast<double*>(h_stage + kStageBytes); }
   BatchArgs buf{};                // device buffers sized for Bmax (pointers only)
   // histogram ring for ecorr (corrcal) / per-batch histograms
   // histogram ring of the ecorr flush: two halves of ring_half entries; batches fill the
@@ -142,8 +143,9 @@ struct Engine {
   bool flush_pend[2] = {false, false};  // a flush of that half may still be running
   int* d_ring_hist = nullptr;     // [ring_cap][ermax]
   double* d_ring_w = nullptr;     // [ring_cap]
-  int* d_ring_nz = nullptr;       // ecorr flush scratch, [2][ring_cap][ermax]: the FP64 flush's occupied-bin
-                                  // lists (bins, counts); the mixed flush's active-bin flags and list
+  int* d_ring_nz = nullptr;       // FP64 flush, [2][ring_cap][ermax]: occupied-bin lists (bins, counts)
+  int* d_ring_act = nullptr;      // flush: the bins' largest counts, the active bins and theirs, their number
+  char* d_ring_digits = nullptr;  // flush: digit planes of the matrix kernels
   int* d_ring_nnz = nullptr;      // [ring_cap] occupied bins per entry
   int* d_ring_valid = nullptr;    // [ring_cap] entry accumulated (no error in its batch)
   double* d_u0 = nullptr;         // [2][Bmax] solute self energies (two batch slots)
@@ -152,7 +154,7 @@ struct Engine {
 
   // ---- status ----------------------------------------------------------------------
   DevStatus* d_status = nullptr;
-  DevStatus* h_status = nullptr;  // pinned
+  DevStatus* h_status = nullptr;  // pinned, at the end of h_stage
   bool status_clean = true;  // d_status holds no result of queued work
   int err_placement = -1, err_molecule = -1;
   double err_energy = 0.0;
@@ -259,6 +261,8 @@ int spectrum_partials(const Engine& e);
 int spectrum64_partials(const Engine& e);
 int mol_tile(const Engine& e);  // molecules per block of the molecule kernels
 int accumulate_max_batch();
+size_t ecorr_digits_bytes(int ermax);
+size_t ecorr_scratch_ints(int ermax);
 size_t frame_cub_bytes(int n);
 cudaError_t launch_frame_bricks(Engine& e);
 double host_spline_value(int order, double x);

@@ -6,6 +6,10 @@
 //                 edens += engnmfc * insdst.  Every FP64 sum runs in placement order, as
 //                 in the reference's sequential loop, so results are bit-reproducible.
 //                 A batch in which any molecule failed a bin check is not accumulated.
+//   ecorr_digits, ecorr_mma   the ecorr update (engproc.F90:841-853) of the placements
+//                 buffered in the ring as exact integer matrix products; the kernels below
+//                 take what these do not (short rings, exact counts, weights too far apart).
+//   ecorr_ff      the same sum by a walk of the placements in float-float registers.
 //   ring_compact  per placement, the ascending list of occupied bins (bin, count).
 //   ecorr_rows    ecorr(iduvp, iduv) += engnmfc * insdst(iduv) * insdst(iduvp)
 //                 (engproc.F90:841-853) for the placements buffered in the ring: each
@@ -417,8 +421,10 @@ static_assert(kSmallBatch == 2, "the counts of two placements tested together");
 
 // occupied-bin list per ring entry: entries (bin << 0) with counts beside them
 __global__ void __launch_bounds__(256) ring_compact_kernel(const int* __restrict__ hist, const int* __restrict__ valid,
-                                                         int ermax, int* __restrict__ nz_bin, int* __restrict__ nz_cnt,
+                                                         int ermax, const int* __restrict__ mma,
+                                                         int* __restrict__ nz_bin, int* __restrict__ nz_cnt,
                                                          int* __restrict__ nnz) {
+  if (mma && *mma) return;  // summed by the matrix kernels
   const int p = blockIdx.x;
   const int* h = hist + (size_t)p * ermax;
   __shared__ int scan[256];
@@ -449,7 +455,9 @@ __global__ void __launch_bounds__(256) ring_compact_kernel(const int* __restrict
 __global__ void __launch_bounds__(256) ecorr_rows_kernel(const int* __restrict__ hist, const int* __restrict__ nz_bin,
                                                        const int* __restrict__ nz_cnt, const int* __restrict__ nnz,
                                                        const double* __restrict__ w, int nring, int ermax, int R,
-                                                       double* __restrict__ ecorr, long long* __restrict__ ecorr_n) {
+                                                       const int* __restrict__ mma, double* __restrict__ ecorr,
+                                                       long long* __restrict__ ecorr_n) {
+  if (mma && *mma) return;  // summed by the matrix kernels
   extern __shared__ double srow[];  // [R][ermax] (+ [R][ermax] int64 mirror)
   long long* srow_n = reinterpret_cast<long long*>(srow + (size_t)R * ermax);
   const int row0 = blockIdx.x * R;
@@ -502,6 +510,14 @@ SmemAttr& ecorr_rows_attr() {
   return attr;
 }
 
+// what the flush's kernels need to know of the ring
+struct RingInfo {
+  int nact;  // active bins
+  int emax;  // binary exponent of the largest weight: w = f 2^emax, f in [1/2, 1)
+  int mma;   // 1: the matrix kernels sum this flush, 0: the walk (weights or bins out of their range)
+};
+
+
 // Mixed path flush, same sum as ecorr_rows_kernel.  A CTA owns kEcRows rows and 256
 // columns of the matrix; thread t owns one column and keeps the flush's contribution
 // to its kEcRows entries in registers as float-float pairs (exact products by fma,
@@ -533,13 +549,14 @@ __device__ __forceinline__ void ff_add_prod(float& hi, float& lo, float wh, floa
 template <bool COUNT>
 __global__ void __launch_bounds__(256, 2) ecorr_ff_kernel(const int* __restrict__ hist, const int* __restrict__ valid,
                                                         const double* __restrict__ w, int nring, int ermax,
-                                                        const int* __restrict__ act, const int* __restrict__ nact_d,
+                                                        const int* __restrict__ act, const RingInfo* __restrict__ info,
                                                         double* __restrict__ ecorr, long long* __restrict__ ecorr_n) {
   extern __shared__ float2 sdyn2[];
   float2* sa = sdyn2;  // [nring][kEcRows]: w_p * hist[p][row r's bin] as a float-float pair
   unsigned* smask = reinterpret_cast<unsigned*>(sa + (size_t)nring * kEcRows);  // [nring]
   int* sci = reinterpret_cast<int*>(smask + nring);  // [nring][kEcRows] counts (count mirror only)
-  const int nact = *nact_d;
+  if (info->mma) return;  // summed by the matrix kernels
+  const int nact = info->nact;
   const int row0 = blockIdx.y * kEcRows;
   if (row0 >= nact) return;  // the grid covers every bin; the active ones come first
   if ((int)(blockIdx.x * blockDim.x + blockDim.x) <= row0) return;  // all below the diagonal
@@ -624,13 +641,12 @@ __global__ void __launch_bounds__(256, 2) ecorr_ff_kernel(const int* __restrict_
   }
 }
 
-// The flush's active bins: flag[i] != 0 when some valid placement of the ring occupies bin
-// i (flag zeroed first).  CTA per (256 bins, 32 placements): the 32 loads of a thread are
-// independent and in flight together; an occupied bin sets its flag (an OR, so the
-// order of the writes does not matter).
+// The flush's active bins: top[i] = the largest count of bin i over the ring's valid placements
+// (top zeroed first; 0: no placement occupies it).  CTA per (256 bins, 32 placements): the 32
+// loads of a thread are independent and in flight together.
 constexpr int kActivePlacements = 32;
 __global__ void __launch_bounds__(256) ring_active_kernel(const int* __restrict__ hist, const int* __restrict__ valid,
-                                                        int nring, int ermax, int* __restrict__ flag) {
+                                                        int nring, int ermax, int* __restrict__ top) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int p0 = blockIdx.y * kActivePlacements;
   if (i >= ermax) return;
@@ -640,40 +656,270 @@ __global__ void __launch_bounds__(256) ring_active_kernel(const int* __restrict_
     const int p = p0 + u;
     c[u] = (p < nring && valid[p]) ? __ldg(hist + (size_t)p * ermax + i) : 0;
   }
-  int any = 0;
+  int most = 0;
 #pragma unroll
-  for (int u = 0; u < kActivePlacements; ++u) any |= c[u];
-  if (any) flag[i] = 1;
+  for (int u = 0; u < kActivePlacements; ++u) most = max(most, c[u]);
+  if (most) atomicMax(&top[i], most);
 }
 
-// Coordinates of at most this many bins walk every bin: on the 33,000-water workload
-// (1,396 bins, about 900 of them active in a flush) the gathered walk over the active
-// ones was slower than the contiguous walk over all.
-constexpr int kActiveMinBins = 2048;
-
-// act[0 .. *nact) = the flagged bins in increasing order (one CTA, chunks of 1024)
-__global__ void __launch_bounds__(1024) ring_active_list_kernel(const int* __restrict__ flag, int ermax,
-                                                              int* __restrict__ act, int* __restrict__ nact) {
-  __shared__ int scan[1024];
+// act[0 .. nact) = the active bins in increasing order, atop their largest counts, and whether
+// the matrix kernels may sum the flush: at most max_bins active bins and positive finite weights
+// whose exponents differ by at most spread (one CTA, chunks of 1024)
+__global__ void __launch_bounds__(1024) ring_active_list_kernel(const int* __restrict__ top, int ermax,
+                                                              const int* __restrict__ valid,
+                                                              const double* __restrict__ w, int nring, int max_bins,
+                                                              int spread, int all, int* __restrict__ act,
+                                                              int* __restrict__ atop, RingInfo* __restrict__ info) {
+  __shared__ int warp_sum[32];
+  __shared__ int s_max, s_min, s_bad;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    s_max = -100000;
+    s_min = 100000;
+    s_bad = 0;
+  }
+  __syncthreads();
   int base = 0;
   for (int c0 = 0; c0 < ermax; c0 += 1024) {
     const int i = c0 + (int)threadIdx.x;
-    const int f = (i < ermax && flag[i] != 0) ? 1 : 0;
-    scan[threadIdx.x] = f;
+    const int t = i < ermax ? (all ? 1 : top[i]) : 0;
+    const unsigned m = __ballot_sync(0xffffffffu, t != 0);
+    if (lane == 0) warp_sum[warp] = __popc(m);
     __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {  // inclusive Hillis-Steele scan
-      const int v = (threadIdx.x >= (unsigned)off) ? scan[threadIdx.x - off] : 0;
-      __syncthreads();
-      scan[threadIdx.x] += v;
-      __syncthreads();
+    int before = __popc(m & ((1u << lane) - 1u)), total = 0;
+    for (int k = 0; k < 32; ++k) {
+      if (k < warp) before += warp_sum[k];
+      total += warp_sum[k];
     }
-    if (f) act[base + scan[threadIdx.x] - 1] = i;
-    const int tot = scan[1023];
-    __syncthreads();  // scan[1023] read by every thread before the next chunk overwrites it
-    base += tot;
+    if (t) {
+      act[base + before] = i;
+      atop[base + before] = t;
+      if (t >= 1 << 24) s_bad = 1;  // more digits than the planes hold
+    }
+    __syncthreads();  // warp_sum read by every thread before the next chunk overwrites it
+    base += total;
   }
-  if (threadIdx.x == 0) *nact = base;
+  int emx = -100000, emn = 100000;
+  for (int p = threadIdx.x; p < nring; p += 1024) {
+    if (!valid[p]) continue;
+    const double x = w[p];
+    if (x == 0.0) continue;
+    if (!(x > 0.0) || isinf(x)) {
+      s_bad = 1;
+      continue;
+    }
+    const int e = ilogb(x) + 1;
+    emx = max(emx, e);
+    emn = min(emn, e);
+  }
+  atomicMax(&s_max, emx);
+  atomicMin(&s_min, emn);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    info->nact = base;
+    info->emax = s_max;
+    info->mma = (!all && !s_bad && base <= max_bins && s_max >= s_min && s_max - s_min <= spread) ? 1 : 0;
+  }
 }
+
+// ---- the flush as exact integer matrix products ------------------------------------------
+// ecorr(i, j) += sum_p w_p h_p(i) h_p(j), a product of (bins x placements) matrices.  With the
+// weights as integers m_p = w_p 2^(T - emax) (T = 56, FP64 path 63: relative to the largest
+// weight 2^-T, and a weight whose exponent is within the spread of the largest keeps 44, FP64
+// path 53, bits), m_p h_p(i) is cut into 7-bit digits and h_p(j) into 8-bit ones: their bf16
+// values are exact, and the FP32 sums of 512 products of two digits are integers below 2^24,
+// exact too.  So mma.sync adds the digit planes without error, and each entry is rounded once
+// per 35 bits of planes when they are joined.  512 placements, with the two kernels before: 168 ->
+// 95 us for 4,000 waters, 294 -> 130 us for 33,000 (float-float sums by the walk below); FP64
+// path, 64 placements of 4,000 waters 253 -> 45 us.
+constexpr int kMmaK = 512;         // placements per pass (a longer ring takes several)
+constexpr int kMmaBins = 2048;     // active bins, at most
+constexpr int kMaxADigits = 13;    // 7-bit digits of m h: T + 24 bits of a count
+constexpr int kMaxBDigits = 3;     // 8-bit digits of a count below 2^24
+constexpr int kMmaMinRing = 48;    // placements in the ring for the matrix kernels to pay
+
+__device__ __forceinline__ int bit_length(int x) { return 32 - __clz(x); }
+__device__ __forceinline__ int a_digits(int T, int top) { return (T + 1 + bit_length(top) + 6) / 7; }
+__device__ __forceinline__ int b_digits(int top) { return (bit_length(top) + 7) / 8; }
+// the largest count of 16 active bins from block ib on (by a whole warp)
+__device__ __forceinline__ int block_top(const int* atop, int nact, int ib) {
+  const int i = 16 * ib + (threadIdx.x & 15);
+  return max(1, __reduce_max_sync(0xffffffffu, i < nact ? atop[i] : 0));
+}
+
+// the digits in the order of mma.m16n8k16's fragments: [plane][block of 16 bins][block of 16
+// placements][lane][8].  A warp per block of 16 x 16: lane (g, t) = (lane / 4, lane % 4) holds
+// bins g and g + 8 and placements 2 t, 2 t + 1, + 8 of it.
+__global__ void __launch_bounds__(256) ecorr_digits_kernel(const int* __restrict__ hist, const int* __restrict__ valid,
+                                                         const double* __restrict__ w, int p0, int n, int ermax, int T,
+                                                         int nbins, const int* __restrict__ act,
+                                                         const int* __restrict__ atop, const RingInfo* __restrict__ info,
+                                                         uint4* __restrict__ A, uint4* __restrict__ B) {
+  const RingInfo I = *info;
+  const int ib = blockIdx.x, kb = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int nkb = (n + 15) / 16;
+  if (!I.mma || 16 * ib >= I.nact || kb >= nkb) return;
+  const int g = lane >> 2, t = lane & 3;
+  const int top = block_top(atop, I.nact, ib);
+  const int na = a_digits(T, top), nb = b_digits(top);
+  unsigned long long lo[8], hi[8];
+  int h[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {  // e = 4 (placement + 8) + 2 (bin + 8) + (placement + 1)
+    const int i = 16 * ib + g + ((e >> 1) & 1) * 8, k = 16 * kb + 2 * t + (e & 1) + (e >> 2) * 8;
+    const int p = p0 + k;
+    h[e] = (k < n && i < I.nact && valid[p]) ? __ldg(hist + (size_t)p * ermax + act[i]) : 0;
+    unsigned long long m = 0;
+    if (h[e]) m = (unsigned long long)__double2ull_rn(ldexp(w[p], T - I.emax));
+    lo[e] = m * (unsigned long long)h[e];
+    hi[e] = __umul64hi(m, (unsigned long long)h[e]);
+  }
+  auto bf = [](unsigned a, unsigned b) {  // two digits below 256 as bf16, exactly
+    return (__float_as_uint((float)a) >> 16) | (__float_as_uint((float)b) & 0xffff0000u);
+  };
+  const size_t nib = (size_t)nbins / 16, at = ((size_t)ib * (kMmaK / 16) + kb) * 32 + lane;
+  const size_t plane = nib * (kMmaK / 16) * 32;
+  for (int l = 0; l < na; ++l) {
+    unsigned d[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      d[e] = (unsigned)lo[e] & 127u;
+      lo[e] = (lo[e] >> 7) | (hi[e] << 57);
+      hi[e] >>= 7;
+    }
+    A[l * plane + at] = make_uint4(bf(d[0], d[1]), bf(d[2], d[3]), bf(d[4], d[5]), bf(d[6], d[7]));
+  }
+  for (int m = 0; m < nb; ++m) {
+    unsigned d[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) d[e] = ((unsigned)h[e] >> (8 * m)) & 255u;
+    // as the second operand: bins g (then g + 8), for each the placements and those + 8
+    B[m * plane + at] = make_uint4(bf(d[0], d[1]), bf(d[4], d[5]), bf(d[2], d[3]), bf(d[6], d[7]));
+  }
+}
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint4& a, unsigned b0, unsigned b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, "
+      "%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+
+// CTA per 32 x 32 active bins on or above the diagonal.  The digit planes' products come from
+// fragments in L2; a warp takes five planes, joined as 64-bit integers, and a quarter of the
+// placements, so that the loads' latency is paid a few times over and not once per plane and
+// round (one warp per tile: twice the time); the warps' integers are added exactly and joined
+// in FP64.  Bound by that latency still: two CTAs to an SM take 67 us a flush of 512 placements
+// of 4,000 waters, one with more loads in flight per warp 120.  Each entry is added at both mirrored positions.
+constexpr int kMmaWarps = 8, kMmaParts = 4;
+__global__ void __launch_bounds__(32 * kMmaWarps, 2) ecorr_mma_kernel(const uint4* __restrict__ A,
+                                                                 const uint4* __restrict__ B, int n, int ermax, int T,
+                                                                 int nbins, const int* __restrict__ act,
+                                                                 const int* __restrict__ atop,
+                                                                 const RingInfo* __restrict__ info,
+                                                                 double* __restrict__ ecorr) {
+  extern __shared__ long long sq[];  // [kMmaWarps][32 entries of a lane][32 lanes]
+  const RingInfo I = *info;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+  if (!I.mma || c0 < r0 || r0 >= I.nact || c0 >= I.nact) return;
+  const int nkb = (n + 15) / 16;
+  const int nblk = (I.nact + 15) / 16;  // blocks of 16 bins written
+  const int rb = r0 / 16, cb = c0 / 16;
+  const bool r1 = rb + 1 < nblk, c1 = cb + 1 < nblk;
+  const size_t row = (size_t)(kMmaK / 16) * 32, plane = (size_t)(nbins / 16) * row;
+  // a block's planes beyond its own digits were not written: each block has its own count
+  const int top0 = block_top(atop, I.nact, rb), top1 = block_top(atop, I.nact, rb + 1);
+  const int cop0 = block_top(atop, I.nact, cb), cop1 = block_top(atop, I.nact, cb + 1);
+  const int na0 = a_digits(T, top0), na1 = r1 ? a_digits(T, top1) : 0, na = max(na0, na1);
+  const int nb0 = b_digits(cop0), nb1 = c1 ? b_digits(cop1) : 0;
+  const int part = warp % kMmaParts, half = warp / kMmaParts;
+  const int nround = (na + 9) / 10;  // two groups of five planes at a time
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (int m = max(nb0, nb1) - 1; m >= 0; --m) {
+    double R[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int round = nround - 1; round >= 0; --round) {
+      const int l0 = 10 * round + 5 * half;
+      long long q[2][4][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) q[i][j][e] = 0;
+      for (int l = min(l0 + 4, na - 1); l >= l0; --l) {
+        float c[2][4][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) c[i][j][e] = 0.f;
+        const uint4* a = A + l * plane + rb * row + lane;
+        const uint4* b = B + m * plane + cb * row + lane;
+#pragma unroll 2
+        for (int kb = part; kb < nkb; kb += kMmaParts) {
+          const uint4 a0 = l < na0 ? __ldg(a + kb * 32) : zero, a1 = l < na1 ? __ldg(a + row + kb * 32) : zero;
+          const uint4 b0 = m < nb0 ? __ldg(b + kb * 32) : zero, b1 = m < nb1 ? __ldg(b + row + kb * 32) : zero;
+          mma_bf16(c[0][0], a0, b0.x, b0.y);
+          mma_bf16(c[0][1], a0, b0.z, b0.w);
+          mma_bf16(c[0][2], a0, b1.x, b1.y);
+          mma_bf16(c[0][3], a0, b1.z, b1.w);
+          mma_bf16(c[1][0], a1, b0.x, b0.y);
+          mma_bf16(c[1][1], a1, b0.z, b0.w);
+          mma_bf16(c[1][2], a1, b1.x, b1.y);
+          mma_bf16(c[1][3], a1, b1.z, b1.w);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) q[i][j][e] = q[i][j][e] * 128 + __float2int_rn(c[i][j][e]);
+      }
+      __syncthreads();  // the round before has been read
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sq[(warp * 32 + i * 16 + j * 4 + e) * 32 + lane] = q[i][j][e];
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int at = warp + 8 * u;  // entry of each lane
+        long long lo = 0, hi = 0;
+#pragma unroll
+        for (int p = 0; p < kMmaParts; ++p) {
+          lo += sq[(p * 32 + at) * 32 + lane];
+          hi += sq[((p + kMmaParts) * 32 + at) * 32 + lane];
+        }
+        R[u] = fma(fma(R[u], 34359738368.0, (double)hi), 34359738368.0, (double)lo);  // 2^35 per five planes
+      }
+    }
+    const double unit = ldexp(1.0, I.emax - T + 8 * m);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      // entry (i, j, e) of the fragments: row 16 i + lane / 4 (+ 8 for e >= 2), column 8 j + 2 (lane % 4) + (e & 1)
+      const int at = warp + 8 * u, i = at >> 4, j = (at >> 2) & 3, e = at & 3;
+      const int ri = r0 + 16 * i + (lane >> 2) + (e >> 1) * 8, ci = c0 + 8 * j + 2 * (lane & 3) + (e & 1);
+      if (ci < ri || ci >= I.nact || R[u] == 0.0) continue;
+      const double v = R[u] * unit;
+      const size_t br = act[ri], bc = act[ci];
+      // one addition per entry and launch: an atomic one only so that no thread waits for it
+      atomicAdd(ecorr + br * ermax + bc, v);
+      if (br != bc) atomicAdd(ecorr + bc * ermax + br, v);
+    }
+  }
+}
+
+// Coordinates of at most this many bins walk every bin in ecorr_ff_kernel: on the 33,000-water
+// workload (1,396 bins, about 900 of them active in a flush) the gathered walk over the active
+// ones was slower than the contiguous walk over all.
+constexpr int kActiveMinBins = 2048;
+
+size_t mma_bins(int ermax) { return ((size_t)std::min(ermax, kMmaBins) + 63) / 64 * 64; }
 
 }  // namespace
 
@@ -735,53 +981,82 @@ cudaError_t launch_accumulate(Engine& e, const BatchArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+size_t ecorr_digits_bytes(int ermax) {
+  return sizeof(uint4) * mma_bins(ermax) / 16 * (kMmaK / 16) * 32 * (kMaxADigits + kMaxBDigits);
+}
+size_t ecorr_scratch_ints(int ermax) { return 3 * (size_t)ermax + sizeof(RingInfo) / sizeof(int); }
+
 cudaError_t launch_ecorr_flush(Engine& e, cudaStream_t s) {
   if (e.ring_fill == 0) return cudaSuccess;
   const int n = e.ring_fill;
+  const bool count = e.d_ecorr_n != nullptr;
+  const int* hist = e.d_ring_hist + (size_t)e.ring_off * e.ermax;
+  const int* valid = e.d_ring_valid + e.ring_off;
+  const double* w = e.d_ring_w + e.ring_off;
+  int* top = e.d_ring_act;              // [ermax] largest counts
+  int* act = top + e.ermax;             // [ermax] the active bins
+  int* atop = act + e.ermax;            // [ermax] their largest counts
+  RingInfo* info = reinterpret_cast<RingInfo*>(atop + e.ermax);
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+  // the matrix kernels, unless the flush is short or the exact counts are wanted too; the walk
+  // below them returns at once when they have summed the flush
+  const bool mma = !count && n >= kMmaMinRing;
+  if (mma || (e.mixed && e.ermax > kActiveMinBins)) {
+    if ((err = cudaMemsetAsync(top, 0, sizeof(int) * e.ermax, s)) != cudaSuccess) return err;
+    ring_active_kernel<<<dim3((e.ermax + 255) / 256, (n + kActivePlacements - 1) / kActivePlacements), 256, 0, s>>>(
+        hist, valid, n, e.ermax, top);
+    e.count_launch();
+  }
+  // (every bin walked on a short coordinate: the list costs more than the bins it could leave out)
+  const int all = !mma && e.ermax <= kActiveMinBins;
+  const int T = e.mixed ? 56 : 63, spread = e.mixed ? 12 : 10;
+  if (mma || e.mixed) {
+    ring_active_list_kernel<<<1, 1024, 0, s>>>(top, e.ermax, valid, w, n, mma ? kMmaBins : -1, spread, all, act, atop,
+                                             info);
+    e.count_launch();
+  }
+  if (mma) {
+    const int nbins = (int)mma_bins(e.ermax);
+    constexpr size_t smem_q = sizeof(long long) * kMmaWarps * 32 * 32;
+    static SmemAttr attr_q;
+    if ((err = attr_q.ensure(ecorr_mma_kernel, smem_q)) != cudaSuccess) return err;
+    uint4* A = reinterpret_cast<uint4*>(e.d_ring_digits);
+    uint4* B = A + (size_t)nbins / 16 * (kMmaK / 16) * 32 * kMaxADigits;
+    for (int p0 = 0; p0 < n; p0 += kMmaK) {
+      const int np = std::min(kMmaK, n - p0);
+      ecorr_digits_kernel<<<dim3(nbins / 16, (np + 127) / 128), 256, 0, s>>>(hist, valid, w, p0, np, e.ermax, T, nbins,
+                                                                            act, atop, info, A, B);
+      ecorr_mma_kernel<<<dim3(nbins / 32, nbins / 32), 32 * kMmaWarps, smem_q, s>>>(A, B, np, e.ermax, T, nbins, act, atop, info,
+                                                                   e.d_ecorr);
+      e.count_launch(2);
+    }
+    if ((err = cudaGetLastError()) != cudaSuccess) return err;
+  }
   if (e.mixed) {
-    const bool count = e.d_ecorr_n != nullptr;
     const size_t smem =
         (size_t)n * (kEcRows * sizeof(float2) + sizeof(unsigned) + (count ? kEcRows * sizeof(int) : 0));
-    cudaError_t err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-    const int* hist = e.d_ring_hist + (size_t)e.ring_off * e.ermax;
-    const int* valid = e.d_ring_valid + e.ring_off;
-    int* flag = e.d_ring_nz;                  // [ermax] occupied by some placement
-    int* act = e.d_ring_nz + e.ermax;         // [ermax] the active bins
-    int* nact = e.d_ring_nz + 2 * e.ermax;    // [1]
-    if (e.ermax > kActiveMinBins) {
-      if ((err = cudaMemsetAsync(flag, 0, sizeof(int) * e.ermax, s)) != cudaSuccess) return err;
-      ring_active_kernel<<<dim3((e.ermax + 255) / 256, (n + kActivePlacements - 1) / kActivePlacements), 256, 0, s>>>(
-          hist, valid, n, e.ermax, flag);
-    } else {  // every bin walked: the list costs more than the bins it could leave out
-      if ((err = cudaMemsetAsync(flag, 0xff, sizeof(int) * e.ermax, s)) != cudaSuccess) return err;
-    }
-    ring_active_list_kernel<<<1, 1024, 0, s>>>(flag, e.ermax, act, nact);
-    e.count_launch(e.ermax > kActiveMinBins ? 2 : 1);
-    void (*kern)(const int*, const int*, const double*, int, int, const int*, const int*, double*, long long*) =
+    void (*kern)(const int*, const int*, const double*, int, int, const int*, const RingInfo*, double*, long long*) =
         count ? ecorr_ff_kernel<true> : ecorr_ff_kernel<false>;
     static SmemAttr attr_ff[2];  // per instantiation; the size set only ever grows
     if ((err = attr_ff[count ? 1 : 0].ensure(kern, smem)) != cudaSuccess) return err;
     dim3 grid((e.ermax + 255) / 256, (e.ermax + kEcRows - 1) / kEcRows);
-    kern<<<grid, 256, smem, s>>>(hist, valid, e.d_ring_w + e.ring_off, n, e.ermax, act, nact, e.d_ecorr, e.d_ecorr_n);
+    kern<<<grid, 256, smem, s>>>(hist, valid, w, n, e.ermax, act, info, e.d_ecorr, e.d_ecorr_n);
     e.count_launch();
     return cudaGetLastError();
   }
   int* nz_bin = e.d_ring_nz;
   int* nz_cnt = e.d_ring_nz + (size_t)e.ring_cap * e.ermax;
-  const int* valid = e.d_ring_valid + e.ring_off;
-  const int* hist = e.d_ring_hist + (size_t)e.ring_off * e.ermax;
-  ring_compact_kernel<<<n, 256, 0, s>>>(hist, valid, e.ermax, nz_bin, nz_cnt, e.d_ring_nnz);
+  ring_compact_kernel<<<n, 256, 0, s>>>(hist, valid, e.ermax, mma ? &info->mma : nullptr, nz_bin, nz_cnt, e.d_ring_nnz);
   e.count_launch();
-  cudaError_t err = cudaGetLastError();
-  if (err != cudaSuccess) return err;
+  if ((err = cudaGetLastError()) != cudaSuccess) return err;
   const size_t per_row = (size_t)e.ermax * (sizeof(double) + (e.d_ecorr_n ? sizeof(long long) : 0));
   int R = (int)std::max<size_t>(1, std::min<size_t>(8, (96 * 1024) / per_row));
   const size_t smem = per_row * R;
   if ((err = ecorr_rows_attr().ensure(ecorr_rows_kernel, smem)) != cudaSuccess) return err;
   const int nblk = (e.ermax + R - 1) / R;
-  ecorr_rows_kernel<<<nblk, 256, smem, s>>>(hist, nz_bin, nz_cnt, e.d_ring_nnz, e.d_ring_w + e.ring_off, n,
-                                                   e.ermax, R, e.d_ecorr, e.d_ecorr_n);
+  ecorr_rows_kernel<<<nblk, 256, smem, s>>>(hist, nz_bin, nz_cnt, e.d_ring_nnz, w, n, e.ermax, R,
+                                            mma ? &info->mma : nullptr, e.d_ecorr, e.d_ecorr_n);
   e.count_launch();
   return cudaGetLastError();
 }
@@ -875,7 +1150,7 @@ cudaError_t launch_ecorr_noalloc(const int* hist, const double* weight, int npla
   err = ecorr_rows_attr().ensure(ecorr_rows_kernel, smem);
   if (err != cudaSuccess) return err;
   ecorr_rows_kernel<<<(ermax + R - 1) / R, 256, smem, s>>>(hist, nz_bin, nz_cnt, nnz, weight, nplace, ermax, R,
-                                                           ecorr, ecorr_count);
+                                                           nullptr, ecorr, ecorr_count);
   return cudaGetLastError();
 }
 
