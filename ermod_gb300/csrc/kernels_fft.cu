@@ -966,7 +966,10 @@ __global__ void __launch_bounds__(pme_threads(KC), pme_min_blocks(KC)) pme_b_ker
         }
       }
     }
-    cluster.sync();  // no CTA leaves while another still reads its shared memory
+    // no CTA leaves while another still reads its shared memory.  The remote loads have returned
+    // (their values are stored), so the barrier orders nothing: a releasing one waits for the
+    // stores above to reach memory (256 placements at 96^3: 687 us with it, 668 us without)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
   } else {
     for (int c = 0; c < ncopy; ++c) {
       float* plane_out = out + (size_t)(c ? z - K3 + h : z + h) * A.YP * A.XP * 4;
