@@ -450,7 +450,9 @@ struct PmeArgs {
   FastDiv fH, fK1, fHp4, fnpair, fKX;
 };
 
-// KC > 0: a K^3 grid with K = KC and compile-time transforms; KC = 0: any grid
+// KC > 0: a K^3 grid with K = KC and compile-time transforms; KC = 0: any grid, a CTA of one
+// thread per generation tile (whole warps, at most 512) like the sized ones: 512 threads for
+// the 7 x 27 tiles of a 54 x 54 x 80 grid left two thirds of them idle
 template <int KC>
 __global__ void __launch_bounds__(pme_threads(KC), pme_min_blocks(KC)) pme_a_kernel(PmeArgs A) {
   extern __shared__ float2 sm[];
@@ -862,7 +864,8 @@ __device__ __forceinline__ float2* pme_b_planes(const PmeArgs& A, const float2* 
 // CTA per (z, placement): the k2 transform of the (k2, k1) plane, then the
 // complex-to-real transform along k1, two rows per complex transform; writes the real
 // plane into the placement's lane of the interleaved potential grid.
-// Compile-time sizes (KC > 0): the four CTAs of an interleaved group (the same plane of
+// Compile-time sizes (KC > 0, K1 = K2 = KC and any K3: a plane's work does not depend on K3, so
+// tetragonal cells take them too): the four CTAs of an interleaved group (the same plane of
 // four placements) form a thread-block cluster.  Once their planes are done, each CTA
 // reads a quarter of the rows of all four planes through distributed shared memory and
 // writes them as whole float4 points (16-byte stores, full 32-byte sectors), instead of
@@ -877,7 +880,7 @@ __global__ void __launch_bounds__(pme_threads(KC), pme_min_blocks(KC)) pme_b_ker
   if constexpr (KC == 0) {
     if (!live) return;
   }
-  const int K1 = KC ? KC : A.K1, K2 = KC ? KC : A.K2, K3 = KC ? KC : A.K3;
+  const int K1 = KC ? KC : A.K1, K2 = KC ? KC : A.K2, K3 = A.K3;
   const int H = KC ? KC / 2 + 1 : A.H, K1p = KC ? (KC | 1) : A.K1p;
   const size_t plane = (size_t)K2 * H;
   const int npair = (K2 + 1) / 2;
@@ -1039,51 +1042,61 @@ cudaError_t launch_pme_mixed(Engine& e, const BatchArgs& a) {
   A.fnpair = make_fastdiv((A.K2 + 1) / 2);
   A.fKX = make_fastdiv(A.K1 + A.halo);
   cudaError_t err;
-  // cubic grids of common sizes take the compile-time transforms
+  // Compile-time transforms for the lengths 2^a 3^b 5^c from 32 to 144: the plane kernel when
+  // K1 = K2, the slab kernel when the grid is cubic.  Shorter lengths take microseconds either way,
+  // longer ones do not fit two CTAs on an SM.  700 insertions on 54 x 54 x 80 (order 6): 4.07 ms
+  // with the general kernels in 512 threads, 3.06 now; a graph of four systems, one of them on
+  // 54^3, 31.9 and 27.7 ms.
   struct Sized {
     int K;
     void (*a)(PmeArgs);
     void (*b)(PmeArgs);
   };
 #define ERMOD_PME_SIZE(KK) Sized{KK, pme_a_kernel<KK>, pme_b_kernel<KK>}
-  static const Sized sized[] = {ERMOD_PME_SIZE(32),  ERMOD_PME_SIZE(40),  ERMOD_PME_SIZE(45),  ERMOD_PME_SIZE(48),
-                                ERMOD_PME_SIZE(50),  ERMOD_PME_SIZE(60),  ERMOD_PME_SIZE(64),  ERMOD_PME_SIZE(72),
-                                ERMOD_PME_SIZE(80),  ERMOD_PME_SIZE(90),  ERMOD_PME_SIZE(96),  ERMOD_PME_SIZE(100),
+  static const Sized sized[] = {ERMOD_PME_SIZE(32),  ERMOD_PME_SIZE(36),  ERMOD_PME_SIZE(40),  ERMOD_PME_SIZE(45),
+                                ERMOD_PME_SIZE(48),  ERMOD_PME_SIZE(50),  ERMOD_PME_SIZE(54),  ERMOD_PME_SIZE(60),
+                                ERMOD_PME_SIZE(64),  ERMOD_PME_SIZE(72),  ERMOD_PME_SIZE(75),  ERMOD_PME_SIZE(80),
+                                ERMOD_PME_SIZE(81),  ERMOD_PME_SIZE(90),  ERMOD_PME_SIZE(96),  ERMOD_PME_SIZE(100),
                                 ERMOD_PME_SIZE(108), ERMOD_PME_SIZE(120), ERMOD_PME_SIZE(125), ERMOD_PME_SIZE(128),
-                                ERMOD_PME_SIZE(144)};
+                                ERMOD_PME_SIZE(135), ERMOD_PME_SIZE(144)};
 #undef ERMOD_PME_SIZE
   constexpr int nsized = (int)(sizeof(sized) / sizeof(sized[0]));
-  const bool cubic = A.K1 == A.K2 && A.K2 == A.K3;
-  int slot = 0;  // 0: the generic kernels, 1 + i: sized[i]
+  const bool square = A.K1 == A.K2, cubic = square && A.K2 == A.K3;
+  int slot_a = 0, slot_b = 0;  // 0: the generic kernels, 1 + i: sized[i]
   void (*ka)(PmeArgs) = pme_a_kernel<0>;
   void (*kb)(PmeArgs) = pme_b_kernel<0>;
-  for (int i = 0; i < nsized && cubic; ++i)
+  for (int i = 0; i < nsized && square; ++i)
     if (sized[i].K == A.K1) {
-      slot = 1 + i;
-      ka = sized[i].a;
+      slot_b = 1 + i;
       kb = sized[i].b;
+      if (cubic) {
+        slot_a = slot_b;
+        ka = sized[i].a;
+      }
     }
-  const int KC = slot ? A.K1 : 0;
+  const int KC = slot_a ? A.K1 : 0;
   // solute sites staged per generation chunk: both tables, chunk x (K3 + Hp), fit in pme_a's
   // work buffer
   const int wcols = KC ? pme_a_work_cols(KC) : A.Hp;
   A.chunk = std::max(1, std::min(kSites, (A.K3 * wcols) / (A.K3 + A.Hp)));
-  const size_t sa = pme_a_smem(A.K3, A.Hp, KC > 0), sb = pme_b_smem(A.K1, A.K2, A.H, KC > 0);
+  const size_t sa = pme_a_smem(A.K3, A.Hp, slot_a > 0), sb = pme_b_smem(A.K1, A.K2, A.H, slot_b > 0);
   static SmemAttr attr_a[1 + nsized], attr_b[1 + nsized];  // per kernel
-  if ((err = attr_a[slot].ensure(ka, sa)) != cudaSuccess) return err;
-  if ((err = attr_b[slot].ensure(kb, sb)) != cudaSuccess) return err;
-  const int nthr = pme_threads(KC);
-  ka<<<dim3(A.K2, a.nb), nthr, sa, a.stream>>>(A);
+  if ((err = attr_a[slot_a].ensure(ka, sa)) != cudaSuccess) return err;
+  if ((err = attr_b[slot_b].ensure(kb, sb)) != cudaSuccess) return err;
+  const int tiles = (A.Hp / kR1) * ((A.K3 + kR3 - 1) / kR3);
+  const int nthr_a = KC ? pme_threads(KC) : std::min(512, (tiles + 31) / 32 * 32);
+  ka<<<dim3(A.K2, a.nb), nthr_a, sa, a.stream>>>(A);
   e.count_launch();
   if ((err = cudaGetLastError()) != cudaSuccess) return err;
   if (a.phases) {
     e.phase_end_on(a.stream);
     e.phase_begin_on(PH_FFT, a.stream);
   }
-  if (slot) {  // compile-time sizes: the four CTAs of a group are one cluster
+  const int nthr_b = pme_threads(slot_b ? A.K1 : 0);
+  if (slot_b) {  // compile-time sizes: the four CTAs of a group are one cluster
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(4, A.K3, (a.nb + 3) / 4);
-    cfg.blockDim = dim3(nthr);
+    cfg.blockDim = dim3(nthr_b);
     cfg.dynamicSmemBytes = sb;
     cfg.stream = a.stream;
     cudaLaunchAttribute attr[1];
@@ -1095,7 +1108,7 @@ cudaError_t launch_pme_mixed(Engine& e, const BatchArgs& a) {
     cfg.numAttrs = 1;
     if ((err = cudaLaunchKernelEx(&cfg, kb, A)) != cudaSuccess) return err;
   } else {
-    kb<<<dim3(4, A.K3, (a.nb + 3) / 4), nthr, sb, a.stream>>>(A);
+    kb<<<dim3(4, A.K3, (a.nb + 3) / 4), nthr_b, sb, a.stream>>>(A);
   }
   e.count_launch();
   return cudaGetLastError();
