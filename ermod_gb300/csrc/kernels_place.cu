@@ -231,73 +231,136 @@ struct Spec64Args {
   const double* engfac;  // [K3][K2][H]
   double2* spec;         // [nb][K3][K2][H]
   double* self_part;     // [nb][spectrum64_partials]
-  int K1, K2, K3, H, Kmax, R;
+  int K1, K2, K3, H, Kmax;
+  int groups;  // groups of kSpecPairs k3 pairs per CTA
 };
 
 // The FP64 spectrum engfac(k) S(k), S = sum_s q_s b1_s(k1) b2_s(k2) b3_s(k3): exactly the R2C
 // transform of the spread charges (recpcal.F90:357-384) without the K^3 grid, the spread and
 // the forward transform, and with the self energy 0.5 sum_k engfac |S|^2 (recpcal.F90:385-394)
-// in the same pass.  CTA per (k2, R values of k3, placement): the R x ns row factors
-// q b2 b3 in shared memory, a thread per point of R rows of H.  Bound by the FP64 pipe: 4 FMA
-// per point and site, which at 2 per clock and SM is 35 us for 12 sites at 96^3; measured 50 us a
-// placement there (4.1 us for 6 sites at 48^3), against 149 us (45 us) for the spread, cuFFT's
-// D2Z and the influence pass in its place, one placement at a time.
-constexpr int kSpec64Threads = 256;
+// in the same pass.
+//
+// Bound by the FP64 pipe (2 FMA per clock and SM), so k3 and K3 - k3 are computed together:
+// b3(K3 - k3) is the conjugate of b3(k3) = c + i s, so with the site's p = q b1 b2,
+// A = sum p c and B = sum p s (real times complex, 2 FMA each) give S(k3) = A + i B and
+// S(K3 - k3) = A - i B: half of the 4 FMA per point and site that each point takes by itself.
+// Pair 0 holds the real b3(0) and b3(K3 / 2) (the latter 0 for odd K3): S(0) = A, S(K3 / 2) = B.
+// CTA per (k2, groups x 4 pairs, placement), a thread per k1 and 4 pairs; p and the pairs'
+// factors of 16 sites at a time in shared memory.  200 insertions on 48^3 (6 sites) 4.83 -> 4.54
+// ms, 32 on 96^3 (12 sites) 6.78 -> 6.16 ms against a thread per point.
+constexpr int kSpecPairs = 4;   // k3 pairs per thread
+constexpr int kSpecSites = 16;  // sites staged at a time
+constexpr int kSpec64Threads = 512;
 __global__ void __launch_bounds__(kSpec64Threads) spectrum64_kernel(Spec64Args A) {
-  extern __shared__ double2 sc[];  // [ns][R]: q_s b2_s(k2) b3_s(k3)
-  const int k2 = blockIdx.x, k3a = blockIdx.y * A.R, b = blockIdx.z;
-  const int nr = min(A.R, A.K3 - k3a);
+  extern __shared__ double2 sc[];
+  double2* sp = sc;                      // [kSpecSites][H]: q_s b1_s(k1) b2_s(k2)
+  double2* sd = sc + kSpecSites * A.H;   // [kSpecSites][groups * kSpecPairs]: the pairs' (c, s)
+  const int k2 = blockIdx.x, b = blockIdx.z;
+  const int npair = (A.K3 + 1) / 2, width = A.groups * kSpecPairs, pair0 = blockIdx.y * width;
   const int ns = A.u_nsite[b];
+  const bool even = (A.K1 % 2) == 0, even3 = (A.K3 % 2) == 0;
   const double2* bv = A.bvec + (size_t)b * kMaxSoluteSites * 3 * A.Kmax;
-  for (int t = threadIdx.x; t < ns * nr; t += blockDim.x) {
-    const int s = t / nr, r = t - s * nr;
-    const double q = A.u_q[(size_t)b * kMaxSoluteSites + s];
-    const double2 b2 = bv[(size_t)(s * 3 + 1) * A.Kmax + k2], b3 = bv[(size_t)(s * 3 + 2) * A.Kmax + k3a + r];
-    const double x = q * b2.x, y = q * b2.y;
-    sc[s * A.R + r] = make_double2(x * b3.x - y * b3.y, x * b3.y + y * b3.x);
-  }
-  __syncthreads();
-  const bool even = (A.K1 % 2) == 0;
+  const int ntask = A.groups * A.H;
   double self = 0.0;
-  for (int t = threadIdx.x; t < nr * A.H; t += blockDim.x) {
-    const int r = t / A.H, k1 = t - r * A.H;
-    double re = 0.0, im = 0.0;
-    for (int s = 0; s < ns; ++s) {
-      const double2 c = sc[s * A.R + r];
-      const double2 e = __ldg(bv + (size_t)s * 3 * A.Kmax + k1);
-      re = fma(c.x, e.x, fma(-c.y, e.y, re));
-      im = fma(c.x, e.y, fma(c.y, e.x, im));
+  for (int t0 = 0; t0 < ntask; t0 += blockDim.x) {  // one round unless H is above the CTA's size
+    const int t = t0 + (int)threadIdx.x;
+    const int gr = t / A.H, k1 = t - gr * A.H;
+    const int pa = pair0 + gr * kSpecPairs;
+    const bool on = t < ntask && pa < npair;
+    double2 a[kSpecPairs], c[kSpecPairs];
+#pragma unroll
+    for (int i = 0; i < kSpecPairs; ++i) a[i] = c[i] = make_double2(0.0, 0.0);
+    for (int s0 = 0; s0 < ns; s0 += kSpecSites) {
+      const int n = min(kSpecSites, ns - s0);
+      __syncthreads();
+      for (int i = threadIdx.x; i < n * A.H; i += blockDim.x) {
+        const int s = i / A.H, k = i - s * A.H;
+        const double2* row = bv + (size_t)(s0 + s) * 3 * A.Kmax;
+        const double q = A.u_q[(size_t)b * kMaxSoluteSites + s0 + s];
+        const double2 b2 = row[A.Kmax + k2], b1 = row[k];
+        const double x = q * b2.x, y = q * b2.y;
+        sp[s * A.H + k] = make_double2(x * b1.x - y * b1.y, x * b1.y + y * b1.x);
+      }
+      for (int i = threadIdx.x; i < n * width; i += blockDim.x) {
+        const int s = i / width, p = pair0 + i - s * width;
+        const double2* row = bv + (size_t)(s0 + s) * 3 * A.Kmax + 2 * A.Kmax;
+        double2 v = make_double2(0.0, 0.0);
+        if (p == 0)
+          v = make_double2(row[0].x, even3 ? row[A.K3 / 2].x : 0.0);
+        else if (p < npair)
+          v = row[p];
+        sd[s * width + p - pair0] = v;
+      }
+      __syncthreads();
+      if (on) {
+        const double2* d = sd + gr * kSpecPairs;
+        for (int s = 0; s < n; ++s) {
+          const double2 p = sp[s * A.H + k1];
+#pragma unroll
+          for (int i = 0; i < kSpecPairs; ++i) {
+            const double2 v = d[s * width + i];
+            a[i].x = fma(p.x, v.x, a[i].x);
+            a[i].y = fma(p.y, v.x, a[i].y);
+            c[i].x = fma(p.x, v.y, c[i].x);
+            c[i].y = fma(p.y, v.y, c[i].y);
+          }
+        }
+      }
     }
-    const size_t at = ((size_t)(k3a + r) * A.K2 + k2) * A.H + k1;
-    const double ef = A.engfac[at];
-    const double en = ef * (re * re + im * im);
-    self += (k1 == 0 || (even && k1 == A.H - 1)) ? 0.5 * en : en;
-    A.spec[(size_t)b * A.K3 * A.K2 * A.H + at] = make_double2(ef * re, ef * im);
+    if (on) {
+      const double w = (k1 == 0 || (even && k1 == A.H - 1)) ? 0.5 : 1.0;
+      const size_t plane = (size_t)A.K2 * A.H, at0 = (size_t)k2 * A.H + k1;
+      double2* out = A.spec + (size_t)b * A.K3 * plane + at0;
+#pragma unroll
+      for (int i = 0; i < kSpecPairs; ++i) {
+        const int p = pa + i;
+        if (p >= npair) break;
+        const int lo = p, hi = p == 0 ? A.K3 / 2 : A.K3 - p;  // odd K3: pair 0 has no upper point
+        const double2 x = p == 0 ? a[i] : make_double2(a[i].x - c[i].y, a[i].y + c[i].x);
+        const double2 y = p == 0 ? c[i] : make_double2(a[i].x + c[i].y, a[i].y - c[i].x);
+        const double fl = A.engfac[(size_t)lo * plane + at0];
+        self += w * fl * (x.x * x.x + x.y * x.y);
+        out[(size_t)lo * plane] = make_double2(fl * x.x, fl * x.y);
+        if (p > 0 || even3) {
+          const double fh = A.engfac[(size_t)hi * plane + at0];
+          self += w * fh * (y.x * y.x + y.y * y.y);
+          out[(size_t)hi * plane] = make_double2(fh * y.x, fh * y.y);
+        }
+      }
+    }
   }
   __shared__ double red[kSpec64Threads / 32];
   for (int o = 16; o > 0; o >>= 1) self += __shfl_xor_sync(0xffffffffu, self, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = self;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < kSpec64Threads / 32; ++w) self += red[w];
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) self += red[w];
     A.self_part[((size_t)b * gridDim.y + blockIdx.y) * A.K2 + k2] = self;
   }
 }
 
-// k3 rows per CTA: the count up to 16 whose R H points leave the fewest of the CTA's thread
-// rounds idle
-int spec64_rows(int H) {
+// Groups of k3 pairs per CTA, fixed for a context, so that a placement's self energy does not
+// depend on its batch: one in solution mode, whose single placement makes few CTAs; otherwise
+// the count of the least FP64 work in whole warps, 16 FMA per thread and site and 4 per staged
+// p (at 96^3 2 x 320 threads of 6 groups; the staging is then 5% of the work).
+int spec64_groups(const Engine& e) {
+  const int H = e.H(), all = ((e.geom.K[2] + 1) / 2 + kSpecPairs - 1) / kSpecPairs;
+  if (e.P.slttype == 1) return 1;
   int best = 1;
-  double use = 0.0;
-  for (int R = 1; R <= 16; ++R) {
-    const int n = R * H, rounds = (n + kSpec64Threads - 1) / kSpec64Threads;
-    const double u = (double)n / (rounds * kSpec64Threads);
-    if (u > use + 1e-9) {
-      use = u;
-      best = R;
+  long long cost = 0;
+  for (int g = 1; g <= all && (g == 1 || g * H <= kSpec64Threads); ++g) {
+    const long long parts = (all + g - 1) / g;
+    const long long c = parts * (16LL * ((g * H + 31) / 32) + 4LL * ((H + 31) / 32));
+    if (g == 1 || c < cost) {
+      cost = c;
+      best = g;
     }
   }
   return best;
+}
+int spec64_parts(const Engine& e) {
+  const int width = spec64_groups(e) * kSpecPairs;
+  return ((e.geom.K[2] + 1) / 2 + width - 1) / width;
 }
 
 Coef make_coef(int order, double screen) {
@@ -345,10 +408,7 @@ cudaError_t launch_place_prep(Engine& e, const BatchArgs& a, const double* sol_x
   return cudaGetLastError();
 }
 
-int spectrum64_partials(const Engine& e) {
-  const int R = spec64_rows(e.H());
-  return e.geom.K[1] * ((e.geom.K[2] + R - 1) / R);
-}
+int spectrum64_partials(const Engine& e) { return e.geom.K[1] * spec64_parts(e); }
 
 cudaError_t launch_spectrum64(Engine& e, const BatchArgs& a) {
   Spec64Args A{};
@@ -363,13 +423,14 @@ cudaError_t launch_spectrum64(Engine& e, const BatchArgs& a) {
   A.K3 = e.geom.K[2];
   A.H = e.H();
   A.Kmax = e.Kmax();
-  A.R = spec64_rows(A.H);
-  const size_t smem = sizeof(double2) * kMaxSoluteSites * A.R;
+  A.groups = spec64_groups(e);
+  const size_t smem = sizeof(double2) * kSpecSites * (A.H + A.groups * kSpecPairs);
   static SmemAttr attr;
   cudaError_t err = attr.ensure(spectrum64_kernel, smem);
   if (err != cudaSuccess) return err;
-  const dim3 grid(A.K2, (A.K3 + A.R - 1) / A.R, a.nb);
-  spectrum64_kernel<<<grid, kSpec64Threads, smem, a.stream>>>(A);
+  const dim3 grid(A.K2, spec64_parts(e), a.nb);
+  const int nthr = std::min(kSpec64Threads, (A.groups * A.H + 31) / 32 * 32);
+  spectrum64_kernel<<<grid, nthr, smem, a.stream>>>(A);
   e.count_launch();
   return cudaGetLastError();
 }
