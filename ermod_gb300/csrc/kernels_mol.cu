@@ -47,6 +47,7 @@ struct MolArgs {
   const float* frame_scal;
   const int* mol_to_k;
   int slvmax, nummol;
+  int max_mol_sites;  // of the solvent molecules
   // LJ tables
   const double* ljene;
   const double* ljlensq;
@@ -299,9 +300,12 @@ __device__ __forceinline__ double pair_fp64(const MolArgs& A, int idx, const dou
 // finds its own again.
 constexpr int kBigList = 1024;
 // a pair: near item (11 bits: at most 8 placements of 256 molecules), solute site (8 bits), site
-// of the solvent molecule (13 bits)
+// of the solvent molecule within a window of 8,192 (13 bits); the pass takes larger molecules
+// window by window
+constexpr int kSiteWindowBits = 13;
+constexpr int kListWindows = 64;  // windows that a listed pair's byte holds beside its FP64 parts
 __device__ __forceinline__ unsigned pair_key(int near, int su, int s) {
-  return ((unsigned)near << 21) | ((unsigned)su << 13) | (unsigned)s;
+  return ((unsigned)near << 21) | ((unsigned)su << kSiteWindowBits) | (unsigned)s;
 }
 constexpr int kPairQueue = 64;  // pairs within the cutoffs waiting in a warp's queue: at most 31 + 32
 // the pass's scratch (ints): the list (values, pairs, their order as 16 bits, their FP64 parts as
@@ -937,12 +941,13 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
     const float scale = A.fx_scale_f, reach2 = A.reach2_f;
     unsigned* queue = squeue + wid * kPairQueue;
     int nq = 0;  // warp-uniform
+    int win = 0;  // the window of 8,192 molecule sites that the queue's pairs lie in (block-uniform)
     // the last n pairs of the warp's queue, one per lane
     auto evaluate = [&](int n) {
       __syncwarp();
       if (lane < n) {
         const unsigned key = queue[nq - n + lane];
-        const int near = key >> 21, su_ = (key >> 13) & 0xff, s = key & 0x1fff;
+        const int near = key >> 21, su_ = (key >> 13) & 0xff, s = (int)(key & 0x1fff) + (win << kSiteWindowBits);
         const int nr = snear[near], site = ss0[nr & 0xff] + s;
         const size_t us = (size_t)(g0 + (nr >> 8)) * kMaxSoluteSites + su_;
         const int4 vp = A.site_pos[site], up = a.u_pos[us];
@@ -953,36 +958,41 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
         if (!(parts & kPairCoulomb)) v += __float2ll_rn(eco * scale);
         if (v != 0) fixed_add(sfix + near, sfix + 256 * G + near, v);
         if (parts) {
-          const int q = atomicAdd(&snlist, 1);
-          if (q < kBigList) {
+          // (a window that the byte cannot hold: the items' threads find all their own again)
+          const int q = win < kListWindows ? atomicAdd(&snlist, 1) : atomicMax(&snlist, kBigList + 1);
+          if (q < kBigList && win < kListWindows) {
             sbig[q] = key;
-            sparts[q] = (unsigned char)parts;
+            sparts[q] = (unsigned char)(parts | win << 2);
           }
         }
       }
       __syncwarp();
       nq -= n;
     };
-    for (int task0 = wid * 32; task0 < nnear * nu_max; task0 += 256) {  // warp-uniform
-      const int task = task0 + lane;
-      const int near = nu_max > 1 ? (int)__umulhi((unsigned)task, magic) : task, su_ = task - near * nu_max;
-      int is0 = 0, ins = 0, b = 0;
-      if (near < nnear) {
-        const int nr = snear[near];
-        b = g0 + (nr >> 8);
-        is0 = ss0[nr & 0xff];
-        if (su_ < a.u_nsite[b]) ins = A.slot_site[tile * TILE + (nr & 0xff) + 1] - is0;
+    for (int wbase = 0; wbase < A.max_mol_sites; wbase += 1 << kSiteWindowBits, ++win) {
+      for (int task0 = wid * 32; task0 < nnear * nu_max; task0 += 256) {  // warp-uniform
+        const int task = task0 + lane;
+        const int near = nu_max > 1 ? (int)__umulhi((unsigned)task, magic) : task, su_ = task - near * nu_max;
+        int is0 = 0, ins = 0, b = 0;
+        if (near < nnear) {
+          const int nr = snear[near];
+          b = g0 + (nr >> 8);
+          is0 = ss0[nr & 0xff];
+          if (su_ < a.u_nsite[b]) ins = A.slot_site[tile * TILE + (nr & 0xff) + 1] - is0;
+        }
+        const int4 up = a.u_pos[(size_t)b * kMaxSoluteSites + su_];
+        ins = min(ins - wbase, 1 << kSiteWindowBits);
+        is0 += wbase;
+        for (int s = 0; __any_sync(0xffffffffu, s < ins); ++s) {
+          const bool in = s < ins && pair_r2(A, A.site_pos[is0 + s], up) <= reach2;
+          const unsigned m = __ballot_sync(0xffffffffu, in);
+          if (in) queue[nq + __popc(m & ((1u << lane) - 1u))] = pair_key(near, su_, s);
+          nq += __popc(m);
+          if (nq >= 32) evaluate(32);
+        }
       }
-      const int4 up = a.u_pos[(size_t)b * kMaxSoluteSites + su_];
-      for (int s = 0; __any_sync(0xffffffffu, s < ins); ++s) {
-        const bool in = s < ins && pair_r2(A, A.site_pos[is0 + s], up) <= reach2;
-        const unsigned m = __ballot_sync(0xffffffffu, in);
-        if (in) queue[nq + __popc(m & ((1u << lane) - 1u))] = pair_key(near, su_, s);
-        nq += __popc(m);
-        if (nq >= 32) evaluate(32);
-      }
+      if (nq > 0) evaluate(nq);
     }
-    if (nq > 0) evaluate(nq);
     __syncthreads();
     // FP64 pass over the listed pair parts (overlapping pairs, left out of the FP32 sums): one
     // per thread, so that every FP64 instruction runs on full warps; an item's values are added
@@ -992,11 +1002,12 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
       for (int q = threadIdx.x; q < nlist; q += 256) {
         const unsigned key = sbig[q];
         int rank = 0;
-        for (int i = 0; i < nlist; ++i) rank += sbig[i] < key ? 1 : 0;
+        for (int i = 0; i < nlist; ++i) rank += sbig[i] < key || (sbig[i] == key && sparts[i] < sparts[q]) ? 1 : 0;
         sorder[rank] = (unsigned short)q;
         const int nr = snear[key >> 21];
         const size_t us = (size_t)(g0 + (nr >> 8)) * kMaxSoluteSites + ((key >> 13) & 0xff);
-        sval[q] = pair_fp64(A, ss0[nr & 0xff] + (int)(key & 0x1fff), a.u_x + us * 3, a.u_q[us], a.u_pos[us].w, sparts[q]);
+        const int s = (int)(key & 0x1fff) + ((sparts[q] >> 2) << kSiteWindowBits);
+        sval[q] = pair_fp64(A, ss0[nr & 0xff] + s, a.u_x + us * 3, a.u_q[us], a.u_pos[us].w, sparts[q] & 3);
       }
       __syncthreads();
     }
@@ -1171,6 +1182,7 @@ static MolArgs make_mol_args(Engine& e, const BatchArgs& a) {
   A.mol_to_k = e.d_mol_to_k;
   A.slvmax = e.slvmax;
   A.nummol = e.nummol;
+  A.max_mol_sites = e.max_mol_sites;
   A.ljene = e.d_ljene;
   A.ljlensq = e.d_ljlensq;
   A.ljene_f = e.d_ljene_f;
