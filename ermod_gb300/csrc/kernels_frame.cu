@@ -376,17 +376,14 @@ __global__ void frame_sites_kernel(SiteArgs A) {
       A.site_x[3 * (size_t)idx + 1] = w[1];
       A.site_x[3 * (size_t)idx + 2] = w[2];
       A.site_q[idx] = q;
-      if constexpr (P == 0) {
-        unsigned int X[3];
-        for (int i = 0; i < 3; ++i) {
-          const double u = w[i] * g.invL[i] * 4294967296.0;
-          X[i] = (unsigned int)(unsigned long long)llrint(u);
-        }
-        A.site_pos[idx] = make_int4((int)X[0], (int)X[1], (int)X[2], A.ljtype[a]);
-        A.site_rec[idx] = make_float4((float)tfrac[0], (float)tfrac[1], (float)tfrac[2], (float)q);
-      } else {
-        A.site_pos[idx] = make_int4(0, 0, 0, A.ljtype[a]);
+      // fixed-point coordinates: the mixed path's pairs, and the FP64 path's test of what is in reach
+      unsigned int X[3];
+      for (int i = 0; i < 3; ++i) {
+        const double u = w[i] * g.invL[i] * 4294967296.0;
+        X[i] = (unsigned int)(unsigned long long)llrint(u);
       }
+      A.site_pos[idx] = make_int4((int)X[0], (int)X[1], (int)X[2], A.ljtype[a]);
+      if constexpr (P == 0) A.site_rec[idx] = make_float4((float)tfrac[0], (float)tfrac[1], (float)tfrac[2], (float)q);
     }
   }
   // the largest molecule radius: a warp maximum first, then one atomic per warp on this

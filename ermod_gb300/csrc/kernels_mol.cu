@@ -328,6 +328,10 @@ __device__ __forceinline__ float pair_r2(const MolArgs& A, const int4& vp, const
   return ex * ex + ey * ey + ez * ez;
 }
 
+// a squared distance in FP32 above this is beyond r2 in FP64 too (the fixed-point and FP32
+// roundings are below 1e-6 of it)
+__device__ __forceinline__ float margin_r2(float r2) { return r2 * 1.0001f + 1e-3f; }
+
 // the FP32 terms of one pair at squared distance r2: LJ (0 beyond its cutoff) and screened or
 // bare Coulomb; returns the parts too large for FP32 (above kFp64Lj / kFp64Coulomb in
 // magnitude, or not finite: the comparisons are false for NaN and inf)
@@ -371,23 +375,28 @@ constexpr long long kKeyNegInf = (long long)0x800fffffffffffffull;  // ordered k
 
 // The plain FP64 path: T = 4 TY threads per (solvent molecule, placement).  FP64 runs at 2
 // FMA per clock and SM on GB300, a warp instruction taking as long with one active lane as
-// with 32, so the work is laid out for full lanes: thread t of a molecule takes the stencil
-// columns c1 = t mod 4, + 4, .. (four consecutive doubles of a grid row side by side in a
-// warp's load, and 21 FP64 instructions per site instead of 148 for the plain triple loop)
-// and the stencil rows c2 = t / 4, + TY, ..; of the real-space pairs it takes every T-th,
-// ordered with the solute site fastest so that neighbouring threads evaluate the same solvent
-// site (the LJ branch is then uniform).  TY = 1 in reference mode, where the batch fills the
-// GPU; TY = 4 for a solution-mode frame of few molecules, whose latency is one molecule's
-// serial chain (mol64_ty).  Per placement, against one thread per molecule and one placement
-// per launch: 148 -> 8.3 us (4,000 waters, 6 sites, 48^3), 260 -> 49 us (33,000 waters, 12
-// sites, 96^3); one frame of 1,000 waters at 32^3 167 -> 33 us.
+// with 32, so the work is laid out for full lanes.  Reciprocal part: thread t of a molecule
+// takes the stencil columns c1 = t mod 4, + 4, .. (four consecutive doubles of a grid row side
+// by side in a warp's load, and 21 FP64 instructions per site instead of 148 for the plain
+// triple loop) and the stencil rows c2 = t / 4, + TY, ...  Real space: the warp tests its near
+// molecules' pairs, 32 at a time, in FP32 (with a margin: the FP64 distances decide), and
+// evaluates those that pass on full warps out of a queue; a molecule's values are added by a
+// segmented scan over the queue's order, which is the order of its pairs.  (Each thread
+// evaluating its share of all pairs in FP64, half of them beyond the cutoffs, 21.5 of 32 lanes
+// active: the FP64 pipe 87% busy for 534 us per 64 placements of 4,000 waters and 801 us per 16
+// of 33,000.  200 insertions into 4,000 waters 4.54 -> 3.78 ms, 32 into 33,000 6.23 -> 5.36 ms.)  TY = 1 in reference mode, where the batch fills the GPU; TY = 4 for
+// a solution-mode frame of few molecules, whose latency is one molecule's serial chain (mol64_ty).
 constexpr int kMol64Threads = 256;
+constexpr int kQueue64 = 64;  // pairs waiting in a warp's queue: at most 31 + 32
 template <int P, int TY>
 __global__ void __launch_bounds__(kMol64Threads) mol_energy_kernel(MolArgs A) {
-  constexpr int T = 4 * TY, kMols = kMol64Threads / T;
+  constexpr int T = 4 * TY, kMols = kMol64Threads / T, kWarps = kMol64Threads / 32, kWarpMols = 32 / T;
+  __shared__ int2 squeue[kWarps][kQueue64];  // {molecule of the warp | solute site << 8, site of the molecule}
+  __shared__ double sreal[kMols];
   const int tile = blockIdx.x, b = blockIdx.y;
   const BatchArgs& a = A.a;
   const int sub = threadIdx.x % T;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m = tile * kMols + threadIdx.x / T;
   const bool valid = m < A.slvmax;
   int k = -1, s0 = 0, ns = 0, species = 0;
@@ -403,82 +412,107 @@ __global__ void __launch_bounds__(kMol64Threads) mol_energy_kernel(MolArgs A) {
   const int kskip = (tg >= 0 && tg < A.nummol) ? A.mol_to_k[tg] : -2;
   // a placement rejected by check_mol_configuration has no molecule (engproc.F90:690-691)
   const bool active = valid && (k != kskip) && !(a.skip && a.skip[b]);
-  double recip = 0.0, real = 0.0;
-  if (active) {
-    // ---- reciprocal part ----
-    if (!A.bare) {  // bare Coulomb: no reciprocal part
-      const double* phi = a.phi64 + (size_t)b * K1 * K2 * K3;
-      for (int s = 0; s < ns; ++s) {
-        const int idx = s0 + s;
-        const double* w = A.site_w + (size_t)idx * 3 * P;
-        const int gp = A.site_grid[idx];
-        const int g1 = gp & 1023, g2 = (gp >> 10) & 1023, g3 = (gp >> 20) & 1023;
-        double w3[P];
-        int z[P];
+  double recip = 0.0;
+  // ---- reciprocal part ----
+  if (active && !A.bare) {  // bare Coulomb: no reciprocal part
+    const double* phi = a.phi64 + (size_t)b * K1 * K2 * K3;
+    for (int s = 0; s < ns; ++s) {
+      const int idx = s0 + s;
+      const double* w = A.site_w + (size_t)idx * 3 * P;
+      const int gp = A.site_grid[idx];
+      const int g1 = gp & 1023, g2 = (gp >> 10) & 1023, g3 = (gp >> 20) & 1023;
+      double w3[P];
+      int z[P];
 #pragma unroll
-        for (int c3 = 0; c3 < P; ++c3) {
-          w3[c3] = w[2 * P + c3];
-          z[c3] = wrapi(g3 - c3, K3);
-        }
-        double site = 0.0;
-#pragma unroll
-        for (int c1 = sub & 3; c1 < P; c1 += 4) {
-          const double* col = phi + wrapi(g1 - c1, K1);
-          double line = 0.0;
-#pragma unroll
-          for (int c2 = sub >> 2; c2 < P; c2 += TY) {
-            const double* row = col + (size_t)wrapi(g2 - c2, K2) * K1;
-            double t = 0.0;
-#pragma unroll
-            for (int c3 = 0; c3 < P; ++c3) t = fma(w3[c3], row[(size_t)z[c3] * K1 * K2], t);
-            line = fma(w[P + c2], t, line);
-          }
-          site = fma(w[c1], line, site);
-        }
-        recip = fma(A.site_q[idx], site, recip);
+      for (int c3 = 0; c3 < P; ++c3) {
+        w3[c3] = w[2 * P + c3];
+        z[c3] = wrapi(g3 - c3, K3);
       }
-    }
-    // ---- real space ----
-    const int nu = a.u_nsite[b];
-    const size_t ub = (size_t)b * kMaxSoluteSites;
-    const float rcut = (float)fmax(A.elecut, A.upljcut) + a.u_radius[b] + A.frame_scal[0];
-    double d0 = 0.0;
-    for (int i = 0; i < 3; ++i) {
-      const double h = 0.5 * g.L[i];
-      const double x = fabs(A.site_x[3 * (size_t)s0 + i] - a.u_x[ub * 3 + i]);
-      const double d = g.periodic ? h - fabs(h - x) : x;
-      d0 += d * d;
-    }
-    if (nu > 0 && d0 <= (double)rcut * (double)rcut) {
-      const int npair = nu * ns;
-      int s = sub / nu, su = sub - s * nu;  // pair s nu + su, advanced by T
-      const int ds = T / nu, du = T - ds * nu;
-      for (int p = sub; p < npair; p += T) {
-        real += pair_fp64(A, s0 + s, a.u_x + (ub + su) * 3, a.u_q[ub + su], a.u_pos[ub + su].w,
-                          kPairLj | kPairCoulomb);
-        s += ds;
-        su += du;
-        if (su >= nu) {
-          su -= nu;
-          ++s;
+      double site = 0.0;
+#pragma unroll
+      for (int c1 = sub & 3; c1 < P; c1 += 4) {
+        const double* col = phi + wrapi(g1 - c1, K1);
+        double line = 0.0;
+#pragma unroll
+        for (int c2 = sub >> 2; c2 < P; c2 += TY) {
+          const double* row = col + (size_t)wrapi(g2 - c2, K2) * K1;
+          double t = 0.0;
+#pragma unroll
+          for (int c3 = 0; c3 < P; ++c3) t = fma(w3[c3], row[(size_t)z[c3] * K1 * K2], t);
+          line = fma(w[P + c2], t, line);
         }
+        site = fma(w[c1], line, site);
       }
+      recip = fma(A.site_q[idx], site, recip);
     }
   }
-  // the T threads' parts, in a fixed tree (every thread of the warp takes part)
 #pragma unroll
-  for (int o = 1; o < T; o <<= 1) {
-    recip += __shfl_xor_sync(0xffffffffu, recip, o);
-    real += __shfl_xor_sync(0xffffffffu, real, o);
+  for (int o = 1; o < T; o <<= 1) recip += __shfl_xor_sync(0xffffffffu, recip, o);  // the T threads' parts
+  // ---- real space (every lane of the warp takes part) ----
+  const int nu = a.u_nsite[b];
+  const size_t ub = (size_t)b * kMaxSoluteSites;
+  const float rcut = A.rc_f + a.u_radius[b] + A.frame_scal[0];
+  const bool near = active && nu > 0 && !(pair_r2(A, A.site_pos[s0], a.u_pos[ub]) > margin_r2(rcut * rcut));
+  if (sub == 0) sreal[threadIdx.x / T] = 0.0;
+  __syncwarp();
+  unsigned nearm = __ballot_sync(0xffffffffu, near && sub == 0);
+  if (nearm) {
+    const float reach2 = margin_r2(A.reach2_f);
+    int2* queue = squeue[warp];
+    int nq = 0;  // warp-uniform
+    // the first n pairs of the warp's queue, one per lane; the others move up
+    auto evaluate = [&](int n) {
+      __syncwarp();
+      const bool on = lane < n;
+      const int2 e = on ? queue[lane] : make_int2(kWarpMols, 0);
+      const int mw = e.x & 0xff, su = e.x >> 8;  // mw = kWarpMols: no pair
+      const int site = __shfl_sync(0xffffffffu, s0, (mw * T) & 31) + e.y;
+      double v = 0.0;
+      if (on)
+        v = pair_fp64(A, site, a.u_x + (ub + su) * 3, a.u_q[ub + su], a.u_pos[ub + su].w, kPairLj | kPairCoulomb);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {  // inclusive scan within each molecule's run of lanes
+        const double up = __shfl_up_sync(0xffffffffu, v, o);
+        const int mo = __shfl_up_sync(0xffffffffu, mw, o);
+        if (lane >= o && mo == mw) v += up;
+      }
+      const int next = __shfl_down_sync(0xffffffffu, mw, 1);
+      if (on && (lane == n - 1 || next != mw)) sreal[warp * kWarpMols + mw] += v;
+      const int2 rest = lane < nq - n ? queue[n + lane] : make_int2(0, 0);
+      __syncwarp();
+      if (lane < nq - n) queue[lane] = rest;
+      __syncwarp();
+      nq -= n;
+    };
+    const unsigned magic = nu > 1 ? (unsigned)((0x100000000ull + nu - 1) / nu) : 0u;
+    for (; nearm; nearm &= nearm - 1) {
+      const int owner = __ffs(nearm) - 1, mw = owner / T;
+      const int is0 = __shfl_sync(0xffffffffu, s0, owner), ins = __shfl_sync(0xffffffffu, ns, owner);
+      // pairs with the solute site fastest (32 x nu pairs, whole solvent sites, at a time keep
+      // the division's operand small)
+      for (int sb = 0; sb < ins; sb += 32) {
+        const int npair = min(32, ins - sb) * nu;
+        for (int p0 = 0; p0 < npair; p0 += 32) {
+          const int p = p0 + lane;
+          const int ds = nu > 1 ? (int)__umulhi((unsigned)p, magic) : p, s = sb + ds, su = p - ds * nu;
+          const bool in = p < npair && !(pair_r2(A, A.site_pos[is0 + s], a.u_pos[ub + su]) > reach2);
+          const unsigned mask = __ballot_sync(0xffffffffu, in);
+          if (in) queue[nq + __popc(mask & ((1u << lane) - 1u))] = make_int2(mw | su << 8, s);
+          nq += __popc(mask);
+          if (nq >= 32) evaluate(32);
+        }
+      }
+    }
+    if (nq > 0) evaluate(nq);
+    __syncwarp();
   }
-  const bool owner = active && sub == 0;
+  const bool mine = active && sub == 0;
   double u = 0.0;
   if (valid && sub == 0) {
     if (active) {
-      // residual_ene + assembly (engproc.F90:741-752); bare Coulomb has no such term
-      const double epcl =
-          A.bare ? 0.0 : kPi * a.u_qmol[b] * A.slot_qmol[m] / A.screen / A.screen / g.volume;
-      u = real + (recip - epcl);
+      // residual_ene + assembly (engproc.F90:741-752); bare Coulomb has no such term (factor 0)
+      const double epcl = A.resid_fac * a.u_qmol[b] * A.slot_qmol[m];
+      u = sreal[threadIdx.x / T] + (recip - epcl);
       // ---- getiduv / binsearch ----
       int sp_off = 0, sp_n = 1, sp_soft = 1, ret = 0;
       if (species >= 1 && species <= A.numslv) {
@@ -496,15 +530,13 @@ __global__ void __launch_bounds__(kMol64Threads) mol_energy_kernel(MolArgs A) {
   }
   // per-species partials {sum, min, max} of this block: fixed trees over the warps, then the
   // warps in order
-  constexpr int kWarps = kMol64Threads / 32;
   __shared__ double wsum[kWarps];
   __shared__ long long wmin[kWarps], wmax[kWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int sp = 1; sp <= A.numslv; ++sp) {
-    const bool mine = owner && species == sp;
-    double s = mine ? u : 0.0;
-    long long mn = mine ? ordered_key(u) : kKeyPosInf, mx = mine ? ordered_key(u) : kKeyNegInf;
-    for (int o = 16; o > 0; o >>= 1) {
+    const bool take = mine && species == sp;
+    double s = take ? u : 0.0;
+    long long mn = take ? ordered_key(u) : kKeyPosInf, mx = take ? ordered_key(u) : kKeyNegInf;
+    for (int o = 16; o >= T; o >>= 1) {  // only a molecule's first lane has values
       s += __shfl_xor_sync(0xffffffffu, s, o);
       mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
       mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
