@@ -697,7 +697,7 @@ int ermod_set_topology(ermod_ctx* c, int nummol, int numatm, const int* mbi, con
   e.tagpt.clear();
   std::vector<int> mol_to_k(nummol, -1);
   e.total_charge_phys = 0.0;
-  e.max_mol_sites = 0;
+  e.max_mol_sites = e.max_solute_sites = 0;
   for (int i = 0; i < nummol; ++i) {
     e.numsite[i] = e.mbi0[i + 1] - e.mbi0[i];
     double s = 0.0;  // mol_charge (setconf.F90:832-834)
@@ -708,6 +708,7 @@ int ermod_set_topology(ermod_ctx* c, int nummol, int numatm, const int* mbi, con
       e.tagpt.push_back(i);
       e.max_mol_sites = std::max(e.max_mol_sites, e.numsite[i]);
     }
+    if (sluvid[i] != 0) e.max_solute_sites = std::max(e.max_solute_sites, e.numsite[i]);
   }
   // volcorrect's charge sum in the reference's order (engproc.F90:880-881)
   for (int i = 0; i < nummol; ++i)

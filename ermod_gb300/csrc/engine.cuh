@@ -38,7 +38,7 @@ struct Engine {
   cudaEvent_t cur_ev[8] = {};
 
   // ---- topology ----------------------------------------------------------------
-  int nummol = 0, numatm = 0, ljtype_max = 0, slvmax = 0, nsite_phys = 0, max_mol_sites = 0;
+  int nummol = 0, numatm = 0, ljtype_max = 0, slvmax = 0, nsite_phys = 0, max_mol_sites = 0, max_solute_sites = 0;
   std::vector<int> mbi0;  // 0-based first atom of each molecule, nummol+1 entries
   std::vector<int> sluvid, uvspec, tagpt, numsite, ljtype0;
   std::vector<double> charge, mol_charge;

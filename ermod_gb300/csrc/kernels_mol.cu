@@ -307,18 +307,24 @@ constexpr int kListWindows = 64;  // windows that a listed pair's byte holds bes
 __device__ __forceinline__ unsigned pair_key(int near, int su, int s) {
   return ((unsigned)near << 21) | ((unsigned)su << kSiteWindowBits) | (unsigned)s;
 }
-constexpr int kPairQueue = 64;  // pairs within the cutoffs waiting in a warp's queue: at most 31 + 32
+// Solutes of at least this many sites take the stage that drops an item's solute sites too far
+// from the whole molecule.  256 insertions of 36 sites into 2,000 waters: 309 us without it, 243
+// with it (4,000 of them 13.3 and 12.5 ms); 12 sites into 33,000 waters the same; 6 sites into
+// 4,000 waters, two thirds of whose items pass, 1% slower with it.
+constexpr int kTwoStageSites = 16;
+constexpr int kPairQueue = 64;  // entries waiting in one of a warp's two queues: at most 31 + 32
 // the pass's scratch (ints): the list (values, pairs, their order as 16 bits, their FP64 parts as
 // bytes), the warps' queues, the fixed-point sums of the near items, the molecules' first
 // sites, and the list of near (molecule, placement) items (16 bits)
-__host__ __device__ constexpr int finish_scratch_ints(int G) {  // for the larger tile, 256
-  return 2 * kBigList + kBigList + kBigList / 2 + kBigList / 4 + 8 * kPairQueue + 2 * 256 * G + 256 + G * 256 / 2;
+__host__ __device__ constexpr int finish_scratch_ints(int G, bool two) {  // for the larger tile, 256
+  return 2 * kBigList + kBigList + kBigList / 2 + kBigList / 4 + (two ? 2 : 1) * 8 * kPairQueue + 2 * 256 * G + 256 +
+         G * 256 / 2;
 }
 // the dynamic shared memory of the finish kernel before its edge keys: the block
 // histograms (when in shared memory) or the real-space pass's scratch, whichever is larger
-__host__ __device__ __forceinline__ int finish_region_ints(int G, int ermax, int hist_global) {
+__host__ __device__ __forceinline__ int finish_region_ints(int G, bool two, int ermax, int hist_global) {
   const int h = hist_global ? 0 : G * ermax;
-  return h > finish_scratch_ints(G) ? h : finish_scratch_ints(G);
+  return h > finish_scratch_ints(G, two) ? h : finish_scratch_ints(G, two);
 }
 
 __device__ __forceinline__ float pair_r2(const MolArgs& A, const int4& vp, const int4& up) {
@@ -814,18 +820,21 @@ __device__ __forceinline__ void species_partials(const MolArgs& A, const BatchAr
 // exactly against the FP64 edges), histograms and per-species partials.
 //
 // The real-space pass: the block's (molecule, placement) items within the solute's bounding
-// sphere + cutoff are compacted into a list (2% of the 33,000-water box's molecules); a thread
-// takes an item and a solute site, and the pairs within the cutoffs -- a fifth of the tested
-// ones for a 36-site solute -- go through a queue per warp, so that the evaluation, ten times
-// as long as the test, runs on full warps.  Its terms are added as fixed-point integers, in
-// any order.  (A few threads per item, each walking its pairs: 19 of 32 lanes active and four
-// times the instructions, 438 us for 256 insertions of a 36-site solute into 2,000 waters,
-// now 280; 12 sites into 33,000 waters 340, now 314.)
+// sphere + cutoff are compacted into a list (2% of the 33,000-water box's molecules).  A thread
+// takes an item and a solute site; for large solutes, those whose first molecule site lies
+// within the cutoff and the largest molecule's radius -- a sixth at 36 sites -- go through a
+// queue per warp to the test of each of the molecule's sites, and the pairs within the cutoffs
+// through another one to the evaluation, so that each stage, several times as long as the one
+// before, runs on full warps.  The terms are added as fixed-point integers, in any order.  (A
+// few threads per item, each walking its pairs: 19 of 32 lanes active, 438 us for 256
+// insertions of a 36-site solute into 2,000 waters, now 243; 12 sites into 33,000 waters 340,
+// now 294.)
 //
 // Four blocks per SM (64 registers): 2-3% faster over a whole run than three of 80.
 // TILE: molecules per block of 256 threads.  64 in solution mode, where a frame's one placement
 // makes few blocks and the real-space pass takes all 256 threads.
-template <int G, int TILE>
+// kTwo: the stage before the pairs' test, for solutes of many sites (kTwoStageSites).
+template <int G, int TILE, bool kTwo>
 __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const float* __restrict__ site_e) {
   extern __shared__ __align__(16) int smem_dyn[];
   // [G][ermax] block histograms, or none when they would not fit beside other blocks: the
@@ -833,13 +842,13 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
   // Before the histograms are zeroed, the same region holds the real-space pass's scratch
   // (finish_scratch_ints ints).
   int* smem_hist = A.hist_global ? nullptr : smem_dyn;
-  int* skeys = smem_dyn + finish_region_ints(G, A.ermax, A.hist_global);  // [ermax] 32-bit edge keys
+  int* skeys = smem_dyn + finish_region_ints(G, kTwo, A.ermax, A.hist_global);  // [ermax] 32-bit edge keys
   double* sval = reinterpret_cast<double*>(smem_dyn);                           // [kBigList] FP64 values of the list
   unsigned* sbig = reinterpret_cast<unsigned*>(sval + kBigList);                // [kBigList] the list's pairs
   unsigned short* sorder = reinterpret_cast<unsigned short*>(sbig + kBigList);  // [kBigList] in the pairs' order
   unsigned char* sparts = reinterpret_cast<unsigned char*>(sorder + kBigList);  // [kBigList] the parts left out
-  unsigned* squeue = reinterpret_cast<unsigned*>(sparts + kBigList);            // [8][kPairQueue]
-  unsigned* sfix = squeue + 8 * kPairQueue;                                     // [2][G * 256] sums, low and high words
+  unsigned* squeue = reinterpret_cast<unsigned*>(sparts + kBigList);            // [1 or 2][8][kPairQueue]
+  unsigned* sfix = squeue + (kTwo ? 16 : 8) * kPairQueue;                                    // [2][G * 256] sums, low and high words
   int* ss0 = reinterpret_cast<int*>(sfix + 2 * 256 * G);                        // [256] first sites
   unsigned short* snear = reinterpret_cast<unsigned short*>(ss0 + 256);         // [G * 256] molecule | placement << 8
   __shared__ int swarp[8];
@@ -971,7 +980,10 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
     const int nu_max = snu;
     const unsigned magic = nu_max > 1 ? (unsigned)((0x100000000ull + nu_max - 1) / nu_max) : 0u;
     const float scale = A.fx_scale_f, reach2 = A.reach2_f;
+    // beyond this a molecule's first site is too far from a solute site for any pair of the two
+    const float mol_reach = sqrtf(reach2) + A.frame_scal[0], mol_reach2 = margin_r2(mol_reach * mol_reach);
     unsigned* queue = squeue + wid * kPairQueue;
+    [[maybe_unused]] unsigned* cand = queue + 8 * kPairQueue;
     int nq = 0;  // warp-uniform
     int win = 0;  // the window of 8,192 molecule sites that the queue's pairs lie in (block-uniform)
     // the last n pairs of the warp's queue, one per lane
@@ -1001,27 +1013,52 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
       __syncwarp();
       nq -= n;
     };
+    const int total = nnear * nu_max;
     for (int wbase = 0; wbase < A.max_mol_sites; wbase += 1 << kSiteWindowBits, ++win) {
-      for (int task0 = wid * 32; task0 < nnear * nu_max; task0 += 256) {  // warp-uniform
-        const int task = task0 + lane;
-        const int near = nu_max > 1 ? (int)__umulhi((unsigned)task, magic) : task, su_ = task - near * nu_max;
-        int is0 = 0, ins = 0, b = 0;
-        if (near < nnear) {
-          const int nr = snear[near];
-          b = g0 + (nr >> 8);
-          is0 = ss0[nr & 0xff];
-          if (su_ < a.u_nsite[b]) ins = A.slot_site[tile * TILE + (nr & 0xff) + 1] - is0;
+      int nc = 0;  // candidates waiting: at most 31 + 32 (warp-uniform)
+      for (int task0 = wid * 32;; task0 += 256) {
+        const bool more = task0 < total;  // warp-uniform
+        bool on = false;                  // the lane's candidate
+        unsigned key = 0u;
+        if (more) {
+          const int task = task0 + lane;
+          const int near = nu_max > 1 ? (int)__umulhi((unsigned)task, magic) : task, su_ = task - near * nu_max;
+          key = pair_key(near, su_, 0);
+          if (near < nnear) {
+            const int nr = snear[near], b = g0 + (nr >> 8);
+            on = su_ < a.u_nsite[b];
+            if (kTwo && on)
+              on = !(pair_r2(A, A.site_pos[ss0[nr & 0xff]], a.u_pos[(size_t)b * kMaxSoluteSites + su_]) > mol_reach2);
+          }
         }
-        const int4 up = a.u_pos[(size_t)b * kMaxSoluteSites + su_];
-        ins = min(ins - wbase, 1 << kSiteWindowBits);
-        is0 += wbase;
+        if constexpr (kTwo) {  // wait for 32 of them
+          const unsigned m = __ballot_sync(0xffffffffu, on);
+          if (on) cand[nc + __popc(m & ((1u << lane) - 1u))] = key;
+          nc += __popc(m);
+          if (more && nc < 32) continue;
+          const int n = min(nc, 32);
+          __syncwarp();
+          on = lane < n;
+          if (on) key = cand[nc - n + lane];
+          __syncwarp();
+          nc -= n;
+        }
+        int is0 = 0, ins = 0;
+        int4 up = make_int4(0, 0, 0, 0);
+        if (on) {
+          const int nr = snear[key >> 21];
+          is0 = ss0[nr & 0xff] + wbase;
+          ins = min(A.slot_site[tile * TILE + (nr & 0xff) + 1] - is0, 1 << kSiteWindowBits);
+          up = a.u_pos[(size_t)(g0 + (nr >> 8)) * kMaxSoluteSites + ((key >> kSiteWindowBits) & 0xff)];
+        }
         for (int s = 0; __any_sync(0xffffffffu, s < ins); ++s) {
           const bool in = s < ins && pair_r2(A, A.site_pos[is0 + s], up) <= reach2;
           const unsigned m = __ballot_sync(0xffffffffu, in);
-          if (in) queue[nq + __popc(m & ((1u << lane) - 1u))] = pair_key(near, su_, s);
+          if (in) queue[nq + __popc(m & ((1u << lane) - 1u))] = key | (unsigned)s;
           nq += __popc(m);
           if (nq >= 32) evaluate(32);
         }
+        if (!more) break;
       }
       if (nq > 0) evaluate(nq);
     }
@@ -1322,19 +1359,24 @@ cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a) {
     e.phase_begin_on(PH_MOL, a.stream);
   }
   // step 2: per-molecule totals and binning (histograms + edge keys in shared memory)
-  const size_t smem_f = sizeof(int) * ((size_t)finish_region_ints(G, e.ermax, A.hist_global) + e.ermax);
+  const bool two = e.tile == 256 && e.max_solute_sites >= kTwoStageSites;
+  const size_t smem_f = sizeof(int) * ((size_t)finish_region_ints(G, two, e.ermax, A.hist_global) + e.ermax);
   dim3 g2((a.nb + G - 1) / G, e.ntile);
-#define ERMOD_FINISH(GG, TILE)                                                                             \
-  if (G == GG && e.tile == TILE) {                                                                         \
-    static SmemAttr attr;                                                                                  \
-    if ((err = attr.ensure(mol_finish_kernel<GG, TILE>, smem_f)) != cudaSuccess) return err;               \
-    mol_finish_kernel<GG, TILE><<<g2, 256, smem_f, a.stream>>>(A, a.site_e);                               \
+#define ERMOD_FINISH(GG, TILE, TWO)                                                                             \
+  if (G == GG && e.tile == TILE && two == TWO) {                                                               \
+    static SmemAttr attr;                                                                                      \
+    if ((err = attr.ensure(mol_finish_kernel<GG, TILE, TWO>, smem_f)) != cudaSuccess) return err;              \
+    mol_finish_kernel<GG, TILE, TWO><<<g2, 256, smem_f, a.stream>>>(A, a.site_e);                              \
   }
-  ERMOD_FINISH(1, 64)
-  ERMOD_FINISH(1, 256)
-  ERMOD_FINISH(2, 256)
-  ERMOD_FINISH(4, 256)
-  ERMOD_FINISH(8, 256)
+  ERMOD_FINISH(1, 64, false)
+  ERMOD_FINISH(1, 256, false)
+  ERMOD_FINISH(2, 256, false)
+  ERMOD_FINISH(4, 256, false)
+  ERMOD_FINISH(8, 256, false)
+  ERMOD_FINISH(1, 256, true)
+  ERMOD_FINISH(2, 256, true)
+  ERMOD_FINISH(4, 256, true)
+  ERMOD_FINISH(8, 256, true)
 #undef ERMOD_FINISH
   e.count_launch();
   return cudaGetLastError();
