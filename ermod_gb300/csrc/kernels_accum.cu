@@ -203,6 +203,7 @@ __device__ int accumulate_scalars(const AccArgs& A) {
     }
     if (nb > 0 && A.rigid && A.scal[6] == 0.0) {
       A.scal[5] = a.u_usreal[0];
+      __threadfence();  // place_prep of a batch on another stream may see the flag
       A.scal[6] = 1.0;
     }
     s_voffset = A.scal[3];

@@ -60,6 +60,8 @@ struct PrepArgs {
   int nummol;
   int bare;  // cltype 0
   unsigned mK[3];  // ceil(2^32 / d): n / d = umulhi(n, m) for n d < 2^32
+  unsigned mKh[3];  // the same for K / 2 + 1
+  const double* usreal_known;  // rigid solutes: nonzero once the context holds realcal_self's value
   DevStatus* status;
 };
 
@@ -73,7 +75,8 @@ __device__ __forceinline__ void wrap_coord(const double* v, double x0raw, const 
 
 // 1-D structure factors of one axis of one placement's solute: FP64 weights
 // (calc_spline_molecule on the raw coordinates) and twiddles; the mixed path rounds them to
-// FP32 once at the end, so that their errors are independent roundings
+// FP32 once at the end, so that their errors are independent roundings.  Half of the range is
+// computed, the other half is its conjugate
 __device__ void structure_factors(const PrepArgs& A, int b, int atom0, int ns, int ax) {
   __shared__ double th[kMaxSoluteSites * kMaxSplineOrder];
   __shared__ int sgrd[kMaxSoluteSites];
@@ -93,9 +96,10 @@ __device__ void structure_factors(const PrepArgs& A, int b, int atom0, int ns, i
   __syncthreads();
   const int Kmax = max(g.K[0], max(g.K[1], g.K[2]));
   const double2* tw = A.twiddle64 + (ax == 0 ? 0 : (ax == 1 ? g.K[0] : g.K[0] + g.K[1]));
-  const unsigned mk = A.mK[ax];
-  for (int t = threadIdx.x; t < ns * K; t += blockDim.x) {
-    const int s = (int)__umulhi((unsigned)t, mk), k = t - s * K;
+  const unsigned mk = A.mK[ax], mh = A.mKh[ax];
+  const int Kh = K / 2 + 1;
+  for (int t = threadIdx.x; t < ns * Kh; t += blockDim.x) {
+    const int s = (int)__umulhi((unsigned)t, mh), k = t - s * Kh;
     const int grd = sgrd[s];
     double re = 0.0, im = 0.0;
     for (int c = 0; c < P; ++c) {
@@ -107,11 +111,16 @@ __device__ void structure_factors(const PrepArgs& A, int b, int atom0, int ns, i
       re = fma(th[s * P + c], w.x, re);
       im = fma(th[s * P + c], w.y, im);
     }
-    const size_t at = (((size_t)b * kMaxSoluteSites + s) * 3 + ax) * Kmax + k;
-    if (A.mixed)
-      a.u_bvec[at] = make_float2((float)re, (float)im);
-    else
-      a.u_bvec64[at] = make_double2(re, im);
+    const size_t row = (((size_t)b * kMaxSoluteSites + s) * 3 + ax) * Kmax;
+    const bool two = k > 0 && 2 * k < K;  // K - k is another point
+    if (A.mixed) {
+      const float2 v = make_float2((float)re, (float)im);
+      a.u_bvec[row + k] = v;
+      if (two) a.u_bvec[row + K - k] = make_float2(v.x, -v.y);
+    } else {
+      a.u_bvec64[row + k] = make_double2(re, im);
+      if (two) a.u_bvec64[row + K - k] = make_double2(re, -im);
+    }
   }
 }
 
@@ -187,31 +196,36 @@ __global__ void __launch_bounds__(256) place_prep_kernel(PrepArgs A) {
   }
   __syncthreads();
   if (threadIdx.x == 0) a.u_radius[b] = __int_as_float(rmax_bits) * 1.0001f + 1e-4f;
-  // realcal_self (realcal.F90:284-328), fixed-order block reduction
-  const bool need_self = (A.self_mode == 1) || (A.self_mode == 2 && b == 0);
+  // realcal_self (realcal.F90:284-328), fixed-order block reduction.  A rigid solute's is taken
+  // from the context's first placement (the accumulation keeps it), so that later batches' blocks
+  // are spared the longest chain of the kernel; it is read here only as a flag
+  const bool need_self =
+      (A.self_mode == 1) || (A.self_mode == 2 && b == 0 && *(const volatile double*)A.usreal_known == 0.0);
   if (need_self && A.bare) {  // realcal_self returns 0 for bare Coulomb (realcal.F90:294)
     if (threadIdx.x == 0) a.u_usreal[b] = 0.0;
     return;
   }
   if (need_self) {
     double acc = 0.0;
-    const int npair = ns * ns;  // (is, js) with js >= is; diagonal gives the atom residual
-    for (int t = threadIdx.x; t < npair; t += blockDim.x) {
-      const int is = t / ns, js = t % ns;
-      if (js < is) continue;
+    for (int is = threadIdx.x; is < ns; is += blockDim.x) {  // the diagonal gives the atoms' residuals
       const double qi = A.charge[atom0 + is];
-      if (js == is) {
-        acc += -qi * qi * A.sc.screen / sqrt(kPi);
-      } else {
-        double d2 = 0.0;
-        for (int i = 0; i < 3; ++i) {
-          const double h = 0.5 * g.L[i];
-          const double d = h - fabs(h - fabs(sx[is][i] - sx[js][i]));
-          d2 += d * d;
-        }
-        const double rst = sqrt(d2);
-        acc += -qi * A.charge[atom0 + js] * erf(A.sc.screen * rst) / rst;
+      acc += -qi * qi * A.sc.screen / sqrt(kPi);
+    }
+    // every pair once, as (is, is + d mod ns), d up to ns / 2 (half of the last row when ns is
+    // even), so that no lane idles through an erf
+    const int half = ns / 2;
+    for (int t = threadIdx.x; t < ns * half; t += blockDim.x) {
+      const int d = t / ns + 1, is = t - (d - 1) * ns;
+      if (2 * d == ns && is >= half) continue;
+      const int js = is + d < ns ? is + d : is + d - ns;
+      double d2 = 0.0;
+      for (int i = 0; i < 3; ++i) {
+        const double h = 0.5 * g.L[i];
+        const double x = h - fabs(h - fabs(sx[is][i] - sx[js][i]));
+        d2 += x * x;
       }
+      const double rst = sqrt(d2);
+      acc += -A.charge[atom0 + is] * A.charge[atom0 + js] * erf(A.sc.screen * rst) / rst;
     }
     red[threadIdx.x] = acc;
     __syncthreads();
@@ -402,7 +416,11 @@ cudaError_t launch_place_prep(Engine& e, const BatchArgs& a, const double* sol_x
   A.nummol = e.nummol;
   A.status = e.d_status;
   auto magic = [](unsigned d) { return (unsigned)((0x100000000ull + d - 1) / d); };
-  for (int i = 0; i < 3; ++i) A.mK[i] = magic((unsigned)e.geom.K[i]);
+  for (int i = 0; i < 3; ++i) {
+    A.mK[i] = magic((unsigned)e.geom.K[i]);
+    A.mKh[i] = magic((unsigned)(e.geom.K[i] / 2 + 1));
+  }
+  A.usreal_known = e.d_scal + 6;
   place_prep_kernel<<<dim3(a.nb, A.bare ? 1 : 4), 256, 0, s>>>(A);
   e.count_launch();
   return cudaGetLastError();
