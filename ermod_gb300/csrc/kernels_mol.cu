@@ -1456,8 +1456,13 @@ struct AdjArgs {
   int* val;                // [slvmax] slot index
 };
 
+// A thread per (molecule, site of the chunk), sites fastest: a molecule's site terms and its
+// derivatives are then consecutive words, and a solution-mode frame's few thousand molecules
+// fill the GPU (a thread per molecule walking the sites: 39 us of latency for 8,000 waters and
+// 16 sites, 32 CTAs).
 __global__ void __launch_bounds__(256) adjoint_mol_kernel(MolArgs A, AdjArgs J) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  const long long task = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int m = (int)(task / J.nchunk), j = (int)(task - (long long)m * J.nchunk);
   if (m >= A.slvmax) return;
   const BatchArgs& a = A.a;
   const int b = J.b;
@@ -1469,7 +1474,7 @@ __global__ void __launch_bounds__(256) adjoint_mol_kernel(MolArgs A, AdjArgs J) 
   const int kskip = (tg >= 0 && tg < A.nummol) ? A.mol_to_k[tg] : -2;
   bool take = (tg + 1 == J.adj_mol) && (k != kskip) && species >= 1 && species <= A.numslv &&
               !(a.skip && a.skip[b]);
-  if (J.first) {
+  if (J.first && j == 0) {
     // the molecule's bin as the finish kernel found it (ermax: not binned)
     const int key = take ? J.mol_bin[m] : A.ermax;
     J.key[m] = key;
@@ -1491,40 +1496,38 @@ __global__ void __launch_bounds__(256) adjoint_mol_kernel(MolArgs A, AdjArgs J) 
   const float dz0 = (float)(int)((unsigned)p0.z - (unsigned)q0.z) * fz;
   const float rcut = A.rc_f + a.u_radius[b] + A.frame_scal[0];
   const bool near = dx0 * dx0 + dy0 * dy0 + dz0 * dz0 <= rcut * rcut;
-  for (int j = 0; j < J.nchunk; ++j) {
-    const int s = J.s_begin + j;
-    float dq = -rq, deps = 0.f, dsig = 0.f;
-    for (int t = 0; t < ns; ++t) dq += J.site_e_ps[(size_t)(s0 + t) * A.ldb + j];
-    if (near) {
-      const int4 up = a.u_pos[ub + s];
-      const float2 par = J.par[s];
-      for (int t = 0; t < ns; ++t) {
-        const int4 vp = A.site_pos[s0 + t];
-        const float ex = (float)(int)((unsigned)vp.x - (unsigned)up.x) * fx;
-        const float ey = (float)(int)((unsigned)vp.y - (unsigned)up.y) * fy;
-        const float ez = (float)(int)((unsigned)vp.z - (unsigned)up.z) * fz;
-        const float r2 = ex * ex + ey * ey + ez * ez;
-        const float ljeps = A.ljene_f[vp.w + A.T * up.w];
-        if (ljeps > 0.f && r2 <= k32.up2) {
-          const float x = A.ljlensq_f[vp.w + A.T * up.w];
-          float va, vb;
-          lj_parts_f(A.ljswitch, k32, x, r2, va, vb);
-          if (par.x > 0.f) deps += 4.f * ljeps * (va - vb) / (2.f * par.x);
-          const float dldx = 4.f * ljeps * (6.f * va - 3.f * vb) / x;
-          const float dxds = (J.cmbrule == 0) ? sqrtf(x) : (par.y > 0.f ? x / par.y : 0.f);
-          dsig += dldx * dxds;
-        }
-        if (r2 <= k32.ele2) {
-          const float r = sqrtf(r2);
-          dq += A.site_rec[s0 + t].w * erfcf(beta * r) / r;
-        }
+  const int s = J.s_begin + j;
+  float dq = -rq, deps = 0.f, dsig = 0.f;
+  for (int t = 0; t < ns; ++t) dq += J.site_e_ps[(size_t)(s0 + t) * A.ldb + j];
+  if (near) {
+    const int4 up = a.u_pos[ub + s];
+    const float2 par = J.par[s];
+    for (int t = 0; t < ns; ++t) {
+      const int4 vp = A.site_pos[s0 + t];
+      const float ex = (float)(int)((unsigned)vp.x - (unsigned)up.x) * fx;
+      const float ey = (float)(int)((unsigned)vp.y - (unsigned)up.y) * fy;
+      const float ez = (float)(int)((unsigned)vp.z - (unsigned)up.z) * fz;
+      const float r2 = ex * ex + ey * ey + ez * ez;
+      const float ljeps = A.ljene_f[vp.w + A.T * up.w];
+      if (ljeps > 0.f && r2 <= k32.up2) {
+        const float x = A.ljlensq_f[vp.w + A.T * up.w];
+        float va, vb;
+        lj_parts_f(A.ljswitch, k32, x, r2, va, vb);
+        if (par.x > 0.f) deps += 4.f * ljeps * (va - vb) / (2.f * par.x);
+        const float dldx = 4.f * ljeps * (6.f * va - 3.f * vb) / x;
+        const float dxds = (J.cmbrule == 0) ? sqrtf(x) : (par.y > 0.f ? x / par.y : 0.f);
+        dsig += dldx * dxds;
+      }
+      if (r2 <= k32.ele2) {
+        const float r = sqrtf(r2);
+        dq += A.site_rec[s0 + t].w * erfcf(beta * r) / r;
       }
     }
-    float* o = J.du + (size_t)m * P + 3 * s;
-    o[0] = dq;
-    o[1] = deps;
-    o[2] = dsig;
   }
+  float* o = J.du + (size_t)m * P + 3 * s;
+  o[0] = dq;
+  o[1] = deps;
+  o[2] = dsig;
 }
 
 // the chunk's unit-charge single-site placements: site s_begin + j of placement b
@@ -1564,6 +1567,85 @@ __global__ void adjoint_reduce_kernel(const int* __restrict__ val, const float* 
     grad[(size_t)p * ermax + bin] += w * acc;
   }
   if (threadIdx.x == 0) wsum[bin] += w * (double)(i1 - i0);
+}
+
+// The same sums without a sort: CTA per bin, which lists its molecules in slot order from the
+// keys, 4,096 at a time, and adds their derivatives, a thread per parameter (at most kAdjPar
+// of each).  Every CTA reads every key: n ermax of them cost less than the sort's six launches
+// until kAdjDirect (8,000 molecules and 1,396 bins, a third of it: 27 us against 23 for the sums of
+// sorted molecules and 40 for the sort and the bounds; the rest is the fullest bin's chain of FP64
+// additions, whose order is the slots').  An adjoint frame of that size 454 -> 372 us with the
+// derivatives' kernel split over the sites.
+// a float as a double by integer operations (exact): the conversion instruction is the FP64 pipe's,
+// 64 clocks of a scheduler for a warp, as long as the addition that it feeds
+__device__ __forceinline__ double widen(float f) {
+  const unsigned u = __float_as_uint(f), mag = u & 0x7fffffffu;
+  if (mag - 1u < 0x007fffffu || mag >= 0x7f800000u) return (double)f;  // subnormal, infinite or NaN
+  const unsigned hi = (u & 0x80000000u) | (mag == 0u ? 0u : (mag >> 3) + 0x38000000u);
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+constexpr int kAdjThreads = 256, kAdjWindow = 4096;
+constexpr int kAdjPar = (3 * kMaxSoluteSites + kAdjThreads - 1) / kAdjThreads;
+constexpr long long kAdjDirect = 1ll << 25;
+__global__ void __launch_bounds__(kAdjThreads) adjoint_bins_kernel(const int* __restrict__ key, int n,
+                                                                   const float* __restrict__ du, int P,
+                                                                   const double* __restrict__ engnmfc, int b, int ermax,
+                                                                   double* grad, double* wsum) {
+  constexpr int kWarps = kAdjThreads / 32, kPer = kAdjWindow / kAdjThreads;
+  __shared__ int list[kAdjWindow];
+  __shared__ int wcount[kWarps];
+  const int bin = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double acc[kAdjPar];
+#pragma unroll
+  for (int i = 0; i < kAdjPar; ++i) acc[i] = 0.0;
+  int count = 0;
+  for (int w0 = 0; w0 < n; w0 += kAdjWindow) {
+    unsigned m[kPer];
+    int own = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {  // the warp's keys in order: 32 kPer consecutive ones
+      const int at = w0 + (warp * kPer + i) * 32 + lane;
+      m[i] = __ballot_sync(0xffffffffu, at < n && __ldg(key + min(at, n - 1)) == bin);
+      own += __popc(m[i]);
+    }
+    if (lane == 0) wcount[warp] = own;
+    if (!__syncthreads_or(own)) continue;  // most bins hold few molecules
+    int at = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      if (w < warp) at += wcount[w];
+      total += wcount[w];
+    }
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      if (m[i] >> lane & 1u) list[at + __popc(m[i] & ((1u << lane) - 1u))] = w0 + (warp * kPer + i) * 32 + lane;
+      at += __popc(m[i]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kAdjPar; ++i) {
+      const int p = threadIdx.x + i * kAdjThreads;
+      if (p >= P) break;
+      for (int q = 0; q < total; q += 16) {  // 16 loads in flight; the adds in slot order
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = q + k < total ? du[(size_t)list[q + k] * P + p] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+          if (q + k < total) acc[i] += widen(v[k]);
+      }
+    }
+    count += total;
+    __syncthreads();  // the list is used again
+  }
+  if (count == 0) return;
+  const double w = engnmfc[b];
+#pragma unroll
+  for (int i = 0; i < kAdjPar; ++i) {
+    const int p = threadIdx.x + i * kAdjThreads;
+    if (p < P) grad[(size_t)p * ermax + bin] += w * acc[i];
+  }
+  if (threadIdx.x == 0) wsum[bin] += w * (double)count;
 }
 
 int key_bits(int ermax) {
@@ -1620,9 +1702,16 @@ cudaError_t launch_adjoint(Engine& e, const BatchArgs& a, cudaStream_t s) {
       J.du = e.d_adj_du;
       J.key = key;
       J.val = val;
-      adjoint_mol_kernel<<<(n + 255) / 256, 256, 0, s>>>(A, J);
+      adjoint_mol_kernel<<<(unsigned)(((long long)n * nch + 255) / 256), 256, 0, s>>>(A, J);
       e.count_launch();
       if ((err = cudaGetLastError()) != cudaSuccess) return err;
+    }
+    if ((long long)n * e.ermax <= kAdjDirect) {
+      adjoint_bins_kernel<<<e.ermax, kAdjThreads, 0, s>>>(key, n, e.d_adj_du, P, a.engnmfc, b, e.ermax, e.d_adj_grad,
+                                                          e.d_adj_w);
+      e.count_launch();
+      if ((err = cudaGetLastError()) != cudaSuccess) return err;
+      continue;
     }
     size_t bytes = e.adj_cub_bytes;
     err = cub::DeviceRadixSort::SortPairs(e.d_adj_cub, bytes, key, key_s, val, val_s, n, 0, key_bits(e.ermax), s);
