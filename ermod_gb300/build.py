@@ -19,9 +19,9 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libermod_gb300.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["engine.cu", "kernels_frame.cu", "kernels_place.cu", "kernels_fft.cu", "kernels_mol.cu",
+SOURCES = ["engine.cu", "kernels_frame.cu", "kernels_place.cu", "kernels_fft.cu", "kernels_fft64.cu", "kernels_mol.cu",
            "kernels_accum.cu", "kernels_insert.cu", "host_setup.cpp"]
-HEADERS = ["engine.cuh", "ermod_internal.cuh", "async_copy.cuh", "bestfit.cuh"]
+HEADERS = ["engine.cuh", "ermod_internal.cuh", "async_copy.cuh", "bestfit.cuh", "dft.cuh"]
 
 
 def nvcc() -> str:

@@ -338,9 +338,14 @@ static int ensure_batch(Engine& e) {
   return ERMOD_OK;
 }
 
-// FP64 path: the batch's inverse transforms, as cuFFT plans of powers of two (a call's last
-// batch may hold any number of placements; each size is planned once, when first needed)
+// FP64 path: the batch's inverse transforms, by the kernels of this library or, for lengths with
+// other factors than 2, 3 and 5, as cuFFT plans of powers of two (a call's last batch may hold
+// any number of placements; each size is planned once, when first needed)
 static int inverse_fft64(Engine& e, const BatchArgs& a) {
+  if (fft64_fits(e.geom.K[0], e.geom.K[1], e.geom.K[2])) {
+    ERMOD_CUDA(launch_fft64(e, a));
+    return ERMOD_OK;
+  }
   const size_t nr = e.grid_real(), nc = e.grid_cplx();
   int done = 0;
   for (int lg = kFp64MaxLog2; lg >= 0; --lg) {

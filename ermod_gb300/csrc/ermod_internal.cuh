@@ -265,6 +265,8 @@ cudaError_t launch_place_prep(Engine& e, const BatchArgs& a, const double* sol_x
 cudaError_t launch_pme_mixed(Engine& e, const BatchArgs& a);
 bool pme_fits(int K1, int K2, int K3);
 cudaError_t launch_spectrum64(Engine& e, const BatchArgs& a);
+bool fft64_fits(int K1, int K2, int K3);  // lengths with factors 2, 3 and 5
+cudaError_t launch_fft64(Engine& e, const BatchArgs& a);
 // per-molecule energies and histograms
 cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a);
 cudaError_t launch_gather(Engine& e, const BatchArgs& a);

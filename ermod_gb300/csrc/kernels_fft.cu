@@ -17,166 +17,13 @@
 // registers), unnormalised, sign +1, exactly the conventions of fft_iface.F90.
 #include <cooperative_groups.h>
 
+#include "dft.cuh"
 #include "engine.cuh"
 
 namespace ermod {
 
 namespace {
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 mul_i(float2 a) { return make_float2(-a.y, a.x); }  // a * i
-
-// ---- in-register inverse DFTs: Y[q] = sum_r v[r] exp(+2 pi i r q / R) ----------------
-template <int R>
-struct Dft;
-
-template <>
-struct Dft<2> {
-  static __device__ __forceinline__ void run(float2* v) {
-    const float2 a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
-  }
-};
-template <>
-struct Dft<3> {
-  static __device__ __forceinline__ void run(float2* v) {
-    const float c = -0.5f, s = 0.86602540378443864676f;  // exp(2 pi i / 3)
-    const float2 a = v[0], b = v[1], d = v[2];
-    const float2 t = cadd(b, d), u = csub(b, d);
-    v[0] = cadd(a, t);
-    const float2 m = make_float2(a.x + c * t.x, a.y + c * t.y);
-    const float2 n = make_float2(-s * u.y, s * u.x);  // i s (b - d)
-    v[1] = cadd(m, n);
-    v[2] = csub(m, n);
-  }
-};
-template <>
-struct Dft<4> {
-  static __device__ __forceinline__ void run(float2* v) {
-    const float2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]);
-    const float2 c = cadd(v[1], v[3]), d = mul_i(csub(v[1], v[3]));
-    v[0] = cadd(a, c);
-    v[2] = csub(a, c);
-    v[1] = cadd(b, d);
-    v[3] = csub(b, d);
-  }
-};
-template <>
-struct Dft<5> {
-  static __device__ __forceinline__ void run(float2* v) {
-    const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
-    const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;
-    const float2 a = v[0];
-    const float2 t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
-    const float2 u1 = csub(v[1], v[4]), u2 = csub(v[2], v[3]);
-    v[0] = cadd(a, cadd(t1, t2));
-    const float2 m1 = make_float2(a.x + c1 * t1.x + c2 * t2.x, a.y + c1 * t1.y + c2 * t2.y);
-    const float2 m2 = make_float2(a.x + c2 * t1.x + c1 * t2.x, a.y + c2 * t1.y + c1 * t2.y);
-    const float2 n1 = make_float2(s1 * u1.x + s2 * u2.x, s1 * u1.y + s2 * u2.y);  // (s1 u1 + s2 u2)
-    const float2 n2 = make_float2(s2 * u1.x - s1 * u2.x, s2 * u1.y - s1 * u2.y);
-    v[1] = cadd(m1, mul_i(n1));
-    v[4] = csub(m1, mul_i(n1));
-    v[2] = cadd(m2, mul_i(n2));
-    v[3] = csub(m2, mul_i(n2));
-  }
-};
-
-// compile-time cos/sin(pi x) for the in-register twiddles (Taylor series after reduction
-// to [-1/2, 1/2]; |error| < 1e-16, folded to float constants)
-constexpr double ct_pi = 3.14159265358979323846;
-constexpr double ct_taylor_cos(double t) {  // cos(t), |t| <= pi/2
-  double term = 1.0, sum = 1.0;
-  for (int k = 1; k < 16; ++k) {
-    term = -term * t * t / ((2.0 * k - 1.0) * (2.0 * k));
-    sum += term;
-  }
-  return sum;
-}
-constexpr double ct_taylor_sin(double t) {  // sin(t), |t| <= pi/2
-  double term = t, sum = t;
-  for (int k = 1; k < 16; ++k) {
-    term = -term * t * t / ((2.0 * k) * (2.0 * k + 1.0));
-    sum += term;
-  }
-  return sum;
-}
-constexpr double ct_cospi(double x) {  // cos(pi x)
-  while (x > 1.0) x -= 2.0;
-  while (x < -1.0) x += 2.0;
-  if (x > 0.5) return -ct_taylor_cos(ct_pi * (1.0 - x));
-  if (x < -0.5) return -ct_taylor_cos(ct_pi * (1.0 + x));
-  return ct_taylor_cos(ct_pi * x);
-}
-constexpr double ct_sinpi(double x) {  // sin(pi x)
-  while (x > 1.0) x -= 2.0;
-  while (x < -1.0) x += 2.0;
-  if (x > 0.5) return ct_taylor_sin(ct_pi * (1.0 - x));
-  if (x < -0.5) return -ct_taylor_sin(ct_pi * (1.0 + x));
-  return ct_taylor_sin(ct_pi * x);
-}
-
-// composite radix A*B in registers (Cooley-Tukey): B DFTs of size A on stride-B
-// subsequences, twiddles exp(+2 pi i a b / R), then A DFTs of size B
-template <int A, int B>
-struct DftCT {
-  static constexpr int R = A * B;
-  static __device__ __forceinline__ void run(float2* v) {
-    float2 t[R];
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-      float2 s[A];
-#pragma unroll
-      for (int a = 0; a < A; ++a) s[a] = v[a * B + b];
-      Dft<A>::run(s);
-#pragma unroll
-      for (int a = 0; a < A; ++a) {
-        if (a * b != 0) {
-          const float cs = (float)ct_cospi(2.0 * (double)(a * b) / (double)R);
-          const float sn = (float)ct_sinpi(2.0 * (double)(a * b) / (double)R);
-          s[a] = cmul(s[a], make_float2(cs, sn));
-        }
-        t[a * B + b] = s[a];
-      }
-    }
-    // t[a*B + b]: A-point results (index a) of subsequence b; now B-point DFTs over b
-#pragma unroll
-    for (int a = 0; a < A; ++a) {
-      float2 s[B];
-#pragma unroll
-      for (int b = 0; b < B; ++b) s[b] = t[a * B + b];
-      Dft<B>::run(s);
-#pragma unroll
-      for (int b = 0; b < B; ++b) v[b * A + a] = s[b];
-    }
-  }
-};
-template <>
-struct Dft<6> : DftCT<2, 3> {};
-template <>
-struct Dft<8> : DftCT<2, 4> {};
-template <>
-struct Dft<9> : DftCT<3, 3> {};
-template <>
-struct Dft<10> : DftCT<2, 5> {};
-template <>
-struct Dft<12> : DftCT<4, 3> {};
-template <>
-struct Dft<15> : DftCT<3, 5> {};
-template <>
-struct Dft<16> : DftCT<4, 4> {};
-
-// n / d for n < 2^16 by a multiply-high (m = ceil(2^32 / d)); d = 1 handled apart
-struct FastDiv {
-  unsigned d, m;
-};
-__host__ __device__ inline FastDiv make_fastdiv(unsigned d) {
-  return FastDiv{d, d <= 1 ? 0u : (unsigned)((0x100000000ull + d - 1) / d)};
-}
 __device__ __forceinline__ int fdiv(int n, FastDiv f) { return f.d <= 1 ? n : (int)__umulhi((unsigned)n, f.m); }
 
 // One Stockham pass of radix R over ncols transforms of length N (elements estride
@@ -233,13 +80,6 @@ __device__ __forceinline__ void run_pass(int R, const float2* A, float2* B, int 
 
 }  // namespace
 
-// radix plan: at most kMaxPasses radices from {16,15,12,10,9,8,6,5,4,3,2}, fewest passes
-constexpr int kMaxPasses = 6;
-struct FftPlan {
-  int n, npass, r[kMaxPasses], ns[kMaxPasses];
-  FastDiv fns[kMaxPasses];
-};
-
 bool make_fft_plan(int n, FftPlan& p) {
   static const int cand[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
   p.n = n;
@@ -291,7 +131,7 @@ static bool finish_plan(FftPlan& p) {
   return ns == p.n;
 }
 
-static bool plan(int n, FftPlan& p) { return make_fft_plan(n, p) && finish_plan(p); }
+bool fft_plan(int n, FftPlan& p) { return make_fft_plan(n, p) && finish_plan(p); }
 
 namespace {
 
@@ -1009,7 +849,7 @@ size_t pme_b_smem(int K1, int K2, int H, bool shared_tw) {
 bool pme_fits(int K1, int K2, int K3) {
   const int H = K1 / 2 + 1, Hp = ((H + kR1 - 1) / kR1) * kR1;
   FftPlan a, b, c;
-  if (!plan(K1, a) || !plan(K2, b) || !plan(K3, c)) return false;
+  if (!fft_plan(K1, a) || !fft_plan(K2, b) || !fft_plan(K3, c)) return false;
   return pme_a_smem(K3, Hp) <= 227 * 1024 && pme_b_smem(K1, K2, H, false) <= 227 * 1024;
 }
 
@@ -1035,7 +875,7 @@ cudaError_t launch_pme_mixed(Engine& e, const BatchArgs& a) {
   A.XP = e.phi_dims[0];
   A.YP = e.phi_dims[1];
   A.ZP = e.phi_dims[2];
-  if (!plan(A.K1, A.p1) || !plan(A.K2, A.p2) || !plan(A.K3, A.p3)) return cudaErrorInvalidValue;
+  if (!fft_plan(A.K1, A.p1) || !fft_plan(A.K2, A.p2) || !fft_plan(A.K3, A.p3)) return cudaErrorInvalidValue;
   A.fH = make_fastdiv(A.H);
   A.fK1 = make_fastdiv(A.K1);
   A.fHp4 = make_fastdiv(A.Hp / kR1);

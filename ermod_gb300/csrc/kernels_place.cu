@@ -246,7 +246,7 @@ struct Spec64Args {
   double2* spec;         // [nb][K3][K2][H]
   double* self_part;     // [nb][spectrum64_partials]
   int K1, K2, K3, H, Kmax;
-  int groups;  // groups of kSpecPairs k3 pairs per CTA
+  int groups;  // groups of the threads' k3 pairs per CTA
 };
 
 // The FP64 spectrum engfac(k) S(k), S = sum_s q_s b1_s(k1) b2_s(k2) b3_s(k3): exactly the R2C
@@ -259,12 +259,14 @@ struct Spec64Args {
 // A = sum p c and B = sum p s (real times complex, 2 FMA each) give S(k3) = A + i B and
 // S(K3 - k3) = A - i B: half of the 4 FMA per point and site that each point takes by itself.
 // Pair 0 holds the real b3(0) and b3(K3 / 2) (the latter 0 for odd K3): S(0) = A, S(K3 / 2) = B.
-// CTA per (k2, groups x 4 pairs, placement), a thread per k1 and 4 pairs; p and the pairs'
+// CTA per (k2, groups x 4 pairs, placement), a thread per k1 and 4 pairs (one in solution mode,
+// whose single placement waits for each warp's chain); p and the pairs'
 // factors of 16 sites at a time in shared memory.  200 insertions on 48^3 (6 sites) 4.83 -> 4.54
 // ms, 32 on 96^3 (12 sites) 6.78 -> 6.16 ms against a thread per point.
-constexpr int kSpecPairs = 4;   // k3 pairs per thread
+constexpr int kSpecPairsMost = 4;  // k3 pairs per thread, in reference mode
 constexpr int kSpecSites = 16;  // sites staged at a time
 constexpr int kSpec64Threads = 512;
+template <int kSpecPairs>
 __global__ void __launch_bounds__(kSpec64Threads) spectrum64_kernel(Spec64Args A) {
   extern __shared__ double2 sc[];
   double2* sp = sc;                      // [kSpecSites][H]: q_s b1_s(k1) b2_s(k2)
@@ -353,13 +355,15 @@ __global__ void __launch_bounds__(kSpec64Threads) spectrum64_kernel(Spec64Args A
   }
 }
 
-// Groups of k3 pairs per CTA, fixed for a context, so that a placement's self energy does not
-// depend on its batch: one in solution mode, whose single placement makes few CTAs; otherwise
-// the count of the least FP64 work in whole warps, 16 FMA per thread and site and 4 per staged
-// p (at 96^3 2 x 320 threads of 6 groups; the staging is then 5% of the work).
+// Pairs per thread and groups of them per CTA, fixed for a context, so that a placement's self
+// energy does not depend on its batch.  Solution mode: 4 groups of one pair (32^3, 6 sites: 14.8 us
+// with one group of 4 pairs); otherwise the groups of the least FP64 work in whole warps, 16 FMA per
+// thread and site and 4 per staged p (at 96^3 2 x 320 threads of 6 groups; the staging is then
+// 5% of the work).
+int spec64_pairs(const Engine& e) { return e.P.slttype == 1 ? 1 : kSpecPairsMost; }
 int spec64_groups(const Engine& e) {
-  const int H = e.H(), all = ((e.geom.K[2] + 1) / 2 + kSpecPairs - 1) / kSpecPairs;
-  if (e.P.slttype == 1) return 1;
+  const int H = e.H(), all = ((e.geom.K[2] + 1) / 2 + kSpecPairsMost - 1) / kSpecPairsMost;
+  if (e.P.slttype == 1) return 4;
   int best = 1;
   long long cost = 0;
   for (int g = 1; g <= all && (g == 1 || g * H <= kSpec64Threads); ++g) {
@@ -373,7 +377,7 @@ int spec64_groups(const Engine& e) {
   return best;
 }
 int spec64_parts(const Engine& e) {
-  const int width = spec64_groups(e) * kSpecPairs;
+  const int width = spec64_groups(e) * spec64_pairs(e);
   return ((e.geom.K[2] + 1) / 2 + width - 1) / width;
 }
 
@@ -442,13 +446,15 @@ cudaError_t launch_spectrum64(Engine& e, const BatchArgs& a) {
   A.H = e.H();
   A.Kmax = e.Kmax();
   A.groups = spec64_groups(e);
-  const size_t smem = sizeof(double2) * kSpecSites * (A.H + A.groups * kSpecPairs);
-  static SmemAttr attr;
-  cudaError_t err = attr.ensure(spectrum64_kernel, smem);
+  const int pairs = spec64_pairs(e);
+  void (*kern)(Spec64Args) = pairs == 1 ? spectrum64_kernel<1> : spectrum64_kernel<kSpecPairsMost>;
+  const size_t smem = sizeof(double2) * kSpecSites * (A.H + A.groups * pairs);
+  static SmemAttr attr1, attr4;
+  cudaError_t err = (pairs == 1 ? attr1 : attr4).ensure(kern, smem);
   if (err != cudaSuccess) return err;
   const dim3 grid(A.K2, spec64_parts(e), a.nb);
   const int nthr = std::min(kSpec64Threads, (A.groups * A.H + 31) / 32 * 32);
-  spectrum64_kernel<<<grid, nthr, smem, a.stream>>>(A);
+  kern<<<grid, nthr, smem, a.stream>>>(A);
   e.count_launch();
   return cudaGetLastError();
 }
