@@ -6,8 +6,8 @@
 // use radices up to 16 (96 points: 12 x 8, 2,100 instructions where 5 N log2 N
 // counts 3,160), and two real rows share one complex transform.  Integer work and
 // shared memory hide behind it, so one kernel serves every length with factors 2, 3 and 5 (others
-// take cuFFT).  16 placements at 96^3: 298, 318 and 350 us (the first two at 88% of the FP64 pipe's
-// rate), cuFFT's three kernels 333, 333 and 834; 64 at 48^3 464 us and 594.
+// take cuFFT).  16 placements at 96^3: 293, 314 and 346 us (the first two at 85% of the FP64 pipe's
+// rate), cuFFT's three kernels 333, 333 and 834; 64 at 48^3 440 us and 594.
 #include "dft.cuh"
 #include "engine.cuh"
 

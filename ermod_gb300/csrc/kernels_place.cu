@@ -325,6 +325,12 @@ __global__ void __launch_bounds__(kSpec64Threads) spectrum64_kernel(Spec64Args A
     }
     if (on) {
       const double w = (k1 == 0 || (even && k1 == A.H - 1)) ? 0.5 : 1.0;
+      double own = 0.0;  // the thread's points share the weight
+      auto put = [&](double2* to, double f, double2 x) {
+        const double2 y = make_double2(f * x.x, f * x.y);
+        own = fma(y.y, x.y, fma(y.x, x.x, own));
+        *to = y;
+      };
       const size_t plane = (size_t)A.K2 * A.H, at0 = (size_t)k2 * A.H + k1;
       double2* out = A.spec + (size_t)b * A.K3 * plane + at0;
 #pragma unroll
@@ -334,15 +340,10 @@ __global__ void __launch_bounds__(kSpec64Threads) spectrum64_kernel(Spec64Args A
         const int lo = p, hi = p == 0 ? A.K3 / 2 : A.K3 - p;  // odd K3: pair 0 has no upper point
         const double2 x = p == 0 ? a[i] : make_double2(a[i].x - c[i].y, a[i].y + c[i].x);
         const double2 y = p == 0 ? c[i] : make_double2(a[i].x + c[i].y, a[i].y - c[i].x);
-        const double fl = A.engfac[(size_t)lo * plane + at0];
-        self += w * fl * (x.x * x.x + x.y * x.y);
-        out[(size_t)lo * plane] = make_double2(fl * x.x, fl * x.y);
-        if (p > 0 || even3) {
-          const double fh = A.engfac[(size_t)hi * plane + at0];
-          self += w * fh * (y.x * y.x + y.y * y.y);
-          out[(size_t)hi * plane] = make_double2(fh * y.x, fh * y.y);
-        }
+        put(out + (size_t)lo * plane, A.engfac[(size_t)lo * plane + at0], x);
+        if (p > 0 || even3) put(out + (size_t)hi * plane, A.engfac[(size_t)hi * plane + at0], y);
       }
+      self = fma(w, own, self);
     }
   }
   __shared__ double red[kSpec64Threads / 32];
