@@ -326,7 +326,9 @@ __global__ void __launch_bounds__(pme_threads(KC), pme_min_blocks(KC)) pme_a_ker
     // first nsc threads those of q b2(k2) per site), then forms and stores them, so that
     // one L2 round trip covers its share (issued one entry at a time, the round trips made
     // the staging about a third of the CTA's time)
-    constexpr int kStage = 2;
+    // three entries of each: 12 sites at 96^3 in one round (2,048 insertions of 33,000 waters 16.46 ms in
+    // rounds of two, 16.26 of three, 16.37 of four)
+    constexpr int kStage = 3;
     const int nd = nsc * K3, n1 = nsc * Hp;
     __shared__ float2 sqb2[kSites];  // q_s b2_s(k2)
     for (int r0 = 0; r0 < max(nd, n1); r0 += kStage * blockDim.x) {
@@ -350,7 +352,7 @@ __global__ void __launch_bounds__(pme_threads(KC), pme_min_blocks(KC)) pme_a_ker
         const float2 b2 = bv[(us * 3 + 1) * A.Kmax + k2];
         sqb2[threadIdx.x] = make_float2(q * b2.x, q * b2.y);
       }
-      __syncthreads();  // sqb2 staged (the loop runs the same number of rounds in every thread)
+      if (r0 == 0) __syncthreads();  // sqb2 staged (the loop runs the same number of rounds in every thread)
 #pragma unroll
       for (int i = 0; i < kStage; ++i) {
         const int t = base + i * blockDim.x;
