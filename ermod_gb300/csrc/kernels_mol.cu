@@ -831,8 +831,9 @@ __device__ __forceinline__ void species_partials(const MolArgs& A, const BatchAr
 // now 294.)
 //
 // Four blocks per SM (64 registers): 2-3% faster over a whole run than three of 80.
-// TILE: molecules per block of 256 threads.  64 in solution mode, where a frame's one placement
-// makes few blocks and the real-space pass takes all 256 threads.
+// TILE: molecules per block of 256 threads.  16 or 64 in solution mode, where a frame's one placement
+// makes few blocks and the real-space pass, the FP64 pairs of the first shell above all, takes
+// all 256 threads.
 // kTwo: the stage before the pairs' test, for solutes of many sites (kTwoStageSites).
 template <int G, int TILE, bool kTwo>
 __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const float* __restrict__ site_e) {
@@ -1324,11 +1325,14 @@ cudaError_t launch_gather(Engine& e, const BatchArgs& a) {
 // one per solute molecule), so its molecules are split further while that still leaves the
 // GPU room; fixed for a context, so that a placement's sums do not depend on its batch
 static int mol64_ty(const Engine& e) { return e.P.slttype == 1 && e.slvmax < 512 * e.num_sm ? 4 : 1; }
-// molecules per block of the molecule kernels: the FP64 path's as above; the mixed path's 256,
-// or 64 in solution mode while that still leaves blocks to fill the GPU
+// molecules per block of the molecule kernels: the FP64 path's as above; the mixed path's 256, or
+// in solution mode 16 while that gives at most a block per SM (a droplet of 300 molecules, a frame
+// of which makes hundreds of FP64 pairs: 145 -> 137 us; 1,000 waters 172.4 -> 171.5; at 8,000 no
+// faster than 64), then 64 while that leaves few
 int mol_tile(const Engine& e) {
   if (!e.mixed) return kMol64Threads / (4 * mol64_ty(e));
-  return e.P.slttype == 1 && e.P.finish_group == 0 && e.slvmax < 64 * 3 * e.num_sm ? 64 : 256;
+  if (e.P.slttype != 1 || e.P.finish_group != 0 || e.slvmax >= 64 * 3 * e.num_sm) return 256;
+  return e.slvmax <= 16 * e.num_sm ? 16 : 64;
 }
 
 // placements per molecule-energy block: the caller's choice (4 or 8), else 4, halved while the
@@ -1368,6 +1372,7 @@ cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a) {
     if ((err = attr.ensure(mol_finish_kernel<GG, TILE, TWO>, smem_f)) != cudaSuccess) return err;              \
     mol_finish_kernel<GG, TILE, TWO><<<g2, 256, smem_f, a.stream>>>(A, a.site_e);                              \
   }
+  ERMOD_FINISH(1, 16, false)
   ERMOD_FINISH(1, 64, false)
   ERMOD_FINISH(1, 256, false)
   ERMOD_FINISH(2, 256, false)
