@@ -31,12 +31,12 @@ MEASURED_TRAFFIC_REFS_LARGE = {
 # peak as ncu reports it) and its duration launched alone (us, one 256-placement launch,
 # serialised and cold, so slower than inside the pipelined step).
 MEASURED_PIPES_REFS_LARGE = {
-    "spectrum": {"kernel": "pme_a_kernel<96>", "issue_active_pct": 62.7, "fma_pipe_pct": 40.8,
-                 "alu_pipe_pct": 21.1, "fp64_pipe_pct": 0.5, "dram_pct": 15.3, "standalone_us": 720.9},
-    "fft_c2r": {"kernel": "pme_b_kernel<96>", "issue_active_pct": 44.9, "fma_pipe_pct": 22.1,
-                "alu_pipe_pct": 25.5, "fp64_pipe_pct": 0.0, "dram_pct": 34.8, "standalone_us": 688.9},
-    "gather": {"kernel": "gather_tma_kernel<4>", "issue_active_pct": 28.2, "fma_pipe_pct": 18.3,
-               "alu_pipe_pct": 4.7, "fp64_pipe_pct": 0.0, "dram_pct": 32.2, "standalone_us": 438.8},
+    "spectrum": {"kernel": "pme_a_kernel<96>", "issue_active_pct": 64.1, "fma_pipe_pct": 42.0,
+                 "alu_pipe_pct": 20.2, "fp64_pipe_pct": 0.5, "dram_pct": 15.9, "standalone_us": 694.4},
+    "fft_c2r": {"kernel": "pme_b_kernel<96>", "issue_active_pct": 46.4, "fma_pipe_pct": 22.7,
+                "alu_pipe_pct": 26.3, "fp64_pipe_pct": 0.0, "dram_pct": 36.0, "standalone_us": 666.7},
+    "gather": {"kernel": "gather_tma_kernel<4>", "issue_active_pct": 36.1, "fma_pipe_pct": 23.8,
+               "alu_pipe_pct": 5.1, "fp64_pipe_pct": 0.0, "dram_pct": 42.8, "standalone_us": 331.8},
 }
 PIPES_SOURCE = "profiles/kernels_refs_large_batch256.md"
 
@@ -60,7 +60,7 @@ def bytes_per_placement(K1: int, K2: int, K3: int, nsite: int, G: int = 8) -> di
 def bytes_per_placement_fp64(K1: int, K2: int, K3: int, nsite: int) -> dict:
     nh, nr = grid_terms(K1, K2, K3)
     d = {
-        "spectrum": 8.0 * nr + 8.0 * nr + 16.0 * nh + 2 * 16.0 * nh,  # spread, D2Z, influence
+        "spectrum": 16.0 * nh,  # written once, from the 1-D structure factors
         "fft_c2r": 16.0 * nh + 8.0 * nr,
         "mol_energy": 8.0 * nr + (24 + 96 + 8 + 8) * nsite,
     }
