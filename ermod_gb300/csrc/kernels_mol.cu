@@ -574,14 +574,18 @@ __global__ void __launch_bounds__(kMol64Threads) mol_energy_kernel(MolArgs A) {
 // Mixed path, step 1 -- gather by bricks.  CTA per (kBrickX x kBrickY x kBrickZ brick of the
 // PME grid, run of placement groups of 4).  One TMA box copy per group brings the
 // brick's stencil halo of the group's interleaved potential grids into shared memory as
-// [z][y][x][4], in kGatherStages buffers so that the next groups' copies are in flight
+// [z][y][x][4], in gather_stages(P) buffers so that the next groups' copies are in flight
 // while this one is used; each thread takes a site of the brick (its B-spline weights
 // computed once for all groups, FP32 stable recursion) and accumulates
 // q theta theta theta phi for the four placements with one 16-byte shared load per
 // stencil point.  Bound by those loads (66% of the shared-memory wavefronts, a launch of 256
 // placements at 96^3 in 340 us); 160-thread CTAs, three to an SM, measured 2% slower.
 constexpr int kGatherThreads = 256;
-constexpr int kGatherStages = 2;  // halo buffers (TMA copies in flight) per gather CTA
+// halo buffers (TMA copies in flight) per gather CTA: two for order 4, whose halos leave an SM room
+// for two CTAs of them; one for orders 6 and 8, where two buffers of 57 and 83 KB would leave it a
+// single CTA, and another CTA hides the copies better (1,024 insertions of 33,000 waters: order 6
+// 11.44 ms with two buffers, 10.62 with one; order 8 16.20 and 15.65)
+constexpr int gather_stages(int P) { return P <= 4 ? 2 : 1; }
 
 template <int P>
 __device__ __forceinline__ void site_setup(int site, const float4* __restrict__ site_rec,
@@ -633,12 +637,12 @@ __global__ void __launch_bounds__(kGatherThreads) gather_tma_kernel(
     const __grid_constant__ CUtensorMap tmap, int nb, int groups_per_cta, const float4* __restrict__ site_rec,
     const int* __restrict__ site_grid, const int* __restrict__ brick_site, const int* __restrict__ brick_start,
     int K1, int K2, int K3, int nbx, int nby, int BX, int ldb, float* __restrict__ site_e, DevStatus* status) {
-  constexpr int BY = kBrickY + P - 1, BZ = kBrickZ + P - 1;
+  constexpr int BY = kBrickY + P - 1, BZ = kBrickZ + P - 1, kStages = gather_stages(P);
   extern __shared__ unsigned char smem_raw[];
-  __shared__ unsigned long long bar[kGatherStages];
+  __shared__ unsigned long long bar[kStages];
   const int npt = BZ * BY * BX;
-  // kGatherStages halo buffers [z][y][x] of float4 (the four placements of a group),
-  // 128-byte aligned; group g lands in buffer (g - g_begin) % kGatherStages
+  // kStages halo buffers [z][y][x] of float4 (the four placements of a group),
+  // 128-byte aligned; group g lands in buffer (g - g_begin) % kStages
   float4* halo_base = reinterpret_cast<float4*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
   const int hstride = (npt + 7) & ~7;  // float4 elements, a multiple of 128 bytes
   const int brick = blockIdx.x;
@@ -647,7 +651,7 @@ __global__ void __launch_bounds__(kGatherThreads) gather_tma_kernel(
   const int g_end = min((nb + 3) / 4, g_begin + groups_per_cta);
   const uint32_t box_bytes = (uint32_t)(npt * sizeof(float4));
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kGatherStages; ++i) mbar_init(&bar[i], 1);
+    for (int i = 0; i < kStages; ++i) mbar_init(&bar[i], 1);
     fence_barrier_init();
     fence_proxy_async_smem();
   }
@@ -655,7 +659,7 @@ __global__ void __launch_bounds__(kGatherThreads) gather_tma_kernel(
   // padded coordinates: the halo of brick (bx, by, bz) starts at (kBrickX bx,
   // kBrickY by, kBrickZ bz), four floats (the group's placements) per x
   if (threadIdx.x == 0) {
-    for (int g = g_begin; g < min(g_end, g_begin + kGatherStages); ++g) {
+    for (int g = g_begin; g < min(g_end, g_begin + kStages); ++g) {
       const int st = g - g_begin;
       mbar_expect_tx(&bar[st], box_bytes);
       tma_load_4d(halo_base + (size_t)st * hstride, &tmap, 4 * bx * kBrickX, by * kBrickY, bz * kBrickZ, g, &bar[st]);
@@ -707,8 +711,8 @@ __global__ void __launch_bounds__(kGatherThreads) gather_tma_kernel(
   if (site0 >= 0) site_setup<P>(site0, site_rec, site_grid, K1, K2, K3, ox, oy, oz, BX, w1, w2, w3, base, q);
   const int n_extra = bucketed ? novf : max(0, n - (int)blockDim.x);
   for (int g = g_begin; g < g_end; ++g) {
-    const int slot = (g - g_begin) % kGatherStages;
-    const uint32_t parity = (uint32_t)(((g - g_begin) / kGatherStages) & 1);
+    const int slot = (g - g_begin) % kStages;
+    const uint32_t parity = (uint32_t)(((g - g_begin) / kStages) & 1);
     bool ok = false;
     for (long it = 0; it < kWaitLimit; ++it)
       if (mbar_try_wait(&bar[slot], parity)) {
@@ -717,9 +721,9 @@ __global__ void __launch_bounds__(kGatherThreads) gather_tma_kernel(
       }
     if (!__syncthreads_and(ok)) {  // flag, let the other copies in flight land (bounded), leave
       if (threadIdx.x == 0) atomicOr(&status->range_fault, 2);
-      for (int g2 = g + 1; g2 < min(g_end, g + kGatherStages); ++g2) {
-        const int s2 = (g2 - g_begin) % kGatherStages;
-        const uint32_t p2 = (uint32_t)(((g2 - g_begin) / kGatherStages) & 1);
+      for (int g2 = g + 1; g2 < min(g_end, g + kStages); ++g2) {
+        const int s2 = (g2 - g_begin) % kStages;
+        const uint32_t p2 = (uint32_t)(((g2 - g_begin) / kStages) & 1);
         for (long it = 0; it < kWaitLimit; ++it)
           if (mbar_try_wait(&bar[s2], p2)) break;
       }
@@ -742,12 +746,12 @@ __global__ void __launch_bounds__(kGatherThreads) gather_tma_kernel(
       *reinterpret_cast<float4*>(site_e + (size_t)site * ldb + b0) =
           make_float4(qs * acc.x, qs * acc.y, qs * acc.z, qs * acc.w);
     }
-    __syncthreads();  // halo[slot] consumed: the copy of group g + kGatherStages may land in it
-    if (threadIdx.x == 0 && g + kGatherStages < g_end) {
+    __syncthreads();  // halo[slot] consumed: the copy of group g + kStages may land in it
+    if (threadIdx.x == 0 && g + kStages < g_end) {
       fence_proxy_async_smem();
       mbar_expect_tx(&bar[slot], box_bytes);
       tma_load_4d(halo_base + (size_t)slot * hstride, &tmap, 4 * bx * kBrickX, by * kBrickY, bz * kBrickZ,
-                  g + kGatherStages, &bar[slot]);
+                  g + kStages, &bar[slot]);
     }
   }
 }
@@ -1304,7 +1308,7 @@ cudaError_t launch_gather(Engine& e, const BatchArgs& a) {
   const int K1 = e.geom.K[0], K2 = e.geom.K[1], K3 = e.geom.K[2];
   const size_t npt = (size_t)e.gbox[0] * e.gbox[1] * e.gbox[2];
   const size_t hstride = (npt + 7) & ~(size_t)7;  // as in the kernel: 128-byte aligned halos
-  const size_t sh = 128 + kGatherStages * hstride * sizeof(float4);
+  const size_t sh = 128 + gather_stages(e.P_order) * hstride * sizeof(float4);
 #define ERMOD_GATHER(PP)                                                                                        \
   if (e.P_order == PP) {                                                                                        \
     static SmemAttr attr;                                                                                       \
