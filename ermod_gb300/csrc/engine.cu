@@ -322,7 +322,7 @@ static int ensure_batch(Engine& e) {
   }
   ERMOD_CUDA(dalloc(&b.part, NS * B * e.ntile * e.numslv * 3));
   e.ring_half = e.P.corrcal ? std::max(2 * B, (512 / B) * B) : B;
-  e.ring_cap = 2 * e.ring_half;
+  e.ring_cap = e.P.corrcal ? 2 * e.ring_half : kBatchSlots * B;  // without ecorr one histogram per slot
   e.ring_fill = 0;
   e.ring_off = 0;
   e.flush_pend[0] = e.flush_pend[1] = false;
@@ -1168,7 +1168,8 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
         e.ring_fill = 0;
       }
     } else {
-      e.ring_off = e.ring_half - e.ring_off;  // two histogram slots, ordered by ev_acc
+      // a histogram per batch slot, whose reuse ev_acc orders
+      e.ring_off = (e.ring_off + B) % (kBatchSlots * B);
     }
   }
   if (e.P.corrcal && e.ring_fill > 0) {
