@@ -322,47 +322,89 @@ __global__ void __launch_bounds__(pme_threads(KC), pme_min_blocks(KC)) pme_a_ker
     const int nsc = min(A.chunk, ns - s0);
     const bool last = s0 + A.chunk >= ns;
     __syncthreads();
-    // staging: each thread first issues the loads of its entries of both tables (and the
-    // first nsc threads those of q b2(k2) per site), then forms and stores them, so that
-    // one L2 round trip covers its share (issued one entry at a time, the round trips made
-    // the staging about a third of the CTA's time)
-    // three entries of each: 12 sites at 96^3 in one round (2,048 insertions of 33,000 waters 16.46 ms in
-    // rounds of two, 16.26 of three, 16.37 of four)
-    constexpr int kStage = 3;
-    const int nd = nsc * K3, n1 = nsc * Hp;
-    __shared__ float2 sqb2[kSites];  // q_s b2_s(k2)
-    for (int r0 = 0; r0 < max(nd, n1); r0 += kStage * blockDim.x) {
-      const int base = r0 + (int)threadIdx.x;
-      float2 b3[kStage], b1[kStage];
+    if constexpr (KC > 0) {
+      // staging: a warp takes two or three sites at a time, its lanes along k3 and k1, and issues all
+      // their loads before it forms and stores the entries, so that one L2 round trip covers them
+      // (against entries dealt to the threads as below, 40 instructions each with their divisions:
+      // four systems in a graph 27.10 -> 26.76 ms, 33,000 waters 16.23 -> 16.16)
+      constexpr int HPC = ((KC / 2 + 1 + kR1 - 1) / kR1) * kR1, TXC = HPC / kR1;
+      constexpr int N3 = (KC + 31) / 32, N1 = (HPC + 31) / 32, kU = KC <= 64 ? 3 : 2;
+      constexpr int kWarps = pme_threads(KC) / 32;
+      const int lane = threadIdx.x & 31;
+      for (int sl0 = (int)(threadIdx.x >> 5); sl0 < nsc; sl0 += kU * kWarps) {
+        float2 b3[kU][N3], b1[kU][N1], b2[kU];
+        float q[kU];
 #pragma unroll
-      for (int i = 0; i < kStage; ++i) {
-        const int t = base + i * blockDim.x;
-        if (t < nd) {
-          const int sl = t / K3, k3 = t - sl * K3;
-          b3[i] = bv[((size_t)(s0 + sl) * 3 + 2) * A.Kmax + k3];
+        for (int u = 0; u < kU; ++u) {
+          const int sl = sl0 + u * kWarps;
+          if (sl >= nsc) break;
+          const float2* row = bv + (size_t)(s0 + sl) * 3 * A.Kmax;
+          q[u] = A.u_qf[(size_t)b * kMaxSoluteSites + s0 + sl];
+          b2[u] = row[A.Kmax + k2];
+#pragma unroll
+          for (int i = 0; i < N3; ++i)
+            if (lane + 32 * i < KC) b3[u][i] = row[2 * A.Kmax + lane + 32 * i];
+#pragma unroll
+          for (int i = 0; i < N1; ++i) b1[u][i] = lane + 32 * i < KC / 2 + 1 ? row[lane + 32 * i] : make_float2(0.f, 0.f);
         }
-        if (t < n1) {
-          const int sl = t / Hp, k1 = t - sl * Hp;
-          b1[i] = (k1 < H) ? bv[((size_t)(s0 + sl) * 3 + 0) * A.Kmax + k1] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          const int sl = sl0 + u * kWarps;
+          if (sl >= nsc) break;
+          const float2 c = make_float2(q[u] * b2[u].x, q[u] * b2[u].y);  // q_s b2_s(k2)
+#pragma unroll
+          for (int i = 0; i < N3; ++i)
+            if (lane + 32 * i < KC) sd[sl * KC + lane + 32 * i] = cmul(c, b3[u][i]);
+#pragma unroll
+          for (int i = 0; i < N1; ++i) {
+            const int k1 = lane + 32 * i;
+            if (k1 < HPC) sb[sl * HPC + (k1 % kR1) * TXC + k1 / kR1] = b1[u][i];
+          }
         }
       }
-      if (r0 == 0 && threadIdx.x < (unsigned)nsc) {
-        const size_t us = (size_t)(s0 + threadIdx.x);
-        const float q = A.u_qf[(size_t)b * kMaxSoluteSites + us];
-        const float2 b2 = bv[(us * 3 + 1) * A.Kmax + k2];
-        sqb2[threadIdx.x] = make_float2(q * b2.x, q * b2.y);
-      }
-      if (r0 == 0) __syncthreads();  // sqb2 staged (the loop runs the same number of rounds in every thread)
+    } else {
+      // staging: each thread first issues the loads of its entries of both tables (and the
+      // first nsc threads those of q b2(k2) per site), then forms and stores them, so that
+      // one L2 round trip covers its share (issued one entry at a time, the round trips made
+      // the staging about a third of the CTA's time)
+      // three entries of each: 12 sites at 96^3 in one round (2,048 insertions of 33,000 waters 16.46 ms in
+      // rounds of two, 16.26 of three, 16.37 of four)
+      constexpr int kStage = 3;
+      const int nd = nsc * K3, n1 = nsc * Hp;
+      __shared__ float2 sqb2[kSites];  // q_s b2_s(k2)
+      for (int r0 = 0; r0 < max(nd, n1); r0 += kStage * blockDim.x) {
+        const int base = r0 + (int)threadIdx.x;
+        float2 b3[kStage], b1[kStage];
 #pragma unroll
-      for (int i = 0; i < kStage; ++i) {
-        const int t = base + i * blockDim.x;
-        if (t < nd) {
-          const int sl = t / K3, k3 = t - sl * K3;
-          sd[sl * K3 + k3] = cmul(sqb2[sl], b3[i]);
+        for (int i = 0; i < kStage; ++i) {
+          const int t = base + i * blockDim.x;
+          if (t < nd) {
+            const int sl = t / K3, k3 = t - sl * K3;
+            b3[i] = bv[((size_t)(s0 + sl) * 3 + 2) * A.Kmax + k3];
+          }
+          if (t < n1) {
+            const int sl = t / Hp, k1 = t - sl * Hp;
+            b1[i] = (k1 < H) ? bv[((size_t)(s0 + sl) * 3 + 0) * A.Kmax + k1] : make_float2(0.f, 0.f);
+          }
         }
-        if (t < n1) {
-          const int sl = t / Hp, k1 = t - sl * Hp;
-          sb[sl * Hp + (k1 % kR1) * TX + k1 / kR1] = b1[i];
+        if (r0 == 0 && threadIdx.x < (unsigned)nsc) {
+          const size_t us = (size_t)(s0 + threadIdx.x);
+          const float q = A.u_qf[(size_t)b * kMaxSoluteSites + us];
+          const float2 b2 = bv[(us * 3 + 1) * A.Kmax + k2];
+          sqb2[threadIdx.x] = make_float2(q * b2.x, q * b2.y);
+        }
+        if (r0 == 0) __syncthreads();  // sqb2 staged (the loop runs the same number of rounds in every thread)
+#pragma unroll
+        for (int i = 0; i < kStage; ++i) {
+          const int t = base + i * blockDim.x;
+          if (t < nd) {
+            const int sl = t / K3, k3 = t - sl * K3;
+            sd[sl * K3 + k3] = cmul(sqb2[sl], b3[i]);
+          }
+          if (t < n1) {
+            const int sl = t / Hp, k1 = t - sl * Hp;
+            sb[sl * Hp + (k1 % kR1) * TX + k1 / kR1] = b1[i];
+          }
         }
       }
     }
