@@ -236,6 +236,14 @@ static int free_bins(Engine& e) {
   return ERMOD_OK;
 }
 
+// Set-up copies and memsets run on the legacy default stream, which the context's non-blocking
+// streams do not wait for (and a copy from pageable memory may return before its bytes have
+// arrived): every set-up call waits for them before it returns or launches.
+static int setup_done() {
+  ERMOD_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  return ERMOD_OK;
+}
+
 // TMA descriptor of the padded potential grids [B/4][ZP][YP][XP][4] (four placements
 // interleaved innermost), as a 4-D tensor whose innermost dimension is a whole row of 4 XP
 // floats; one box = the gather halo of a brick for 4 placements, landing in shared memory as
@@ -308,7 +316,7 @@ static int ensure_batch(Engine& e) {
     e.gbox[2] = kBrickZ + h;
     const size_t np = (size_t)e.phi_dims[0] * e.phi_dims[1] * e.phi_dims[2];
     ERMOD_CUDA(dalloc(&b.phi, NS * np * B));
-    ERMOD_CUDA(cudaMemset(b.phi, 0, sizeof(float) * NS * np * B));
+    ERMOD_CUDA(cudaMemsetAsync(b.phi, 0, sizeof(float) * NS * np * B, e.stream));  // the batch streams fork from it
     for (int s = 0; s < kBatchSlots; ++s) {
       const int st = make_phi_tmap(e, b.phi + (size_t)s * np * B, &e.phi_tmap[s]);
       if (st) return st;
@@ -574,6 +582,10 @@ int ermod_create(const ermod_params* p_in, int device, ermod_ctx** out) {
   cudaMemcpy(e.d_splfc, splfc.data(), sizeof(double) * splfc.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(e.d_twiddle, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(e.d_twiddle64, tw64.data(), sizeof(double2) * tw64.size(), cudaMemcpyHostToDevice);
+  if (const int st = setup_done()) {
+    ermod_destroy(c);
+    return st;
+  }
   *out = c;
   return ERMOD_OK;
 }
@@ -796,6 +808,7 @@ int ermod_set_topology(ermod_ctx* c, int nummol, int numatm, const int* mbi, con
   ERMOD_CUDA(dalloc(&e.d_site_x, 3 * (size_t)e.nsite_phys));
   ERMOD_CUDA(dalloc(&e.d_site_q, e.nsite_phys));
   ERMOD_CUDA(dalloc(&e.d_frame_scal, 4));
+  if (const int st = setup_done()) return st;
   e.green_valid = false;
   e.topo_ready = true;
   return ERMOD_OK;
@@ -888,6 +901,7 @@ int ermod_set_bins(ermod_ctx* c, int numslv, const int* uvmax, const int* uvsoft
   ERMOD_CUDA(cudaMemset(e.d_edens, 0, sizeof(double) * ermax));
   ERMOD_CUDA(cudaMemset(e.d_eself, 0, sizeof(double) * std::max(esmax, 1)));
   ERMOD_CUDA(cudaMemset(e.d_slnuv, 0, sizeof(double) * numslv));
+  if (const int st = setup_done()) return st;
   e.warn_bin_firsttime = true;
   e.bins_ready = true;
   return ERMOD_OK;
@@ -1426,6 +1440,7 @@ int ermod_set_solute_library(ermod_ctx* c, int nconf, int nsite, const double* c
   ERMOD_CUDA(dalloc(&e.d_lib_acc, (size_t)nconf + 1));
   ERMOD_CUDA(cudaMemcpy(e.d_lib, conf, sizeof(double) * 3 * nsite * (size_t)nconf, cudaMemcpyHostToDevice));
   if (nwt) ERMOD_CUDA(cudaMemcpy(e.d_lib_wt, weight, sizeof(double) * nwt, cudaMemcpyHostToDevice));
+  if (const int st = setup_done()) return st;
   e.lib_nconf = nconf;
   e.lib_ns = nsite;
   e.lib_nwt = nwt;
@@ -1467,7 +1482,7 @@ int ermod_set_aggregate(ermod_ctx* c, const int* host_mol, const double* sitemas
   if (!e.d_site_mass) ERMOD_CUDA(dalloc(&e.d_site_mass, (size_t)e.numatm));
   ERMOD_CUDA(cudaMemcpy(e.d_agg_mass, hm.data(), sizeof(double) * e.numatm, cudaMemcpyHostToDevice));
   ERMOD_CUDA(cudaMemcpy(e.d_site_mass, sitemass, sizeof(double) * e.numatm, cudaMemcpyHostToDevice));
-  return ERMOD_OK;
+  return setup_done();
 }
 
 // load_refstructure (insertion.F90:619-700): refspec atoms and the reference solute
@@ -1509,6 +1524,7 @@ int ermod_set_reference_structure(ermod_ctx* c, const int* ref_mol, const double
   if (nh > 0) ERMOD_CUDA(cudaMemcpy(e.d_ref_atoms, atoms.data(), sizeof(int) * nh, cudaMemcpyHostToDevice));
   ERMOD_CUDA(cudaMemcpy(e.d_ref_host, host.data(), sizeof(double) * host.size(), cudaMemcpyHostToDevice));
   ERMOD_CUDA(cudaMemcpy(e.d_ref_slt, slt.data(), sizeof(double) * slt.size(), cudaMemcpyHostToDevice));
+  if (const int st = setup_done()) return st;
   e.ref_nh = nh;
   e.ref_ns = refslt_natom;
   return ERMOD_OK;
@@ -1565,7 +1581,7 @@ int ermod_intermediate_enable(ermod_ctx* c, const double* refs_density) {
   ERMOD_CUDA(dalloc(&e.d_edintm, (size_t)e.ermax + e.numslv + 3));
   ERMOD_CUDA(cudaMemcpy(e.d_int_mask, mask.data(), e.ermax, cudaMemcpyHostToDevice));
   ERMOD_CUDA(cudaMemset(e.d_edintm, 0, sizeof(double) * ((size_t)e.ermax + e.numslv + 3)));
-  return ERMOD_OK;
+  return setup_done();
 }
 
 int ermod_intermediate_get(ermod_ctx* c, double* edintm, double* uvintm, double* totals) {
@@ -1644,6 +1660,7 @@ int ermod_adjoint_enable(ermod_ctx* c, int solute_mol, int cmbrule) {
   ERMOD_CUDA(cudaMemset(e.d_adj_grad, 0, sizeof(double) * 3 * (size_t)ns * e.ermax));
   ERMOD_CUDA(cudaMemset(e.d_adj_w, 0, sizeof(double) * e.ermax));
   ERMOD_CUDA(cudaMemset(e.d_ps_qf, 0, sizeof(float) * (size_t)B * kMaxSoluteSites));
+  if (const int st = setup_done()) return st;
   e.adj_mol = solute_mol;
   e.adj_ns = ns;
   e.adj_cmbrule = cmbrule;
