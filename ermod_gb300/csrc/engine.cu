@@ -1014,6 +1014,7 @@ int ermod_frame(ermod_ctx* c, const double* sitepos, const double* cell, double 
   if (staged) ERMOD_CUDA(cudaEventRecord(e.ev_stage, e.stream));
   st = frame_launch(e);
   if (st) return st;
+  e.queued = true;
   if (!staged) ERMOD_CUDA(cudaStreamSynchronize(e.stream));
   return ERMOD_OK;
 }
@@ -1254,6 +1255,7 @@ int ermod_sync(ermod_ctx* c) {
   ERMOD_CUDA(cudaStreamSynchronize(e.stream));
   const int st = decode_status(e);
   const int rs = reset_status(e);  // the next calls start a new sequence
+  e.queued = true;
   return st ? st : rs;
 }
 
@@ -1952,7 +1954,12 @@ int ermod_graph_launch(ermod_graph* g, void* stream) {
   if (!g || !g->exec) return fail_param("null graph");
   cudaSetDevice(g->device);
   g->launched = (cudaStream_t)stream;
-  for (ermod_ctx* c : g->ctx) c->e.status_clean = false;
+  for (ermod_ctx* c : g->ctx) {
+    Engine& e = c->e;
+    if (e.queued && e.stream != g->launched) ERMOD_CUDA(cudaStreamSynchronize(e.stream));
+    e.queued = false;
+    e.status_clean = false;
+  }
   ERMOD_CUDA(cudaGraphLaunch(g->exec, g->launched));
   return ERMOD_OK;
 }

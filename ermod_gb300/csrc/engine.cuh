@@ -156,6 +156,9 @@ struct Engine {
   DevStatus* d_status = nullptr;
   DevStatus* h_status = nullptr;  // pinned, at the end of h_stage
   bool status_clean = true;  // d_status holds no result of queued work
+  // a host call has returned with work queued on the stream (a small frame, the status reset): a
+  // graph's launch, on a stream of its own, waits for it
+  bool queued = false;
   int err_placement = -1, err_molecule = -1;
   double err_energy = 0.0;
   int call_b0 = 0;
