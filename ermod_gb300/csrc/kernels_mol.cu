@@ -322,10 +322,17 @@ __host__ __device__ constexpr int finish_scratch_ints(int G, bool two) {  // for
 }
 // the dynamic shared memory of the finish kernel before its edge keys: the block
 // histograms (when in shared memory) or the real-space pass's scratch, whichever is larger
-__host__ __device__ __forceinline__ int finish_region_ints(int G, bool two, int ermax, int hist_global) {
+__host__ __device__ constexpr int finish_region_ints(int G, bool two, int ermax, int hist_global) {
   const int h = hist_global ? 0 : G * ermax;
   return h > finish_scratch_ints(G, two) ? h : finish_scratch_ints(G, two);
 }
+
+// its dynamic shared memory in bytes, and an upper bound of its static one (the totals of 256 molecules)
+constexpr size_t finish_smem(int G, bool two, int ermax, int hist_global) {
+  return sizeof(int) * ((size_t)finish_region_ints(G, two, ermax, hist_global) + ermax);
+}
+constexpr size_t finish_static_smem(int G) { return 2112 * (size_t)G + 512; }
+constexpr size_t kMaxSmem = 227 * 1024;  // per block
 
 __device__ __forceinline__ float pair_r2(const MolArgs& A, const int4& vp, const int4& up) {
   const float ex = (float)(int)((unsigned)vp.x - (unsigned)up.x) * A.fxf[0];
@@ -1357,18 +1364,24 @@ cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a) {
   e.count_launch();
   cudaError_t err = cudaSuccess;
   if (!e.mixed) return mol64_ty(e) == 4 ? launch_mol64<4>(e, A) : launch_mol64<1>(e, A);
-  const int G = finish_group(e, a.nb);
+  int G = finish_group(e, a.nb);
+  bool two = e.tile == 256 && e.max_solute_sites >= kTwoStageSites;
   // block histograms in shared memory up to 64 KB (three blocks per SM fit); beyond that, and
   // for the few molecules of a small tile, the counts go straight to global memory
   A.hist_global = (e.tile < 256 || (size_t)G * e.ermax * sizeof(int) > 64 * 1024) ? 1 : 0;
+  // the keys of a coordinate of tens of thousands of bins may leave no room for the scratch of G
+  // placements (48,788 bins leave it for 4): one placement and one stage need the least, up to 52,268
+  if (finish_smem(G, two, e.ermax, A.hist_global) + finish_static_smem(G) > kMaxSmem) {
+    G = 1;
+    two = false;
+  }
   if (e.P.cltype != 0 && (err = launch_gather(e, a)) != cudaSuccess) return err;
   if (a.phases) {
     e.phase_end_on(a.stream);
     e.phase_begin_on(PH_MOL, a.stream);
   }
   // step 2: per-molecule totals and binning (histograms + edge keys in shared memory)
-  const bool two = e.tile == 256 && e.max_solute_sites >= kTwoStageSites;
-  const size_t smem_f = sizeof(int) * ((size_t)finish_region_ints(G, two, e.ermax, A.hist_global) + e.ermax);
+  const size_t smem_f = finish_smem(G, two, e.ermax, A.hist_global);
   dim3 g2((a.nb + G - 1) / G, e.ntile);
 #define ERMOD_FINISH(GG, TILE, TWO)                                                                             \
   if (G == GG && e.tile == TILE && two == TWO) {                                                               \
