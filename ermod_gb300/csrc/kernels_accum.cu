@@ -725,9 +725,9 @@ __global__ void __launch_bounds__(1024) ring_active_list_kernel(const int* __res
 
 // ---- the flush as exact integer matrix products ------------------------------------------
 // ecorr(i, j) += sum_p w_p h_p(i) h_p(j), a product of (bins x placements) matrices.  With the
-// weights as integers m_p = w_p 2^(T - emax) (T = 56, FP64 path 63: relative to the largest
-// weight 2^-T, and a weight whose exponent is within the spread of the largest keeps 44, FP64
-// path 53, bits), m_p h_p(i) is cut into 7-bit digits and h_p(j) into 8-bit ones: their bf16
+// weights as integers m_p = w_p 2^(T - emax) (T = 60, FP64 path 63: a weight whose exponent is
+// within the spread of the largest, 12 or 10, keeps 48 bits, as the walk's float-float pairs hold
+// it, or all 53), m_p h_p(i) is cut into 7-bit digits and h_p(j) into 8-bit ones: their bf16
 // values are exact, and the FP32 sums of 512 products of two digits are integers below 2^24,
 // exact too.  So mma.sync adds the digit planes without error, and each entry is rounded once
 // per 35 bits of planes when they are joined.  512 placements, with the two kernels before: 168 ->
@@ -1013,7 +1013,7 @@ cudaError_t launch_ecorr_flush(Engine& e, cudaStream_t s) {
   }
   // (every bin walked on a short coordinate: the list costs more than the bins it could leave out)
   const int all = !mma && e.ermax <= kActiveMinBins;
-  const int T = e.mixed ? 56 : 63, spread = e.mixed ? 12 : 10;
+  const int T = e.mixed ? 60 : 63, spread = e.mixed ? 12 : 10;
   if (mma || e.mixed) {
     ring_active_list_kernel<<<1, 1024, 0, s>>>(top, e.ermax, valid, w, n, mma ? kMmaBins : -1, spread, all, act, atop,
                                              info);

@@ -1,5 +1,6 @@
 """The ecorr flush's weights at the ends of their range (GPU, against the sum over the placements' own
-histograms): as small as a normal double holds them in FP64."""
+histograms): as small as a normal double holds them in FP64, and 48-bit weights of 2^-12 of the
+largest, the widest spread that the matrix kernels take."""
 import numpy as np
 import pytest
 
@@ -32,3 +33,19 @@ def test_smallest_weights(gpu_lib, scale):
     want = (H * sw[:, None]).T @ H
     np.testing.assert_array_equal(got != 0.0, want != 0.0)
     np.testing.assert_allclose(got, want, rtol=1e-12)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_spread_weights_keep_48_bits(gpu_lib, precision):
+    n = 64
+    k = 2 ** 47 + np.random.default_rng(9).integers(0, 2 ** 46, n) * 2 + 1  # 48 bits, the last one set
+    spread = 12 if precision == "mixed" else 10
+    k_hi = k >> 24 << 24
+    exps = np.full(n, -spread)
+    exps[5] = 0
+    scale = 2.0 ** (exps - 47.0)
+    got, H = _flush(precision, k * scale)
+    # the weights' halves of 24 bits: sums of exact products, rounded once when they are joined
+    want = (H * (k_hi * scale)[:, None]).T @ H + (H * ((k - k_hi) * scale)[:, None]).T @ H
+    # every weight is a multiple of the matrix kernels' unit, so only the joining rounds: twice
+    np.testing.assert_allclose(got, want, rtol=2.0 ** -50)
