@@ -838,6 +838,7 @@ __global__ void __launch_bounds__(32 * kMmaWarps, 2) ecorr_mma_kernel(const uint
   const int part = warp % kMmaParts, half = warp / kMmaParts;
   const int nround = (na + 9) / 10;  // two groups of five planes at a time
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  double S[4] = {0.0, 0.0, 0.0, 0.0};  // the entries, all digits of the second operand joined
   for (int m = max(nb0, nb1) - 1; m >= 0; --m) {
     double R[4] = {0.0, 0.0, 0.0, 0.0};
     for (int round = nround - 1; round >= 0; --round) {
@@ -899,21 +900,23 @@ __global__ void __launch_bounds__(32 * kMmaWarps, 2) ecorr_mma_kernel(const uint
         R[u] = fma(fma(R[u], 34359738368.0, (double)hi), 34359738368.0, (double)lo);  // 2^35 per five planes
       }
     }
-    // (weights below 1e-304 have no unit in a double: their entries are scaled by ldexp)
-    const int ex = I.emax - T + 8 * m;
-    const double unit = ldexp(1.0, ex);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      // entry (i, j, e) of the fragments: row 16 i + lane / 4 (+ 8 for e >= 2), column 8 j + 2 (lane % 4) + (e & 1)
-      const int at = warp + 8 * u, i = at >> 4, j = (at >> 2) & 3, e = at & 3;
-      const int ri = r0 + 16 * i + (lane >> 2) + (e >> 1) * 8, ci = c0 + 8 * j + 2 * (lane & 3) + (e & 1);
-      if (ci < ri || ci >= I.nact || R[u] == 0.0) continue;
-      const double v = unit > 0.0 ? R[u] * unit : ldexp(R[u], ex);
-      const size_t br = act[ri], bc = act[ci];
-      // one addition per entry and launch: an atomic one only so that no thread waits for it
-      atomicAdd(ecorr + br * ermax + bc, v);
-      if (br != bc) atomicAdd(ecorr + bc * ermax + br, v);
-    }
+    for (int u = 0; u < 4; ++u) S[u] = fma(S[u], 256.0, R[u]);
+  }
+  // (weights below 1e-304 have no unit in a double: their entries are scaled by ldexp)
+  const int ex = I.emax - T;
+  const double unit = ldexp(1.0, ex);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    // entry (i, j, e) of the fragments: row 16 i + lane / 4 (+ 8 for e >= 2), column 8 j + 2 (lane % 4) + (e & 1)
+    const int at = warp + 8 * u, i = at >> 4, j = (at >> 2) & 3, e = at & 3;
+    const int ri = r0 + 16 * i + (lane >> 2) + (e >> 1) * 8, ci = c0 + 8 * j + 2 * (lane & 3) + (e & 1);
+    if (ci < ri || ci >= I.nact || S[u] == 0.0) continue;
+    const double v = unit > 0.0 ? S[u] * unit : ldexp(S[u], ex);
+    const size_t br = act[ri], bc = act[ci];
+    // one addition per entry and launch: an atomic one only so that no thread waits for it
+    atomicAdd(ecorr + br * ermax + bc, v);
+    if (br != bc) atomicAdd(ecorr + bc * ermax + br, v);
   }
 }
 
