@@ -370,17 +370,41 @@ __device__ __forceinline__ int pair_fp32(const MolArgs& A, const int4& vp, const
   return (fabsf(elj) <= kFp64Lj ? 0 : kPairLj) | (fabsf(eco) <= kFp64Coulomb ? 0 : kPairCoulomb);
 }
 
-// Sums of FP32 terms as 64-bit integers of 2^-A.fx_bits kcal/mol (2^-44 unless the molecules'
-// pairs could overflow it: no term is above 16): exact additions, so that the sum does not
-// depend on the order in which a block's threads add.  Two words, the low one's carry passed on.
+// Sums of FP32 terms as integers of 1 / A.fx_scale_f kcal/mol: exact additions, so that the sum does
+// not depend on the order in which a block's threads add.  A pair adds an LJ and a Coulomb term, at
+// most kFixedTerm together.  Two words, the low one's carry passed on, while they leave the unit at
+// 2^-48 kcal/mol or finer for every pair of the largest molecule with a solute (1,365 pairs; 2^-53 for
+// water and 12 sites); three words of 2^-58 beyond.  (Float-float sums hold 48 bits.  With a unit of 2^-44
+// for water the small terms of distant pairs lost theirs; adding them costs 1% of this kernel at 36
+// solute sites, 4.98 -> 5.04 ms of 4,000 insertions into 2,000 waters.)
+constexpr float kFixedTerm = kFp64Lj + kFp64Coulomb;
+constexpr int kFixedNarrowBits = 48, kFixedWideBits = 58;
+static_assert(kFixedTerm < 32.f, "a pair's terms in 63 bits at kFixedWideBits");
 __device__ __forceinline__ void fixed_add(unsigned* lo, unsigned* hi, long long v) {
   const unsigned l = (unsigned)v, old = atomicAdd(lo, l);
   atomicAdd(hi, (unsigned)((unsigned long long)v >> 32) + (old + l < old ? 1u : 0u));
+}
+__device__ __forceinline__ void fixed_add_wide(unsigned* lo, unsigned* hi, unsigned* top, long long v) {
+  const unsigned l = (unsigned)v, old = atomicAdd(lo, l), c = old + l < old ? 1u : 0u;
+  const unsigned m = (unsigned)((unsigned long long)v >> 32), mc = m + c, oldm = atomicAdd(hi, mc);
+  const unsigned t = (v < 0 ? ~0u : 0u) + (mc < m || oldm + mc < oldm ? 1u : 0u);
+  if (t) atomicAdd(top, t);
 }
 __device__ __forceinline__ ff fixed_to_ff(unsigned lo, unsigned hi, float unit) {
   const long long v = (long long)(((unsigned long long)hi << 32) | lo);
   const float h = __ll2float_rn(v);
   return ff{h * unit, __ll2float_rn(v - __float2ll_rn(h)) * unit};
+}
+// three words: the magnitude's upper and lower 64 bits as doubles (rounded at 53 bits)
+__device__ __noinline__ ff fixed_to_ff_wide(unsigned lo, unsigned hi, unsigned top, float unit) {
+  unsigned long long v = ((unsigned long long)hi << 32) | lo;
+  const bool neg = (int)top < 0;
+  if (neg) {
+    v = ~v + 1ull;
+    top = ~top + (v == 0ull ? 1u : 0u);
+  }
+  const double x = fma((double)top, 18446744073709551616.0, (double)v) * (double)unit;
+  return ff_from_double(neg ? -x : x);
 }
 
 constexpr long long kKeyPosInf = 0x7ff0000000000000ll;
@@ -846,7 +870,9 @@ __device__ __forceinline__ void species_partials(const MolArgs& A, const BatchAr
 // makes few blocks and the real-space pass, the FP64 pairs of the first shell above all, takes
 // all 256 threads.
 // kTwo: the stage before the pairs' test, for solutes of many sites (kTwoStageSites).
-template <int G, int TILE, bool kTwo>
+// kWide: the sums of the pair terms take three words (fixed_add_wide); a parameter, so that the usual
+// kernels keep their registers.
+template <int G, int TILE, bool kTwo, bool kWide>
 __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const float* __restrict__ site_e) {
   extern __shared__ __align__(16) int smem_dyn[];
   // [G][ermax] block histograms, or none when they would not fit beside other blocks: the
@@ -861,6 +887,7 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
   unsigned char* sparts = reinterpret_cast<unsigned char*>(sorder + kBigList);  // [kBigList] the parts left out
   unsigned* squeue = reinterpret_cast<unsigned*>(sparts + kBigList);            // [1 or 2][8][kPairQueue]
   unsigned* sfix = squeue + (kTwo ? 16 : 8) * kPairQueue;                                    // [2][G * 256] sums, low and high words
+  [[maybe_unused]] unsigned* stop = reinterpret_cast<unsigned*>(sval);                           // [G * 256] their third ones, read before sval is written
   int* ss0 = reinterpret_cast<int*>(sfix + 2 * 256 * G);                        // [256] first sites
   unsigned short* snear = reinterpret_cast<unsigned short*>(ss0 + 256);         // [G * 256] molecule | placement << 8
   __shared__ int swarp[8];
@@ -980,7 +1007,10 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
       nnear += swarp[w2];
     }
     for (unsigned q = nearm; q; q &= q - 1) snear[near0++] = (unsigned short)(threadIdx.x | ((__ffs(q) - 1) << 8));
-    for (int i = threadIdx.x; i < nnear; i += 256) sfix[i] = sfix[256 * G + i] = 0u;
+    for (int i = threadIdx.x; i < nnear; i += 256) {
+      sfix[i] = sfix[256 * G + i] = 0u;
+      if constexpr (kWide) stop[i] = 0u;
+    }
     if (threadIdx.x == 0) {
       snlist = 0;
       snu = 0;
@@ -1012,7 +1042,12 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
         long long v = 0;
         if (!(parts & kPairLj)) v = __float2ll_rn(elj * scale);
         if (!(parts & kPairCoulomb)) v += __float2ll_rn(eco * scale);
-        if (v != 0) fixed_add(sfix + near, sfix + 256 * G + near, v);
+        if (v != 0) {
+          if constexpr (kWide)
+            fixed_add_wide(sfix + near, sfix + 256 * G + near, stop + near, v);
+          else
+            fixed_add(sfix + near, sfix + 256 * G + near, v);
+        }
         if (parts) {
           // (a window that the byte cannot hold: the items' threads find all their own again)
           const int q = win < kListWindows ? atomicAdd(&snlist, 1) : atomicMax(&snlist, kBigList + 1);
@@ -1075,6 +1110,23 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
       if (nq > 0) evaluate(nq);
     }
     __syncthreads();
+    auto add_sums = [&] {
+      for (int near = threadIdx.x; near < nnear; near += 256) {
+        const int t = snear[near] & 0xff, j = snear[near] >> 8;
+        const unsigned lo = sfix[near], hi = sfix[256 * G + near];
+        ff r;
+        if constexpr (kWide)
+          r = fixed_to_ff_wide(lo, hi, stop[near], 1.f / scale);
+        else
+          r = fixed_to_ff(lo, hi, 1.f / scale);
+        const ff x = ff_add2(ff{su[j][t], sul[j][t]}, r);
+        su[j][t] = x.hi;
+        sul[j][t] = x.lo;
+      }
+      __syncthreads();
+    };
+    static_assert(sizeof(unsigned) * 256 * G <= sizeof(double) * kBigList, "the third words in sval's place");
+    if constexpr (kWide) add_sums();  // before sval takes the third words' place
     // FP64 pass over the listed pair parts (overlapping pairs, left out of the FP32 sums): one
     // per thread, so that every FP64 instruction runs on full warps; an item's values are added
     // in the order of its pairs (solute site, molecule site), by the thread of the first
@@ -1092,14 +1144,7 @@ __global__ void __launch_bounds__(256, 4) mol_finish_kernel(MolArgs A, const flo
       }
       __syncthreads();
     }
-    for (int near = threadIdx.x; near < nnear; near += 256) {
-      const int t = snear[near] & 0xff, j = snear[near] >> 8;
-      const ff r = fixed_to_ff(sfix[near], sfix[256 * G + near], 1.f / scale);
-      const ff x = ff_add2(ff{su[j][t], sul[j][t]}, r);
-      su[j][t] = x.hi;
-      sul[j][t] = x.lo;
-    }
-    __syncthreads();
+    if constexpr (!kWide) add_sums();
     if (nlist <= kBigList) {
       for (int r = threadIdx.x; r < nlist; r += 256) {
         const unsigned near = sbig[sorder[r]] >> 21;
@@ -1247,6 +1292,15 @@ cudaError_t launch_mol64(Engine& e, const MolArgs& A) {
 
 }  // namespace
 
+// bits below the binary point that two words leave the sums of the largest molecule's pairs with the
+// largest solute (the device API may name any molecule as one): their sum stays below 2^63 units
+static int fixed_bits(const Engine& e) {
+  const double most = (double)kFixedTerm * e.max_mol_sites *
+                      std::min(kMaxSoluteSites, std::max(e.max_mol_sites, e.max_solute_sites));
+  return 63 - (std::ilogb(most) + 1);
+}
+static bool fixed_wide(const Engine& e) { return fixed_bits(e) < kFixedNarrowBits; }
+
 static MolArgs make_mol_args(Engine& e, const BatchArgs& a) {
   MolArgs A{};
   A.site_pos = e.d_site_pos;
@@ -1292,10 +1346,7 @@ static MolArgs make_mol_args(Engine& e, const BatchArgs& a) {
   A.k64 = make_k64(A);
   A.k32 = to_f32(A.k64);
   A.reach2_f = std::max(A.k32.up2, A.k32.ele2);
-  // terms of at most 16 = 2^4: 2^(44 + 4) each, 2^15 pairs of a molecule with a solute in 63 bits
-  int fx_bits = 44;
-  for (long long pairs = (long long)e.max_mol_sites * kMaxSoluteSites; pairs > (1 << 15); pairs /= 2) --fx_bits;
-  A.fx_scale_f = std::ldexp(1.f, fx_bits);
+  A.fx_scale_f = std::ldexp(1.f, fixed_wide(e) ? kFixedWideBits : fixed_bits(e));
   A.a = a;
   A.ntile = e.ntile;
   A.status = e.d_status;
@@ -1383,22 +1434,27 @@ cudaError_t launch_mol_energy(Engine& e, const BatchArgs& a) {
   // step 2: per-molecule totals and binning (histograms + edge keys in shared memory)
   const size_t smem_f = finish_smem(G, two, e.ermax, A.hist_global);
   dim3 g2((a.nb + G - 1) / G, e.ntile);
-#define ERMOD_FINISH(GG, TILE, TWO)                                                                             \
-  if (G == GG && e.tile == TILE && two == TWO) {                                                               \
+#define ERMOD_FINISH(GG, TILE, TWO, WIDE)                                                                       \
+  if (G == GG && e.tile == TILE && two == TWO && wide == WIDE) {                                               \
     static SmemAttr attr;                                                                                      \
-    if ((err = attr.ensure(mol_finish_kernel<GG, TILE, TWO>, smem_f)) != cudaSuccess) return err;              \
-    mol_finish_kernel<GG, TILE, TWO><<<g2, 256, smem_f, a.stream>>>(A, a.site_e);                              \
+    if ((err = attr.ensure(mol_finish_kernel<GG, TILE, TWO, WIDE>, smem_f)) != cudaSuccess) return err;        \
+    mol_finish_kernel<GG, TILE, TWO, WIDE><<<g2, 256, smem_f, a.stream>>>(A, a.site_e);                        \
   }
-  ERMOD_FINISH(1, 16, false)
-  ERMOD_FINISH(1, 64, false)
-  ERMOD_FINISH(1, 256, false)
-  ERMOD_FINISH(2, 256, false)
-  ERMOD_FINISH(4, 256, false)
-  ERMOD_FINISH(8, 256, false)
-  ERMOD_FINISH(1, 256, true)
-  ERMOD_FINISH(2, 256, true)
-  ERMOD_FINISH(4, 256, true)
-  ERMOD_FINISH(8, 256, true)
+#define ERMOD_FINISH_ALL(WIDE)        \
+  ERMOD_FINISH(1, 16, false, WIDE)    \
+  ERMOD_FINISH(1, 64, false, WIDE)    \
+  ERMOD_FINISH(1, 256, false, WIDE)   \
+  ERMOD_FINISH(2, 256, false, WIDE)   \
+  ERMOD_FINISH(4, 256, false, WIDE)   \
+  ERMOD_FINISH(8, 256, false, WIDE)   \
+  ERMOD_FINISH(1, 256, true, WIDE)    \
+  ERMOD_FINISH(2, 256, true, WIDE)    \
+  ERMOD_FINISH(4, 256, true, WIDE)    \
+  ERMOD_FINISH(8, 256, true, WIDE)
+  const bool wide = fixed_wide(e);
+  ERMOD_FINISH_ALL(false)
+  ERMOD_FINISH_ALL(true)
+#undef ERMOD_FINISH_ALL
 #undef ERMOD_FINISH
   e.count_launch();
   return cudaGetLastError();
