@@ -134,8 +134,9 @@ struct SmemAttr {
   }
 };
 
-// the molecules sorted by counting their spatial codes: at most this many, whose codes (at most
-// 4 per molecule) have at most this many bits per axis
+// the molecules sorted by counting their spatial codes: at most this many (beyond, the cluster's
+// threads have too many each, and the radix sort's grid-wide passes are the faster), whose codes (at
+// most 4 per molecule) have at most three times this many bits
 constexpr int kSortMaxMol = 98304;
 constexpr int kSortMaxBits = 6;
 static_assert(4LL * kSortMaxMol < 1LL << (3 * (kSortMaxBits + 1)), "the codes' counts");

@@ -83,14 +83,22 @@ __device__ __forceinline__ void wrap_atom(const double* __restrict__ pos, int a,
   out[2] = x[2];
 }
 
-__device__ __forceinline__ unsigned int spread3(unsigned int v) {
-  v &= 0x3ff;
-  v = (v | (v << 16)) & 0x030000ff;
-  v = (v | (v << 8)) & 0x0300f00f;
-  v = (v | (v << 4)) & 0x030c30c3;
-  v = (v | (v << 2)) & 0x09249249;
-  return v;
-}
+// n[i] cells along axis i, their Morton code of bits[i] bits an axis: the axes' bits in turn while an
+// axis has any, so that a long box has no more codes than cells (rounded up to powers of two)
+struct CodeGrid {
+  int n[3], bits[3];
+  __host__ __device__ __forceinline__ int total() const { return bits[0] + bits[1] + bits[2]; }
+  __device__ __forceinline__ unsigned code(const int (&c)[3]) const {
+    const int most = max(bits[0], max(bits[1], bits[2]));
+    unsigned k = 0u;
+    int at = 0;
+    for (int b = 0; b < most; ++b)
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        if (b < bits[i]) k |= (unsigned)((c[i] >> b) & 1) << at++;
+    return k;
+  }
+};
 
 // the coordinates of atom a as the pair terms take them
 __device__ __forceinline__ void normalised(const double* __restrict__ pos, int a, const FrameGeom& g, double out[3]) {
@@ -104,7 +112,7 @@ __device__ __forceinline__ void normalised(const double* __restrict__ pos, int a
 // the Morton codes and their counts (count zeroed before); also zeroes what the later kernels
 // of the frame add to (the brick counts and the largest molecule radius)
 __global__ void frame_key_kernel(const double* __restrict__ pos, const int* __restrict__ mol_atom0, int slvmax,
-                                 FrameGeom g, int3 ncell, unsigned int* __restrict__ key, int* __restrict__ val,
+                                 FrameGeom g, CodeGrid cells, unsigned int* __restrict__ key, int* __restrict__ val,
                                  int* __restrict__ count, int* __restrict__ brick_count, int nbricks,
                                  float* __restrict__ frame_scal) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -114,14 +122,13 @@ __global__ void frame_key_kernel(const double* __restrict__ pos, const int* __re
   double w[3];
   normalised(pos, mol_atom0[k], g, w);
   int c[3];
-  const int n[3] = {ncell.x, ncell.y, ncell.z};
   for (int i = 0; i < 3; ++i) {
     // non-periodic coordinates lie in (-L/2, L/2) of the virtual cube
     const double f = w[i] * g.invL[i] + (g.periodic ? 0.0 : 0.5);
-    int ci = (int)(f * (double)n[i]);
-    c[i] = min(max(ci, 0), n[i] - 1);
+    int ci = (int)(f * (double)cells.n[i]);
+    c[i] = min(max(ci, 0), cells.n[i] - 1);
   }
-  const unsigned code = spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2);
+  const unsigned code = cells.code(c);
   key[k] = code;
   if (count)
     atomicAdd(&count[code], 1);
@@ -563,6 +570,14 @@ cudaError_t launch_max_abs(Engine& e, const double* x_d, size_t n, double* host_
 // 3,000 sites 5.7 us with one CTA, of 12,000 12.5 with the cluster)
 constexpr int kSortSharedCodes = 32768;
 constexpr int kSortOneCta = 3 * kSortThreads;
+// and by counting at all for up to kSortMaxMol molecules while the ordering of a code's molecules, each
+// against all others of its code, stays within kSortReads reads a thread, with a code's cell as full
+// as a liquid packs it (kDenseVolume cubic Angstrom a molecule; water has 30).  Beyond, the radix sort
+// takes the 4 A cells as they are.  Frames of one cluster of molecules and one molecule 1,000 A away,
+// counting and radix sort: 2,000 molecules (3,900 reads) 46 and 50 us, 3,000 (8,800) 66 and 56, 5,000 (3,000,
+// by the cluster) 70 and 108, 10,000 (12,200) 133 and 133, 20,000 (48,800) 297 and 178.
+constexpr double kSortReads = 8192.0;
+constexpr double kDenseVolume = 25.0;
 
 template <class... Params, class... Args>
 static cudaError_t launch_cluster(void (*kern)(Params...), cudaStream_t s, Args... args) {
@@ -581,24 +596,31 @@ static cudaError_t launch_cluster(void (*kern)(Params...), cudaStream_t s, Args.
 }
 
 cudaError_t launch_frame_sort(Engine& e) {
-  int nc[3], bits = 1;
+  CodeGrid cells;  // of 4 A
   for (int i = 0; i < 3; ++i) {
-    nc[i] = std::max(1, std::min(1024, (int)(e.geom.L[i] / 4.0)));
-    while ((1 << bits) < nc[i]) ++bits;
+    cells.n[i] = std::max(1, std::min(1024, (int)(e.geom.L[i] / 4.0)));
+    cells.bits[i] = 0;
+    while ((1 << cells.bits[i]) < cells.n[i]) ++cells.bits[i];
   }
-  // sparse cells (a droplet in its virtual cube): no more codes than 4 per molecule, by doubling
-  // the cell's edge (300 waters, 32,768 codes: 56 us of scanning)
-  while (bits > 1 && (1ll << (3 * bits)) > std::max(4096ll, 4ll * e.slvmax)) {
-    --bits;
-    for (int& n : nc) n = (n + 1) / 2;
+  // Sorting by counting takes no more codes than 4 per molecule (300 waters in their virtual cube, 32,768
+  // codes: 56 us of scanning), by doubling the cells' shortest edge.
+  CodeGrid few = cells;
+  auto edge = [&](int i) { return e.geom.L[i] / few.n[i]; };
+  while ((1ll << few.total()) > std::max(4096ll, 4ll * e.slvmax)) {
+    int ax = -1;
+    for (int i = 0; i < 3; ++i)
+      if (few.bits[i] > 0 && (ax < 0 || edge(i) < edge(ax))) ax = i;
+    few.n[ax] = (few.n[ax] + 1) / 2;
+    --few.bits[ax];
   }
-  // up to kSortMaxMol molecules are sorted by counting (their codes then have at most
-  // kSortMaxBits bits per axis); beyond, the cluster's threads have too many each, and the
-  // radix sort's grid-wide passes are the faster
-  const bool counted = e.slvmax <= kSortMaxMol;
-  const int ncode = 1 << (3 * std::min(bits, kSortMaxBits));
+  const double most = std::min<double>(e.slvmax, edge(0) * edge(1) * edge(2) / kDenseVolume + 1.0);
+  const bool one = e.slvmax <= kSortOneCta && (1 << few.total()) <= kSortSharedCodes;
+  const bool counted = e.slvmax <= kSortMaxMol &&
+                       e.slvmax * most <= kSortReads * kSortThreads * (one ? 1 : kSortCluster);
+  if (counted) cells = few;
+  const int ncode = 1 << cells.total();
   frame_key_kernel<<<nblk(e.slvmax, 256), 256, 0, e.stream>>>(
-      e.d_sitepos, e.d_mol_atom0, e.slvmax, e.geom, make_int3(nc[0], nc[1], nc[2]), e.d_sort_key, e.d_sort_val,
+      e.d_sitepos, e.d_mol_atom0, e.slvmax, e.geom, cells, e.d_sort_key, e.d_sort_val,
       counted ? e.d_sort_count : nullptr, e.d_brick_count, e.nbricks, e.d_frame_scal);
   e.count_launch();
   cudaError_t err = cudaGetLastError();
@@ -620,7 +642,7 @@ cudaError_t launch_frame_sort(Engine& e) {
     A.slot_qmol = e.d_slot_qmol;
     A.slot_site = e.d_slot_site;
     e.count_launch();
-    if (e.slvmax <= kSortOneCta && ncode <= kSortSharedCodes) {
+    if (one) {
       static SmemAttr attr;
       const size_t smem = sizeof(int) * ncode;
       if ((err = attr.ensure(frame_sort_kernel<1>, smem)) != cudaSuccess) return err;
@@ -631,7 +653,7 @@ cudaError_t launch_frame_sort(Engine& e) {
   }
   size_t bytes = e.cub_tmp_bytes;
   err = cub::DeviceRadixSort::SortPairs(e.d_cub_tmp, bytes, e.d_sort_key, e.d_sort_key_alt, e.d_sort_val,
-                                        e.d_slot_mol, e.slvmax, 0, 3 * bits, e.stream);
+                                        e.d_slot_mol, e.slvmax, 0, std::max(1, cells.total()), e.stream);
   if (err != cudaSuccess) return err;
   frame_slot_kernel<<<nblk(e.slvmax, 256), 256, 0, e.stream>>>(e.d_slot_mol, e.d_mol_nsite, e.d_mol_species,
                                                               e.d_mol_qmol, e.slvmax, e.d_sort_val_alt,
