@@ -1133,8 +1133,9 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
     if (ibatch >= kBatchSlots) ERMOD_CUDA(cudaStreamWaitEvent(bst, e.ev_acc[slot], 0));  // slot free again
     if (!single) ERMOD_CUDA(cudaStreamWaitEvent(bst, e.ev_prep[slot], 0));
     const int half = e.ring_off ? 1 : 0;
-    if (e.flush_pend[half]) {  // the first batch in this half waits for its previous flush
-      ERMOD_CUDA(cudaStreamWaitEvent(bst, e.ev_flush[half], 0));
+    if (e.flush_pend[half]) {  // every batch in this half, on whichever stream, waits for its previous flush
+      for (int k = 0; k < (dual ? kBatchStreams : 1); ++k)
+        ERMOD_CUDA(cudaStreamWaitEvent(dual ? e.bs[k] : bst, e.ev_flush[half], 0));
       e.flush_pend[half] = false;
     }
     ERMOD_CUDA(cudaMemsetAsync(a.hist, 0, sizeof(int) * (size_t)nb * e.ermax, bst));
