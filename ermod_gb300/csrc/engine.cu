@@ -808,6 +808,8 @@ int ermod_set_topology(ermod_ctx* c, int nummol, int numatm, const int* mbi, con
   ERMOD_CUDA(dalloc(&e.d_site_x, 3 * (size_t)e.nsite_phys));
   ERMOD_CUDA(dalloc(&e.d_site_q, e.nsite_phys));
   ERMOD_CUDA(dalloc(&e.d_frame_scal, 4));
+  // a rigid solute's real-space self energy, kept from its first placement, was the old topology's
+  if (e.bins_ready) ERMOD_CUDA(cudaMemset(e.d_scal + 5, 0, 2 * sizeof(double)));
   if (const int st = setup_done()) return st;
   e.green_valid = false;
   e.topo_ready = true;
