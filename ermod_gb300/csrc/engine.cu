@@ -5,8 +5,8 @@
 // Per batch of B placements:
 //   [mixed] place_prep (prep stream) -> pme_a -> pme_b -> gather -> finish (one of two
 //           batch streams) -> reduce + accumulate (aux stream)
-//   [fp64]  place_prep (prep stream) -> spectrum64 -> Z2D -> mol_energy (caller's stream) ->
-//           reduce + accumulate (aux stream)
+//   [fp64]  place_prep (prep stream) -> spectrum64 -> fft64 (lengths with other factors than 2, 3
+//           and 5: cuFFT) -> mol_energy (caller's stream) -> reduce + accumulate (aux stream)
 // and, when ecorr is on, a flush of the histogram ring every `ring_half` placements on
 // the flush stream while the next batches fill the ring's other half.
 // Status is reported once per call (host API) or per ermod_sync (device API).
@@ -1048,7 +1048,7 @@ static int run_placements(Engine& e, int nplace, const int* d_tag, const double*
   const int nbatch = (nplace + B - 1) / B;
   const size_t parts = e.mixed ? (size_t)spectrum_partials(e) : (size_t)spectrum64_partials(e);
   // batches run on two alternating streams (mixed path) or on the caller's stream (FP64
-  // path, whose cuFFT plans are bound to it); every stream starts after what is
+  // path, whose batches share one set of grids); every stream starts after what is
   // already queued on the caller's stream
   const bool dual = e.mixed;
   // solution mode: the placements check_mol_configuration skips (engproc.F90:389-390)

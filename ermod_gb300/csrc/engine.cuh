@@ -148,9 +148,9 @@ struct Engine {
   char* d_ring_digits = nullptr;  // flush: digit planes of the matrix kernels
   int* d_ring_nnz = nullptr;      // [ring_cap] occupied bins per entry
   int* d_ring_valid = nullptr;    // [ring_cap] entry accumulated (no error in its batch)
-  double* d_u0 = nullptr;         // [2][Bmax] solute self energies (two batch slots)
-  float* d_site_e = nullptr;      // [2][nsite_phys][Bmax] reciprocal site terms (mixed path)
-  int* d_self_bin = nullptr;      // [2][Bmax]
+  double* d_u0 = nullptr;         // [kBatchSlots][Bmax] solute self energies
+  float* d_site_e = nullptr;      // [kBatchSlots][nsite_phys][Bmax] reciprocal site terms (mixed path)
+  int* d_self_bin = nullptr;      // [kBatchSlots][Bmax]
 
   // ---- status ----------------------------------------------------------------------
   DevStatus* d_status = nullptr;

@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(1024) ring_active_list_kernel(const int* __res
 // values are exact, and the FP32 sums of 512 products of two digits are integers below 2^24,
 // exact too.  So mma.sync adds the digit planes without error, and each entry is rounded once
 // per 35 bits of planes when they are joined.  512 placements, with the two kernels before: 168 ->
-// 95 us for 4,000 waters, 294 -> 130 us for 33,000 (float-float sums by the walk below); FP64
+// 97 us for 4,000 waters, 294 -> 130 us for 33,000 (float-float sums by the walk below); FP64
 // path, 64 placements of 4,000 waters 253 -> 45 us.
 constexpr int kMmaK = 512;         // placements per pass (a longer ring takes several)
 constexpr int kMmaBins = 2048;     // active bins, at most
@@ -811,7 +811,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint4& a, unsigned
 // fragments in L2; a warp takes five planes, joined as 64-bit integers, and a quarter of the
 // placements, so that the loads' latency is paid a few times over and not once per plane and
 // round (one warp per tile: twice the time); the warps' integers are added exactly and joined
-// in FP64.  Bound by that latency still: two CTAs to an SM take 67 us a flush of 512 placements
+// in FP64.  Bound by that latency still: two CTAs to an SM take 68 us a flush of 512 placements
 // of 4,000 waters, one with more loads in flight per warp 120.  Each entry is added at both mirrored positions.
 constexpr int kMmaWarps = 8, kMmaParts = 4;
 __global__ void __launch_bounds__(32 * kMmaWarps, 2) ecorr_mma_kernel(const uint4* __restrict__ A,

@@ -1,7 +1,7 @@
 // kernels_mol.cu -- per-molecule solute-solvent energies, fused with the binning.
 //
-// One thread owns one solvent molecule (a "slot" of the frame's spatially sorted
-// order) and G placements of the batch.  For each placement it computes
+// For every placement of the batch and solvent molecule (a "slot" of the frame's spatially
+// sorted order):
 //   recip   sum over its sites of q * sum_{c1,c2,c3} theta theta theta phi(g - c)
 //           (recpcal_energy, recpcal.F90:451-502), phi being the solute's PME potential;
 //   real    LJ (4 switch forms) + q q erfc(beta r) / r against every solute site within
@@ -9,14 +9,15 @@
 //           the molecule is inside the solute's bounding sphere + cutoff, so the cell
 //           list of the reference (realcal.F90:373-582) is not needed;
 //   resid   -pi Q_u Q_j / (beta^2 V) (residual_ene, engproc.F90:859-869);
-// then the FP64 total u = real + (resid + recip) (get_uv_energy, engproc.F90:736-753)
-// is binned exactly as getiduv/binsearch do (engproc.F90:927-1020), with integer keys
-// of the FP64 values, into a shared-memory histogram per placement (insdst,
-// engproc.F90:813-830).  Per-species sum/min/max go to per-block partials reduced in
-// a fixed tree, so every result is run-to-run deterministic.
+// then the total u = real + (resid + recip) (get_uv_energy, engproc.F90:736-753) is binned
+// exactly as getiduv/binsearch do (engproc.F90:927-1020), with integer keys, into the
+// placement's histogram (insdst, engproc.F90:813-830).  Per-species sum/min/max go to
+// per-block partials reduced in a fixed tree, so every result is run-to-run deterministic.
 //
-// Mixed path: fixed-point positions, FP32 pair terms and grid gather, FP64 per-site and
-// per-molecule totals.  FP64 path: everything in FP64 with the reference's formulas.
+// Mixed path: the gather, then a thread per molecule and up to 8 placements; fixed-point
+// positions, FP32 pair terms and grid gather, float-float totals, block histograms in shared
+// memory.  FP64 path: 4 or 16 threads per molecule and placement, everything in FP64 with the
+// reference's formulas, counts straight into the batch's histograms.
 #include <cub/device/device_radix_sort.cuh>
 
 #include "async_copy.cuh"

@@ -8,7 +8,7 @@
 //                     b_{s,a}(k) = sum_c theta_{s,a,c} exp(-2 pi i k (g_{s,a} - c) / K_a);
 //                 (the mixed path's spectrum and transforms are in kernels_fft.cu);
 //   spectrum64    the plain FP64 path's spectrum engfac S(k) from those vectors, with the
-//                 self energy; its inverse transform is a batched cuFFT Z2D.
+//                 self energy; its inverse transforms are in kernels_fft64.cu.
 #include "engine.cuh"
 
 namespace ermod {

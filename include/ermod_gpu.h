@@ -58,7 +58,7 @@ typedef enum ermod_status {
 
 /* Arithmetic of the per-placement path. */
 enum {
-  ERMOD_PRECISION_FP64 = 0,  /* plain path: FP64 everywhere, spread + D2Z/Z2D, one placement at a time */
+  ERMOD_PRECISION_FP64 = 0,  /* plain path: FP64 everywhere, in batches of up to 64 placements */
   ERMOD_PRECISION_MIXED = 1  /* batched path: FP32 grids and pair terms, FP64 totals and sums */
 };
 
@@ -92,14 +92,14 @@ typedef struct ermod_ctx ermod_ctx;
 void ermod_default_params(ermod_params* p);
 
 /* Context on CUDA device `device`.  Replaces recpcal_init's allocations
- * (recpcal.F90:42-85); the cuFFT plans are created here. */
+ * (recpcal.F90:42-85); buffers sized by topology and bins are made by the first call. */
 int ermod_create(const ermod_params* p, int device, ermod_ctx** out);
 int ermod_destroy(ermod_ctx* ctx);
 
 /* Optional: order all work of this context on an existing cudaStream_t.  A placement call
  * forks from it onto the context's own streams (solute preparation, two batch streams,
  * the ordered accumulation and, with ecorr on, the flush) and joins them back into it
- * before it returns, so the caller sees one stream. */
+ * before it returns, so the caller sees one stream; a call of one batch runs on it alone. */
 int ermod_set_stream(ermod_ctx* ctx, void* cuda_stream);
 
 /* Topology (engmain.F90:252-277).  mol_begin_index has nummol+1 entries (1-based),
@@ -155,7 +155,8 @@ int ermod_set_configuration_check(ermod_ctx* ctx, int insposition, double lwreg,
 
 /* engconst prologue: cell inverse (engproc.F90:898-919), Green function when the
  * cell changed (recpcal.F90:111-152), solvent splines (recpcal.F90:328-340,408-442)
- * and the frame's solvent layout.  sitepos is (3, numatm), cell (3,3). */
+ * and the frame's solvent layout.  sitepos is (3, numatm), cell (3,3).  ermod_frame has taken
+ * sitepos when it returns; its kernels may still be queued on the context's stream. */
 int ermod_frame(ermod_ctx* ctx, const double* sitepos, const double* cell,
                 double stat_weight_system);
 int ermod_frame_device(ermod_ctx* ctx, const double* sitepos_device, const double* cell,
@@ -169,7 +170,8 @@ int ermod_frame_device(ermod_ctx* ctx, const double* sitepos_device, const doubl
  * get_uv_energy in tagpt order, uvengy(0) the solute self energy -- and
  * flceng_out (numslv, nplace).  Results accumulate into the context's
  * accumulators.  On an error status the accumulators keep the state of the last
- * complete batch and ermod_error_info tells which placement/molecule failed. */
+ * complete batch (FP64: of the last placement before the failing one) and ermod_error_info
+ * tells which placement/molecule failed. */
 int ermod_placements(ermod_ctx* ctx, int nplace, const int* tagslt, const double* solute_sitepos,
                      const double* stat_weight_solute, double* uvengy_out, double* flceng_out);
 /* Same with tagslt/solute_sitepos/stat_weight_solute in device memory; the optional
